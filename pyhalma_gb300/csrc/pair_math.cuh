@@ -109,11 +109,11 @@ __device__ __forceinline__ float pair_term_fast_masked(float4 q, float px, float
     return fmaf(q.w, keep ? ri : 0.0f, acc);
 }
 
-// The reference's float32 statement, each operation rounded on its own (no FMA):
+// The reference's float32 term, each operation rounded on its own (no FMA):
 //   r = sqrt((xj-xi)**2 + (yj-yi)**2 + (zj-zi)**2); phi = phi + m / r
-// (particle_subroutines.f90:502-505), guarded by the mask of f90:499-501.
-__device__ __forceinline__ float pair_term_reference(float4 q, float px, float py, float pz,
-                                                     float acc) {
+// (particle_subroutines.f90:502-505); +0, which leaves the sum as it is, where the mask of
+// f90:499-501 drops the pair (the sum starts at +0 and can never become -0).
+__device__ __forceinline__ float pair_term_reference(float4 q, float px, float py, float pz) {
     if (q.x != px && q.y != py && q.z != pz) {
         float dx = __fsub_rn(q.x, px);
         float dy = __fsub_rn(q.y, py);
@@ -121,10 +121,9 @@ __device__ __forceinline__ float pair_term_reference(float4 q, float px, float p
         float s = __fmul_rn(dx, dx);
         s = __fadd_rn(s, __fmul_rn(dy, dy));
         s = __fadd_rn(s, __fmul_rn(dz, dz));
-        float r = __fsqrt_rn(s);
-        acc = __fadd_rn(acc, __fdiv_rn(q.w, r));
+        return __fdiv_rn(q.w, __fsqrt_rn(s));
     }
-    return acc;
+    return 0.0f;
 }
 
 }  // namespace halma

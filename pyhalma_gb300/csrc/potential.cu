@@ -22,33 +22,205 @@ __device__ __forceinline__ float4 load_source(const float *__restrict__ m, const
     return make_float4(kPadCoord, kPadCoord, kPadCoord, 0.0f);
 }
 
-// HALMA_POT_REFERENCE: one target per lane, sources in order, bit-identical to the
-// Fortran loop body (f90:497-510).
-__global__ void __launch_bounds__(256) bf_potential_reference_kernel(
+// ---- HALMA_POT_REFERENCE ------------------------------------------------------------------
+// The Fortran loop body (f90:497-510) bit for bit: per target a float32 sum over the sources
+// in order, every operation rounded on its own, a term m / sqrt(s) only where the source's x, y
+// and z all differ from the target's.
+//
+// Only the additions have to follow one another; the terms do not depend on them.  So a block
+// takes TL targets: eight warps compute the terms of 256 sources at a time into shared memory
+// and a ninth adds the previous 256 in order (double buffered, one barrier a stage).  One
+// warp doing both in turn left the GPU waiting on single dependent chains: 2,000 targets x
+// 20,000 sources took 2.20 ms, 40,000 x 100,000 12.2 ms (2.2 warps on an SM's scheduler).
+//
+// Bound of the terms: the FP32 pipe, 18 two-lane instructions for two terms.  Square root and
+// quotient come from one rsqrt y of s by Markstein's correction steps (P. Markstein, Computation
+// of elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990):
+// g = s y, r = g + (s - g g) y / 2;  z = y + y (1 - r y);  q = m z, t = q + (m - r q) z.  r is the
+// rounded square root for every mantissa (checked over all 2^24 of two binades, in five
+// scalings), z the rounded reciprocal of r -- where the theorem makes t the rounded quotient --
+// except for four mantissas of s; of those, checked over all 2^23 mantissas of m, t is wrong
+// for one m, a power of two, when r's mantissa is all ones.  Those pairs (looked for when a mass is a
+// power of two), squared distances under 2^-90, coordinates or masses outside the ranges below
+// and values that are not finite take the plain operations instead.
+constexpr int kRefWarps = 8;                      // warps that compute terms; one more adds them
+constexpr int kRefStage = 256;                    // sources of one stage
+constexpr int kRefQuads = kRefStage / 4;
+constexpr int kRefThreads = (kRefWarps + 1) * 32;
+constexpr float kRefFar = 1.0e15f;                // sources past the end: m = 0 here gives +0 terms
+constexpr float kRefMaxCoord = 0x1p48f, kRefMinMass = 0x1p-40f, kRefMaxMass = 0x1p80f, kRefMinS = 0x1p-90f;
+enum { kRefPlain = 1, kRefPow2 = 2 };             // bits of the flags word
+
+struct __align__(16) Src4 {   // four consecutive sources
+    float4 x, y, z, m;
+};
+
+// The sources four by four, padded to whole stages, and the flags: kRefPlain when a coordinate or a
+// mass is outside the ranges of the correction steps, kRefPow2 when a mass is a power of two.
+__global__ void __launch_bounds__(256) ref_pack_kernel(
     const float *__restrict__ m, const float *__restrict__ x, const float *__restrict__ y,
-    const float *__restrict__ z, int64_t ns, const float *__restrict__ tx,
-    const float *__restrict__ ty, const float *__restrict__ tz, int64_t nt, float *__restrict__ out) {
-    __shared__ float4 buf[kWarpsPerBlock][32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t gwarp = (int64_t)blockIdx.x * kWarpsPerBlock + w;
-    const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
-    const int64_t ntiles = (nt + 31) / 32;
-    for (int64_t tile = gwarp; tile < ntiles; tile += nwarps) {
-        const int64_t i = tile * 32 + lane;
-        const bool valid = i < nt;
-        const float px = valid ? tx[i] : 0.f, py = valid ? ty[i] : 0.f, pz = valid ? tz[i] : 0.f;
-        float acc = 0.0f;
-        float4 nxt = load_source(m, x, y, z, lane, ns);
-        for (int64_t j0 = 0; j0 < ns; j0 += 32) {
-            __syncwarp();
-            buf[w][lane] = nxt;
-            __syncwarp();
-            nxt = load_source(m, x, y, z, j0 + 32 + lane, ns);
-            const int cnt = (int)min((int64_t)32, ns - j0);
-            for (int k = 0; k < cnt; ++k) acc = pair_term_reference(buf[w][k], px, py, pz, acc);
+    const float *__restrict__ z, int64_t ns, int64_t nquads, const float *__restrict__ tx,
+    const float *__restrict__ ty, const float *__restrict__ tz, int64_t nt, Src4 *__restrict__ src,
+    int *__restrict__ flags) {
+    int f = 0;
+    auto coord = [&](float v) {
+        if (!(fabsf(v) < kRefMaxCoord)) f |= kRefPlain;
+        return v;
+    };
+    const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t q = i0; q < nquads; q += step) {
+        float v[4][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int64_t j = 4 * q + k;
+            const bool in = j < ns;
+            v[0][k] = in ? coord(x[j]) : kRefFar;
+            v[1][k] = in ? coord(y[j]) : kRefFar;
+            v[2][k] = in ? coord(z[j]) : kRefFar;
+            const float mj = in ? m[j] : 0.f;
+            v[3][k] = mj;
+            if (mj != 0.f) {   // true for NaN
+                if (!(fabsf(mj) >= kRefMinMass && fabsf(mj) <= kRefMaxMass)) f |= kRefPlain;
+                if ((__float_as_int(mj) & 0x7fffff) == 0) f |= kRefPow2;
+            }
         }
-        if (valid) out[i] = acc;
+        Src4 o;
+        o.x = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
+        o.y = make_float4(v[1][0], v[1][1], v[1][2], v[1][3]);
+        o.z = make_float4(v[2][0], v[2][1], v[2][2], v[2][3]);
+        o.m = make_float4(v[3][0], v[3][1], v[3][2], v[3][3]);
+        src[q] = o;
     }
+    for (int64_t i = i0; i < nt; i += step) {
+        coord(tx[i]);
+        coord(ty[i]);
+        coord(tz[i]);
+    }
+    f = __reduce_or_sync(0xffffffffu, f);
+    if (f && (threadIdx.x & 31) == 0) atomicOr(flags, f);
+}
+
+// Two terms by the correction steps (+0 where the mask drops the pair); smin follows the smallest
+// s met, ones is set when a square root's mantissa is all ones (ONES).  The squares are
+// multiply-adds of nz = -0, a kernel argument: the compiler contracts a two-lane product and the
+// sum that takes it (also with .rn, and when it knows the -0), which would leave the product unrounded.
+template <bool ONES>
+__device__ __forceinline__ f2x ref_terms2(f2x X, f2x Y, f2x Z, float m0, float m1, f2x tx, f2x ty, f2x tz, f2x nz,
+                                          float &smin, bool &ones) {
+    const f2x dx = sub2(X, tx), dy = sub2(Y, ty), dz = sub2(Z, tz);
+    const f2x s = add2(add2(fma2(dx, dx, nz), fma2(dy, dy, nz)), fma2(dz, dz, nz));
+    float a0, a1, b0, b1, c0, c1, s0, s1;
+    unpack2(dx, a0, a1);
+    unpack2(dy, b0, b1);
+    unpack2(dz, c0, c1);
+    unpack2(s, s0, s1);
+    // x, y and z all differ <=> no difference is zero (subnormals are kept)
+    const bool k0 = fminf(fminf(fabsf(a0), fabsf(b0)), fabsf(c0)) > 0.f;
+    const bool k1 = fminf(fminf(fabsf(a1), fabsf(b1)), fabsf(c1)) > 0.f;
+    smin = fminf(fminf(smin, s0), s1);
+    const f2x M = pack2(k0 ? m0 : 0.f, k1 ? m1 : 0.f);
+    const f2x y = pack2(rsqrt_ftz(s0), rsqrt_ftz(s1));
+    const f2x g = mul2(s, y), ng = mul2(g, pack2(-1.f, -1.f));
+    const f2x nr = fma2(fma2(ng, g, s), mul2(y, pack2(-0.5f, -0.5f)), ng);   // minus the square root
+    if (ONES) {
+        float r0, r1;
+        unpack2(nr, r0, r1);
+        ones |= ((~__float_as_int(r0) & 0x7fffff) == 0) | ((~__float_as_int(r1) & 0x7fffff) == 0);
+    }
+    const f2x iz = fma2(y, fma2(nr, y, pack2(1.f, 1.f)), y);
+    const f2x q = mul2(M, iz);
+    return fma2(fma2(nr, q, M), iz, q);
+}
+
+// The lane's quads q0, q0 + step, .. (N of them) of the stage against its target, terms to out[quad][TL].
+template <int TL, int N, bool ONES>
+__device__ __forceinline__ bool ref_quads(const Src4 *__restrict__ src, int q0, float px, float py, float pz, float nzero,
+                                          float4 *__restrict__ out, int t) {
+    const f2x tx = pack2(px, px), ty = pack2(py, py), tz = pack2(pz, pz), nz = pack2(nzero, nzero);
+    float smin = kRefMaxCoord;
+    bool ones = false;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int q = q0 + i * (32 / TL);
+        const float4 X = __ldg(&src[q].x), Y = __ldg(&src[q].y), Z = __ldg(&src[q].z), M = __ldg(&src[q].m);
+        const f2x lo = ref_terms2<ONES>(pack2(X.x, X.y), pack2(Y.x, Y.y), pack2(Z.x, Z.y), M.x, M.y, tx, ty, tz,
+                                        nz, smin, ones);
+        const f2x hi = ref_terms2<ONES>(pack2(X.z, X.w), pack2(Y.z, Y.w), pack2(Z.z, Z.w), M.z, M.w, tx, ty, tz,
+                                        nz, smin, ones);
+        float4 v;
+        unpack2(lo, v.x, v.y);
+        unpack2(hi, v.z, v.w);
+        out[q * TL + t] = v;
+    }
+    return smin < kRefMinS || ones;
+}
+
+// The same with the plain operations.
+template <int TL, int N>
+__device__ __noinline__ void ref_quads_plain(const Src4 *__restrict__ src, int q0, float px, float py, float pz,
+                                             float4 *__restrict__ out, int t) {
+    for (int i = 0; i < N; ++i) {
+        const int q = q0 + i * (32 / TL);
+        const float4 X = __ldg(&src[q].x), Y = __ldg(&src[q].y), Z = __ldg(&src[q].z), M = __ldg(&src[q].m);
+        float4 v;
+        v.x = pair_term_reference(make_float4(X.x, Y.x, Z.x, M.x), px, py, pz);
+        v.y = pair_term_reference(make_float4(X.y, Y.y, Z.y, M.y), px, py, pz);
+        v.z = pair_term_reference(make_float4(X.z, Y.z, Z.z, M.z), px, py, pz);
+        v.w = pair_term_reference(make_float4(X.w, Y.w, Z.w, M.w), px, py, pz);
+        out[q * TL + t] = v;
+    }
+}
+
+template <int TL>
+__global__ void __launch_bounds__(kRefThreads) ref_potential_kernel(const Src4 *__restrict__ src, int64_t nstages,
+                                                                    const float *__restrict__ tx,
+                                                                    const float *__restrict__ ty,
+                                                                    const float *__restrict__ tz, int64_t nt,
+                                                                    const int *__restrict__ flags,
+                                                                    float nzero, float *__restrict__ out) {
+    extern __shared__ float4 ref_terms[];   // [2][kRefQuads][TL]
+    constexpr int G = 32 / TL, N = kRefQuads / kRefWarps / G;
+    static_assert(N >= 1 && N * kRefWarps * G == kRefQuads, "a stage is split evenly over the lanes");
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int t = lane % TL;
+    const int64_t i = (int64_t)blockIdx.x * TL + t;
+    const int64_t it = i < nt ? i : nt - 1;
+    const float px = tx[it], py = ty[it], pz = tz[it];
+    const int fl = *flags;
+    const int q0 = w * (kRefQuads / kRefWarps) + lane / TL;
+    float acc = 0.f;
+    for (int64_t st = 0; st <= nstages; ++st) {
+        if (w < kRefWarps) {
+            if (st < nstages) {
+                float4 *buf = ref_terms + (st & 1) * kRefQuads * TL;
+                const Src4 *s = src + st * kRefQuads;
+                bool again = (fl & kRefPlain) != 0;
+                if (!again)
+                    again = (fl & kRefPow2) ? ref_quads<TL, N, true>(s, q0, px, py, pz, nzero, buf, t)
+                                            : ref_quads<TL, N, false>(s, q0, px, py, pz, nzero, buf, t);
+                if (again) ref_quads_plain<TL, N>(s, q0, px, py, pz, buf, t);
+            }
+        } else if (st > 0 && lane < TL) {
+            const float4 *buf = ref_terms + ((st - 1) & 1) * kRefQuads * TL;
+#pragma unroll 8
+            for (int q = 0; q < kRefQuads; ++q) {
+                const float4 v = buf[q * TL + t];
+                acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, v.x), v.y), v.z), v.w);
+            }
+        }
+        __syncthreads();
+    }
+    if (w == kRefWarps && lane < TL && i < nt) out[i] = acc;
+}
+
+template <int TL>
+static int launch_reference(const Src4 *src, int64_t nstages, const float *tx, const float *ty, const float *tz,
+                            int64_t nt, const int *flags, float *out, cudaStream_t st) {
+    constexpr int smem = 2 * kRefQuads * TL * (int)sizeof(float4);
+    HALMA_CUDA(cudaFuncSetAttribute(ref_potential_kernel<TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    HALMA_LAUNCH(ref_potential_kernel<TL>, (unsigned)((nt + TL - 1) / TL), kRefThreads, smem, st, src, nstages, tx, ty, tz, nt,
+                 flags, -0.0f, out);
+    return HALMA_OK;
 }
 
 // HALMA_POT_FAST: T targets per lane, FP32 rsqrt pair terms with the reference mask, each
@@ -350,17 +522,26 @@ extern "C" int halma_bf_potential_f32(int64_t ntotal, const float *total_mass, c
     sg.add(test_y, ntest, true, false, &ty);
     sg.add(test_z, ntest, true, false, &tz);
     sg.add((const float *)binding_energy, ntest, false, true, &out);
+    const int64_t nstages = (ntotal + kRefStage - 1) / kRefStage, nquads = nstages * kRefQuads;
     Layout L;
     sg.plan(L);
+    const size_t o_src = L.add(sizeof(Src4) * (size_t)nquads), o_flags = L.add(sizeof(int));
     void *base = nullptr;
     HALMA_TRY(workspace(L.total, &base, st));
     HALMA_TRY(sg.bind_and_upload(base, st));
     if (ntotal == 0) {
         HALMA_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * ntest, st));
     } else {
-        const int64_t ntiles = (ntest + 31) / 32;
-        const int grid = (int)std::min<int64_t>((ntiles + kWarpsPerBlock - 1) / kWarpsPerBlock, (int64_t)device_sm_count() * 16);
-        HALMA_LAUNCH(bf_potential_reference_kernel, grid, 256, 0, st, m, x, y, z, ntotal, tx, ty, tz, ntest, out);
+        Src4 *src = at<Src4>(base, o_src);
+        int *flags = at<int>(base, o_flags);
+        HALMA_CUDA(cudaMemsetAsync(flags, 0, sizeof(int), st));
+        const int sms = device_sm_count();
+        HALMA_LAUNCH(ref_pack_kernel, grid_for(std::max(nquads, ntest), 256, sms * 8), 256, 0, st, m, x, y, z, ntotal,
+                     nquads, tx, ty, tz, ntest, src, flags);
+        if (ntest <= (int64_t)8 * 3 * sms)
+            HALMA_TRY(launch_reference<8>(src, nstages, tx, ty, tz, ntest, flags, out, st));
+        else
+            HALMA_TRY(launch_reference<32>(src, nstages, tx, ty, tz, ntest, flags, out, st));
     }
     return sg.download(st);
 }

@@ -141,3 +141,40 @@ def test_self_set_potential_symmetric_route(cuda, nt, ns, self_mask):
                                mask=oracle.MASK_SELF if self_mask else oracle.MASK_NONE)
     assert np.max(np.abs(phi / ref - 1.0)) <= RTOL_FAST
     assert np.max(np.abs(phi.astype(np.float64) / tile - 1.0)) <= RTOL_FAST
+
+
+def _reference_inputs(kind, ns, nt, seed):
+    """float32 sources and targets; half of the targets are sources (coincident points)."""
+    rng = np.random.default_rng(seed)
+    scale = {"tiny": 1e-30, "huge": 1e18}.get(kind, 0.05)
+    s = (rng.normal(0.0, scale, (ns, 3)) + (3.0 if kind == "offset" else 0.0)).astype(np.float32)
+    t = (rng.normal(0.0, scale, (nt, 3)) + (3.0 if kind == "offset" else 0.0)).astype(np.float32)
+    k = min(ns, nt // 2)
+    t[:k] = s[rng.permutation(ns)[:k]]
+    m = np.exp(rng.normal(np.log(1e5), 1.0, ns)).astype(np.float32)
+    if kind == "signs":
+        m *= rng.choice([-1.0, 0.0, 1.0], ns).astype(np.float32)
+    if kind == "ones":   # square roots whose mantissa is all ones, masses a power of two
+        t[: nt // 2 + 1] = 0.0
+        s[rng.random(ns) < 0.5] = np.float32([2.0 - 2.0 ** -23, 1e-7, 1e-7])
+        m = (2.0 ** rng.integers(-2, 3, ns)).astype(np.float32)
+    if kind == "masses":
+        m = (10.0 ** rng.uniform(-37, 37, ns)).astype(np.float32)
+    if kind == "nonfinite":
+        s[rng.integers(0, ns), 0] = np.inf
+        t[0, 1] = np.nan
+        m[rng.integers(0, ns)] = np.inf
+    return s, t, m
+
+
+@pytest.mark.parametrize("kind,ns,nt", [
+    ("offset", 1, 1), ("offset", 255, 7), ("offset", 256, 8), ("offset", 257, 9), ("centred", 1023, 33),
+    ("centred", 511, 3648), ("centred", 300, 3649), ("offset", 2049, 4863), ("tiny", 700, 65), ("huge", 700, 65),
+    ("signs", 513, 3700), ("ones", 600, 50), ("ones", 300, 4000), ("masses", 600, 129), ("nonfinite", 400, 40)])
+def test_reference_mode_split_over_sources(cuda, kind, ns, nt):
+    """Terms computed by several warps and added in order: bit for bit the sequential loop."""
+    s, t, m = _reference_inputs(kind, ns, nt, 7)
+    got = halo_gas.bf_potential(m, *s.T, *t.T, mode="reference")
+    with np.errstate(all="ignore"):
+        ref = oracle.bf_potential_f32(m, *s.T, *t.T)
+    np.testing.assert_array_equal(got, ref)
