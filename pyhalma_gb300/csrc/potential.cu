@@ -33,7 +33,10 @@ __device__ __forceinline__ float4 load_source(const float *__restrict__ m, const
 // warp doing both in turn left the GPU waiting on single dependent chains: 2,000 targets x
 // 20,000 sources took 2.20 ms, 40,000 x 100,000 12.2 ms (2.2 warps on an SM's scheduler).
 //
-// Bound of the terms: the FP32 pipe, 18 two-lane instructions for two terms.  Square root and
+// So: 0.065 ms and 3.7 ms.
+//
+// Bound of the terms: the FP32 pipe, 18 two-lane instructions for two terms (measured: 57 % of it
+// busy, 3.6 terms per SM-cycle).  Square root and
 // quotient come from one rsqrt y of s by Markstein's correction steps (P. Markstein, Computation
 // of elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990):
 // g = s y, r = g + (s - g g) y / 2;  z = y + y (1 - r y);  q = m z, t = q + (m - r q) z.  r is the
@@ -43,10 +46,6 @@ __device__ __forceinline__ float4 load_source(const float *__restrict__ m, const
 // for one m, a power of two, when r's mantissa is all ones.  Those pairs (looked for when a mass is a
 // power of two), squared distances under 2^-90, coordinates or masses outside the ranges below
 // and values that are not finite take the plain operations instead.
-constexpr int kRefWarps = 8;                      // warps that compute terms; one more adds them
-constexpr int kRefStage = 256;                    // sources of one stage
-constexpr int kRefQuads = kRefStage / 4;
-constexpr int kRefThreads = (kRefWarps + 1) * 32;
 constexpr float kRefFar = 1.0e15f;                // sources past the end: m = 0 here gives +0 terms
 constexpr float kRefMaxCoord = 0x1p48f, kRefMinMass = 0x1p-40f, kRefMaxMass = 0x1p80f, kRefMinS = 0x1p-90f;
 enum { kRefPlain = 1, kRefPow2 = 2 };             // bits of the flags word
@@ -132,9 +131,10 @@ __device__ __forceinline__ f2x ref_terms2(f2x X, f2x Y, f2x Z, float m0, float m
     return fma2(fma2(nr, q, M), iz, q);
 }
 
-// The lane's quads q0, q0 + step, .. (N of them) of the stage against its target, terms to out[quad][TL].
+// The lane's quads q0, q0 + step, .. (N of them) of its warp's sources against its target, terms to
+// out[quad][TL].
 template <int TL, int N, bool ONES>
-__device__ __forceinline__ bool ref_quads(const Src4 *__restrict__ src, int q0, float px, float py, float pz, float nzero,
+__device__ __forceinline__ bool ref_quads(const Src4 *src, int q0, float px, float py, float pz, float nzero,
                                           float4 *__restrict__ out, int t) {
     const f2x tx = pack2(px, px), ty = pack2(py, py), tz = pack2(pz, pz), nz = pack2(nzero, nzero);
     float smin = kRefMaxCoord;
@@ -142,7 +142,7 @@ __device__ __forceinline__ bool ref_quads(const Src4 *__restrict__ src, int q0, 
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         const int q = q0 + i * (32 / TL);
-        const float4 X = __ldg(&src[q].x), Y = __ldg(&src[q].y), Z = __ldg(&src[q].z), M = __ldg(&src[q].m);
+        const float4 X = src[q].x, Y = src[q].y, Z = src[q].z, M = src[q].m;
         const f2x lo = ref_terms2<ONES>(pack2(X.x, X.y), pack2(Y.x, Y.y), pack2(Z.x, Z.y), M.x, M.y, tx, ty, tz,
                                         nz, smin, ones);
         const f2x hi = ref_terms2<ONES>(pack2(X.z, X.w), pack2(Y.z, Y.w), pack2(Z.z, Z.w), M.z, M.w, tx, ty, tz,
@@ -157,11 +157,11 @@ __device__ __forceinline__ bool ref_quads(const Src4 *__restrict__ src, int q0, 
 
 // The same with the plain operations.
 template <int TL, int N>
-__device__ __noinline__ void ref_quads_plain(const Src4 *__restrict__ src, int q0, float px, float py, float pz,
+__device__ __noinline__ void ref_quads_plain(const Src4 *src, int q0, float px, float py, float pz,
                                              float4 *__restrict__ out, int t) {
     for (int i = 0; i < N; ++i) {
         const int q = q0 + i * (32 / TL);
-        const float4 X = __ldg(&src[q].x), Y = __ldg(&src[q].y), Z = __ldg(&src[q].z), M = __ldg(&src[q].m);
+        const float4 X = src[q].x, Y = src[q].y, Z = src[q].z, M = src[q].m;
         float4 v;
         v.x = pair_term_reference(make_float4(X.x, Y.x, Z.x, M.x), px, py, pz);
         v.y = pair_term_reference(make_float4(X.y, Y.y, Z.y, M.y), px, py, pz);
@@ -171,55 +171,107 @@ __device__ __noinline__ void ref_quads_plain(const Src4 *__restrict__ src, int q
     }
 }
 
+// TL targets a block.  Wide (32): eight warps compute, the ninth adds, for target counts that keep
+// the SMs busy; there the terms are the bound (at most three such blocks fit an SM).  Narrow (8):
+// for fewer targets the additions are, 4.1 cycles each at best; six warps compute, and the adding
+// warp has a scheduler (every fourth warp) to itself: it shares it only with the adding warps of
+// the SM's other blocks (sharing it with computing warps: 7 us more of 65 at 2,000 x 20,000).
 template <int TL>
-__global__ void __launch_bounds__(kRefThreads) ref_potential_kernel(const Src4 *__restrict__ src, int64_t nstages,
-                                                                    const float *__restrict__ tx,
-                                                                    const float *__restrict__ ty,
-                                                                    const float *__restrict__ tz, int64_t nt,
-                                                                    const int *__restrict__ flags,
-                                                                    float nzero, float *__restrict__ out) {
-    extern __shared__ float4 ref_terms[];   // [2][kRefQuads][TL]
-    constexpr int G = 32 / TL, N = kRefQuads / kRefWarps / G;
-    static_assert(N >= 1 && N * kRefWarps * G == kRefQuads, "a stage is split evenly over the lanes");
+struct RefShape {
+    static constexpr bool wide = TL == 32;
+    static constexpr int computing = wide ? 8 : 6, warps = wide ? 9 : 8;
+    static constexpr int take = wide ? 8 : 16;       // quads of a warp in one stage
+    static constexpr int quads = computing * take;   // of all
+    __device__ static int computes(int w) { return wide ? w : (w % 4 == 3 ? -1 : w - w / 4); }   // its share, or -1
+    __device__ static bool adds(int w) { return w == (wide ? 8 : 3); }
+};
+
+template <int TL>
+__global__ void __launch_bounds__(RefShape<TL>::warps * 32) ref_potential_kernel(
+    const Src4 *__restrict__ src, int64_t nstages, const float *__restrict__ tx, const float *__restrict__ ty,
+    const float *__restrict__ tz, int64_t nt, const int *__restrict__ flags, float nzero, float *__restrict__ out) {
+    using S = RefShape<TL>;
+    constexpr int N = S::take * TL / 32;    // quads of a lane in one stage
+    extern __shared__ float4 ref_terms[];    // [2][S::quads][TL]
+    __shared__ Src4 quads[S::computing][2][S::take];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int share = w < S::warps - (S::wide ? 1 : 0) ? S::computes(w) : -1;
     const int t = lane % TL;
     const int64_t i = (int64_t)blockIdx.x * TL + t;
     const int64_t it = i < nt ? i : nt - 1;
     const float px = tx[it], py = ty[it], pz = tz[it];
     const int fl = *flags;
-    const int q0 = w * (kRefQuads / kRefWarps) + lane / TL;
+    // every warp copies its own next sources while it computes
+    auto fetch = [&](int64_t st) {
+        if (st < nstages) {
+            const float4 *from = reinterpret_cast<const float4 *>(src + st * S::quads + share * S::take);
+            float4 *to = reinterpret_cast<float4 *>(quads[share][st & 1]);
+#pragma unroll
+            for (int k = lane; k < S::take * 4; k += 32)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                 (unsigned)__cvta_generic_to_shared(to + k)),
+                             "l"(from + k)
+                             : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (share >= 0) fetch(0);
     float acc = 0.f;
     for (int64_t st = 0; st <= nstages; ++st) {
-        if (w < kRefWarps) {
-            if (st < nstages) {
-                float4 *buf = ref_terms + (st & 1) * kRefQuads * TL;
-                const Src4 *s = src + st * kRefQuads;
-                bool again = (fl & kRefPlain) != 0;
-                if (!again)
-                    again = (fl & kRefPow2) ? ref_quads<TL, N, true>(s, q0, px, py, pz, nzero, buf, t)
-                                            : ref_quads<TL, N, false>(s, q0, px, py, pz, nzero, buf, t);
-                if (again) ref_quads_plain<TL, N>(s, q0, px, py, pz, buf, t);
-            }
-        } else if (st > 0 && lane < TL) {
-            const float4 *buf = ref_terms + ((st - 1) & 1) * kRefQuads * TL;
-#pragma unroll 8
-            for (int q = 0; q < kRefQuads; ++q) {
-                const float4 v = buf[q * TL + t];
-                acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, v.x), v.y), v.z), v.w);
+        if (share >= 0 && st < nstages) {
+            fetch(st + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncwarp();
+            float4 *buf = ref_terms + ((st & 1) * S::quads + share * S::take) * TL;
+            const Src4 *s = quads[share][st & 1];
+            bool again = (fl & kRefPlain) != 0;
+            if (!again)
+                again = (fl & kRefPow2) ? ref_quads<TL, N, true>(s, lane / TL, px, py, pz, nzero, buf, t)
+                                        : ref_quads<TL, N, false>(s, lane / TL, px, py, pz, nzero, buf, t);
+            if (again) ref_quads_plain<TL, N>(s, lane / TL, px, py, pz, buf, t);
+        } else if (S::adds(w) && st > 0 && lane < TL) {
+            const float4 *buf = ref_terms + ((st - 1) & 1) * S::quads * TL;
+            // the next eight loads are in flight during the 32 additions of the last eight
+            float4 v[8], u[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = buf[k * TL + t];
+#pragma unroll
+            for (int q = 0; q < S::quads; q += 8) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (q + 8 < S::quads) u[k] = buf[(q + 8 + k) * TL + t];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    acc = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(acc, v[k].x), v[k].y), v[k].z), v[k].w);
+                    v[k] = u[k];
+                }
             }
         }
         __syncthreads();
     }
-    if (w == kRefWarps && lane < TL && i < nt) out[i] = acc;
+    if (S::adds(w) && lane < TL && i < nt) out[i] = acc;
+}
+
+// Packs the sources and runs the kernel; src holds ref_quads_of(ntotal) quads.
+template <int TL>
+static int64_t ref_quads_of(int64_t ns) {
+    const int64_t q = RefShape<TL>::quads;
+    return ((ns + 3) / 4 + q - 1) / q * q;
 }
 
 template <int TL>
-static int launch_reference(const Src4 *src, int64_t nstages, const float *tx, const float *ty, const float *tz,
-                            int64_t nt, const int *flags, float *out, cudaStream_t st) {
-    constexpr int smem = 2 * kRefQuads * TL * (int)sizeof(float4);
+static int launch_reference(const float *m, const float *x, const float *y, const float *z, int64_t ns, const float *tx,
+                            const float *ty, const float *tz, int64_t nt, Src4 *src, int *flags, float *out,
+                            cudaStream_t st) {
+    using S = RefShape<TL>;
+    const int64_t nquads = ref_quads_of<TL>(ns);
+    HALMA_CUDA(cudaMemsetAsync(flags, 0, sizeof(int), st));
+    HALMA_LAUNCH(ref_pack_kernel, grid_for(std::max(nquads, nt), 256, device_sm_count() * 8), 256, 0, st, m, x, y, z, ns,
+                 nquads, tx, ty, tz, nt, src, flags);
+    constexpr int smem = 2 * S::quads * TL * (int)sizeof(float4);
     HALMA_CUDA(cudaFuncSetAttribute(ref_potential_kernel<TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    HALMA_LAUNCH(ref_potential_kernel<TL>, (unsigned)((nt + TL - 1) / TL), kRefThreads, smem, st, src, nstages, tx, ty, tz, nt,
-                 flags, -0.0f, out);
+    HALMA_LAUNCH(ref_potential_kernel<TL>, (unsigned)((nt + TL - 1) / TL), S::warps * 32, smem, st, src,
+                 nquads / S::quads, tx, ty, tz, nt, flags, -0.0f, out);
     return HALMA_OK;
 }
 
@@ -522,10 +574,13 @@ extern "C" int halma_bf_potential_f32(int64_t ntotal, const float *total_mass, c
     sg.add(test_y, ntest, true, false, &ty);
     sg.add(test_z, ntest, true, false, &tz);
     sg.add((const float *)binding_energy, ntest, false, true, &out);
-    const int64_t nstages = (ntotal + kRefStage - 1) / kRefStage, nquads = nstages * kRefQuads;
+    // narrow blocks while three of them an SM hold all targets: 2,000 x 20,000 takes 75 us so and 115 us
+    // in wide ones, 4,500 x 20,000 128 and 115 us
+    const bool narrow = ntest <= (int64_t)8 * 3 * device_sm_count();
     Layout L;
     sg.plan(L);
-    const size_t o_src = L.add(sizeof(Src4) * (size_t)nquads), o_flags = L.add(sizeof(int));
+    const size_t o_src = L.add(sizeof(Src4) * (size_t)(narrow ? ref_quads_of<8>(ntotal) : ref_quads_of<32>(ntotal)));
+    const size_t o_flags = L.add(sizeof(int));
     void *base = nullptr;
     HALMA_TRY(workspace(L.total, &base, st));
     HALMA_TRY(sg.bind_and_upload(base, st));
@@ -534,14 +589,8 @@ extern "C" int halma_bf_potential_f32(int64_t ntotal, const float *total_mass, c
     } else {
         Src4 *src = at<Src4>(base, o_src);
         int *flags = at<int>(base, o_flags);
-        HALMA_CUDA(cudaMemsetAsync(flags, 0, sizeof(int), st));
-        const int sms = device_sm_count();
-        HALMA_LAUNCH(ref_pack_kernel, grid_for(std::max(nquads, ntest), 256, sms * 8), 256, 0, st, m, x, y, z, ntotal,
-                     nquads, tx, ty, tz, ntest, src, flags);
-        if (ntest <= (int64_t)8 * 3 * sms)
-            HALMA_TRY(launch_reference<8>(src, nstages, tx, ty, tz, ntest, flags, out, st));
-        else
-            HALMA_TRY(launch_reference<32>(src, nstages, tx, ty, tz, ntest, flags, out, st));
+        HALMA_TRY(narrow ? launch_reference<8>(m, x, y, z, ntotal, tx, ty, tz, ntest, src, flags, out, st)
+                         : launch_reference<32>(m, x, y, z, ntotal, tx, ty, tz, ntest, src, flags, out, st));
     }
     return sg.download(st);
 }
