@@ -13,13 +13,15 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "pair_math.cuh"
 
 namespace halma {
 namespace {
 
-constexpr int kGWarps = 8;
+constexpr int kGWarps = 4, kGT = 2;
 constexpr float kFarG = 3.0e30f;
 
 __device__ __forceinline__ float4 load_b(const float *__restrict__ x, const float *__restrict__ y,
@@ -72,76 +74,143 @@ __device__ __forceinline__ void fold2(float &s, float &c, f2x v) {
     two_sum_acc(s, c, lo + hi);
 }
 
-// One warp per tile of 32*T particles a against all partners b, streamed in chunks of 32
-// through a per-warp shared buffer; chunk partials folded into TwoSum-compensated sums.
+// One warp per item: a tile of 32*T particles a against one slice of the partners b, streamed in
+// chunks of 32 through a per-warp shared buffer; chunk partials folded into TwoSum-compensated sums.
+// A slice's sums go to part[(slice * na + a) * NV + v] (v: the scalar sum if wanted, then the vector), added
+// in slice order by adjoint_reduce_kernel; with one slice they are the result.
+//
+// Bound: the FP32 pipe (12 or 13 lane-operations a pair, 10 pairs per SM-cycle).  The partners are sliced so
+// that several items wait for every warp slot (choose_slices): one item per tile left 94 warps for 3,000
+// cells (150 us a sweep, now 15) and 2.06 blocks an SM, the third round nearly empty, for 160,000
+// (19.6 ms, now 11.5).
 template <int T, bool WANT_S>
-__global__ void __launch_bounds__(256, 3) adjoint_kernel(
+__global__ void __launch_bounds__(32 * kGWarps) adjoint_kernel(
     const float *__restrict__ bx, const float *__restrict__ by, const float *__restrict__ bz,
     const float *__restrict__ bw, int64_t nb, const float *__restrict__ ax, const float *__restrict__ ay,
-    const float *__restrict__ az, int64_t na, float eps2, int self_mask, int64_t self_off,
-    const float *__restrict__ vscale, float *__restrict__ out_s, float *__restrict__ out_v) {
+    const float *__restrict__ az, int64_t na, float eps2, int self_mask, int64_t self_off, int n_split,
+    int64_t split_len, const float *__restrict__ vscale, float *__restrict__ out_s, float *__restrict__ out_v,
+    double *__restrict__ part) {
     __shared__ float4 buf[kGWarps][32];
+    constexpr int NV = WANT_S ? 4 : 3;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float *sa = reinterpret_cast<float *>(buf[w]);        // 16 float4: x/y pairs
     float *sb = reinterpret_cast<float *>(buf[w] + 16);   // 16 float4: z/w pairs
     const int kp = lane >> 1, hf = lane & 1;
     const f2x e2 = pack2(eps2, eps2);
     const int64_t ntiles = (na + 32 * T - 1) / (32 * T);
-    for (int64_t tile = (int64_t)blockIdx.x * kGWarps + w; tile < ntiles; tile += (int64_t)gridDim.x * kGWarps) {
-        f2x px[T], py[T], pz[T];
-        float ss[T], sc[T], vxs[T], vxc[T], vys[T], vyc[T], vzs[T], vzc[T];
-        int64_t self[T];
+    const int64_t item = (int64_t)blockIdx.x * kGWarps + w;
+    if (item >= ntiles * n_split) return;
+    const int64_t tile = item % ntiles;
+    const int64_t slice = item / ntiles;
+    const int64_t jb = slice * split_len, je = jb + split_len < nb ? jb + split_len : nb;
+    f2x px[T], py[T], pz[T];
+    float ss[T], sc[T], vxs[T], vxc[T], vys[T], vyc[T], vzs[T], vzc[T];
+    int64_t self[T];
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        const int64_t a = tile * 32 * T + t * 32 + lane;
+        const bool v = a < na;
+        const float x = v ? ax[a] : kFarG, y = v ? ay[a] : kFarG, z = v ? az[a] : kFarG;
+        px[t] = pack2(x, x);
+        py[t] = pack2(y, y);
+        pz[t] = pack2(z, z);
+        self[t] = (v && self_mask) ? a + self_off : -1;
+        ss[t] = sc[t] = vxs[t] = vxc[t] = vys[t] = vyc[t] = vzs[t] = vzc[t] = 0.f;
+    }
+    // partner indices self[t] lie in [lo_self, lo_self + 32 * T) for this tile
+    const int64_t lo_self = tile * 32 * T + self_off;
+    float4 nxt = load_b(bx, by, bz, bw, jb + lane, je);
+    for (int64_t j0 = jb; j0 < je; j0 += 32) {
+        __syncwarp();
+        sa[kp * 4 + hf] = nxt.x;
+        sa[kp * 4 + 2 + hf] = nxt.y;
+        sb[kp * 4 + hf] = nxt.z;
+        sb[kp * 4 + 2 + hf] = nxt.w;
+        __syncwarp();
+        nxt = load_b(bx, by, bz, bw, j0 + 32 + lane, je);
+        f2x ps[T], pvx[T], pvy[T], pvz[T];
+#pragma unroll
+        for (int t = 0; t < T; ++t) ps[t] = pvx[t] = pvy[t] = pvz[t] = pack2(0.f, 0.f);
+        const bool self_chunk = self_mask && j0 + 32 > lo_self && j0 < lo_self + 32 * T;
+        if (self_chunk)
+            adjoint_chunk<T, WANT_S, true>(buf[w], buf[w] + 16, px, py, pz, e2, j0, self, ps, pvx, pvy, pvz);
+        else
+            adjoint_chunk<T, WANT_S, false>(buf[w], buf[w] + 16, px, py, pz, e2, j0, self, ps, pvx, pvy, pvz);
 #pragma unroll
         for (int t = 0; t < T; ++t) {
-            const int64_t a = tile * 32 * T + t * 32 + lane;
-            const bool v = a < na;
-            const float x = v ? ax[a] : kFarG, y = v ? ay[a] : kFarG, z = v ? az[a] : kFarG;
-            px[t] = pack2(x, x);
-            py[t] = pack2(y, y);
-            pz[t] = pack2(z, z);
-            self[t] = (v && self_mask) ? a + self_off : -1;
-            ss[t] = sc[t] = vxs[t] = vxc[t] = vys[t] = vyc[t] = vzs[t] = vzc[t] = 0.f;
-        }
-        // partner indices self[t] lie in [lo_self, lo_self + 32 * T) for this tile
-        const int64_t lo_self = tile * 32 * T + self_off;
-        float4 nxt = load_b(bx, by, bz, bw, lane, nb);
-        for (int64_t j0 = 0; j0 < nb; j0 += 32) {
-            __syncwarp();
-            sa[kp * 4 + hf] = nxt.x;
-            sa[kp * 4 + 2 + hf] = nxt.y;
-            sb[kp * 4 + hf] = nxt.z;
-            sb[kp * 4 + 2 + hf] = nxt.w;
-            __syncwarp();
-            nxt = load_b(bx, by, bz, bw, j0 + 32 + lane, nb);
-            f2x ps[T], pvx[T], pvy[T], pvz[T];
-#pragma unroll
-            for (int t = 0; t < T; ++t) ps[t] = pvx[t] = pvy[t] = pvz[t] = pack2(0.f, 0.f);
-            const bool self_chunk = self_mask && j0 + 32 > lo_self && j0 < lo_self + 32 * T;
-            if (self_chunk)
-                adjoint_chunk<T, WANT_S, true>(buf[w], buf[w] + 16, px, py, pz, e2, j0, self, ps, pvx, pvy, pvz);
-            else
-                adjoint_chunk<T, WANT_S, false>(buf[w], buf[w] + 16, px, py, pz, e2, j0, self, ps, pvx, pvy, pvz);
-#pragma unroll
-            for (int t = 0; t < T; ++t) {
-                if (WANT_S) fold2(ss[t], sc[t], ps[t]);
-                fold2(vxs[t], vxc[t], pvx[t]);
-                fold2(vys[t], vyc[t], pvy[t]);
-                fold2(vzs[t], vzc[t], pvz[t]);
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < T; ++t) {
-            const int64_t a = tile * 32 * T + t * 32 + lane;
-            if (a >= na) continue;
-            if (WANT_S && out_s) out_s[a] = ss[t] + sc[t];
-            if (out_v) {
-                const float sc_ = vscale[a];
-                out_v[3 * a + 0] = sc_ * (vxs[t] + vxc[t]);
-                out_v[3 * a + 1] = sc_ * (vys[t] + vyc[t]);
-                out_v[3 * a + 2] = sc_ * (vzs[t] + vzc[t]);
-            }
+            if (WANT_S) fold2(ss[t], sc[t], ps[t]);
+            fold2(vxs[t], vxc[t], pvx[t]);
+            fold2(vys[t], vyc[t], pvy[t]);
+            fold2(vzs[t], vzc[t], pvz[t]);
         }
     }
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        const int64_t a = tile * 32 * T + t * 32 + lane;
+        if (a >= na) continue;
+        if (n_split > 1) {
+            double *p = part + (slice * na + a) * NV;
+            if (WANT_S) p[0] = (double)ss[t] + (double)sc[t];
+            p[NV - 3] = (double)vxs[t] + (double)vxc[t];
+            p[NV - 2] = (double)vys[t] + (double)vyc[t];
+            p[NV - 1] = (double)vzs[t] + (double)vzc[t];
+            continue;
+        }
+        if (WANT_S && out_s) out_s[a] = ss[t] + sc[t];
+        if (out_v) {
+            const float sc_ = vscale[a];
+            out_v[3 * a + 0] = sc_ * (vxs[t] + vxc[t]);
+            out_v[3 * a + 1] = sc_ * (vys[t] + vyc[t]);
+            out_v[3 * a + 2] = sc_ * (vzs[t] + vzc[t]);
+        }
+    }
+}
+
+// The slices' sums in slice order (FP64), rounded to FP32 as a single slice's are, and scaled.
+template <bool WANT_S>
+__global__ void __launch_bounds__(256) adjoint_reduce_kernel(const double *__restrict__ part, int n_split, int64_t na,
+                                                             const float *__restrict__ vscale,
+                                                             float *__restrict__ out_s, float *__restrict__ out_v) {
+    constexpr int NV = WANT_S ? 4 : 3;
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < na * NV; k += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t a = k / NV;
+        const int v = (int)(k - a * NV) - (NV - 3);   // -1: the scalar sum
+        double acc = 0.0;
+#pragma unroll 8
+        for (int s = 0; s < n_split; ++s) acc += part[(int64_t)s * na * NV + k];
+        if (v < 0) {
+            if (out_s) out_s[a] = (float)acc;
+        } else if (out_v) {
+            out_v[3 * a + v] = vscale[a] * (float)acc;
+        }
+    }
+}
+
+// Slices of the partners: about eight items per warp slot (16 warps an SM), at least 128 partners each, and
+// at most 2^23 partial sums (64 MB) in all.
+void choose_slices(int64_t na, int64_t nb, int T, int nv, int *n_split, int64_t *split_len) {
+    const int64_t ntiles = (na + 32 * T - 1) / (32 * T);
+    int64_t s = ((int64_t)device_sm_count() * 16 * 8 + ntiles - 1) / ntiles;
+    s = std::min(s, std::min<int64_t>(nb / 128, (1ll << 23) / (na * nv)));
+    s = std::max<int64_t>(s, 1);
+    const int64_t len = ((nb + s - 1) / s + 31) / 32 * 32;
+    *n_split = (int)((nb + len - 1) / len);
+    *split_len = len;
+}
+
+template <bool WANT_S>
+int launch_adjoint(const float *bx, const float *by, const float *bz, const float *bw, int64_t nb, const float *ax,
+                   const float *ay, const float *az, int64_t na, float eps2, int self_mask, int64_t self_off,
+                   int n_split, int64_t split_len, const float *vscale, float *out_s, float *out_v, double *part,
+                   cudaStream_t st) {
+    constexpr int T = kGT, NV = WANT_S ? 4 : 3;
+    const int64_t items = (na + 32 * T - 1) / (32 * T) * n_split;
+    HALMA_LAUNCH((adjoint_kernel<T, WANT_S>), (unsigned)((items + kGWarps - 1) / kGWarps), 32 * kGWarps, 0, st, bx, by,
+                 bz, bw, nb, ax, ay, az, na, eps2, self_mask, self_off, n_split, split_len, vscale, out_s, out_v, part);
+    if (n_split > 1)
+        HALMA_LAUNCH(adjoint_reduce_kernel<WANT_S>, grid_for(na * NV, 256, device_sm_count() * 8), 256, 0, st, part,
+                     n_split, na, vscale, out_s, out_v);
+    return HALMA_OK;
 }
 
 }  // namespace
@@ -190,25 +259,23 @@ extern "C" int halma_potential_grad_f32(int64_t ns, const float *m_, const float
     sg.add((const float *)grad_m, grad_m ? ns : 0, false, true, &gm);
     sg.add((const float *)grad_src, grad_src ? 3 * ns : 0, false, true, &gs);
     sg.add((const float *)grad_tgt, grad_tgt ? 3 * nt : 0, false, true, &gt);
+    int split_t = 1, split_s = 1;
+    int64_t len_t = ns, len_s = nt;
+    if (grad_tgt) choose_slices(nt, ns, kGT, 3, &split_t, &len_t);
+    if (grad_m || grad_src) choose_slices(ns, nt, kGT, 4, &split_s, &len_s);
     Layout L;
     sg.plan(L);
+    const size_t o_part = L.add(8 * (size_t)std::max(split_t > 1 ? 3 * nt * split_t : 0, split_s > 1 ? 4 * ns * split_s : 0));
     void *base = nullptr;
     HALMA_TRY(workspace(L.total, &base, st));
     HALMA_TRY(sg.bind_and_upload(base, st));
+    double *part = at<double>(base, o_part);
     const int self = mask == HALMA_MASK_SELF;
-    constexpr int T = 2;
-    const int cap = device_sm_count() * 8;
-    if (gt) {
-        const int64_t tiles = (nt + 32 * T - 1) / (32 * T);
-        const int grid = (int)std::min<int64_t>((tiles + kGWarps - 1) / kGWarps, cap);
-        HALMA_LAUNCH((adjoint_kernel<T, false>), grid, 256, 0, st, sx, sy, sz, m, ns, tx, ty, tz, nt, (float)eps2,
-                     self, self_offset, g, (float *)nullptr, gt);
-    }
-    if (gm || gs) {
-        const int64_t tiles = (ns + 32 * T - 1) / (32 * T);
-        const int grid = (int)std::min<int64_t>((tiles + kGWarps - 1) / kGWarps, cap);
-        HALMA_LAUNCH((adjoint_kernel<T, true>), grid, 256, 0, st, tx, ty, tz, g, nt, sx, sy, sz, ns, (float)eps2,
-                     self, -self_offset, m, gm, gs);
-    }
+    if (gt)
+        HALMA_TRY(launch_adjoint<false>(sx, sy, sz, m, ns, tx, ty, tz, nt, (float)eps2, self, self_offset, split_t, len_t,
+                                        g, nullptr, gt, part, st));
+    if (gm || gs)
+        HALMA_TRY(launch_adjoint<true>(tx, ty, tz, g, nt, sx, sy, sz, ns, (float)eps2, self, -self_offset, split_s, len_s,
+                                       m, gm, gs, part, st));
     return sg.download(st);
 }

@@ -86,29 +86,6 @@ __device__ __forceinline__ float2 df_from_acc(float s, float c) { return df_fast
 
 __device__ __forceinline__ double df_to_double(float2 a) { return (double)a.x + (double)a.y; }
 
-// One softened pair term m / sqrt(r^2 + eps2) with the FP32 special-function rsqrt.
-__device__ __forceinline__ float pair_term_fast(float4 q, float px, float py, float pz, float eps2,
-                                                float acc) {
-    float dx = q.x - px;
-    float dy = q.y - py;
-    float dz = q.z - pz;
-    float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-    return fmaf(q.w, rsqrtf(r2), acc);
-}
-
-// Same, with the reference's pair mask: the term counts only when the source's x, y and z
-// all differ from the target's (particle_subroutines.f90:499-501).
-__device__ __forceinline__ float pair_term_fast_masked(float4 q, float px, float py, float pz,
-                                                       float eps2, float acc) {
-    float dx = q.x - px;
-    float dy = q.y - py;
-    float dz = q.z - pz;
-    float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-    float ri = rsqrtf(r2);
-    bool keep = (q.x != px) & (q.y != py) & (q.z != pz);
-    return fmaf(q.w, keep ? ri : 0.0f, acc);
-}
-
 // The reference's float32 term, each operation rounded on its own (no FMA):
 //   r = sqrt((xj-xi)**2 + (yj-yi)**2 + (zj-zi)**2); phi = phi + m / r
 // (particle_subroutines.f90:502-505); +0, which leaves the sum as it is, where the mask of

@@ -275,11 +275,56 @@ static int launch_reference(const float *m, const float *x, const float *y, cons
     return HALMA_OK;
 }
 
-// HALMA_POT_FAST: T targets per lane, FP32 rsqrt pair terms with the reference mask, each
-// 32-source chunk summed in FP32 and folded into a TwoSum-compensated accumulator.
+// HALMA_POT_FAST and the softened potential: T targets per lane, FP32 rsqrt pair terms, each 32-source
+// chunk summed in FP32 and folded into a TwoSum-compensated accumulator.
 // MASK: HALMA_MASK_COORD (reference mask), HALMA_MASK_SELF (skip j == i + self_offset) or
-// HALMA_MASK_NONE.
-template <int T, int MASK>
+// HALMA_MASK_NONE.  FTZ: eps2 is a normal float, so that no r^2 is subnormal and the rsqrt that
+// flushes subnormal arguments gives the same values (one instruction instead of five).
+//
+// Bound: the special-function unit (one rsqrt a term) and the FP32 pipe (7 lane-operations) together, as
+// the unbinding's tile kernel: two sources per two-lane instruction.  With one-lane instructions the
+// star terms of a 160,000-cell gas halo (6.4e9) took 2.29 ms, now 1.6.
+template <bool FTZ>
+__device__ __forceinline__ float pot_rsqrt(float v) {
+    return FTZ ? rsqrt_ftz(v) : rsqrtf(v);
+}
+
+// The chunk's 32 sources (sa[kp] = {x, x, y, y} of sources 2 kp and 2 kp + 1, sb[kp] = {z, z, m, m}) against
+// the lane's T targets.  SELF: source number self[t] of the chunk is skipped.
+template <int T, int MASK, bool FTZ, bool SELF>
+__device__ __forceinline__ void pot_chunk(const float4 *sa, const float4 *sb, const f2x (&px)[T], const f2x (&py)[T],
+                                          const f2x (&pz)[T], f2x e2, const int (&self)[T], f2x (&acc)[T]) {
+#pragma unroll 4
+    for (int kp = 0; kp < 16; ++kp) {
+        const float4 a = sa[kp], b = sb[kp];
+        const f2x X = pack2(a.x, a.y), Y = pack2(a.z, a.w), Z = pack2(b.x, b.y), M = pack2(b.z, b.w);
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            const f2x dx = sub2(X, px[t]), dy = sub2(Y, py[t]), dz = sub2(Z, pz[t]);
+            f2x r2 = fma2(dz, dz, e2);
+            r2 = fma2(dy, dy, r2);
+            r2 = fma2(dx, dx, r2);
+            float r0, r1;
+            unpack2(r2, r0, r1);
+            float i0 = pot_rsqrt<FTZ>(r0), i1 = pot_rsqrt<FTZ>(r1);
+            if (MASK == HALMA_MASK_COORD) {   // the coordinates themselves: equal infinities drop the pair too
+                float qx, qy, qz, hi;
+                unpack2(px[t], qx, hi);
+                unpack2(py[t], qy, hi);
+                unpack2(pz[t], qz, hi);
+                if (!((a.x != qx) & (a.z != qy) & (b.x != qz))) i0 = 0.f;
+                if (!((a.y != qx) & (a.w != qy) & (b.y != qz))) i1 = 0.f;
+            }
+            if (SELF) {
+                if (2 * kp == self[t]) i0 = 0.f;
+                if (2 * kp + 1 == self[t]) i1 = 0.f;
+            }
+            acc[t] = fma2(M, pack2(i0, i1), acc[t]);
+        }
+    }
+}
+
+template <int T, int MASK, bool FTZ>
 __global__ void __launch_bounds__(256) bf_potential_fast_kernel(
     const float *__restrict__ m, const float *__restrict__ x, const float *__restrict__ y,
     const float *__restrict__ z, int64_t ns, const float *__restrict__ tx,
@@ -288,6 +333,10 @@ __global__ void __launch_bounds__(256) bf_potential_fast_kernel(
     double *__restrict__ partial) {
     __shared__ float4 buf[kWarpsPerBlock][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float *sa = reinterpret_cast<float *>(buf[w]);        // 16 float4: x and y pairs
+    float *sb = reinterpret_cast<float *>(buf[w] + 16);   // 16 float4: z and m pairs
+    const int kp = lane >> 1, hf = lane & 1;
+    const f2x e2 = pack2(eps2, eps2);
     const int64_t gwarp = (int64_t)blockIdx.x * kWarpsPerBlock + w;
     const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
     const int64_t ntiles = (nt + 32 * T - 1) / (32 * T);
@@ -297,57 +346,50 @@ __global__ void __launch_bounds__(256) bf_potential_fast_kernel(
         const int s = (int)(item - tile * n_split);
         const int64_t jb = (int64_t)s * split_len;
         const int64_t je = min(ns, jb + split_len);
-        float px[T], py[T], pz[T], sum[T], comp[T];
+        f2x px[T], py[T], pz[T];
+        float sum[T], comp[T];
 #pragma unroll
         for (int t = 0; t < T; ++t) {
             const int64_t i = tile * 32 * T + t * 32 + lane;
             const bool v = i < nt;
-            px[t] = v ? tx[i] : kPadCoord;
-            py[t] = v ? ty[i] : kPadCoord;
-            pz[t] = v ? tz[i] : kPadCoord;
+            const float cx = v ? tx[i] : kPadCoord, cy = v ? ty[i] : kPadCoord, cz = v ? tz[i] : kPadCoord;
+            px[t] = pack2(cx, cx);
+            py[t] = pack2(cy, cy);
+            pz[t] = pack2(cz, cz);
             sum[t] = 0.f;
             comp[t] = 0.f;
         }
+        // the tile's self pairs are with the sources lo_self .. lo_self + 32 T - 1
+        const int64_t lo_self = tile * 32 * T + self_offset;
         float4 nxt = load_source(m, x, y, z, jb + lane, je);
         for (int64_t j0 = jb; j0 < je; j0 += 32) {
             __syncwarp();
-            buf[w][lane] = nxt;
+            sa[kp * 4 + hf] = nxt.x;
+            sa[kp * 4 + 2 + hf] = nxt.y;
+            sb[kp * 4 + hf] = nxt.z;
+            sb[kp * 4 + 2 + hf] = nxt.w;
             __syncwarp();
             nxt = load_source(m, x, y, z, j0 + 32 + lane, je);
-            float part[T];
+            f2x acc[T];
+            int self[T];
 #pragma unroll
-            for (int t = 0; t < T; ++t) part[t] = 0.f;
-            if (MASK == HALMA_MASK_COORD) {
-#pragma unroll 8
-                for (int k = 0; k < 32; ++k) {
-                    const float4 q = buf[w][k];
+            for (int t = 0; t < T; ++t) {
+                acc[t] = pack2(0.f, 0.f);
+                self[t] = -1;
+            }
+            if (MASK == HALMA_MASK_SELF && j0 + 32 > lo_self && j0 < lo_self + 32 * T) {
 #pragma unroll
-                    for (int t = 0; t < T; ++t) part[t] = pair_term_fast_masked(q, px[t], py[t], pz[t], eps2, part[t]);
-                }
-            } else if (MASK == HALMA_MASK_NONE) {
-#pragma unroll 8
-                for (int k = 0; k < 32; ++k) {
-                    const float4 q = buf[w][k];
-#pragma unroll
-                    for (int t = 0; t < T; ++t) part[t] = pair_term_fast(q, px[t], py[t], pz[t], eps2, part[t]);
-                }
+                for (int t = 0; t < T; ++t) self[t] = (int)(lo_self + t * 32 + lane - j0);
+                pot_chunk<T, MASK, FTZ, true>(buf[w], buf[w] + 16, px, py, pz, e2, self, acc);
             } else {
-                // source index of target t's self pair relative to this chunk
-                int64_t rel[T];
-#pragma unroll
-                for (int t = 0; t < T; ++t) rel[t] = tile * 32 * T + t * 32 + lane + self_offset - j0;
-#pragma unroll 4
-                for (int k = 0; k < 32; ++k) {
-                    const float4 q = buf[w][k];
-#pragma unroll
-                    for (int t = 0; t < T; ++t) {
-                        const float v = pair_term_fast(q, px[t], py[t], pz[t], eps2, part[t]);
-                        part[t] = (rel[t] == k) ? part[t] : v;
-                    }
-                }
+                pot_chunk<T, MASK, FTZ, false>(buf[w], buf[w] + 16, px, py, pz, e2, self, acc);
             }
 #pragma unroll
-            for (int t = 0; t < T; ++t) two_sum_acc(sum[t], comp[t], part[t]);
+            for (int t = 0; t < T; ++t) {
+                float a0, a1;
+                unpack2(acc[t], a0, a1);
+                two_sum_acc(sum[t], comp[t], a0 + a1);
+            }
         }
 #pragma unroll
         for (int t = 0; t < T; ++t) {
@@ -366,6 +408,7 @@ __global__ void reduce_partials_kernel(const double *__restrict__ partial, int n
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nt;
          i += (int64_t)gridDim.x * blockDim.x) {
         double acc = 0.0;
+#pragma unroll 8
         for (int s = 0; s < n_split; ++s) acc += partial[(int64_t)s * nt + i];
         out[i] = (float)acc;
     }
@@ -402,16 +445,21 @@ __global__ void __launch_bounds__(256) potential_f64_kernel(
     if (valid) phi[i] = acc;
 }
 
-// Number of source slices so that (target tiles x slices) keeps every SM busy.
+constexpr int64_t kMaxPartials = 1ll << 21;   // partial sums of one call, from the finer slices below
+
+// Number of source slices so that (target tiles x slices) keeps every SM busy.  Slices have at least
+// 2048 sources, or 128 while the partial sums stay within kMaxPartials: 3,000 targets x 4,000
+// sources took 248 us in one slice (24 warps), 13 us in 32.
 static void choose_split(int64_t ns, int64_t nt, int T, int *n_split, int64_t *split_len) {
     const int sms = device_sm_count();
     const int64_t ntiles = (nt + 32 * T - 1) / (32 * T);
     const int64_t want_items = (int64_t)sms * 64;   // ~2 waves of resident warps
     int64_t s = 1;
     if (ntiles < want_items) s = (want_items + ntiles - 1) / ntiles;
-    const int64_t max_s = std::max<int64_t>(1, ns / 2048);   // keep slices >= 2048 sources
-    s = std::min(s, max_s);
     s = std::min<int64_t>(s, 1024);
+    const int64_t coarse = std::min(s, std::max<int64_t>(1, ns / 2048));
+    const int64_t fine = std::min(s, std::min(ns / 128, kMaxPartials / nt));
+    s = std::max(coarse, fine);
     int64_t len = (ns + s - 1) / s;
     len = (len + 31) / 32 * 32;
     s = std::max<int64_t>(1, (ns + len - 1) / len);
@@ -419,25 +467,36 @@ static void choose_split(int64_t ns, int64_t nt, int T, int *n_split, int64_t *s
     *split_len = std::max<int64_t>(len, 32);
 }
 
-template <int T>
-static int launch_fast(const float *m, const float *x, const float *y, const float *z, int64_t ns,
-                       const float *tx, const float *ty, const float *tz, int64_t nt, float eps2,
-                       int n_split, int64_t split_len, int mask, int64_t self_offset, float *out,
-                       double *partial, cudaStream_t st) {
+template <int T, bool FTZ>
+static int launch_fast_mask(const float *m, const float *x, const float *y, const float *z, int64_t ns,
+                            const float *tx, const float *ty, const float *tz, int64_t nt, float eps2,
+                            int n_split, int64_t split_len, int mask, int64_t self_offset, float *out,
+                            double *partial, cudaStream_t st) {
     const int64_t ntiles = (nt + 32 * T - 1) / (32 * T);
     const int64_t nitems = ntiles * n_split;
     const int sms = device_sm_count();
     const int grid = (int)std::min<int64_t>((nitems + kWarpsPerBlock - 1) / kWarpsPerBlock, (int64_t)sms * 8);
     if (mask == HALMA_MASK_COORD)
-        HALMA_LAUNCH((bf_potential_fast_kernel<T, HALMA_MASK_COORD>), grid, 256, 0, st, m, x, y, z, ns, tx, ty, tz,
-                     nt, eps2, n_split, split_len, self_offset, out, partial);
+        HALMA_LAUNCH((bf_potential_fast_kernel<T, HALMA_MASK_COORD, FTZ>), grid, 256, 0, st, m, x, y, z, ns, tx, ty,
+                     tz, nt, eps2, n_split, split_len, self_offset, out, partial);
     else if (mask == HALMA_MASK_SELF)
-        HALMA_LAUNCH((bf_potential_fast_kernel<T, HALMA_MASK_SELF>), grid, 256, 0, st, m, x, y, z, ns, tx, ty, tz,
+        HALMA_LAUNCH((bf_potential_fast_kernel<T, HALMA_MASK_SELF, FTZ>), grid, 256, 0, st, m, x, y, z, ns, tx, ty, tz,
                      nt, eps2, n_split, split_len, self_offset, out, partial);
     else
-        HALMA_LAUNCH((bf_potential_fast_kernel<T, HALMA_MASK_NONE>), grid, 256, 0, st, m, x, y, z, ns, tx, ty, tz,
+        HALMA_LAUNCH((bf_potential_fast_kernel<T, HALMA_MASK_NONE, FTZ>), grid, 256, 0, st, m, x, y, z, ns, tx, ty, tz,
                      nt, eps2, n_split, split_len, self_offset, out, partial);
     return HALMA_OK;
+}
+
+template <int T>
+static int launch_fast(const float *m, const float *x, const float *y, const float *z, int64_t ns,
+                       const float *tx, const float *ty, const float *tz, int64_t nt, float eps2,
+                       int n_split, int64_t split_len, int mask, int64_t self_offset, float *out,
+                       double *partial, cudaStream_t st) {
+    return eps2 >= 0x1p-126f ? launch_fast_mask<T, true>(m, x, y, z, ns, tx, ty, tz, nt, eps2, n_split, split_len,
+                                                         mask, self_offset, out, partial, st)
+                             : launch_fast_mask<T, false>(m, x, y, z, ns, tx, ty, tz, nt, eps2, n_split, split_len,
+                                                          mask, self_offset, out, partial, st);
 }
 
 // Stages the caller's arrays and runs the FP32-compensated kernel with the given mask.
@@ -496,6 +555,7 @@ __global__ void sym_finish_kernel(int64_t nt, int nblk, int64_t npad, const floa
                                   const float *__restrict__ m, double self_scale, float *__restrict__ out) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nt; i += (int64_t)gridDim.x * blockDim.x) {
         double acc = 0.0;
+#pragma unroll 8   // loads in flight: one at a time took 232 us of the 160,000-cell gas halo's forward
         for (int b = 0; b < nblk; ++b) {
             const float2 v = part[(int64_t)b * npad + i];
             acc += (double)v.x + (double)v.y;
