@@ -2,21 +2,25 @@
 //
 // Pipeline (all on one stream):
 //   1. bounding box (FP64) -> host picks the cell geometry (cell side = ll * (1 + 2^-20));
-//   2. each particle gets a row-major cell key; keys are radix-sorted with their indices;
-//   3. per sorted particle: a float4 record (position inside its cell in units of ll, and
-//      the original index), run heads of equal keys -> cell table -> per cell the first
-//      positions and counts of its 13 forward neighbour cells, found by lower bounds in the
-//      sorted cell keys (the key grid is padded so that a neighbour key is a constant offset);
-//   4. work items = 32-particle chunks of a cell; one warp per item tests its particles
-//      against the same cell and the 13 neighbour cells that sort after it, staging each
-//      neighbour chunk in shared memory (coalesced float4 loads, broadcast reads);
-//   5. a pair whose float32 distance is clearly inside (outside) the linking length is
-//      accepted (rejected); pairs in a +-1e-5 band are re-tested with the exact FP64
-//      predicate ((dx*dx + dy*dy) + dz*dz) <= ll*ll, every operation rounded on its own;
-//   6. accepted pairs join a lock-free union-find over sorted positions (atomicCAS hooks
-//      the larger root under the smaller one, path halving on every find);
-//   7. each component's label = the smallest ORIGINAL index among its members
-//      (atomicMin), -1 for particles that never linked.
+//   2. each particle gets a row-major cell key with its half-cell (2 x 2 x 2) below it; keys are
+//      radix-sorted with their indices;
+//   3. the particles of one half-cell lie within sqrt(3)/2 of the linking length of each other, so they
+//      are one component whatever their positions: a node.  One pass over the sorted keys numbers
+//      cells and nodes and gathers the particles' records (position inside the cell in units of ll,
+//      original index);
+//   4. per cell, its occupied forward neighbours among 13, found by lower bounds in the sorted cell
+//      keys (the key grid is padded so that a neighbour key is a constant offset), in one list of
+//      cell pairs;
+//   5. links in a lock-free union-find over nodes (atomicCAS, randomised linking, path halving): every node joins
+//      the first two nodes ahead of it that it is linked to, which leaves about one in a hundred pairs of
+//      neighbouring nodes in different sets; those are listed by a sweep over the nodes and each is tested
+//      particle by particle up to its first link.
+//      A pair of particles whose float32 distance is clearly inside (outside) the linking length is accepted
+//      (rejected); pairs in a +-1e-5 band are re-tested with the exact FP64 predicate
+//      ((dx*dx + dy*dy) + dz*dz) <= ll*ll, every operation rounded on its own.  Pairs of crowded nodes without
+//      a link among their first tests go to a list that blocks work off;
+//   6. each component's label = the smallest ORIGINAL index among its members (atomicMin over nodes), -1
+//      for particles alone.
 // The result is the reference's partition exactly: same components, same canonical labels.
 #include <math.h>
 #include <limits.h>
@@ -30,7 +34,6 @@ namespace halma {
 
 namespace {
 
-constexpr int kFofWarps = 8;
 constexpr int kUfCapDefault = 1 << 26;   // bound on any union-find loop (never reached in practice)
 // The bound the kernels use: halma_set_union_find_cap changes it (a debug knob, so that tests
 // can make the loops run out); pushed to each device before its next FoF.
@@ -45,7 +48,7 @@ struct FofGeom {
     // empty pad cell, so that a neighbour's key is the cell's key plus a constant that never
     // wraps onto an occupied cell (a wrap lands on a pad cell or past the last slab)
     long long ky, kz;
-    int sb;   // low key bits holding the 4 x 4 x 4 sub-cell (Morton order) within the cell: 6 or 0
+    int sb;   // low key bits holding the half-cell (x, y, z) within the cell: 3, or 0 when nodes are particles
 };
 
 // Segmented FoF (links only inside a segment): every segment gets its own origin (the
@@ -75,57 +78,28 @@ __device__ __forceinline__ int uf_find(int *parent, int v, int *err) {
     return v;
 }
 
-// The cached walk below, continued from p = parent[v] loaded earlier (so that the caller can
-// issue that load next to other independent ones).
-__device__ __forceinline__ int uf_find_from(int *parent, int v, int p, int *err) {
-    int guard = 0;
-    const int cap = c_uf_cap;
-    while (p != v) {
-        const int gp = parent[p];
-        if (gp != p) __stcg(parent + v, gp);
-        v = p;
-        p = gp;
-        if (++guard > cap) {
-            atomicOr(err, 1);
-            break;
-        }
-    }
-    return v;
+// A random order of the nodes (a bijection of 32-bit integers by multiplications and shifts).  Neighbouring nodes
+// have neighbouring numbers: hooked in the order of their numbers they make chains as long as a group, and
+// a walk is one dependent memory access a step; hooked in random order, trees are logarithmically deep (A. Goel,
+// S. Khanna, D. Larkin, R. E. Tarjan, Disjoint set union with randomized linking, SODA 2014).
+__device__ __forceinline__ unsigned uf_rank(int v) {
+    unsigned h = (unsigned)v;
+    h ^= h >> 16;
+    h *= 0x85ebca6bu;
+    h ^= h >> 13;
+    h *= 0xc2b2ae35u;
+    return h ^ (h >> 16);
 }
 
-// Same walk with L1-cached loads, for the linking kernel.  A value read from L1 may be older
-// than the one in L2 (another SM hooked or compressed since), which is harmless there: an
-// older parent is still an ancestor (parents only move toward the root, and every value in a
-// chain is smaller than the last), equal roots still prove the same set, and any hook goes
-// through an atomicCAS on L2 that sees the current value.  The final labels are read by a
-// later kernel.
-__device__ __forceinline__ int uf_find_cached(int *parent, int v, int *err) {
-    int p = parent[v];
-    int guard = 0;
-    const int cap = c_uf_cap;
-    while (p != v) {
-        const int gp = parent[p];
-        if (gp != p) __stcg(parent + v, gp);
-        v = p;
-        p = gp;
-        if (++guard > cap) {
-            atomicOr(err, 1);
-            break;
-        }
-    }
-    return v;
-}
-
-// Joins the sets of two ancestors a and b (roots or not): hooks the larger root under the
-// smaller, retrying from the current roots when the CAS finds that a is no longer a root.
-// Every root of a tree is its smallest sorted position.  Returns the node hooked under (or
-// the common root when the two are one set already): an ancestor of every member of both
-// sets, which the caller may use in place of a fresh find.
+// Joins the sets of two ancestors a and b (roots or not): hooks the root of the larger rank under that of
+// the smaller, retrying from the current roots when the CAS finds that a is no longer a root.
+// Returns the node hooked under (or the common root when the two are one set already): an ancestor
+// of every member of both sets, which the caller may use in place of a fresh find.
 __device__ __forceinline__ int uf_union(int *parent, int a, int b, int *err) {
     int guard = 0;
     const int cap = c_uf_cap;
     while (a != b) {
-        if (a < b) {
+        if (uf_rank(a) < uf_rank(b)) {
             const int t = a;
             a = b;
             b = t;
@@ -140,6 +114,45 @@ __device__ __forceinline__ int uf_union(int *parent, int a, int b, int *err) {
         }
     }
     return a;
+}
+
+// The same for a whole warp: every lane with need joins its a and b, all lanes one step at a time (one step of
+// both walks, or the hook).  In nested loops of their own the lanes ran one after another (3.7 of 32
+// active).  Returns each lane's node as above.
+__device__ __forceinline__ int uf_union_warp(int *parent, int a, int b, bool need, int *err) {
+    const int cap = c_uf_cap;
+    int guard = 0, xa = -1, xb = -1;   // the nodes before a and b on their walks
+    while (__any_sync(0xffffffffu, need)) {
+        if (need) {
+            const int pa = __ldcg(parent + a), pb = __ldcg(parent + b);
+            if (pa == a && pb == b) {
+                if (a != b) {
+                    const bool swap = uf_rank(a) < uf_rank(b);
+                    const int hi = swap ? b : a, lo = swap ? a : b;
+                    const int old = atomicCAS(parent + hi, hi, lo);
+                    a = old == hi ? lo : old;
+                    b = lo;
+                    xa = xb = -1;
+                    need = old != hi;
+                } else {
+                    need = false;
+                }
+            } else {   // path halving: pa and pb are ancestors of xa and xb
+                if (pa != a && xa >= 0) __stcg(parent + xa, pa);
+                if (pb != b && xb >= 0) __stcg(parent + xb, pb);
+                xa = a;
+                xb = b;
+                a = pa;
+                b = pb;
+                if (a == b) need = false;
+            }
+            if (need && ++guard > cap) {
+                atomicOr(err, 1);
+                need = false;
+            }
+        }
+    }
+    return b;
 }
 
 // Doubles as order-preserving signed 64-bit integers (sign-magnitude turned into two's
@@ -319,8 +332,7 @@ __device__ __forceinline__ void quarter_split_fixed(long long t, long long qmax,
     w = __int_as_float((fe << 23) | (int)(((v << lz) >> 40) & 0x7fffff));
 }
 
-// Sort key: row-major cell index, then (when there is room) the particle's 4 x 4 x 4 sub-cell in
-// Morton order, so that each 32-particle chunk of a crowded cell is spatially compact.  The
+// Sort key: row-major cell index, then (with g.sb) the particle's half-cell per axis.  The
 // order of particles inside a cell does not change the partition.  The kernel also writes the
 // particle's position inside its cell in units of the linking length (pre[i], in input order,
 // with the index in .w), so that the sorted records are one 16-byte gather.
@@ -375,219 +387,101 @@ __global__ void keys_kernel(const double *__restrict__ x, const double *__restri
         }
         const long long cx = qx >> 2, cy = qy >> 2, cz = qz >> 2;
         uint64_t key = ((uint64_t)(x0 + cx) * (uint64_t)g.ky + (uint64_t)cy) * (uint64_t)g.kz + (uint64_t)cz;
-        if (g.sb) {
-            const int sx = (int)(qx & 3), sy = (int)(qy & 3), sz = (int)(qz & 3);
-            const int mort = ((sx >> 1) << 5) | ((sy >> 1) << 4) | ((sz >> 1) << 3) | ((sx & 1) << 2) |
-                             ((sy & 1) << 1) | (sz & 1);
-            key = (key << 6) | (uint64_t)mort;
-        }
+        if (g.sb)
+            key = (key << 3) | (uint64_t)(((qx >> 1) & 1) << 2 | ((qy >> 1) & 1) << 1 | ((qz >> 1) & 1));
         keys[i] = key;
         vals[i] = i;
         pre[i] = make_float4(wx * cs4, wy * cs4, wz * cs4, __int_as_float(i));
     }
 }
 
-// Sorted records, run heads, union-find / label initialisation.
-// Sorted records, cell heads and label slots.  With runstart (sub-cells in the key), the
-// sub-cell runs' starts for the run-head scan (see subrun below) instead of the union-find
-// initialisation, which preunion_kernel then writes.
-__global__ void prep_kernel(int n, int sb, const uint64_t *__restrict__ keys, const int *__restrict__ idx,
-                            const float4 *__restrict__ pre, float4 *__restrict__ rec, int *__restrict__ head,
-                            int *__restrict__ parent, unsigned char *__restrict__ has, int *__restrict__ minidx,
-                            int *__restrict__ runstart) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const uint64_t full = keys[k], prev = k > 0 ? keys[k - 1] : ~full;
-        rec[k] = pre[idx[k]];
-        head[k] = (k == 0 || (prev >> sb) != (full >> sb)) ? 1 : 0;
-        if (runstart) {
-            runstart[k] = (k == 0 || prev != full) ? k : 0;
-        } else {
-            parent[k] = k;
-            has[k] = 0;
-        }
-        minidx[k] = INT_MAX;
-    }
-}
+// ---- cells and nodes -----------------------------------------------------------------------
+// Sorted position k starts a cell when its cell key differs from its predecessor's, and a node when its
+// full key does (without half-cells in the key, every particle is a node).  A warp numbers kScanRun
+// consecutive positions with ballots; head_count_kernel leaves cells << 32 | nodes per warp, whose
+// exclusive scan is where head_apply_kernel's warp starts.  Together they replaced eight passes (records and
+// run heads, two scans, run joins, cell table, one-component flags): 0.50 of 11.5 ms at 2e7 particles
+// became 0.31.
+constexpr int kScanRun = 512;
 
-// Particles with the same full key (cell and 4 x 4 x 4 sub-cell) lie at most sqrt(3)/4 of a
-// cell (0.44 LL) apart, so they are friends whatever the rounding: each such run is joined
-// up front, every member under the run's first sorted position (which keeps "a root is the
-// smallest position of its tree").  runstart[k] = k at a run's first position, else 0
-// (prep_kernel); an inclusive max-scan turns it into the run head of every position.
-
-__global__ void preunion_kernel(int n, const uint64_t *__restrict__ keys, const int *__restrict__ runhead,
-                                int *__restrict__ parent, unsigned char *__restrict__ has) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        parent[k] = runhead[k];
-        const bool friend_before = k > 0 && keys[k - 1] == keys[k];
-        const bool friend_after = k + 1 < n && keys[k + 1] == keys[k];
-        has[k] = (friend_before || friend_after) ? 1 : 0;
-    }
-}
-
-// Dense cells (>= kDenseMin particles): the occupied 4 x 4 x 4 sub-cells of a cell (side
-// cell/4) are joined without pair tests when every pair of their points is closer than the
-// linking length: for a sub-cell offset d, the largest distance is sqrt(sum_i (|d_i|+1)^2)/4
-// cells, and offsets with sum_i (|d_i|+1)^2 <= 15 stay below 0.97 LL (the rounding of the
-// sub-cell assignment moves a point by ~1e-8 cells at most).  One warp per dense cell finds
-// the components of its occupied sub-cells under those offsets (bitmask flood fill, see
-// subcell_dilate), hooks every run head under the smallest run head of its component (a
-// smaller sorted position, so a root stays the smallest position of its tree), marks the
-// particles of multi-particle components as having friends, and records whether the whole
-// cell is one component (conn[c]).  Smaller cells are connected when all their particles
-// share one run.
-constexpr int kDenseMin = 32;
-
-__device__ __forceinline__ int lower_bound_key(const uint64_t *__restrict__ keys, int lo, int hi, uint64_t k) {
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (keys[mid] < k) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// Cells of fewer than kDenseMin particles, one thread each: one component when the first and
-// last particles share a sub-cell run; the dense cells are listed for dense_cell_kernel (the
-// list order does not matter: each dense cell only joins runs of its own).
-__global__ void small_cell_kernel(const int *__restrict__ ncell_p, const int *__restrict__ cell_start,
-                                  const uint64_t *__restrict__ keys, unsigned char *__restrict__ conn,
-                                  int *__restrict__ dense, int *__restrict__ ndense) {
-    const int nc = *ncell_p;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-        const int cs = cell_start[c], ce = cell_start[c + 1];
-        if (ce - cs < kDenseMin) conn[c] = keys[cs] == keys[ce - 1] ? 1 : 0;
-        else dense[atomicAdd(ndense, 1)] = c;
-    }
-}
-
-// Sub-cell sets as 64-bit masks, bit 16 x + 4 y + z for sub-cell (x, y, z).  subcell_dilate
-// adds every sub-cell within the guaranteed-link offsets of the set: the 3 x 3 x 3 cube, and
-// +-2 along one axis with at most one of the other two offsets +-1 ((3,2,2) gives 17 > 15).
-__device__ __forceinline__ unsigned long long subcell_dilate(unsigned long long m) {
-    constexpr unsigned long long Z0 = 0x1111111111111111ull, Z1 = Z0 << 1, Z2 = Z0 << 2, Z3 = Z0 << 3;
-    constexpr unsigned long long Y0 = 0x000F000F000F000Full, Y1 = Y0 << 4, Y2 = Y0 << 8, Y3 = Y0 << 12;
-    const unsigned long long zl = ((m << 1) & ~Z0) | ((m >> 1) & ~Z3);   // z +- 1
-    const unsigned long long yl = ((m << 4) & ~Y0) | ((m >> 4) & ~Y3);   // y +- 1
-    const unsigned long long xl = (m << 16) | (m >> 16);                 // x +- 1
-    const unsigned long long a = m | zl;
-    const unsigned long long b = a | ((a << 4) & ~Y0) | ((a >> 4) & ~Y3);
-    const unsigned long long cube = b | (b << 16) | (b >> 16);
-    const unsigned long long cyz = a | yl, cxz = a | xl, cxy = m | xl | yl;   // plus shapes
-    return cube | (cyz << 32) | (cyz >> 32) | ((cxz << 8) & ~(Y0 | Y1)) | ((cxz >> 8) & ~(Y2 | Y3)) |
-           ((cxy << 2) & ~(Z0 | Z1)) | ((cxy >> 2) & ~(Z2 | Z3));
-}
-
-// Bit of Morton sub-cell code m (x1 y1 z1 x0 y0 z0) in the mask layout.
-__device__ __forceinline__ int subcell_bit(int m) {
-    const int x = (((m >> 5) & 1) << 1) | ((m >> 2) & 1), y = (((m >> 4) & 1) << 1) | ((m >> 1) & 1),
-              z = (((m >> 3) & 1) << 1) | (m & 1);
-    return (x << 4) | (y << 2) | z;
-}
-
-__global__ void __launch_bounds__(256) dense_cell_kernel(const int *__restrict__ ndense_p, const int *__restrict__ dense,
-                                                         const int *__restrict__ cell_start,
-                                                         const uint64_t *__restrict__ keys, int *__restrict__ parent,
-                                                         unsigned char *__restrict__ has, unsigned char *__restrict__ conn) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int nd = *ndense_p;
-    const int warps = gridDim.x * (blockDim.x >> 5);
-    const int bit0 = subcell_bit(lane), bit1 = subcell_bit(lane + 32);
-    for (int di = blockIdx.x * (blockDim.x >> 5) + w; di < nd; di += warps) {
-        const int c = dense[di];
-        const int cs = cell_start[c], ce = cell_start[c + 1];
-        const uint64_t ck = keys[cs] & ~63ull;   // the cell's key with the sub-cell bits cleared
-        int lo[2], hi[2];
-        bool occ[2];
-        for (int r = 0; r < 2; ++r) {
-            const int m = lane + 32 * r;
-            lo[r] = lower_bound_key(keys, cs, ce, ck | (uint64_t)m);
-            hi[r] = lower_bound_key(keys, lo[r], ce, (ck | (uint64_t)m) + 1);
-            occ[r] = hi[r] > lo[r];
-        }
-        const unsigned long long mine = (occ[0] ? 1ull << bit0 : 0ull) | (occ[1] ? 1ull << bit1 : 0ull);
-        const unsigned long long occm =
-            (unsigned long long)__reduce_or_sync(0xffffffffu, (unsigned)mine) |
-            ((unsigned long long)__reduce_or_sync(0xffffffffu, (unsigned)(mine >> 32)) << 32);
-        unsigned long long rem = occm;
-        bool first = true, one = false;
-        while (rem) {   // one component per round, from its lowest remaining sub-cell (warp-uniform)
-            unsigned long long comp = rem & (~rem + 1ull);
-            for (;;) {
-                const unsigned long long grown = subcell_dilate(comp) & occm;
-                if (grown == comp) break;
-                comp = grown;
-            }
-            if (first) one = comp == occm;
-            first = false;
-            rem &= ~comp;
-            const bool in0 = occ[0] && ((comp >> bit0) & 1ull), in1 = occ[1] && ((comp >> bit1) & 1ull);
-            // the component's smallest run head (sorted positions grow with the Morton code)
-            const int L = __reduce_min_sync(0xffffffffu, in0 ? lo[0] : (in1 ? lo[1] : INT_MAX));
-            const bool multi = (comp & (comp - 1ull)) != 0;
-            for (int r = 0; r < 2; ++r) {
-                if (!(r == 0 ? in0 : in1)) continue;
-                if (L != lo[r]) parent[lo[r]] = L;   // run head under the component's smallest run head
-                if (multi || hi[r] - lo[r] > 1)
-                    for (int q = lo[r]; q < hi[r]; ++q) has[q] = 1;
-            }
-        }
-        if (lane == 0) conn[c] = one ? 1 : 0;
-    }
-}
-
-// Start and key of every occupied cell (cells in sorted order), from the exclusive scan of
-// the run heads.
-__global__ void cell_table_kernel(int n, int sb, const uint64_t *__restrict__ keys, const int *__restrict__ head,
-                                  const int *__restrict__ cellpos, int *__restrict__ cell_start,
-                                  uint64_t *__restrict__ cell_key, int *__restrict__ ncell) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        if (head[k]) {
-            const int c = cellpos[k];
-            cell_start[c] = k;
-            cell_key[c] = keys[k] >> sb;
-        }
-        if (k == n - 1) {
-            const int m = cellpos[k] + head[k];
-            *ncell = m;
-            cell_start[m] = n;
-        }
-    }
-}
-
-// Marks the first particle of every 32-particle chunk of every cell that has linking work
-// (bit 13 of its neighbour mask, see nbmask_kernel).
-__global__ void itemflag_kernel(int n, const int *__restrict__ head, const int *__restrict__ cellpos,
-                                const int *__restrict__ cell_start, const int *__restrict__ cmask,
-                                int *__restrict__ flag) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const int c = cellpos[k] + head[k] - 1;
-        flag[k] = ((cmask[c] >> 13) & 1) && ((k - cell_start[c]) & 31) == 0 ? 1 : 0;
-    }
-}
-
-// A work item as the linking kernel reads it, in one 16-byte load: the chunk's first sorted
-// position, the cell's end with the cell's one-component flag in bit 31, and the cell's index
-// (its row of the neighbour table).
-struct __align__(16) ItemRec {
-    int k0, ce_conn, cell, pad;
+struct Heads {
+    bool cell, node;
 };
 
-__global__ void items_kernel(int n, const int *__restrict__ head, const int *__restrict__ cellpos,
-                             const int *__restrict__ flag, const int *__restrict__ itempos,
-                             const int *__restrict__ cell_start, const unsigned char *__restrict__ conn,
-                             ItemRec *__restrict__ items, int *__restrict__ nitems) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        if (flag[k]) {
-            const int c = cellpos[k] + head[k] - 1;
-            ItemRec r;
-            r.k0 = k;
-            r.ce_conn = cell_start[c + 1] | (conn[c] ? (int)0x80000000u : 0);
-            r.cell = c;
-            r.pad = 0;
-            items[itempos[k]] = r;
+__device__ __forceinline__ Heads heads_at(const uint64_t *__restrict__ keys, int sb, int k, int n) {
+    Heads h{false, false};
+    if (k < n) {
+        const uint64_t full = keys[k], prev = k > 0 ? keys[k - 1] : ~full;
+        h.cell = (prev >> sb) != (full >> sb);
+        h.node = sb == 0 || prev != full;
+    }
+    return h;
+}
+
+__global__ void __launch_bounds__(256) head_count_kernel(int n, int sb, const uint64_t *__restrict__ keys,
+                                                         int64_t *__restrict__ counts, int nruns) {
+    const int lane = threadIdx.x & 31;
+    const int run = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (run >= nruns) return;
+    int cells = 0, nodes = 0;
+#pragma unroll 4
+    for (int r = 0; r < kScanRun; r += 32) {
+        const Heads h = heads_at(keys, sb, run * kScanRun + r + lane, n);
+        cells += __popc(__ballot_sync(0xffffffffu, h.cell));
+        nodes += __popc(__ballot_sync(0xffffffffu, h.node));
+    }
+    if (lane == 0) counts[run] = (int64_t)cells << 32 | nodes;
+}
+
+// Node m: first sorted position node_start[m], cell node_cell[m], first particle's record
+// node_rec[m], half-cell node_sub[m], union-find parent and smallest original
+// index (the sort is stable, so the first particle's).  Cell c: first node cell_node[c], key cell_key[c].
+// The entries past the last node and cell close the ranges; cnt[0] = cells, cnt[1] = nodes.
+__global__ void __launch_bounds__(256) head_apply_kernel(
+    int n, int sb, const uint64_t *__restrict__ keys, const int *__restrict__ idx, const float4 *__restrict__ pre,
+    const int64_t *__restrict__ base, int nruns, float4 *__restrict__ rec, int *__restrict__ node_of,
+    int *__restrict__ node_start, int *__restrict__ node_cell, unsigned char *__restrict__ node_sub,
+    float4 *__restrict__ node_rec, int *__restrict__ parent, int *__restrict__ minidx, unsigned char *__restrict__ multi, int *__restrict__ cell_node,
+    uint64_t *__restrict__ cell_key, int *__restrict__ cnt) {
+    const int lane = threadIdx.x & 31;
+    const unsigned upto = 0xffffffffu >> (31 - lane);
+    const int run = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (run >= nruns) return;
+    int cells = (int)(base[run] >> 32), nodes = (int)(base[run] & 0xffffffffll);
+#pragma unroll 2
+    for (int r = 0; r < kScanRun; r += 32) {
+        const int k = run * kScanRun + r + lane;
+        const Heads h = heads_at(keys, sb, k, n);
+        const unsigned cb = __ballot_sync(0xffffffffu, h.cell), nb = __ballot_sync(0xffffffffu, h.node);
+        if (k < n) {
+            const int i = idx[k];
+            const int m = nodes + __popc(nb & upto) - 1;
+            const float4 r = pre[i];
+            rec[k] = r;
+            node_of[k] = m;
+            if (h.node) {
+                node_rec[m] = r;
+                node_start[m] = k;
+                node_cell[m] = cells + __popc(cb & upto) - 1;
+                node_sub[m] = sb ? (unsigned char)(keys[k] & 7) : 0;
+                parent[m] = m;
+                minidx[m] = i;
+                multi[m] = 0;
+            }
+            if (h.cell) {
+                const int c = cells + __popc(cb & upto) - 1;
+                cell_node[c] = m;
+                cell_key[c] = keys[k] >> sb;
+            }
         }
-        if (k == n - 1) *nitems = itempos[k] + flag[k];
+        cells += __popc(cb);
+        nodes += __popc(nb);
+    }
+    if (run == nruns - 1 && lane == 0) {
+        cnt[0] = cells;
+        cnt[1] = nodes;
+        cell_node[cells] = nodes;
+        node_start[nodes] = n;
     }
 }
 
@@ -602,10 +496,6 @@ __device__ __forceinline__ bool exact_link(const double *__restrict__ x, const d
     s = __dadd_rn(s, __dmul_rn(dz, dz));
     return s <= r2;
 }
-
-__constant__ int c_stencil[13][3] = {{0, 0, 1},  {0, 1, -1}, {0, 1, 0},  {0, 1, 1},  {1, -1, -1},
-                                     {1, -1, 0}, {1, -1, 1}, {1, 0, -1}, {1, 0, 0},  {1, 0, 1},
-                                     {1, 1, -1}, {1, 1, 0},  {1, 1, 1}};
 
 // Lower bound of q in the sorted keys[lo, n), searched forward from lo: doubling steps, then
 // bisection of the last step.
@@ -627,349 +517,422 @@ __device__ __forceinline__ int gallop_lower_bound(const uint64_t *__restrict__ k
     return a;
 }
 
-// The 13 forward neighbours of every cell, found in the sorted cell keys, one thread per cell.
-// On the padded key grid a neighbour's key is the cell's key plus a constant, so (0, 0, +1) is
-// the next cell or none, and for each of the stencil's four columns (0, 1), (1, -1), (1, 0),
-// (1, 1), whose bases increase, one lower bound of the column's z - 1 key -- galloping forward
-// from the cell itself, then from the previous column's bound -- gives its three z neighbours
-// in order.  nbinfo[13 c + j] = (first sorted position, count | one-component flag << 31) of
-// stencil cell j, (0, 0) when it holds no particle; cmask[c] = the 13-bit mask of occupied
-// neighbours, and bit 13 when the cell has linking work: an occupied neighbour, or more than
-// one particle in a cell that is not one component already.  Cells without work (isolated
-// particles, isolated one-component cells) get no work item.
-__global__ void nbtab_kernel(const int *__restrict__ ncell_p, const int *__restrict__ cell_start,
-                             const uint64_t *__restrict__ cell_key, const unsigned char *__restrict__ conn,
-                             long long ky, long long kz, int2 *__restrict__ nbinfo, int *__restrict__ cmask) {
-    const int nc = *ncell_p;
+// The pairs of cells, listed per cell: the cell itself when it holds more than one node, and its occupied forward
+// neighbours, one thread per cell.  On the padded key grid a neighbour's key is the cell's key plus
+// a constant, so (0, 0, +1) is the next cell or none, and for each of the stencil's four columns (0, 1),
+// (1, -1), (1, 0), (1, 1), whose bases increase, one lower bound of the column's z - 1 key -- galloping
+// forward from the cell itself, then from the previous column's bound -- gives its three z
+// neighbours in order.  A cell's entries are together, in key order: cell_list[c] = first << 4 | count; the
+// order of the cells in the list does not matter.  (A table row of 13 entries per cell,
+// mostly empty, took 0.68 ms at 2e7 particles.)
+// With half-cells an entry is the second cell's nodes as the linking kernels read them: first node, and nodes - 1
+// (at most 7) in bits 0-2, the cell's offset in bits 3-7 (see entry_offset), bit 8 for the cell itself.  Without,
+// it is the two cells.
+template <bool NODES>
+__global__ void __launch_bounds__(256) cell_pair_kernel(const int *__restrict__ cnt, const int *__restrict__ cell_node,
+                                                        const uint64_t *__restrict__ cell_key, long long ky, long long kz,
+                                                        int2 *__restrict__ pairs, long long *__restrict__ cell_list,
+                                                        unsigned long long *__restrict__ npairs) {
+    const int nc = cnt[0];
+    const int lane = threadIdx.x & 31;
     const uint64_t zrow = (uint64_t)kz, slab = (uint64_t)ky * (uint64_t)kz;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-        const uint64_t key = cell_key[c];
-        int2 *row = nbinfo + (int64_t)c * 13;
-        int m = 0;
-        auto put = [&](int j, int d) {
-            int2 v = make_int2(0, 0);
-            if (d >= 0) {
-                const int s0 = cell_start[d];
-                v = make_int2(s0, (cell_start[d + 1] - s0) | (conn[d] ? (int)0x80000000u : 0));
-                m |= 1 << j;
-            }
-            row[j] = v;
-        };
-        put(0, (c + 1 < nc && cell_key[c + 1] == key + 1) ? c + 1 : -1);
-        const uint64_t base[4] = {key + zrow, key + slab - zrow, key + slab, key + slab + zrow};
-        int lb = c + 1;
+    for (int64_t c0 = blockIdx.x * (int64_t)blockDim.x; c0 < nc; c0 += (int64_t)gridDim.x * blockDim.x) {
+        const int c = (int)(c0 + threadIdx.x);
+        int at[4] = {0, 0, 0, 0}, occ = 0;   // first cell of each column, occupied neighbours as a mask
+        if (c < nc) {
+            const uint64_t key = cell_key[c];
+            if (cell_node[c + 1] - cell_node[c] > 1) occ = 1;
+            if (c + 1 < nc && cell_key[c + 1] == key + 1) occ |= 2;
+            const uint64_t base[4] = {key + zrow, key + slab - zrow, key + slab, key + slab + zrow};
+            int lb = c + 1;
 #pragma unroll
-        for (int col = 0; col < 4; ++col) {
-            lb = gallop_lower_bound(cell_key, lb, nc, base[col] - 1);
-            int at_ = lb;
+            for (int col = 0; col < 4; ++col) {
+                lb = gallop_lower_bound(cell_key, lb, nc, base[col] - 1);
+                at[col] = lb;
+                int q = lb;
 #pragma unroll
-            for (int dz = -1; dz <= 1; ++dz) {
-                int d = -1;
-                if (at_ < nc && cell_key[at_] == base[col] + (uint64_t)(long long)dz) d = at_++;
-                put(1 + 3 * col + (dz + 1), d);
+                for (int dz = 0; dz < 3; ++dz)
+                    if (q < nc && cell_key[q] == base[col] - 1 + (uint64_t)dz) {
+                        occ |= 4 << (3 * col + dz);
+                        ++q;
+                    }
             }
         }
-        const int count = cell_start[c + 1] - cell_start[c];
-        const bool work = m != 0 || (count > 1 && !conn[c]);
-        cmask[c] = m | (work ? 1 << 13 : 0);
-    }
-}
-
-// One warp per item (a chunk of up to 32 particles of one cell).  The candidates of the item
-// are the later particles of its own cell (j > k) and every particle of the 13 forward
-// neighbour cells; they are concatenated into one list ("segments" 0..12 = stencil cells, 13 =
-// the home cell from the chunk start) and walked 32 at a time, so a sparse region costs one
-// or two rounds of loads per item instead of one per neighbour cell.  Each candidate is moved
-// into the home cell's frame when it is loaded.
-//
-// Segment of a candidate: the non-empty segments are ranked in lane order (a per-warp table
-// maps rank -> segment); in a round, the segments that start inside it set one bit each of a
-// start mask (one OR-reduction), and a candidate's rank is the rank of the round's first
-// segment plus the starts at or before it.
-//
-// Pair tests: the candidates that need a test (within reach of the home chunk's bounding box,
-// not already in the home chunk's set) are tested one at a time against all home particles,
-// or -- when the chunk holds fewer particles than that (sparse cells) -- the home particles
-// one at a time against all those candidates.
-constexpr int kHomeSeg = 13;
-
-__global__ void __launch_bounds__(256, 6) link_kernel(
-    const float4 *__restrict__ rec, const ItemRec *__restrict__ items, const int *__restrict__ nitems_p, int *item_counter, const int2 *__restrict__ nbinfo, FofGeom g,
-    const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ z,
-    int *parent, unsigned char *has, int *err) {
-    __shared__ float4 buf[kFofWarps][32];    // candidates of the round (candidate-major tests)
-    __shared__ float4 hbuf[kFofWarps][32];   // home particles of the item (home-major tests)
-    __shared__ int rbuf[kFofWarps][32];
-    __shared__ int jbuf[kFofWarps][32];
-    __shared__ int segtab[kFofWarps][16];    // rank of a non-empty segment -> segment (lane)
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    const int nitems = *nitems_p;
-    // items come from a counter: their cost varies by orders of magnitude (dense cores).  The
-    // next item's number, its record and its row of the neighbour table (lanes 0..12) are
-    // fetched while the current item is processed.
-    int nxt = 0;
-    if (lane == 0) nxt = atomicAdd(item_counter, 1);
-    int item = __shfl_sync(0xffffffffu, nxt, 0);
-    int4 ia_next = make_int4(0, 0, 0, 0);
-    int2 nb_next = make_int2(0, 0);
-    if (item < nitems) {
-        ia_next = __ldg(reinterpret_cast<const int4 *>(items + item));
-        if (lane < 13) nb_next = __ldg(nbinfo + (int64_t)ia_next.z * 13 + lane);
-    }
-    if (lane == 0) nxt = atomicAdd(item_counter, 1);
-    for (;;) {
-        if (item >= nitems) break;
-        const int4 ia = ia_next;
-        const int2 nbr = nb_next;   // this lane's neighbour cell (lanes 0..12): first position, count | flag
-        item = __shfl_sync(0xffffffffu, nxt, 0);
-        if (item < nitems) {
-            ia_next = __ldg(reinterpret_cast<const int4 *>(items + item));
-            if (lane == 0) nxt = atomicAdd(item_counter, 1);
-        }
-        const int k0 = ia.x;
-        const int ce = ia.y & 0x7fffffff;
-        const bool home_conn = ia.y < 0;
-        const int k = k0 + lane;
-        const bool hv = k < ce;
-        const float4 hp = hv ? rec[k] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const int pk0 = hv ? parent[k] : -1;   // issued with the record; walked further below
-        const int hidx = __float_as_int(hp.w);
-        const unsigned homes = __ballot_sync(0xffffffffu, hv);
-        const int nhome = __popc(homes);
-        // lane s < 13 owns stencil cell s, lane 13 the rest of the home cell
-        int sjs = 0, sn = 0, soff = 0x15;   // soff: stencil offset + 1 per axis, 2 bits each
-        bool sconn = false;                 // the segment's cell is one component
-        if (lane < 13) {   // an empty neighbour has count 0
-            soff = (c_stencil[lane][0] + 1) | (c_stencil[lane][1] + 1) << 2 | (c_stencil[lane][2] + 1) << 4;
-            sjs = nbr.x;
-            sn = nbr.y & 0x7fffffff;
-            sconn = nbr.y < 0;
-        } else if (lane == kHomeSeg && !home_conn) {   // a cell that is one component has no new pair inside
-            sjs = k0 + 1;
-            sn = ce - sjs;
-        }
-        // exclusive prefix of the segment lengths over lanes 0..13
-        int incl = sn;
-        for (int o = 1; o < 16; o <<= 1) {
+        const int mine = __popc(occ);
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
             const int u = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += u;
         }
-        const int spre = incl - sn;
-        const int total = __shfl_sync(0xffffffffu, incl, kHomeSeg);
-        const bool nonempty = lane <= kHomeSeg && sn > 0;
-        const unsigned ne_mask = __ballot_sync(0xffffffffu, nonempty);
-        __syncwarp();
-        if (nonempty) segtab[w][__popc(ne_mask & lt_mask)] = lane;
-        hbuf[w][lane] = hp;
-        __syncwarp();
-        // bounding box of the home chunk: a candidate farther than the linking length from it
-        // cannot link to any home particle
-        float bl[3] = {hv ? hp.x : INFINITY, hv ? hp.y : INFINITY, hv ? hp.z : INFINITY};
-        float bh[3] = {hv ? hp.x : -INFINITY, hv ? hp.y : -INFINITY, hv ? hp.z : -INFINITY};
+        unsigned long long w = 0;
+        if (lane == 31 && incl > 0) w = atomicAdd(npairs, (unsigned long long)incl);
+        w = __shfl_sync(0xffffffffu, w, 31) + (unsigned long long)(incl - mine);
+        auto put = [&](int d, int ox, int oy, int oz) {
+            if (NODES) {
+                const int t0 = cell_node[d];
+                pairs[w++] = make_int2(t0, (cell_node[d + 1] - t0 - 1) | ox << 3 | (oy + 1) << 4 | (oz + 1) << 6 |
+                                               (d == c ? 1 << 8 : 0));
+            } else {
+                pairs[w++] = make_int2(c, d);
+            }
+        };
+        if (c < nc) cell_list[c] = (long long)w << 4 | mine;
+        if (occ & 1) put(c, 0, 0, 0);
+        if (occ & 2) put(c + 1, 0, 0, 1);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
+        for (int col = 0; col < 4; ++col) {
+            int q = at[col];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                bl[d] = fminf(bl[d], __shfl_xor_sync(0xffffffffu, bl[d], o));
-                bh[d] = fmaxf(bh[d], __shfl_xor_sync(0xffffffffu, bh[d], o));
+            for (int dz = 0; dz < 3; ++dz)
+                if (occ & (4 << (3 * col + dz))) put(q++, col > 0 ? 1 : 0, col == 0 ? 1 : col - 2, dz - 1);
+        }
+    }
+}
+
+__device__ __forceinline__ int3 entry_offset(int e) {
+    return make_int3((e >> 3) & 1, ((e >> 4) & 3) - 1, ((e >> 6) & 3) - 1);
+}
+
+// Offset of cell d (key kd) from cell c (key kc <= kd), per axis; d is c or one of its forward neighbours.
+__device__ __forceinline__ int3 cell_offset(uint64_t kc, uint64_t kd, long long ky, long long kz) {
+    const long long d = (long long)(kd - kc), slab = ky * kz;
+    int3 o;
+    o.x = d >= slab - kz - 1 && slab > 1 ? 1 : 0;
+    long long r = d - (o.x ? slab : 0);             // dy * kz + dz
+    o.y = r > 1 ? 1 : (r < -1 ? -1 : 0);
+    o.z = (int)(r - (long long)o.y * kz);
+    return o;
+}
+
+// A list entry for the blocks: sorted positions [a, a + na) against [b, b + nb), cell b shifted by off (2 bits
+// an axis, offset + 1); without shift and with a == b, pairs j > i of one range.
+struct __align__(8) HeavyPair {
+    int a, na, b, nb, off, pad;
+};
+
+constexpr int kQuickTests = 1024;   // tests a thread makes for one pair of nodes before it leaves it to a block
+constexpr int kQuickNodes = 4096;   // pairs of particles a thread goes through for one cell pair (particles as nodes)
+constexpr int kHookLinks = 2, kHookTests = 16;   // links and candidates of a node in hook_kernel
+
+struct LinkArgs {
+    const int *cnt;                 // [0] cells [1] nodes
+    const int2 *pairs;
+    const unsigned long long *npairs;
+    const long long *cell_list;
+    const int *cell_node, *node_start, *node_cell;
+    const unsigned char *node_sub;
+    const uint64_t *cell_key;
+    const float4 *rec, *node_rec;
+    const double *x, *y, *z;
+    int *parent, *err;
+    HeavyPair *heavy;
+    int *nheavy;
+    int heavy_cap;
+};
+
+// The half-cells of a cell at offset o that can hold a friend of half-cell hs: half-cell offsets reach 3 only
+// between the far halves of neighbouring cells, which are more than ll apart.  near(ts) below.
+struct NearHalves {
+    int up, dn;
+    __device__ __forceinline__ NearHalves(int3 o, int hs) {
+        const int plus = (o.x > 0 ? 4 : 0) | (o.y > 0 ? 2 : 0) | (o.z > 0 ? 1 : 0);
+        const int minus = (o.x < 0 ? 4 : 0) | (o.y < 0 ? 2 : 0) | (o.z < 0 ? 1 : 0);
+        up = plus & ~hs;
+        dn = minus & hs;
+    }
+    __device__ __forceinline__ bool near(int ts) const { return !((ts & up) | (~ts & dn)); }
+};
+
+// First link between the particles of two nodes (q shifted into p's frame): 1, 0 for none, -1 when the budget
+// of tests (left, lowered by those made) ran out before it was decided.
+__device__ __forceinline__ int node_link(const LinkArgs &A, const FofGeom &g, int p0, int p1, int q0, int q1, float sx,
+                                         float sy, float sz, int &left) {
+    for (int p = p0; p < p1; ++p) {
+        const float4 a = A.rec[p];
+        for (int q = q0; q < q1; ++q) {
+            if (left == 0) return -1;
+            --left;
+            const float4 b = A.rec[q];
+            const float dx = (b.x + sx) - a.x, dy = (b.y + sy) - a.y, dz = (b.z + sz) - a.z;
+            const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            if (d2 <= g.hi &&
+                (d2 < g.lo || exact_link(A.x, A.y, A.z, __float_as_int(a.w), __float_as_int(b.w), g.r2)))
+                return 1;
+        }
+    }
+    return 0;
+}
+
+__device__ __forceinline__ bool push_heavy(const LinkArgs &A, int a, int na, int b, int nb, int3 o) {
+    const int k = atomicAdd(A.nheavy, 1);
+    if (k >= A.heavy_cap) return false;
+    A.heavy[k] = HeavyPair{a, na, b, nb, (o.x + 1) | (o.y + 1) << 2 | (o.z + 1) << 4, 0};
+    return true;
+}
+
+// One thread per node: joins it with the first kHookLinks nodes ahead of it (its cell's, then the forward
+// neighbours' in key order) whose first particle is a friend of its own first particle, of at most
+// kHookTests nodes looked at.
+// Bound, as the whole linking: the latency of dependent loads, hidden by many threads, as long as a warp's lanes
+// stay in step.  So a candidate is one 16-byte record, and the joins come after the search, one step of all
+// lanes' walks at a time: 0.077 ms at 2e6 and 0.58 ms at 2e7 particles.  With the joins made where they were
+// found it took 0.23 and 2.4 ms; all pairs of a cell pair in one thread, find by find, 4.3 and 37 ms.
+__global__ void __launch_bounds__(256) hook_kernel(LinkArgs A, FofGeom g) {
+    const int nn = A.cnt[1];
+    for (int64_t v0 = blockIdx.x * (int64_t)blockDim.x; v0 < nn; v0 += (int64_t)gridDim.x * blockDim.x) {
+        const bool in = v0 + threadIdx.x < nn;
+        const int h = (int)(in ? v0 + threadIdx.x : nn - 1);
+        const long long range = in ? A.cell_list[A.node_cell[h]] : 0;
+        const int2 *list = A.pairs + (range >> 4), *end = list + (range & 15);
+        const float4 a = A.node_rec[h];
+        int found[kHookLinks] = {0, 0}, links = 0, looked = 0;
+        bool more = list != end;
+        while (__any_sync(0xffffffffu, more)) {
+            if (!more) continue;
+            const int2 e = *list++;
+            const int3 o = entry_offset(e.y);
+            const int t0 = e.y >> 8 ? h + 1 : e.x, t1 = e.x + (e.y & 7) + 1;
+            const float sx = (float)o.x * g.cs - a.x, sy = (float)o.y * g.cs - a.y, sz = (float)o.z * g.cs - a.z;
+            for (int t = t0; t < t1 && links < kHookLinks; ++t) {
+                const float4 b = A.node_rec[t];
+                const float dx = b.x + sx, dy = b.y + sy, dz = b.z + sz;
+                if (fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < g.lo) {   // the band is left to the sweep
+                    if (links == 0) found[0] = t;
+                    else found[1] = t;
+                    ++links;
+                }
+            }
+            looked += t1 - t0;
+            more = list != end && links < kHookLinks && looked < kHookTests;
+        }
+        const int r = uf_union_warp(A.parent, h, links > 0 ? found[0] : h, links > 0, A.err);
+        uf_union_warp(A.parent, links > 1 ? r : h, links > 1 ? found[1] : h, links > 1, A.err);
+    }
+}
+
+// Roots as they are after hook_kernel, for the sweep (in an array of their own, see root_kernel).
+__global__ void __launch_bounds__(256) flatten_kernel(const int *__restrict__ cnt, int *parent, int *__restrict__ root,
+                                                      int *err) {
+    const int nn = cnt[1];
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nn; k += (int64_t)gridDim.x * blockDim.x)
+        root[k] = uf_find(parent, (int)k, err);
+}
+
+// Whether two nodes (of roots rh and rt) are in different sets and linked.
+__device__ __forceinline__ bool nodes_linked(const LinkArgs &A, const FofGeom &g, int h, int t, int3 o, int &rh,
+                                             int &rt) {
+    rh = uf_find(A.parent, h, A.err);
+    rt = uf_find(A.parent, t, A.err);
+    if (rh == rt) return false;
+    const float sx = (float)o.x * g.cs, sy = (float)o.y * g.cs, sz = (float)o.z * g.cs;
+    const int p0 = A.node_start[h], p1 = A.node_start[h + 1], q0 = A.node_start[t], q1 = A.node_start[t + 1];
+    int left = kQuickTests;
+    int hit = node_link(A, g, p0, p1, q0, q1, sx, sy, sz, left);
+    if (hit < 0 && !push_heavy(A, p0, p1 - p0, q0, q1 - q0, o)) {
+        hit = 0;   // the blocks' list is full: row by row in place
+        for (int p = p0; p < p1 && hit <= 0; ++p) {
+            left = q1 - q0;
+            hit = node_link(A, g, p, p + 1, q0, q1, sx, sy, sz, left);
+        }
+    }
+    return hit > 0;
+}
+
+__device__ __forceinline__ void link_nodes(const LinkArgs &A, const FofGeom &g, int h, int t, int3 o) {
+    int rh, rt;
+    if (nodes_linked(A, g, h, t, o, rh, rt)) uf_union(A.parent, rh, rt, A.err);
+}
+
+// One thread per node: the pairs with nodes ahead of it that are near enough and whose roots differ, to the list
+// as h << 32 | t (tested in place when the list is full).  The block's pairs are gathered in shared memory, so
+// that it takes its place in the list with one atomic.
+constexpr int kSweepBuf = 1024;
+
+__global__ void __launch_bounds__(256) sweep_kernel(LinkArgs A, FofGeom g, const int *__restrict__ root,
+                                                    unsigned long long *__restrict__ list, long long cap,
+                                                    unsigned long long *__restrict__ nlist) {
+    __shared__ unsigned long long buf[kSweepBuf], place;
+    __shared__ int nbuf;
+    const int nn = A.cnt[1];
+    for (int64_t v0 = blockIdx.x * (int64_t)blockDim.x; v0 < nn; v0 += (int64_t)gridDim.x * blockDim.x) {
+        if (threadIdx.x == 0) nbuf = 0;
+        __syncthreads();
+        const int64_t v = v0 + threadIdx.x;
+        if (v < nn) {
+            const int h = (int)v;
+            const long long range = A.cell_list[A.node_cell[h]];
+            const int2 *ent = A.pairs + (range >> 4), *end = ent + (range & 15);
+            const int rh = root[h], hs = A.node_sub[h];
+            for (; ent != end; ++ent) {
+                const int2 e = *ent;
+                const int t0 = e.y >> 8 ? h + 1 : e.x, t1 = e.x + (e.y & 7) + 1;
+                unsigned other = 0;   // nodes of the entry in another set
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (t0 + j < t1 && root[t0 + j] != rh) other |= 1u << j;
+                if (!other) continue;
+                const int3 o = entry_offset(e.y);
+                const NearHalves halves(o, hs);
+                for (; other; other &= other - 1) {
+                    const int t = t0 + __ffs(other) - 1;
+                    if (!halves.near(A.node_sub[t])) continue;
+                    const unsigned long long pr = (unsigned long long)h << 32 | (unsigned)t;
+                    const int k = atomicAdd(&nbuf, 1);
+                    if (k < kSweepBuf) {
+                        buf[k] = pr;
+                    } else {
+                        const unsigned long long q = atomicAdd(nlist, 1ull);
+                        if ((long long)q < cap) list[q] = pr;
+                        else link_nodes(A, g, h, t, o);
+                    }
+                }
             }
         }
-        // the next item's neighbour row, now that its record has arrived
-        if (item < nitems && lane < 13) nb_next = __ldg(nbinfo + (int64_t)ia_next.z * 13 + lane);
-        int myroot = hv ? uf_find_from(parent, k, pk0, err) : -1;
-        int next = 0;
-        for (int v0 = 0; v0 < total; v0 = next) {
-            next = v0 + 32;
-            // rank of the segment holding candidate v0, and the segments starting in this round
-            const int rfirst = __popc(__ballot_sync(0xffffffffu, nonempty && spre <= v0)) - 1;
-            const int so = spre - v0;
-            const unsigned starts =
-                __reduce_or_sync(0xffffffffu, (nonempty && so > 0 && so < 32) ? (1u << so) : 0u);
-            // a round starting in a neighbour cell that is one component, already in the set of a
-            // home chunk that is itself in one set, skips the rest of that cell
-            {
-                const int seg0 = segtab[w][rfirst];
-                const int n0 = __shfl_sync(0xffffffffu, sn, seg0);
-                const int js = __shfl_sync(0xffffffffu, sjs, seg0);
-                const int end0 = __shfl_sync(0xffffffffu, spre, seg0) + n0;
-                if (seg0 < kHomeSeg && n0 >= 16 && __shfl_sync(0xffffffffu, (int)sconn, seg0)) {
-                    if (v0 > 0 && hv) myroot = uf_find_cached(parent, k, err);
-                    const int r0 = __shfl_sync(0xffffffffu, myroot, 0);
-                    if (__all_sync(0xffffffffu, !hv || myroot == r0)) {
-                        int rr = -1;
-                        if (lane == 0) rr = uf_find_cached(parent, js, err);
-                        rr = __shfl_sync(0xffffffffu, rr, 0);
-                        if (rr == r0) {
-                            next = end0;   // > v0: the loop always moves forward
-                            continue;
-                        }
-                    }
-                }
+        __syncthreads();
+        const int m = min(nbuf, kSweepBuf);
+        if (threadIdx.x == 0 && m > 0) place = atomicAdd(nlist, (unsigned long long)m);
+        __syncthreads();
+        for (int k = threadIdx.x; k < m; k += blockDim.x) {
+            const unsigned long long q = place + k;
+            if ((long long)q < cap) {
+                list[q] = buf[k];
+            } else {
+                const int h = (int)(buf[k] >> 32), t = (int)(buf[k] & 0xffffffffu);
+                link_nodes(A, g, h, t, cell_offset(A.cell_key[A.node_cell[h]], A.cell_key[A.node_cell[t]], g.ky, g.kz));
             }
-            const int v = v0 + lane;
-            bool cv = v < total;
-            // candidate v's segment: the round's first segment plus the starts at or before v
-            const unsigned upto = lane == 31 ? 0xffffffffu : ((2u << lane) - 1u);
-            const int seg = segtab[w][rfirst + __popc(starts & upto)];
-            const int jl = __shfl_sync(0xffffffffu, sjs, seg) + v - __shfl_sync(0xffffffffu, spre, seg);
-            const int off = __shfl_sync(0xffffffffu, soff, seg);
-            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-            int rql = -1;
-            // the candidates' parents and the home particles' own are loaded next to the
-            // candidate records, so that the root walks below start without another round trip
-            const int pj = cv ? parent[jl] : -1;
-            const int pk = (v0 > 0 && hv) ? parent[k] : -1;
-            if (cv) {
-                q = rec[jl];
-                q.x += (float)((off & 3) - 1) * g.cs;
-                q.y += (float)(((off >> 2) & 3) - 1) * g.cs;
-                q.z += (float)(((off >> 4) & 3) - 1) * g.cs;
-                const float ex = fmaxf(0.f, fmaxf(bl[0] - q.x, q.x - bh[0]));
-                const float ey = fmaxf(0.f, fmaxf(bl[1] - q.y, q.y - bh[1]));
-                const float ez = fmaxf(0.f, fmaxf(bl[2] - q.z, q.z - bh[2]));
-                cv = fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= g.hi;
-            }
-            if (!__any_sync(0xffffffffu, cv)) continue;
-            // roots of the candidates, found once per round instead of once per hit; a root
-            // read here may be outdated by later unions, which is safe: equal roots prove the
-            // same set, unequal ones are re-checked by uf_union
-            if (cv) rql = uf_find_from(parent, jl, pj, err);
-            // pick up unions made by other warps since the last look
-            if (v0 > 0 && hv) myroot = uf_find_from(parent, k, pk, err);
-            // when every home particle is in one set, candidates already in it need no test
-            const int r0 = __shfl_sync(0xffffffffu, myroot, 0);   // lane 0 is always a home particle
-            const bool uniform = __all_sync(0xffffffffu, !hv || myroot == r0);
-            const bool mine = cv && !(uniform && rql == r0);
-            unsigned todo = __ballot_sync(0xffffffffu, mine);
-            if (!todo) continue;
-            const int jb = seg == kHomeSeg ? jl : ~jl;   // home-cell candidates keep the j > k test
-            if (__popc(todo) > nhome) {
-                // home-major: each home particle against all candidates of the round
-                unsigned hm = homes;
-                while (hm) {
-                    const int p = __ffs(hm) - 1;
-                    hm &= hm - 1;
-                    const float4 pp = hbuf[w][p];
-                    const int kp = k0 + p;
-                    bool hit = false;
-                    if (mine) {
-                        const float dx = q.x - pp.x, dy = q.y - pp.y, dz = q.z - pp.z;
-                        const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                        hit = d2 <= g.hi && (jb < 0 || jb > kp);
-                        if (hit && d2 >= g.lo) hit = exact_link(x, y, z, __float_as_int(pp.w), __float_as_int(q.w), g.r2);
-                    }
-                    if (!__any_sync(0xffffffffu, hit)) continue;
-                    // the candidates' roots as this round knows them against home particle p's
-                    const int rp = __shfl_sync(0xffffffffu, myroot, p);
-                    const bool need = hit && rql != rp;
-                    const unsigned nm = __ballot_sync(0xffffffffu, need);
-                    if (!nm) continue;
-                    // one union per distinct candidate root among the lanes that hit
-                    const unsigned peers = __match_any_sync(0xffffffffu, need ? rql : ~lane);
-                    const bool leader = need && lane == __ffs(peers) - 1;
-                    int nr = 0;
-                    if (leader) nr = uf_union(parent, rp, rql, err);
-                    if (need) has[jb < 0 ? ~jb : jb] = 1;
-                    if (lane == p) has[k] = 1;
-                    // the joined sets' members now carry the node each union returned
-                    unsigned lm = __ballot_sync(0xffffffffu, leader);
-                    while (lm) {
-                        const int l = __ffs(lm) - 1;
-                        lm &= lm - 1;
-                        const int old = __shfl_sync(0xffffffffu, rql, l);
-                        const int nw = __shfl_sync(0xffffffffu, nr, l);
-                        if (myroot == old || myroot == rp) myroot = nw;
-                        if (rql == old || rql == rp) rql = nw;
-                    }
-                }
-                continue;
-            }
-            __syncwarp();
-            buf[w][lane] = q;
-            rbuf[w][lane] = rql;
-            jbuf[w][lane] = jb;
-            __syncwarp();
-            while (todo) {
-                const int t = __ffs(todo) - 1;
-                todo &= todo - 1;
-                const float4 qq = buf[w][t];
-                const int jt = jbuf[w][t];
-                const float dx = qq.x - hp.x, dy = qq.y - hp.y, dz = qq.z - hp.z;
+        }
+        __syncthreads();   // the buffer is reused
+    }
+}
+
+// One thread per listed pair of nodes.
+__global__ void __launch_bounds__(256) link_kernel(LinkArgs A, FofGeom g, const unsigned long long *__restrict__ list,
+                                                   long long cap, const unsigned long long *__restrict__ nlist) {
+    const long long nl = (long long)*nlist < cap ? (long long)*nlist : cap;
+    for (long long k0 = blockIdx.x * (long long)blockDim.x; k0 < nl; k0 += (long long)gridDim.x * blockDim.x) {
+        const long long k = k0 + threadIdx.x;
+        int rh = 0, rt = 0;
+        bool join = false;
+        if (k < nl) {
+            const int h = (int)(list[k] >> 32), t = (int)(list[k] & 0xffffffffu);
+            const int3 o = cell_offset(A.cell_key[A.node_cell[h]], A.cell_key[A.node_cell[t]], g.ky, g.kz);
+            join = nodes_linked(A, g, h, t, o, rh, rt);
+        }
+        uf_union_warp(A.parent, rh, rt, join, A.err);
+    }
+}
+
+// Particles as nodes (coincident points only, or no room for half-cells in the key): one thread per cell pair
+// tests all its particles; crowded pairs go to the blocks' list.
+__global__ void __launch_bounds__(256) link_particles_kernel(LinkArgs A, FofGeom g) {
+    const long long np = (long long)*A.npairs;
+    for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < np; w += (long long)gridDim.x * blockDim.x) {
+        const int2 pr = A.pairs[w];
+        const bool same = pr.x == pr.y;
+        const int h0 = A.cell_node[pr.x], h1 = A.cell_node[pr.x + 1];
+        const int t0 = A.cell_node[pr.y], t1 = A.cell_node[pr.y + 1];
+        int3 o = make_int3(0, 0, 0);
+        if (!same) o = cell_offset(A.cell_key[pr.x], A.cell_key[pr.y], g.ky, g.kz);
+        if ((long long)(h1 - h0) * (t1 - t0) > kQuickNodes && push_heavy(A, h0, h1 - h0, t0, t1 - t0, o)) continue;
+        for (int h = h0; h < h1; ++h)
+            for (int t = same ? h + 1 : t0; t < t1; ++t) link_nodes(A, g, h, t, o);
+    }
+}
+
+// The list's entries: tiles of 256 x 256 particles, an entry of more than kHuge tiles spread over all blocks, the
+// others one block each.  A thread holds one particle of the first range; the second range's records
+// and roots are staged in shared memory.  Candidates already in the thread's set need no test.
+constexpr int kHuge = 64;
+
+__global__ void __launch_bounds__(256) heavy_kernel(LinkArgs A, FofGeom g, const int *__restrict__ node_of) {
+    __shared__ float4 qrec[256];
+    __shared__ int qroot[256];
+    const int ne = min(*A.nheavy, A.heavy_cap);
+    for (int e = 0; e < ne; ++e) {
+        const HeavyPair hp = A.heavy[e];
+        const long long ta = (hp.na + 255) / 256, tb = (hp.nb + 255) / 256, tiles = ta * tb;
+        const bool huge = tiles > kHuge;
+        if (!huge && e % (int)gridDim.x != (int)blockIdx.x) continue;
+        const bool same = hp.a == hp.b;
+        const float sx = (float)((hp.off & 3) - 1) * g.cs, sy = (float)(((hp.off >> 2) & 3) - 1) * g.cs,
+                    sz = (float)(((hp.off >> 4) & 3) - 1) * g.cs;
+        for (long long tile = huge ? blockIdx.x : 0; tile < tiles; tile += huge ? gridDim.x : 1) {
+            const int p = hp.a + (int)(tile / tb) * 256 + threadIdx.x;
+            const int q = hp.b + (int)(tile % tb) * 256 + threadIdx.x;
+            const bool pv = p < hp.a + hp.na, qv = q < hp.b + hp.nb;
+            __syncthreads();   // the last tile's staging has been read
+            qrec[threadIdx.x] = qv ? A.rec[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+            qroot[threadIdx.x] = qv ? uf_find(A.parent, node_of[q], A.err) : -1;
+            __syncthreads();
+            if (!pv) continue;
+            const float4 a = A.rec[p];
+            const int np = node_of[p];
+            int rp = uf_find(A.parent, np, A.err);
+            const int q0 = q - threadIdx.x, cnt = min(256, hp.b + hp.nb - q0);
+            for (int k = 0; k < cnt; ++k) {
+                if (qroot[k] == rp || (same && q0 + k <= p)) continue;
+                const float4 b = qrec[k];
+                const float dx = (b.x + sx) - a.x, dy = (b.y + sy) - a.y, dz = (b.z + sz) - a.z;
                 const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                bool hit = hv && d2 <= g.hi && (jt < 0 || jt > k);
-                if (hit && d2 >= g.lo) hit = exact_link(x, y, z, hidx, __float_as_int(qq.w), g.r2);
-                if (!__any_sync(0xffffffffu, hit)) continue;
-                // the candidate's root as this round knows it: refreshed after every union of
-                // the round below, without a memory round trip; a root another warp has hooked
-                // since is still an ancestor, which uf_union handles
-                const int rq = rbuf[w][t];
-                const bool need = hit && myroot != rq;
-                const unsigned nm = __ballot_sync(0xffffffffu, need);
-                if (!nm) continue;
-                // one union per distinct root among the home particles that hit: in a crowded
-                // cell most of the 32 share one, and their unions would all contend for it
-                const unsigned peers = __match_any_sync(0xffffffffu, need ? myroot : ~lane);
-                const bool leader = need && lane == __ffs(peers) - 1;
-                int nr = 0;
-                if (leader) nr = uf_union(parent, myroot, rq, err);
-                if (need) has[k] = 1;
-                if (lane == __ffs(nm) - 1) has[jt < 0 ? ~jt : jt] = 1;
-                // the joined sets' members (home particles, the round's candidates) now carry
-                // the node each union returned
-                unsigned lm = __ballot_sync(0xffffffffu, leader);
-                while (lm) {
-                    const int l = __ffs(lm) - 1;
-                    lm &= lm - 1;
-                    const int old = __shfl_sync(0xffffffffu, myroot, l);
-                    const int nw = __shfl_sync(0xffffffffu, nr, l);
-                    if (myroot == old || myroot == rq) myroot = nw;
-                    if (rql == old || rql == rq) rql = nw;
-                }
-                rbuf[w][lane] = rql;
-                __syncwarp();
+                if (!(d2 <= g.hi) ||
+                    !(d2 < g.lo || exact_link(A.x, A.y, A.z, __float_as_int(a.w), __float_as_int(b.w), g.r2)))
+                    continue;
+                rp = uf_union(A.parent, rp, qroot[k], A.err);
             }
         }
     }
 }
 
-// Root of every sorted position, and per root the smallest original index of its members.
-// Consecutive sorted positions mostly share a root (a cell, a group), so the lanes of a warp
-// first take the minimum per distinct root and issue one atomicMin each.  The loop runs the
-// same number of rounds on every lane of a warp (blockDim.x is a multiple of 32).
-__global__ void root_kernel(int n, const int *__restrict__ idx, int *parent,
-                            const unsigned char *__restrict__ has, int *__restrict__ root,
-                            int *__restrict__ minidx, int *err) {
+// Root of every node (in an array of its own: another thread's path halving may still write an older ancestor
+// into parent), and per root the smallest original index and whether the component has
+// more than one particle.  Consecutive nodes mostly share a root, so the lanes of a warp first take the
+// minimum per distinct root and issue one atomicMin each.
+__global__ void __launch_bounds__(256) root_kernel(const int *__restrict__ cnt, const int *__restrict__ node_start,
+                                                   int *parent, int *__restrict__ root, int *minidx,
+                                                   unsigned char *__restrict__ multi, int *err) {
+    const int nn = cnt[1];
     const int lane = threadIdx.x & 31;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k - lane < n;
-         k += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k - lane < nn; k += (int64_t)gridDim.x * blockDim.x) {
         int r = -1, v = INT_MAX;
-        if (k < n) {
-            r = uf_find(parent, (int)k, err);
-            root[k] = r;
-            if (has[k]) v = idx[k];
+        bool many = false;
+        if (k < nn) {
+            const int m = (int)k;
+            r = uf_find(parent, m, err);
+            root[m] = r;
+            if (r != m) v = minidx[m];   // only roots' entries are lowered
+            many = r != m || node_start[m + 1] - node_start[m] > 1;
         }
-        unsigned todo = __ballot_sync(0xffffffffu, v != INT_MAX);
+        unsigned todo = __ballot_sync(0xffffffffu, many);
         while (todo) {
             const int rl = __shfl_sync(0xffffffffu, r, __ffs(todo) - 1);
-            const bool mine = r == rl && v != INT_MAX;
-            const int m = __reduce_min_sync(0xffffffffu, mine ? v : INT_MAX);
+            const bool mine = many && r == rl;
+            const int lo = __reduce_min_sync(0xffffffffu, mine ? v : INT_MAX);
             const unsigned grp = __ballot_sync(0xffffffffu, mine);
-            if (lane == __ffs(grp) - 1) atomicMin(minidx + rl, m);
+            if (lane == __ffs(grp) - 1) {
+                if (lo != INT_MAX) atomicMin(minidx + rl, lo);
+                multi[rl] = 1;
+            }
             todo &= ~grp;
         }
     }
 }
 
-__global__ void label_kernel(int n, const int *__restrict__ idx, const unsigned char *__restrict__ has,
-                             const int *__restrict__ root, const int *__restrict__ minidx,
-                             int *__restrict__ labels, int *__restrict__ ngroups) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+__global__ void __launch_bounds__(256) label_kernel(int n, const int *__restrict__ idx, const int *__restrict__ node_of,
+                                                    const int *__restrict__ root, const int *__restrict__ minidx,
+                                                    const unsigned char *__restrict__ multi, int *__restrict__ labels,
+                                                    int *__restrict__ ngroups) {
+    const int lane = threadIdx.x & 31;
+    int groups = 0;
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
         const int i = idx[k];
-        const int r = root[k];
-        labels[i] = has[k] ? minidx[r] : -1;
-        if (has[k] && r == k) atomicAdd(ngroups, 1);
+        const int r = root[node_of[k]];
+        const int l = multi[r] ? minidx[r] : -1;
+        labels[i] = l;
+        groups += l == i ? 1 : 0;   // one particle a group carries its own index
     }
+    for (int o = 16; o > 0; o >>= 1) groups += __shfl_xor_sync(0xffffffffu, groups, o);
+    if (lane == 0 && groups) atomicAdd(ngroups, groups);
 }
 
 int bits_for(uint64_t v) {
@@ -1145,25 +1108,26 @@ int fof_core(int n, const double *x, const double *y, const double *z, FofGeom g
     if (cells > 4.0e18L)
         return fail(HALMA_ERR_CAPACITY, "cell grid too large (%lld x %lld x %lld cells)", g.ncx, g.ncy, g.ncz);
     const int cell_bits = bits_for((uint64_t)(g.ncx * g.ky * g.kz - 1));
-    g.sb = cell_bits <= 58 ? 6 : 0;
+    // half-cells in the key when there is room for them and the linking length is positive
+    g.sb = cell_bits <= 61 && g.lo > 0.f ? 3 : 0;
     const int end_bit = cell_bits + g.sb;
     const int sms = device_sm_count();
 
+    const int nruns = (n + kScanRun - 1) / kScanRun;
+    const int heavy_cap = std::max(4096, n / 64);
     const size_t sort_b = sort_pairs_u64_i32_bytes(n, end_bit);
-    const size_t scan_b = std::max(exclusive_sum_i32_bytes(n), inclusive_max_i32_bytes(n));
+    const size_t scan_b = exclusive_sum_i64_bytes(nruns);
     Layout M;
     const size_t o_kin = M.add(8ull * n), o_kout = M.add(8ull * n);
     const size_t o_vin = M.add(4ull * n), o_vout = M.add(4ull * n);
     const size_t o_rec = M.add(16ull * n), o_pre = M.add(16ull * n);
-    const size_t o_head = M.add(4ull * n), o_cpos = M.add(4ull * n);
-    const size_t o_par = M.add(4ull * n), o_has = M.add(1ull * n), o_root = M.add(4ull * n);
-    const size_t o_min = M.add(4ull * n);
-    const size_t o_cst = M.add(4ull * (n + 1)), o_ckey = M.add(8ull * n);
-    const size_t o_cm = M.add(4ull * n);   // occupied-neighbour mask and work flag per cell
-    const size_t o_flag = M.add(4ull * n), o_ipos = M.add(4ull * n);
-    const size_t o_items = M.add(sizeof(ItemRec) * (size_t)n);
-    const size_t o_cnt = M.add(64), o_conn = M.add(1ull * n);
-    const size_t o_dlist = M.add(4ull * ((uint64_t)n / kDenseMin + 1));   // cells of >= kDenseMin particles
+    const size_t o_run = M.add(8ull * nruns), o_base = M.add(8ull * nruns);
+    const size_t o_nof = M.add(4ull * n), o_nst = M.add(4ull * (n + 1)), o_sub = M.add(1ull * n);
+    const size_t o_nrec = M.add(16ull * n), o_ncell = M.add(4ull * n), o_clist = M.add(8ull * n);
+    const size_t o_par = M.add(4ull * n), o_root = M.add(4ull * n), o_min = M.add(4ull * n), o_multi = M.add(1ull * n);
+    const size_t o_cnode = M.add(4ull * (n + 1)), o_ckey = M.add(8ull * n);
+    const size_t o_heavy = M.add(sizeof(HeavyPair) * (size_t)heavy_cap);
+    const size_t o_cnt = M.add(64);
     const size_t o_tmp = M.add(std::max(sort_b, scan_b));
     void *base = nullptr;
     HALMA_TRY(push_uf_cap(st));
@@ -1171,15 +1135,16 @@ int fof_core(int n, const double *x, const double *y, const double *z, FofGeom g
     auto *kin = at<uint64_t>(base, o_kin), *kout = at<uint64_t>(base, o_kout);
     auto *vin = at<int>(base, o_vin), *vout = at<int>(base, o_vout);
     auto *rec = at<float4>(base, o_rec), *pre = at<float4>(base, o_pre);
-    auto *head = at<int>(base, o_head), *cpos = at<int>(base, o_cpos);
-    auto *parent = at<int>(base, o_par), *root = at<int>(base, o_root), *minidx = at<int>(base, o_min);
-    auto *has = at<unsigned char>(base, o_has);
-    auto *cst = at<int>(base, o_cst);
-    auto *ckey = at<uint64_t>(base, o_ckey);
-    auto *cmask = at<int>(base, o_cm);
-    auto *flag = at<int>(base, o_flag), *ipos = at<int>(base, o_ipos);
-    auto *items = at<ItemRec>(base, o_items);
-    int *cnt = at<int>(base, o_cnt);   // [0] ncell [1] nitems [2] ngroups [3] err [5] link item counter [8] dense cells
+    auto *runs = at<int64_t>(base, o_run), *rbase = at<int64_t>(base, o_base);
+    int *node_of = at<int>(base, o_nof), *node_start = at<int>(base, o_nst);
+    int *parent = at<int>(base, o_par), *root = at<int>(base, o_root), *minidx = at<int>(base, o_min);
+    auto *node_sub = at<unsigned char>(base, o_sub), *multi = at<unsigned char>(base, o_multi);
+    int *cell_node = at<int>(base, o_cnode);
+    auto *cell_key = at<uint64_t>(base, o_ckey);
+    int *cnt = at<int>(base, o_cnt);   // [0] cells [1] nodes [2] groups [3] error [4] heavy pairs [6..7] cell pairs [8..9] listed pairs of nodes
+    auto *npairs = at<unsigned long long>(base, o_cnt + 24), *nlist = npairs + 1;
+    auto *cell_list = at<long long>(base, o_clist);
+    int *node_cell = at<int>(base, o_ncell);
     void *tmp = at<void>(base, o_tmp);
     const int g1 = std::min(sms * 8, grid_for(n, 256));
 
@@ -1204,46 +1169,46 @@ int fof_core(int n, const double *x, const double *y, const double *z, FofGeom g
     HALMA_TRY(mark(1));
     HALMA_TRY(sort_pairs_u64_i32(tmp, sort_b, kin, kout, vin, vout, n, end_bit, st));
     HALMA_TRY(mark(2));
-    const bool runs = g.sb != 0 && g.lo > 0.f;   // sub-cells in the key and a positive linking length
-    HALMA_LAUNCH(prep_kernel, g1, 256, 0, st, n, g.sb, kout, vout, pre, rec, head, parent, has, minidx,
-                 runs ? flag : nullptr);
-    if (runs) {
-        HALMA_TRY(inclusive_max_i32(tmp, scan_b, flag, root, n, st));
-        HALMA_LAUNCH(preunion_kernel, g1, 256, 0, st, n, kout, root, parent, has);
-    }
+    const int gr = grid_for(nruns, 8);
+    HALMA_LAUNCH(head_count_kernel, gr, 256, 0, st, n, g.sb, kout, runs, nruns);
+    HALMA_TRY(exclusive_sum_i64(tmp, scan_b, runs, rbase, nruns, st));
+    HALMA_LAUNCH(head_apply_kernel, gr, 256, 0, st, n, g.sb, kout, vout, pre, rbase, nruns, rec, node_of, node_start,
+                 node_cell, node_sub, at<float4>(base, o_nrec), parent, minidx, multi, cell_node, cell_key, cnt);
     HALMA_TRY(mark(3));
-    HALMA_TRY(exclusive_sum_i32(tmp, scan_b, head, cpos, n, st));
-    HALMA_LAUNCH(cell_table_kernel, g1, 256, 0, st, n, g.sb, kout, head, cpos, cst, ckey, cnt + 0);
-    // one-component cells (sub-cells in the key and a positive linking length only)
-    unsigned char *conn = at<unsigned char>(base, o_conn);
-    int *dlist = at<int>(base, o_dlist);
-    if (g.sb != 0 && g.lo > 0.f) {
-        HALMA_LAUNCH(small_cell_kernel, g1, 256, 0, st, cnt + 0, cst, kout, conn, dlist, cnt + 8);
-        HALMA_LAUNCH(dense_cell_kernel, sms * 8, 256, 0, st, cnt + 8, dlist, cst, kout, parent, has, conn);
-    } else {
-        HALMA_CUDA(cudaMemsetAsync(conn, 0, n, st));
+    // the list of cell pairs (at most 14 x 8 bytes per occupied cell) in its own cached buffer, sized from the cell
+    // count; up to 2^25 particles (3.8 GB) the particle count saves that round trip (25 us)
+    int ncell = n;
+    if (n > (1 << 25)) {
+        HALMA_CUDA(cudaMemcpyAsync(&ncell, cnt + 0, sizeof(int), cudaMemcpyDeviceToHost, st));
+        HALMA_CUDA(cudaStreamSynchronize(st));
     }
-    // the neighbour table (13 x 8 bytes per occupied cell) in its own cached buffer, sized from
-    // the cell count
-    int ncell = 0;
-    HALMA_CUDA(cudaMemcpyAsync(&ncell, cnt + 0, sizeof(int), cudaMemcpyDeviceToHost, st));
-    HALMA_CUDA(cudaStreamSynchronize(st));
-    void *nbbase = nullptr;
-    HALMA_TRY(workspace(sizeof(int2) * 13 * (size_t)std::max(ncell, 1), &nbbase, st, 10));
-    int2 *nbinfo = static_cast<int2 *>(nbbase);
-    HALMA_LAUNCH(nbtab_kernel, std::min(sms * 8, grid_for(ncell, 256)), 256, 0, st, cnt + 0, cst, ckey, conn, g.ky,
-                 g.kz, nbinfo, cmask);
+    void *pbase = nullptr;
+    HALMA_TRY(workspace(sizeof(int2) * 14 * (size_t)std::max(ncell, 1), &pbase, st, 10));
+    int2 *pairs = static_cast<int2 *>(pbase);
+    const int gc = std::min(sms * 8, grid_for(ncell, 256));
     HALMA_TRY(mark(4));
-    HALMA_LAUNCH(itemflag_kernel, g1, 256, 0, st, n, head, cpos, cst, cmask, flag);
-    HALMA_TRY(exclusive_sum_i32(tmp, scan_b, flag, ipos, n, st));
-    HALMA_LAUNCH(items_kernel, g1, 256, 0, st, n, head, cpos, flag, ipos, cst, conn, items, cnt + 1);
+    if (g.sb)
+        HALMA_LAUNCH(cell_pair_kernel<true>, gc, 256, 0, st, cnt, cell_node, cell_key, g.ky, g.kz, pairs, cell_list,
+                     npairs);
+    else
+        HALMA_LAUNCH(cell_pair_kernel<false>, gc, 256, 0, st, cnt, cell_node, cell_key, g.ky, g.kz, pairs, cell_list,
+                     npairs);
     HALMA_TRY(mark(5));
-    HALMA_LAUNCH(link_kernel, sms * 8, 32 * kFofWarps, 0, st, rec, items, cnt + 1, cnt + 5, nbinfo, g, x, y, z,
-                 parent, has, cnt + 3);
+    LinkArgs A{cnt, pairs, npairs, cell_list, cell_node, node_start, node_cell, node_sub, cell_key, rec,
+               at<float4>(base, o_nrec), x, y, z, parent, cnt + 3, at<HeavyPair>(base, o_heavy), cnt + 4, heavy_cap};
+    if (g.sb) {
+        auto *list = reinterpret_cast<unsigned long long *>(kin);   // the sort's input is no longer needed: n entries
+        HALMA_LAUNCH(hook_kernel, g1, 256, 0, st, A, g);
+        HALMA_LAUNCH(flatten_kernel, g1, 256, 0, st, cnt, parent, root, cnt + 3);
+        HALMA_LAUNCH(sweep_kernel, g1, 256, 0, st, A, g, root, list, (long long)n, nlist);
+        HALMA_LAUNCH(link_kernel, g1, 256, 0, st, A, g, list, (long long)n, nlist);
+    } else {
+        HALMA_LAUNCH(link_particles_kernel, std::min(sms * 8, grid_for(4ll * ncell, 256)), 256, 0, st, A, g);
+    }
+    HALMA_LAUNCH(heavy_kernel, sms * 4, 256, 0, st, A, g, node_of);
     HALMA_TRY(mark(6));
-    // the sorted original indices (4 bytes a position) rather than the records' 16
-    HALMA_LAUNCH(root_kernel, g1, 256, 0, st, n, vout, parent, has, root, minidx, cnt + 3);
-    HALMA_LAUNCH(label_kernel, g1, 256, 0, st, n, vout, has, root, minidx, labels, cnt + 2);
+    HALMA_LAUNCH(root_kernel, g1, 256, 0, st, cnt, node_start, parent, root, minidx, multi, cnt + 3);
+    HALMA_LAUNCH(label_kernel, g1, 256, 0, st, n, vout, node_of, root, minidx, multi, labels, cnt + 2);
     HALMA_TRY(mark(7));
     int hc[4];
     HALMA_CUDA(cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));

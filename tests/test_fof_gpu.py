@@ -167,3 +167,47 @@ def test_groups_reject_labels_that_are_not_particle_indices(cuda):
             fof.fof_groups(torch.from_numpy(bad).to(cuda))
     off, mem = fof.fof_groups(np.array([0, 0, -1, 3, 3, 3], dtype=np.int32))
     assert off.tolist() == [0, 2, 5] and mem.tolist() == [0, 1, 3, 4, 5]
+
+
+def _clumps(n, sep, spread, seed):
+    """Two clumps of n points on x = 0 and x = sep (Mpc), spread in y and z only."""
+    rng = np.random.default_rng(seed)
+    p = np.zeros((2 * n, 3))
+    p[n:, 0] = sep
+    p[:, 1:] = rng.uniform(0.0, spread, (2 * n, 2))
+    return np.ascontiguousarray(p[rng.permutation(2 * n)].T)
+
+
+@pytest.mark.parametrize("n,sep,spread", [
+    (31, 1.5e-3, 1e-4), (33, 1.5001e-3, 1e-4), (700, 1.49999e-3, 2e-4), (3000, 1.4999999e-3, 5e-4),
+    (3000, 1.50001e-3, 5e-4), (20000, 1.50001e-3, 6e-4)])
+def test_crowded_half_cells_a_linking_length_apart(cuda, n, sep, spread):
+    """Pairs of nodes with more than a thread's share of tests, with few links or none between them."""
+    ll = 1.5e-3
+    x, y, z = _clumps(n, sep, spread, 3)
+    x += 0.11
+    lab = fof.fof_labels(x, y, z, ll)
+    # a clump is one group (its spread is below the linking length); they join where a pair is near enough
+    left = x < 0.11 + sep / 2
+    d2 = np.inf
+    for b in range(0, n, 2000):   # the smallest separation squared, in the predicate's own order of operations
+        i, j = np.nonzero(left)[0][b:b + 2000], np.nonzero(~left)[0]
+        dx, dy, dz = (a[i][:, None] - a[j][None, :] for a in (x, y, z))
+        d2 = min(d2, ((dx * dx + dy * dy) + dz * dz).min())
+    first = [np.nonzero(left)[0][0], np.nonzero(~left)[0][0]]
+    want = np.where(left, first[0], first[1]) if d2 > ll * ll else np.zeros(2 * n, dtype=np.int64)
+    assert np.array_equal(lab, want)
+
+
+@pytest.mark.parametrize("ll,box,n", [(0.0, 1.0, 9000), (4.0 / 1.45e6, 4.0, 5000), (5000.0 / 1.4e6, 5000.0, 20000)])
+def test_particles_as_nodes(cuda, ll, box, n):
+    """No half-cells in the key: coincident points only (ll = 0, crowded cells), and grids whose keys leave
+    no room for them."""
+    rng = np.random.default_rng(11)
+    p = rng.uniform(0.0, box, (n // 3, 3))
+    p = np.concatenate([p, p[rng.integers(0, len(p), n // 3)], np.full((n // 3, 3), box / 3)])
+    if ll > 0:
+        p[n // 3:2 * (n // 3)] += rng.normal(0.0, 0.4 * ll, (n // 3, 3))
+    p = p[rng.permutation(len(p))]
+    x, y, z = (np.ascontiguousarray(c) for c in p.T)
+    assert np.array_equal(fof.fof_labels(x, y, z, ll), oracle.fof_labels(x, y, z, ll))
