@@ -63,7 +63,7 @@ def _catalogue(lo, hi, target_pairs, seed, alpha=0.0):
 
 def _time_pass(arrs, repeats):
     from .unbinding import UnbindOptions, unbind_batched
-    opt = UnbindOptions(eps=1e-4, max_iter=1)
+    opt = UnbindOptions(eps=1e-4, max_iter=1, incremental=False)   # every halo on the pass kernels
     unbind_batched(*arrs, opt)          # warm-up (graph capture for this shape)
     ms = []
     pairs = 0.0

@@ -168,13 +168,14 @@ __global__ void __launch_bounds__(kSegThreads) ub_reduce_seg_kernel(
     }
 }
 
-// One warp per halo: chunk sums added in a fixed order (lane-strided, then the warp tree);
+// One warp per ordered halo: chunk sums added in a fixed order (lane-strided, then the warp tree);
 // sets the bound mass, centre of mass, bulk velocity and bound count.
-__global__ void ub_reduce_fin_kernel(int nh, const int *__restrict__ cstart, const double *__restrict__ part,
-                                     int force, HaloState *hs) {
-    const int h = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+__global__ void ub_reduce_fin_kernel(int nh, const int *__restrict__ order, const int *__restrict__ cstart,
+                                     const double *__restrict__ part, int force, HaloState *hs) {
+    const int q = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
-    if (h >= nh) return;
+    if (q >= nh) return;
+    const int h = order[q];
     if (!force && !hs[h].active) return;
     double v[kRedSums] = {0, 0, 0, 0, 0, 0, 0, 0};
     for (int c = cstart[h] + lane; c < cstart[h + 1]; c += 32)
@@ -925,6 +926,72 @@ struct SegDF {
     double rm, rmx, rmy, rmz, rmvx, rmvy, rmvz;   // FP64 sums over the removed particles
 };
 
+// One slot's potential of the pass (full pass: the sum itself; incremental pass: the previous potential minus the
+// removed particles' contribution), kinetic energy per unit mass and cut: u is the packed velocity
+// offset and mass, w the halo's bulk-velocity offset.  True when the particle is kept.
+struct SlotEnergy {
+    float2 p;
+    float pf, ek;
+    bool keep;
+};
+
+__device__ __forceinline__ SlotEnergy slot_energy(float2 p, float4 u, float wx, float wy, float wz, float gfac) {
+    SlotEnergy s;
+    s.p = p;
+    s.pf = p.x + p.y;
+    const float dx = u.x - wx, dy = u.y - wy, dz = u.z - wz;
+    s.ek = 0.5f * (dx * dx + dy * dy + dz * dz);
+    const float e = s.ek - gfac * s.pf;
+    s.keep = !(e > 0.f);
+    return s;
+}
+
+// FP64 sums (m, m x, m v) over the listed particles, one warp; lane 0 holds the totals.
+__device__ __forceinline__ void removed_sums(const int *list, int nrem, const double *__restrict__ x,
+                                             const double *__restrict__ y, const double *__restrict__ z,
+                                             const double *__restrict__ vx, const double *__restrict__ vy,
+                                             const double *__restrict__ vz, const double *__restrict__ m, int lane,
+                                             double (&a)[7]) {
+#pragma unroll
+    for (int k = 0; k < 7; ++k) a[k] = 0.0;
+    for (int k = lane; k < nrem; k += 32) {
+        const int i = list[k];
+        const double mi = m[i];
+        a[0] += mi;
+        a[1] += mi * x[i];
+        a[2] += mi * y[i];
+        a[3] += mi * z[i];
+        a[4] += mi * vx[i];
+        a[5] += mi * vy[i];
+        a[6] += mi * vz[i];
+    }
+    if (nrem > 0)
+#pragma unroll
+        for (int k = 0; k < 7; ++k) a[k] = warp_sum(a[k]);
+}
+
+// The halo's state after a pass that removed something: keep_run particles remain, a are the removed ones' sums.
+__device__ __forceinline__ void subtract_removed(HaloState &o, int keep_run, const double (&a)[7]) {
+    o.nb = keep_run;
+    if (keep_run == 0) {
+        o.M = o.sx = o.sy = o.sz = o.px = o.py = o.pz = 0.0;
+    } else {
+        o.M -= a[0];
+        o.sx -= a[1]; o.sy -= a[2]; o.sz -= a[3];
+        o.px -= a[4]; o.py -= a[5]; o.pz -= a[6];
+    }
+    const double M = o.M;
+    if (M > 0) {
+        o.cx = o.sx / M; o.cy = o.sy / M; o.cz = o.sz / M;
+        o.vx = o.px / M; o.vy = o.py / M; o.vz = o.pz / M;
+    } else {
+        o.cx = o.cy = o.cz = o.vx = o.vy = o.vz = 0.0;
+    }
+    o.wx = (float)(o.vx - o.v0x);
+    o.wy = (float)(o.vy - o.v0y);
+    o.wz = (float)(o.vz - o.v0z);
+}
+
 __device__ __forceinline__ float2 df_warp_sum(float2 v) {
     for (int o = 16; o > 0; o >>= 1)
         v = df_add(v, make_float2(__shfl_down_sync(0xffffffffu, v.x, o), __shfl_down_sync(0xffffffffu, v.y, o)));
@@ -1002,22 +1069,16 @@ __global__ void __launch_bounds__(kSegThreads) ub_energy_df_kernel(
                 gone[slot] = 0;
                 continue;
             }
-            // full pass: the sum itself; incremental pass: previous potential minus the removed
-            // particles' contribution
-            const float2 p = inc ? df_sub(phi_prev[pb + r[j]], d[j]) : d[j];
-            phi_cur[pb + r[j]] = p;
-            const float pf = p.x + p.y;
-            const float dx = u[j].x - wx, dy = u[j].y - wy, dz = u[j].z - wz;
-            const float ek = 0.5f * (dx * dx + dy * dy + dz * dz);
-            const float e = ek - gfac * pf;
-            const bool keep = !(e > 0.f);
-            keepf[pb + r[j]] = keep ? 1 : 0;
-            gone[slot] = keep ? 0 : 1;
-            if (keep) {
+            const SlotEnergy se_ =
+                slot_energy(inc ? df_sub(phi_prev[pb + r[j]], d[j]) : d[j], u[j], wx, wy, wz, gfac);
+            phi_cur[pb + r[j]] = se_.p;
+            keepf[pb + r[j]] = se_.keep ? 1 : 0;
+            gone[slot] = se_.keep ? 0 : 1;
+            if (se_.keep) {
                 ++kept;
-                two_sum_acc(ek_s, ek_c, u[j].w * ek);
-                two_sum_acc(ep_s, ep_c, u[j].w * pf);
-                if (phi_out) phi_out[pidx[pb + r[j]]] = df_to_double(p);
+                two_sum_acc(ek_s, ek_c, u[j].w * se_.ek);
+                two_sum_acc(ep_s, ep_c, u[j].w * se_.pf);
+                if (phi_out) phi_out[pidx[pb + r[j]]] = df_to_double(se_.p);
             } else {
                 ++removed;
                 const int i = pidx[pb + r[j]];
@@ -1053,21 +1114,8 @@ __global__ void __launch_bounds__(kSegThreads) ub_energy_df_kernel(
                     base += __popc(bal);
                 }
             __syncwarp();
-            double a[7] = {0, 0, 0, 0, 0, 0, 0};
-            for (int k = lane; k < nrem; k += 32) {
-                const int i = rlist[k];
-                const double mi = m[i];
-                a[0] += mi;
-                a[1] += mi * x[i];
-                a[2] += mi * y[i];
-                a[3] += mi * z[i];
-                a[4] += mi * vx[i];
-                a[5] += mi * vy[i];
-                a[6] += mi * vz[i];
-            }
-            if (nrem > 0)
-#pragma unroll
-                for (int k = 0; k < 7; ++k) a[k] = warp_sum(a[k]);
+            double a[7];
+            removed_sums(rlist, nrem, x, y, z, vx, vy, vz, m, lane, a);
             if (lane == 0) {
                 SegDF o;
                 o.removed = nrem;
@@ -1141,24 +1189,7 @@ __global__ void ub_finalize_df_kernel(int nh, const int *__restrict__ order, con
         if (rem_run == 0) {
             o.active = 0;
         } else {
-            o.nb = keep_run;
-            if (keep_run == 0) {
-                o.M = o.sx = o.sy = o.sz = o.px = o.py = o.pz = 0.0;
-            } else {
-                o.M -= a[0];
-                o.sx -= a[1]; o.sy -= a[2]; o.sz -= a[3];
-                o.px -= a[4]; o.py -= a[5]; o.pz -= a[6];
-            }
-            const double M = o.M;
-            if (M > 0) {
-                o.cx = o.sx / M; o.cy = o.sy / M; o.cz = o.sz / M;
-                o.vx = o.px / M; o.vy = o.py / M; o.vz = o.pz / M;
-            } else {
-                o.cx = o.cy = o.cz = o.vx = o.vy = o.vz = 0.0;
-            }
-            o.wx = (float)(o.vx - o.v0x);
-            o.wy = (float)(o.vy - o.v0y);
-            o.wz = (float)(o.vz - o.v0z);
+            subtract_removed(o, keep_run, a);
         }
     }
 }
@@ -1236,6 +1267,298 @@ __global__ void __launch_bounds__(kSegThreads) ub_compact_df_kernel(
     }
 }
 
+// Haloes of at most kSmallMax members, all passes in one block each: the halo's packed slots, its removed
+// particles and its state stay in shared memory, and the passes follow one another without a launch.  Every sum is
+// formed in the order of the pass kernels above (reduction, pack, tile kernel with one slice, energy, finalize), so
+// the result is theirs bit for bit.
+// Bound: latency -- of a pass's barriers and FP64 steps for a single small catalogue, hidden by the other blocks of
+// an SM for large ones.  24 haloes of 50 to 1,000 took 16 passes x 9 launches; of 10,000 haloes of which 9,500 are
+// this small, a block of 256 threads per halo and kernel was mostly empty.
+// P slots, THREADS threads (slot = j * THREADS + thread, as the energy kernel has it: P <= THREADS, or 256 threads).
+constexpr int kSmallMax = kSymBlock;
+
+template <int P, int THREADS>
+struct SmallShared {
+    float4 src[P];       // 32-slot chunks as pairs: 16 x {x, x, y, y}, 16 x {z, z, m, m}
+    float4 pv[P];        // velocity offsets and masses
+    int idx[P];
+    union {
+        double red[kRedSums - 1][THREADS];   // before the first pass
+        struct {
+            float4 rem[P];   // the last pass's removed particles, as src
+            float2 phi[P];
+            int rlist[P];
+        };
+    };
+    double q4[kRedSums][4];
+    float2 se[2][THREADS / 32];
+    int cnt[2][(P + THREADS - 1) / THREADS][THREADS / 32];
+    HaloState hs;
+};
+
+template <int P>
+__device__ __forceinline__ void put_pair_slot(float4 *chunks, int r, float x, float y, float z, float m) {
+    float *c = reinterpret_cast<float *>(chunks + (r >> 5) * 32);
+    const int kp = (r & 31) >> 1, hf = r & 1;
+    c[kp * 4 + hf] = x;
+    c[kp * 4 + 2 + hf] = y;
+    c[64 + kp * 4 + hf] = z;
+    c[64 + kp * 4 + 2 + hf] = m;
+}
+
+__device__ __forceinline__ float4 get_pair_slot(const float4 *chunks, int r) {
+    const float *c = reinterpret_cast<const float *>(chunks + (r >> 5) * 32);
+    const int kp = (r & 31) >> 1, hf = r & 1;
+    return make_float4(c[kp * 4 + hf], c[kp * 4 + 2 + hf], c[64 + kp * 4 + hf], c[64 + kp * 4 + 2 + hf]);
+}
+
+// 32 * T targets from group g0 on against the sources' chunks; the potentials go to phi (minus them when inc).
+template <int T>
+__device__ __forceinline__ void small_pairs(const float4 *tgt, const float4 *src, int nb, int ns, int g0, bool inc,
+                                            float eps2, float2 *phi, int lane) {
+    f2x tx[T], ty[T], tz[T];
+    float sum[T], comp[T];
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        const int r = (g0 + t) * 32 + lane;
+        const float4 p = r < nb ? get_pair_slot(tgt, r) : make_float4(kFar, kFar, kFar, 0.f);
+        tx[t] = pack2(p.x, p.x);
+        ty[t] = pack2(p.y, p.y);
+        tz[t] = pack2(p.z, p.z);
+        sum[t] = 0.f;
+        comp[t] = 0.f;
+    }
+    const f2x e2 = pack2(eps2, eps2);
+    for (int c = 0; c < (ns + 31) >> 5; ++c) {
+        const float4 *buf = src + c * 32;
+        f2x acc[T];
+#pragma unroll
+        for (int t = 0; t < T; ++t) acc[t] = pack2(0.f, 0.f);
+        const int ts = c - g0;
+        if (!inc && ts >= 0 && ts < T) chunk_pairs<T, true>(buf, buf + 16, tx, ty, tz, e2, acc, ts, lane);
+        else chunk_pairs<T, false>(buf, buf + 16, tx, ty, tz, e2, acc, ts, lane);
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            float a0, a1;
+            unpack2(acc[t], a0, a1);
+            two_sum_acc(sum[t], comp[t], a0 + a1);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        const int r = (g0 + t) * 32 + lane;
+        if (r >= nb) continue;
+        const float2 d = df_add(make_float2(0.f, 0.f), df_from_acc(sum[t], comp[t]));   // as one slice is added
+        phi[r] = inc ? df_sub(phi[r], d) : d;
+    }
+}
+
+template <int P, int THREADS>
+__global__ void __launch_bounds__(THREADS) ub_small_kernel(
+    const int *__restrict__ list, const int64_t *__restrict__ off, const double *__restrict__ x,
+    const double *__restrict__ y, const double *__restrict__ z, const double *__restrict__ vx,
+    const double *__restrict__ vy, const double *__restrict__ vz, const double *__restrict__ m, float eps2, double gfac,
+    int max_iter, unsigned char *__restrict__ bound, double *__restrict__ phi_out, HaloState *__restrict__ hs) {
+    constexpr int J = (P + THREADS - 1) / THREADS, W = THREADS / 32;
+    static_assert(J == 1 || THREADS == kSegThreads, "slots are laid out as in the energy kernel");
+    extern __shared__ __align__(16) unsigned char small_raw[];
+    auto &sh = *reinterpret_cast<SmallShared<P, THREADS> *>(small_raw);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int h = list[blockIdx.x];
+    const int64_t b = off[h];
+    const int n = (int)(off[h + 1] - b);
+    const float gfac_f = (float)gfac;
+    // ---- FP64 mass, centre and bulk velocity (ub_reduce_seg_kernel, ub_reduce_fin_kernel)
+    double f[J][7];
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        const int r = j * THREADS + threadIdx.x;
+        const int64_t i = b + (r < n ? r : 0);
+        const bool in = r < n;
+        f[j][0] = in ? m[i] : 0.0;
+        f[j][1] = in ? x[i] : 0.0;
+        f[j][2] = in ? y[i] : 0.0;
+        f[j][3] = in ? z[i] : 0.0;
+        f[j][4] = in ? vx[i] : 0.0;
+        f[j][5] = in ? vy[i] : 0.0;
+        f[j][6] = in ? vz[i] : 0.0;
+    }
+    {
+        double v[kRedSums - 1] = {0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            if (j * THREADS + (int)threadIdx.x >= n) continue;
+            const double mi = f[j][0];
+            v[0] += mi;
+#pragma unroll
+            for (int k = 1; k < 7; ++k) v[k] += mi * f[j][k];
+        }
+#pragma unroll
+        for (int k = 0; k < kRedSums - 1; ++k) sh.red[k][threadIdx.x] = v[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4 * (kRedSums - 1)) {
+        const int k = threadIdx.x % (kRedSums - 1), run = threadIdx.x / (kRedSums - 1);
+        double t = 0.0;
+        const int u1 = min(min(THREADS, n), (run + 1) * (kSegThreads / 4));   // threads past n hold zeros
+        for (int u = run * (kSegThreads / 4); u < u1; ++u) t += sh.red[k][u];
+        sh.q4[k][run] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < kRedSums - 1) {
+        const int k = threadIdx.x;
+        sh.q4[k][0] = ((sh.q4[k][0] + sh.q4[k][1]) + sh.q4[k][2]) + sh.q4[k][3];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        HaloState s{};
+        const double M = sh.q4[0][0];
+        s.M = M;
+        s.nb = n;
+        s.sx = sh.q4[1][0]; s.sy = sh.q4[2][0]; s.sz = sh.q4[3][0];
+        s.px = sh.q4[4][0]; s.py = sh.q4[5][0]; s.pz = sh.q4[6][0];
+        if (M > 0) {
+            s.cx = s.sx / M; s.cy = s.sy / M; s.cz = s.sz / M;
+            s.vx = s.px / M; s.vy = s.py / M; s.vz = s.pz / M;
+        }
+        s.v0x = s.vx; s.v0y = s.vy; s.v0z = s.vz;
+        sh.hs = s;
+    }
+    __syncthreads();
+    // ---- packing (ub_pack_kernel)
+    {
+        const double cx = sh.hs.cx, cy = sh.hs.cy, cz = sh.hs.cz;
+        const double v0x = sh.hs.v0x, v0y = sh.hs.v0y, v0z = sh.hs.v0z;
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int r = j * THREADS + threadIdx.x;
+            if (r < n) {
+                put_pair_slot<P>(sh.src, r, (float)(f[j][1] - cx), (float)(f[j][2] - cy), (float)(f[j][3] - cz),
+                                 (float)f[j][0]);
+                sh.pv[r] = make_float4((float)(f[j][4] - v0x), (float)(f[j][5] - v0y), (float)(f[j][6] - v0z),
+                                       (float)f[j][0]);
+                sh.idx[r] = (int)(b + r);
+            } else if (r < ((n + 31) & ~31)) {
+                put_pair_slot<P>(sh.src, r, kFar, kFar, kFar, 0.f);
+            }
+        }
+    }
+    __syncthreads();
+    int nb = n, nrem = 0;
+    for (int it = 0; it < max_iter; ++it) {
+        // ---- pair terms
+        const bool inc = it > 0;
+        const int groups = (nb + 31) >> 5, ns = inc ? nrem : nb;
+        const float4 *src = inc ? sh.rem : sh.src;
+        if (groups <= W) {
+            if (w < groups) small_pairs<1>(sh.src, src, nb, ns, w, inc, eps2, sh.phi, lane);
+        } else if (groups <= 2 * W) {
+            if (2 * w < groups) small_pairs<2>(sh.src, src, nb, ns, 2 * w, inc, eps2, sh.phi, lane);
+        } else {
+            if (4 * w < groups) small_pairs<4>(sh.src, src, nb, ns, 4 * w, inc, eps2, sh.phi, lane);
+        }
+        __syncthreads();
+        // ---- energies and the cut (ub_energy_df_kernel)
+        const float wx = sh.hs.wx, wy = sh.hs.wy, wz = sh.hs.wz;
+        float ek_s = 0.f, ek_c = 0.f, ep_s = 0.f, ep_c = 0.f;
+        float4 u[J], pos[J];
+        float2 ph[J];
+        int id[J];
+        unsigned kb[J], gb[J];
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int r = j * THREADS + threadIdx.x;
+            const bool ok = r < nb;
+            bool keep = false;
+            if (ok) {
+                u[j] = sh.pv[r];
+                pos[j] = get_pair_slot(sh.src, r);
+                id[j] = sh.idx[r];
+                const SlotEnergy e = slot_energy(sh.phi[r], u[j], wx, wy, wz, gfac_f);
+                ph[j] = e.p;
+                keep = e.keep;
+                if (keep) {
+                    two_sum_acc(ek_s, ek_c, u[j].w * e.ek);
+                    two_sum_acc(ep_s, ep_c, u[j].w * e.pf);
+                } else {
+                    bound[id[j]] = 0;
+                }
+            }
+            kb[j] = __ballot_sync(0xffffffffu, keep);
+            gb[j] = __ballot_sync(0xffffffffu, ok && !keep);
+            if (lane == 0) {
+                sh.cnt[0][j][w] = __popc(kb[j]);
+                sh.cnt[1][j][w] = __popc(gb[j]);
+            }
+        }
+        const float2 ekv = df_warp_sum(df_from_acc(ek_s, ek_c));
+        const float2 epv = df_warp_sum(df_from_acc(ep_s, ep_c));
+        if (lane == 0) {
+            sh.se[0][w] = ekv;
+            sh.se[1][w] = epv;
+        }
+        __syncthreads();
+        // ---- survivors and removed particles in slot order (ub_compact_df_kernel)
+        int kept = 0, gone = 0;
+        const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            int kr = kept, gr = gone;
+#pragma unroll
+            for (int k = 0; k < W; ++k) {
+                if (k < w) {
+                    kr += sh.cnt[0][j][k];
+                    gr += sh.cnt[1][j][k];
+                }
+                kept += sh.cnt[0][j][k];
+                gone += sh.cnt[1][j][k];
+            }
+            if (kb[j] >> lane & 1) {
+                kr += __popc(kb[j] & lt);
+                put_pair_slot<P>(sh.src, kr, pos[j].x, pos[j].y, pos[j].z, pos[j].w);   // every slot was read before the barrier
+                sh.pv[kr] = u[j];
+                sh.idx[kr] = id[j];
+                sh.phi[kr] = ph[j];
+            } else if (gb[j] >> lane & 1) {
+                gr += __popc(gb[j] & lt);
+                put_pair_slot<P>(sh.rem, gr, pos[j].x, pos[j].y, pos[j].z, pos[j].w);
+                sh.rlist[gr] = id[j];
+            }
+        }
+        if (threadIdx.x < 32) {   // padding of both lists to whole chunks
+            const int rk = kept + threadIdx.x, rg = gone + threadIdx.x;
+            if (rk < ((kept + 31) & ~31)) put_pair_slot<P>(sh.src, rk, kFar, kFar, kFar, 0.f);
+            if (rg < ((gone + 31) & ~31)) put_pair_slot<P>(sh.rem, rg, kFar, kFar, kFar, 0.f);
+        }
+        __syncthreads();
+        // ---- energies of the pass, and the next pass's mass and bulk velocity (ub_finalize_df_kernel)
+        if (w == 0) {
+            double a[7];
+            removed_sums(sh.rlist, gone, x, y, z, vx, vy, vz, m, lane, a);
+            if (lane == 0) {
+                float2 e0 = make_float2(0.f, 0.f), e1 = make_float2(0.f, 0.f);
+                for (int k = 0; k < W; ++k) {
+                    e0 = df_add(e0, sh.se[0][k]);
+                    e1 = df_add(e1, sh.se[1][k]);
+                }
+                HaloState &o = sh.hs;
+                o.iter += 1;
+                o.ekin = df_to_double(df_add(make_float2(0.f, 0.f), e0));
+                o.epot = -0.5 * gfac * df_to_double(df_add(make_float2(0.f, 0.f), e1));
+                if (gone > 0) subtract_removed(o, kept, a);
+            }
+        }
+        nb = kept;
+        nrem = gone;
+        if (gone == 0) break;   // the same for all threads
+        __syncthreads();
+    }
+    __syncthreads();
+    if (phi_out)
+        for (int r = threadIdx.x; r < nb; r += THREADS) phi_out[sh.idx[r]] = df_to_double(sh.phi[r]);
+    if (threadIdx.x == 0) hs[h] = sh.hs;   // active = 0
+}
+
 // Plain FP64 pair kernel for one halo (targets = sources = its packed slots).
 __global__ void __launch_bounds__(256) ub_pair_f64_kernel(const double4 *__restrict__ pk, int nb, double eps2,
                                                           double *__restrict__ phi) {
@@ -1291,9 +1614,10 @@ GraphCache &graph_cache() {
 }
 
 // Number of haloes still active after a chunk of passes (the host stops replaying at 0).
-__global__ void ub_active_kernel(int nh, const HaloState *__restrict__ hs, int *__restrict__ count) {
+__global__ void ub_active_kernel(int nh, const int *__restrict__ order, const HaloState *__restrict__ hs,
+                                 int *__restrict__ count) {
     int a = 0;
-    for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < nh; h += gridDim.x * blockDim.x) a += hs[h].active;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nh; q += gridDim.x * blockDim.x) a += hs[order[q]].active;
     for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
     if ((threadIdx.x & 31) == 0 && a) atomicAdd(count, a);
 }
@@ -1371,6 +1695,19 @@ int sym_self_potential_device(const float4 *pk, int nb, float eps2, float2 *part
     return HALMA_OK;
 }
 
+template <int P, int THREADS>
+static int launch_small(const int *list, int count, const int64_t *off, const double *x, const double *y,
+                        const double *z, const double *vx, const double *vy, const double *vz, const double *m,
+                        const halma_unbind_params &p, double gfac, unsigned char *bound, double *phi_out, HaloState *hs,
+                        cudaStream_t st) {
+    if (count <= 0) return HALMA_OK;
+    constexpr int smem = (int)sizeof(SmallShared<P, THREADS>);
+    HALMA_CUDA(cudaFuncSetAttribute(ub_small_kernel<P, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    HALMA_LAUNCH((ub_small_kernel<P, THREADS>), count, THREADS, smem, st, list, off, x, y, z, vx, vy, vz, m,
+                 (float)(p.eps * p.eps), gfac, p.max_iter, bound, phi_out, hs);
+    return HALMA_OK;
+}
+
 // Device-array implementation shared by halma_unbind_batched and the pipeline.
 int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off, const double *x, const double *y,
                   const double *z, const double *vx, const double *vy, const double *vz, const double *m,
@@ -1380,16 +1717,31 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
     const bool f64 = p.precision == HALMA_UNBIND_FP64;
     // source slice length (a multiple of 32); the FP64 path sums a halo in one piece
     const int slice_len = f64 ? (1 << 30) : tab.slice;
+    // incremental passes subtract the removed particles' potential instead of recomputing
+    const bool incremental = !(p.flags & HALMA_UNBIND_FULL_RECOMPUTE);
+    // Haloes of at most kSmallMax members run all their passes in one block (ub_small_kernel), which forms the
+    // sums as the pass kernels do with one slice; the pass kernels take the others, nb_ of them.
+    const bool use_small = !f64 && incremental && slice_len >= kSmallMax;
+    auto is_small = [&](int h) { return use_small && h_off[h + 1] - h_off[h] <= kSmallMax; };
     // host-side plan: padded slot offsets, per-slice partial-sum offsets, size order
     std::vector<int64_t> poff(nh + 1), qoff(nh + 1);
-    std::vector<int> order(nh);
+    std::vector<int> order;
+    order.reserve(nh);
     poff[0] = 0;
     qoff[0] = 0;
     int64_t segcap = 0;   // energy segments at most (initial sizes)
     std::vector<int> cstart(nh + 1), chunk_h;   // member chunks of kSeg (reduce and first pack)
+    std::vector<int> by_size(use_small ? kSmallMax + 2 : 0, 0);   // small haloes by size
     for (int h = 0; h < nh; ++h) {
         const int64_t c = h_off[h + 1] - h_off[h];
         cstart[h] = (int)chunk_h.size();
+        if (is_small(h)) {
+            poff[h + 1] = poff[h];
+            qoff[h + 1] = qoff[h];
+            ++by_size[kSmallMax - c + 1];
+            continue;
+        }
+        order.push_back(h);
         for (int64_t k = 0; k < (c + kSeg - 1) / kSeg; ++k) chunk_h.push_back(h);
         const int64_t npad = ((c + 31) / 32) * 32;
         int64_t nsl = std::max<int64_t>(1, (c + slice_len - 1) / slice_len);
@@ -1401,17 +1753,30 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
     cstart[nh] = (int)chunk_h.size();
     const int nchunks = (int)chunk_h.size();
     if (segcap >= (1ll << 31)) return fail(HALMA_ERR_CAPACITY, "too many energy segments");
-    std::iota(order.begin(), order.end(), 0);
+    const int nb_ = (int)order.size();
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
         return (h_off[a + 1] - h_off[a]) > (h_off[b + 1] - h_off[b]);
     });
+    // the small haloes follow in the same order (counting sort); their size classes are runs of it
+    constexpr int kClass[3] = {128, 256, kSmallMax};
+    int first[4] = {nb_, nb_, nb_, nb_};   // first[c]: first small halo of at most kClass[c] members
+    if (use_small) {
+        for (int k = 1; k <= kSmallMax + 1; ++k) by_size[k] += by_size[k - 1];
+        order.resize(nh);
+        for (int c = 0; c < 3; ++c) first[c] = nb_ + by_size[kSmallMax - kClass[c]];
+        first[3] = nb_;
+        for (int h = 0; h < nh; ++h)
+            if (is_small(h)) order[nb_ + by_size[kSmallMax - (h_off[h + 1] - h_off[h])]++] = h;
+    }
     const int64_t P = std::max<int64_t>(poff[nh], 32);
     const int64_t Q = std::max<int64_t>(qoff[nh], 32);
     Layout L;
     const size_t o_hs = L.add(sizeof(HaloState) * (size_t)std::max(nh, 1));
-    const size_t o_poff = L.add(sizeof(int64_t) * (nh + 1));
-    const size_t o_qoff = L.add(sizeof(int64_t) * (nh + 1));
-    const size_t o_order = L.add(sizeof(int) * std::max(nh, 1));
+    // the plan's arrays in one piece, uploaded by one copy
+    const size_t pl_poff = 0, pl_qoff = sizeof(int64_t) * (nh + 1), pl_cst = 2 * pl_qoff,
+                 pl_order = pl_cst + sizeof(int) * (nh + 1), pl_chh = pl_order + sizeof(int) * nh,
+                 pl_bytes = pl_chh + sizeof(int) * nchunks;
+    const size_t o_plan = L.add(pl_bytes);
     const size_t vsz = f64 ? sizeof(double4) : sizeof(float4);
     const size_t o_pk = L.add(vsz * P), o_pk2 = L.add(vsz * P);       // packed slots, double-buffered
     const size_t o_pidx = L.add(sizeof(int) * P), o_pidx2 = L.add(sizeof(int) * P);
@@ -1426,27 +1791,23 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
     const size_t o_pv = L.add(f64 ? 0 : sizeof(float4) * P), o_pv2 = L.add(f64 ? 0 : sizeof(float4) * P);
     const size_t o_sown = L.add(sizeof(int) * segcap);
     const size_t o_spre = L.add(sizeof(int2) * segcap);
-    const size_t o_cst = L.add(sizeof(int) * (nh + 1));
-    const size_t o_chh = L.add(sizeof(int) * std::max(nchunks, 1));
     const size_t o_rpart = L.add(sizeof(double) * kRedSums * std::max(nchunks, 1));
     const size_t o_cnt = L.add(64);
     const size_t o_pairs = L.add(sizeof(unsigned long long) * 2 * p.max_iter);
     const size_t o_ystart = L.add(sizeof(int) * (nh + 1));
     const size_t o_off = d_off ? 0 : L.add(sizeof(int64_t) * (nh + 1));
     const size_t o_icnt = L.add(sizeof(int4) * std::max(nh, 1)), o_ipre = L.add(sizeof(int4) * std::max(nh, 1));
-    const size_t iscan_bytes = exclusive_sum_int3_bytes(std::max(nh, 1));
+    const size_t iscan_bytes = exclusive_sum_int3_bytes(std::max(nb_, 1));
     const size_t o_iscan = L.add(iscan_bytes);
     void *base = nullptr;
     HALMA_TRY(workspace(L.total, &base, st));
     auto *hs = at<HaloState>(base, o_hs);
-    auto *dpoff = at<int64_t>(base, o_poff);
-    auto *dqoff = at<int64_t>(base, o_qoff);
-    auto *dorder = at<int>(base, o_order);
+    auto *dpoff = at<int64_t>(base, o_plan + pl_poff);
+    auto *dqoff = at<int64_t>(base, o_plan + pl_qoff);
+    auto *dorder = at<int>(base, o_plan + pl_order);
     int *pidxb[2] = {at<int>(base, o_pidx), at<int>(base, o_pidx2)};
     auto *keepf = at<unsigned char>(base, o_keep);
     auto *phic = at<double>(base, o_phic), *phin = at<double>(base, o_phin);
-    // incremental passes subtract the removed particles' potential instead of recomputing
-    const bool incremental = !(p.flags & HALMA_UNBIND_FULL_RECOMPUTE);
     auto *phi = at<double>(base, o_phi);
     auto *istart = at<int>(base, o_istart);
     auto *sstart = at<int>(base, o_sstart);
@@ -1454,8 +1815,8 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
     auto *ssum = at<double>(base, o_ssum);
     auto *sown = at<int>(base, o_sown);
     auto *segpre = at<int2>(base, o_spre);
-    auto *dcst = at<int>(base, o_cst);
-    auto *dchh = at<int>(base, o_chh);
+    auto *dcst = at<int>(base, o_plan + pl_cst);
+    auto *dchh = at<int>(base, o_plan + pl_chh);
     auto *rpart = at<double>(base, o_rpart);
     int *cnt = at<int>(base, o_cnt);   // [0] nitems [1] counter [2] energy segments
     const int sgrid = (int)segcap;
@@ -1473,23 +1834,26 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
         HALMA_CUDA(cudaMemcpyAsync(o, h_off, sizeof(int64_t) * (nh + 1), cudaMemcpyHostToDevice, st));
         off = o;
     }
-    HALMA_CUDA(cudaMemcpyAsync(dpoff, poff.data(), sizeof(int64_t) * (nh + 1), cudaMemcpyHostToDevice, st));
-    HALMA_CUDA(cudaMemcpyAsync(dqoff, qoff.data(), sizeof(int64_t) * (nh + 1), cudaMemcpyHostToDevice, st));
-    HALMA_CUDA(cudaMemcpyAsync(dorder, order.data(), sizeof(int) * nh, cudaMemcpyHostToDevice, st));
-    HALMA_CUDA(cudaMemcpyAsync(dcst, cstart.data(), sizeof(int) * (nh + 1), cudaMemcpyHostToDevice, st));
-    if (nchunks > 0)
-        HALMA_CUDA(cudaMemcpyAsync(dchh, chunk_h.data(), sizeof(int) * nchunks, cudaMemcpyHostToDevice, st));
-    const int fgrid = grid_for((int64_t)nh * 32, 256);   // one warp per halo
+    {
+        std::vector<unsigned char> plan(pl_bytes);
+        memcpy(plan.data() + pl_poff, poff.data(), sizeof(int64_t) * (nh + 1));
+        memcpy(plan.data() + pl_qoff, qoff.data(), sizeof(int64_t) * (nh + 1));
+        memcpy(plan.data() + pl_cst, cstart.data(), sizeof(int) * (nh + 1));
+        memcpy(plan.data() + pl_order, order.data(), sizeof(int) * nh);
+        memcpy(plan.data() + pl_chh, chunk_h.data(), sizeof(int) * nchunks);
+        HALMA_CUDA(cudaMemcpyAsync(dpoff, plan.data(), pl_bytes, cudaMemcpyHostToDevice, st));
+    }
+    const int fgrid = grid_for((int64_t)nb_ * 32, 256);   // one warp per halo
     // the pass's work list (count, scan, fill; see ub_items_count_kernel)
     auto *icount = at<int4>(base, o_icnt), *ipre = at<int4>(base, o_ipre);
     void *iscan_tmp = at<void>(base, o_iscan);
-    const int igrid = std::min(grid_for(nh, 256), device_sm_count() * 4);
+    const int igrid = std::min(grid_for(nb_, 256), device_sm_count() * 4);
     auto items = [&](cudaStream_t rs, int inc, int sym_ok, unsigned long long *pairs) -> int {
         if (pairs) HALMA_CUDA(cudaMemsetAsync(pairs, 0, 2 * sizeof(unsigned long long), rs));
-        HALMA_LAUNCH(ub_items_count_kernel, igrid, 256, 0, rs, nh, dorder, hs, tab, slice_len, inc, sym_ok, icount,
+        HALMA_LAUNCH(ub_items_count_kernel, igrid, 256, 0, rs, nb_, dorder, hs, tab, slice_len, inc, sym_ok, icount,
                      idesc, pairs);
-        HALMA_TRY(exclusive_sum_int3(iscan_tmp, iscan_bytes, icount, ipre, nh, rs));
-        HALMA_LAUNCH(ub_items_fill_kernel, igrid, 256, 0, rs, nh, icount, ipre, istart, ystart, sstart, sown, cnt);
+        HALMA_TRY(exclusive_sum_int3(iscan_tmp, iscan_bytes, icount, ipre, nb_, rs));
+        HALMA_LAUNCH(ub_items_fill_kernel, igrid, 256, 0, rs, nb_, icount, ipre, istart, ystart, sstart, sown, cnt);
         return HALMA_OK;
     };
     // FP64 bound mass, centre and bulk velocity per halo (active ones, or all with force);
@@ -1506,7 +1870,7 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                 HALMA_LAUNCH(ub_reduce_seg_kernel<0>, nchunks, kSegThreads, 0, rs, off, dcst, dchh, x, y, z, vx, vy,
                              vz, m, bound, hs, force, rpart);
         }
-        HALMA_LAUNCH(ub_reduce_fin_kernel, fgrid, 256, 0, rs, nh, dcst, rpart, force, hs);
+        HALMA_LAUNCH(ub_reduce_fin_kernel, fgrid, 256, 0, rs, nb_, dorder, dcst, rpart, force, hs);
         return HALMA_OK;
     };
     const double gfac = p.G * p.factor_v * p.factor_v;
@@ -1515,7 +1879,17 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                  n, bound, nh, hs);
     if (phi_out) HALMA_CUDA(cudaMemsetAsync(phi_out, 0, sizeof(double) * n, st));
 
-    if (!f64) {
+    auto small = [&]() -> int {
+        HALMA_TRY((launch_small<128, 128>(dorder + first[0], nh - first[0], off, x, y, z, vx, vy, vz, m, p, gfac, bound,
+                                          phi_out, hs, st)));
+        HALMA_TRY((launch_small<256, 256>(dorder + first[1], first[0] - first[1], off, x, y, z, vx, vy, vz, m, p, gfac,
+                                          bound, phi_out, hs, st)));
+        return launch_small<kSmallMax, 256>(dorder + first[2], first[1] - first[2], off, x, y, z, vx, vy, vz, m, p,
+                                            gfac, bound, phi_out, hs, st);
+    };
+    // velocities that may still be arriving: after the big haloes' first pass has waited for them
+    if (use_small && !vel_ready) HALMA_TRY(small());
+    if (!f64 && nb_ > 0) {
         float4 *pkb[2] = {at<float4>(base, o_pk), at<float4>(base, o_pk2)};
         float4 *pvb[2] = {at<float4>(base, o_pv), at<float4>(base, o_pv2)};
         auto *part2 = reinterpret_cast<float2 *>(phi);   // double-float partials and potentials
@@ -1558,10 +1932,10 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                 // full passes: the big haloes' block pairs first (the longest items), then the
                 // tiles of the small ones; incremental passes have only tiles
                 if (!inc)
-                    HALMA_LAUNCH(ub_pair_sym_kernel, ygrid, 128, kSymSmem, rs, pkb[a], dpoff, dqoff, hs, nh, ystart,
+                    HALMA_LAUNCH(ub_pair_sym_kernel, ygrid, 128, kSymSmem, rs, pkb[a], dpoff, dqoff, hs, nb_, ystart,
                                  idesc, cnt, cnt + 4, eps2, part2);
                 if (profiling) HALMA_CUDA(cudaEventRecordWithFlags(prof.evm[it], rs, cudaEventRecordExternal));
-                HALMA_LAUNCH(ub_pair_kernel, pgrid, 256, 0, rs, pkb[a], rk, inc, dpoff, dqoff, hs, nh, istart, idesc,
+                HALMA_LAUNCH(ub_pair_kernel, pgrid, 256, 0, rs, pkb[a], rk, inc, dpoff, dqoff, hs, nb_, istart, idesc,
                              cnt, cnt + 1, eps2, slice_len / 32, part2);
                 if (profiling) HALMA_CUDA(cudaEventRecordWithFlags(prof.ev1[it], rs, cudaEventRecordExternal));
                 if (it == 0 && vel_ready) {
@@ -1574,12 +1948,12 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                 HALMA_LAUNCH(ub_energy_df_kernel, egrid, kSegThreads, 0, rs, sstart, sown, idesc, cnt + 2, dpoff, dqoff,
                              inc, pidxb[a], pvb[a], part2, phin2, phic2, x, y, z, vx, vy, vz, m, gfac_f, hs, bound,
                              phi_out, keepf, sdf);
-                HALMA_LAUNCH(ub_finalize_df_kernel, fgrid, 256, 0, rs, nh, dorder, sstart, sdf, gfac, hs, segpre);
+                HALMA_LAUNCH(ub_finalize_df_kernel, fgrid, 256, 0, rs, nb_, dorder, sstart, sdf, gfac, hs, segpre);
                 HALMA_LAUNCH(ub_compact_df_kernel, cgrid, kSegThreads, 0, rs, sstart, sown, idesc, cnt + 2, dpoff, hs,
                              keepf, segpre, pkb[a], pvb[a], pidxb[a], phic2, pkb[b], pvb[b], pidxb[b], phin2, rk);
             }
             HALMA_CUDA(cudaMemsetAsync(cnt + 6, 0, sizeof(int), rs));
-            HALMA_LAUNCH(ub_active_kernel, std::min(grid_for(nh, 256), 64), 256, 0, rs, nh, hs, cnt + 6);
+            HALMA_LAUNCH(ub_active_kernel, std::min(grid_for(nb_, 256), 64), 256, 0, rs, nb_, dorder, hs, cnt + 6);
             return HALMA_OK;
         };
         int passes_run = p.max_iter;
@@ -1601,6 +1975,7 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
             key.push_back((uintptr_t)slice_len);
             key.push_back((uintptr_t)incremental);
             key.push_back((uintptr_t)nchunks);
+            key.push_back((uintptr_t)nb_);
             key.push_back((uintptr_t)vel_ready);
             for (int c = 0; c < tab.n; ++c) {
                 key.push_back((uintptr_t)tab.upper[c]);
@@ -1667,6 +2042,8 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                 prof.passes.push_back({(double)hp[2 * it], (double)ms, (double)hp[2 * it + 1], (double)sms});
             }
         }
+    } else if (!f64) {
+        if (profiling) prof.passes.clear();
     } else {
         // plain FP64 path: per pass, one pair launch per active halo, host checks convergence
         double4 *pkb[2] = {at<double4>(base, o_pk), at<double4>(base, o_pk2)};
@@ -1697,6 +2074,10 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                          hs, keepf, segpre, pkb[a], pidxb[a], phic, pkb[b], pidxb[b], phin, rk);
         }
         HALMA_TRY(reduce(st, 1));
+    }
+    if (use_small && vel_ready) {
+        HALMA_CUDA(cudaStreamWaitEvent(st, vel_ready, 0));
+        HALMA_TRY(small());
     }
     if (halo_out) HALMA_LAUNCH(ub_output_kernel, grid_for(nh, 256), 256, 0, st, nh, hs, halo_out);
     return HALMA_OK;

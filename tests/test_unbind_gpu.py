@@ -185,3 +185,36 @@ def test_device_tensors(catalogue, cuda):
     bound_h, halo_h, _ = unbind_batched(*_arrays(catalogue), UnbindOptions(eps=EPS, max_iter=50))
     assert np.array_equal(bound_d.cpu().numpy(), bound_h)
     assert np.array_equal(halo_d.cpu().numpy(), halo_h)
+
+
+def test_small_haloes_equal_the_pass_kernels(cuda):
+    """Haloes that run all passes in one block, at the sizes where its layout changes (warps, size classes,
+    slots a thread): bit for bit what the pass kernels give with the halo in one slice.  Source slices of
+    992 slots, below the block's limit, send every halo to the pass kernels."""
+    from pyhalma_gb300 import autotune
+    sizes = [0, 1, 2, 31, 32, 33, 63, 127, 128, 129, 255, 256, 257, 300, 511, 512, 513, 800, 991, 992]
+    cat = synth.powerlaw_catalogue(1, seed=12, n_min=sum(sizes), n_max=sum(sizes), contaminant_frac=0.15)
+    rng = np.random.default_rng(5)
+    perm = rng.permutation(sum(sizes))
+    cols = [np.ascontiguousarray(a[perm]) for a in (cat.x, cat.y, cat.z, cat.vx, cat.vy, cat.vz, cat.mass)]
+    cols[6] = cols[6] * rng.uniform(0.5, 2.0, sum(sizes))
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    for h in range(len(sizes)):   # shrunk with its mass, so that a halo loses members over several passes
+        sl = slice(off[h], off[h + 1])
+        for k in range(3):
+            c = cols[k][sl].mean() if sizes[h] else 0.0
+            cols[k][sl] = c + (cols[k][sl] - c) * (max(sizes[h], 1) / sum(sizes))
+    upper, t, slice_len = autotune.get_table()
+    assert slice_len >= 1024
+    for max_iter in (1, 2, 3, 30):
+        opt = UnbindOptions(eps=EPS, max_iter=max_iter)
+        got = unbind_batched(off, *cols, opt, want_phi=True)
+        try:
+            autotune.set_table(upper, t, 992)
+            want = unbind_batched(off, *cols, opt, want_phi=True)
+        finally:
+            autotune.set_table(upper, t, slice_len)
+        for g, w in zip(got, want):
+            np.testing.assert_array_equal(g, w)
+        if max_iter == 30:
+            assert len(set(got[1][:, 8])) > 3   # haloes of one, two, .. passes
