@@ -965,9 +965,12 @@ __device__ __forceinline__ void removed_sums(const int *list, int nrem, const do
         a[5] += mi * vy[i];
         a[6] += mi * vz[i];
     }
-    if (nrem > 0)
+    // the tree of warp_sum without the levels that add nothing but zeros
+    for (int o = 16; o > 0; o >>= 1) {
+        if (o >= nrem) continue;
 #pragma unroll
-        for (int k = 0; k < 7; ++k) a[k] = warp_sum(a[k]);
+        for (int k = 0; k < 7; ++k) a[k] += __shfl_down_sync(0xffffffffu, a[k], o);
+    }
 }
 
 // The halo's state after a pass that removed something: keep_run particles remain, a are the removed ones' sums.
@@ -1291,9 +1294,10 @@ struct SmallShared {
         };
     };
     double q4[kRedSums][4];
+    double centre[6];    // centre of mass and bulk velocity before the first pass
+    float w[3];          // current bulk velocity relative to that
     float2 se[2][THREADS / 32];
     int cnt[2][(P + THREADS - 1) / THREADS][THREADS / 32];
-    HaloState hs;
 };
 
 template <int P>
@@ -1364,6 +1368,9 @@ __global__ void __launch_bounds__(THREADS) ub_small_kernel(
     extern __shared__ __align__(16) unsigned char small_raw[];
     auto &sh = *reinterpret_cast<SmallShared<P, THREADS> *>(small_raw);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // the size classes' launches are independent: the next may start as soon as this one's blocks all run, and
+    // ends after it (the wait below), so that what follows in the stream follows all of them
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int h = list[blockIdx.x];
     const int64_t b = off[h];
     const int n = (int)(off[h + 1] - b);
@@ -1405,30 +1412,22 @@ __global__ void __launch_bounds__(THREADS) ub_small_kernel(
         sh.q4[k][run] = t;
     }
     __syncthreads();
-    if (threadIdx.x < kRedSums - 1) {
-        const int k = threadIdx.x;
-        sh.q4[k][0] = ((sh.q4[k][0] + sh.q4[k][1]) + sh.q4[k][2]) + sh.q4[k][3];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        HaloState s{};
-        const double M = sh.q4[0][0];
-        s.M = M;
-        s.nb = n;
-        s.sx = sh.q4[1][0]; s.sy = sh.q4[2][0]; s.sz = sh.q4[3][0];
-        s.px = sh.q4[4][0]; s.py = sh.q4[5][0]; s.pz = sh.q4[6][0];
-        if (M > 0) {
-            s.cx = s.sx / M; s.cy = s.sy / M; s.cz = s.sz / M;
-            s.vx = s.px / M; s.vy = s.py / M; s.vz = s.pz / M;
-        }
-        s.v0x = s.vx; s.v0y = s.vy; s.v0z = s.vz;
-        sh.hs = s;
+    // Warp 0 keeps the halo's sums, one a lane (0: M, 1..3: m x, 4..6: m v), so that a division or a subtraction is one
+    // FP64 instruction for all of them: this GPU's FP64 pipe takes 16 cycles an instruction, and seven lanes cost
+    // what one does.
+    double val = 0.0, v0 = 0.0;
+    auto per_mass = [&](double M) { return M > 0 ? val / M : 0.0; };
+    if (w == 0) {
+        if (lane < kRedSums - 1) val = ((sh.q4[lane][0] + sh.q4[lane][1]) + sh.q4[lane][2]) + sh.q4[lane][3];
+        v0 = per_mass(__shfl_sync(0xffffffffu, val, 0));
+        if (lane >= 1 && lane < 7) sh.centre[lane - 1] = v0;
+        if (lane < 3) sh.w[lane] = 0.f;
     }
     __syncthreads();
     // ---- packing (ub_pack_kernel)
     {
-        const double cx = sh.hs.cx, cy = sh.hs.cy, cz = sh.hs.cz;
-        const double v0x = sh.hs.v0x, v0y = sh.hs.v0y, v0z = sh.hs.v0z;
+        const double cx = sh.centre[0], cy = sh.centre[1], cz = sh.centre[2];
+        const double v0x = sh.centre[3], v0y = sh.centre[4], v0z = sh.centre[5];
 #pragma unroll
         for (int j = 0; j < J; ++j) {
             const int r = j * THREADS + threadIdx.x;
@@ -1444,7 +1443,8 @@ __global__ void __launch_bounds__(THREADS) ub_small_kernel(
         }
     }
     __syncthreads();
-    int nb = n, nrem = 0;
+    int nb = n, nrem = 0, iter = 0;
+    double ekin = 0.0, epot = 0.0;   // lane 0 of warp 0
     for (int it = 0; it < max_iter; ++it) {
         // ---- pair terms
         const bool inc = it > 0;
@@ -1459,7 +1459,7 @@ __global__ void __launch_bounds__(THREADS) ub_small_kernel(
         }
         __syncthreads();
         // ---- energies and the cut (ub_energy_df_kernel)
-        const float wx = sh.hs.wx, wy = sh.hs.wy, wz = sh.hs.wz;
+        const float wx = sh.w[0], wy = sh.w[1], wz = sh.w[2];
         float ek_s = 0.f, ek_c = 0.f, ep_s = 0.f, ep_c = 0.f;
         float4 u[J], pos[J];
         float2 ph[J];
@@ -1532,20 +1532,29 @@ __global__ void __launch_bounds__(THREADS) ub_small_kernel(
         }
         __syncthreads();
         // ---- energies of the pass, and the next pass's mass and bulk velocity (ub_finalize_df_kernel)
+        ++iter;
+        const bool last = gone == 0 || it + 1 == max_iter;
         if (w == 0) {
-            double a[7];
-            removed_sums(sh.rlist, gone, x, y, z, vx, vy, vz, m, lane, a);
-            if (lane == 0) {
+            if (gone > 0) {   // subtract_removed, a lane per sum; the centre is formed after the last pass
+                double a[7], mine = 0.0;
+                removed_sums(sh.rlist, gone, x, y, z, vx, vy, vz, m, lane, a);
+#pragma unroll
+                for (int k = 0; k < 7; ++k) {
+                    const double t = __shfl_sync(0xffffffffu, a[k], 0);
+                    if (lane == k) mine = t;
+                }
+                val = kept == 0 ? 0.0 : val - mine;
+                const double v = per_mass(__shfl_sync(0xffffffffu, val, 0));
+                if (lane >= 4 && lane < 7) sh.w[lane - 4] = (float)(v - v0);
+            }
+            if (last && lane == 0) {   // the energies of the last pass are the halo's
                 float2 e0 = make_float2(0.f, 0.f), e1 = make_float2(0.f, 0.f);
                 for (int k = 0; k < W; ++k) {
                     e0 = df_add(e0, sh.se[0][k]);
                     e1 = df_add(e1, sh.se[1][k]);
                 }
-                HaloState &o = sh.hs;
-                o.iter += 1;
-                o.ekin = df_to_double(df_add(make_float2(0.f, 0.f), e0));
-                o.epot = -0.5 * gfac * df_to_double(df_add(make_float2(0.f, 0.f), e1));
-                if (gone > 0) subtract_removed(o, kept, a);
+                ekin = df_to_double(df_add(make_float2(0.f, 0.f), e0));
+                epot = -0.5 * gfac * df_to_double(df_add(make_float2(0.f, 0.f), e1));
             }
         }
         nb = kept;
@@ -1556,7 +1565,19 @@ __global__ void __launch_bounds__(THREADS) ub_small_kernel(
     __syncthreads();
     if (phi_out)
         for (int r = threadIdx.x; r < nb; r += THREADS) phi_out[sh.idx[r]] = df_to_double(sh.phi[r]);
-    if (threadIdx.x == 0) hs[h] = sh.hs;   // active = 0
+    if (w == 0) {
+        const double v = per_mass(__shfl_sync(0xffffffffu, val, 0));
+        HaloState o{};   // what ub_output_kernel reads
+        o.M = __shfl_sync(0xffffffffu, val, 0);
+        o.cx = __shfl_sync(0xffffffffu, v, 1); o.cy = __shfl_sync(0xffffffffu, v, 2); o.cz = __shfl_sync(0xffffffffu, v, 3);
+        o.vx = __shfl_sync(0xffffffffu, v, 4); o.vy = __shfl_sync(0xffffffffu, v, 5); o.vz = __shfl_sync(0xffffffffu, v, 6);
+        o.nb = nb;
+        o.iter = iter;
+        o.ekin = ekin;
+        o.epot = epot;
+        if (lane == 0) hs[h] = o;
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Plain FP64 pair kernel for one halo (targets = sources = its packed slots).
@@ -1699,12 +1720,23 @@ template <int P, int THREADS>
 static int launch_small(const int *list, int count, const int64_t *off, const double *x, const double *y,
                         const double *z, const double *vx, const double *vy, const double *vz, const double *m,
                         const halma_unbind_params &p, double gfac, unsigned char *bound, double *phi_out, HaloState *hs,
-                        cudaStream_t st) {
+                        bool beside_last, cudaStream_t st) {
     if (count <= 0) return HALMA_OK;
     constexpr int smem = (int)sizeof(SmallShared<P, THREADS>);
     HALMA_CUDA(cudaFuncSetAttribute(ub_small_kernel<P, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    HALMA_LAUNCH((ub_small_kernel<P, THREADS>), count, THREADS, smem, st, list, off, x, y, z, vx, vy, vz, m,
-                 (float)(p.eps * p.eps), gfac, p.max_iter, bound, phi_out, hs);
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)count);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = beside_last ? 1 : 0;
+    HALMA_CUDA(cudaLaunchKernelEx(&cfg, ub_small_kernel<P, THREADS>, list, off, x, y, z, vx, vy, vz, m,
+                                  (float)(p.eps * p.eps), gfac, p.max_iter, bound, phi_out, hs));
+    count_launch();
     return HALMA_OK;
 }
 
@@ -1879,13 +1911,14 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                  n, bound, nh, hs);
     if (phi_out) HALMA_CUDA(cudaMemsetAsync(phi_out, 0, sizeof(double) * n, st));
 
+    // the longest blocks first; each class may start beside the one launched before it
     auto small = [&]() -> int {
-        HALMA_TRY((launch_small<128, 128>(dorder + first[0], nh - first[0], off, x, y, z, vx, vy, vz, m, p, gfac, bound,
-                                          phi_out, hs, st)));
+        HALMA_TRY((launch_small<kSmallMax, 256>(dorder + first[2], first[1] - first[2], off, x, y, z, vx, vy, vz, m, p,
+                                                gfac, bound, phi_out, hs, false, st)));
         HALMA_TRY((launch_small<256, 256>(dorder + first[1], first[0] - first[1], off, x, y, z, vx, vy, vz, m, p, gfac,
-                                          bound, phi_out, hs, st)));
-        return launch_small<kSmallMax, 256>(dorder + first[2], first[1] - first[2], off, x, y, z, vx, vy, vz, m, p,
-                                            gfac, bound, phi_out, hs, st);
+                                          bound, phi_out, hs, first[1] > first[2], st)));
+        return launch_small<128, 128>(dorder + first[0], nh - first[0], off, x, y, z, vx, vy, vz, m, p, gfac, bound,
+                                      phi_out, hs, first[0] > first[2], st);
     };
     // velocities that may still be arriving: after the big haloes' first pass has waited for them
     if (use_small && !vel_ready) HALMA_TRY(small());
