@@ -185,11 +185,14 @@ constexpr int kTile = 1024;
 // Block per group: the FP32 inertia tensor in particle order (f90:183-200), its
 // normalisation, Jacobi, the decreasing sort (f90:129-157) and the square roots.  Members
 // are staged in shared memory a tile at a time; the nine tensor sums and the mass sum are
-// independent chains, so threads 0..9 each add one of them in member order.
+// independent chains, so threads 0..9 each add one of them in member order.  A chain is bound by its additions
+// (4 cycles each): the eight products of a step are formed before they are added (one at a time, 26 cycles a
+// member, the group of 19,500 members took 248 us).  Tiles are padded with zero masses, whose terms leave a
+// sum that starts at +0 as it is.
 __global__ void __launch_bounds__(256) pr_shape_kernel(int G, const int64_t *__restrict__ off,
                                                        const double *__restrict__ g, int64_t nm,
                                                        const double *__restrict__ cen, double *__restrict__ out) {
-    __shared__ float sr[4][kTile];   // x, y, z relative to the centre (FP32), mass
+    __shared__ __align__(16) float sr[4][kTile];   // x, y, z relative to the centre (FP32), mass
     __shared__ float acc[10];
     for (int h = blockIdx.x; h < G; h += gridDim.x) {
         const double *c = cen + (int64_t)h * kCenFields;
@@ -204,12 +207,18 @@ __global__ void __launch_bounds__(256) pr_shape_kernel(int G, const int64_t *__r
                 sr[2][q] = (float)__dsub_rn(g[2 * nm + k], c[2]);
                 sr[3][q] = (float)g[6 * nm + k];
             }
+            if (t < 8 && cnt + t < ((cnt + 7) & ~7)) sr[0][cnt + t] = sr[1][cnt + t] = sr[2][cnt + t] = sr[3][cnt + t] = 0.f;
             __syncthreads();
-            if (t < 9) {
-                const int i = t % 3, j = t / 3;
-                for (int q = 0; q < cnt; ++q) a = __fadd_rn(a, __fmul_rn(__fmul_rn(sr[3][q], sr[i][q]), sr[j][q]));
-            } else if (t == 9) {
-                for (int q = 0; q < cnt; ++q) a = __fadd_rn(a, sr[3][q]);
+            if (t < 10) {
+                const float *ri = sr[t % 3], *rj = sr[(t / 3) % 3];
+                for (int q = 0; q < cnt; q += 8) {
+                    float p[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        p[u] = t < 9 ? __fmul_rn(__fmul_rn(sr[3][q + u], ri[q + u]), rj[q + u]) : sr[3][q + u];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) a = __fadd_rn(a, p[u]);
+                }
             }
             __syncthreads();
         }
@@ -317,7 +326,8 @@ __global__ void __launch_bounds__(256) pr_kin1_kernel(int G, int S, const int64_
 }
 
 // Phase 2: kappa_co (kinematic_morphology, halo_properties.py:483-517) and the Tully-Fisher
-// shell velocity (tully_fisher_velocity, :63-96); the last block writes the group's outputs.
+// shell velocity (tully_fisher_velocity, :63-96); the last block writes the group's outputs.  Bound: the FP64 pipe
+// (two square roots and a division fewer a member took it from 209 to 120 us at 4e5 members).
 __global__ void __launch_bounds__(256) pr_kin2_kernel(int G, int S, const int64_t *__restrict__ off,
                                                       const double *__restrict__ g, int64_t nm,
                                                       const double *__restrict__ cen, double *__restrict__ out,
@@ -334,6 +344,7 @@ __global__ void __launch_bounds__(256) pr_kin2_kernel(int G, int S, const int64_
     const double r05 = o[HALMA_PROP_R05];
     const double *jv = jvec + (int64_t)h * 8;
     const double ex = jv[4], ey = jv[5], ez = jv[6];
+    const double shell_lo = 0.81 * (1.0 - 1e-12) * r05 * r05, shell_hi = 1.21 * (1.0 + 1e-12) * r05 * r05;
     double s[4] = {0, 0, 0, 0};   // kin_corot, kin_total, v_TF, mass in the shell
     for (int64_t k = b + threadIdx.x; k < e; k += blockDim.x) {
         const double rx = g[k] - c[0], ry = g[nm + k] - c[1], rz = g[2 * nm + k] - c[2];
@@ -344,12 +355,12 @@ __global__ void __launch_bounds__(256) pr_kin2_kernel(int G, int S, const int64_
         const double lz = llx * ex + lly * ey + llz * ez;
         const double zi = rx * ex + ry * ey + rz * ez;
         const double r2 = rx * rx + ry * ry + rz * rz;
-        const double R = sqrt(r2 - zi * zi);
+        const double R2 = r2 - zi * zi;
         s[1] += 0.5 * mk * (vvx * vvx + vvy * vvy + vvz * vvz);
-        if (lz > 0.0) {
-            const double q = lz / (mk * R);
-            s[0] += 0.5 * mk * q * q;
-        }
+        // 1/2 m (lz / (m R))^2 without the root (NaN, as there, where rounding leaves R^2 negative)
+        if (lz > 0.0) s[0] += R2 < 0.0 ? NAN : 0.5 * (lz * lz) / (mk * R2);
+        // the shell's bounds on squares, with a margin that the roots then decide
+        if (!(r2 > shell_lo && r2 < shell_hi)) continue;
         const double dist = sqrt(r2);
         if (0.9 * r05 < dist && dist < 1.1 * r05) {
             // R_ip = r - (r.u)u, u_R = R_ip/|R_ip|, v_rot = v - (v.u)u - (v.u_R)u_R
@@ -479,19 +490,21 @@ __global__ void pr_cells_kernel(int ncell, int64_t nm, const int *__restrict__ r
         float sd = 0.f, vc = 0.f;
         for (int k0 = b; k0 < e; k0 += 32) {
             const int k = k0 + lane;
-            float v = 0.f, m = 0.f;
+            float vm = 0.f, m = 0.f;
             if (k < e) {
                 const int mk = vals[k] - a * (int)nm;
                 const double *o = out + (int64_t)owner[mk] * HALMA_PROP_NFIELDS;
-                v = (float)__dsub_rn(g[(3 + a) * nm + mk], o[HALMA_PROP_VX + a]);
                 m = (float)g[6 * nm + mk];
+                vm = __fmul_rn((float)__dsub_rn(g[(3 + a) * nm + mk], o[HALMA_PROP_VX + a]), m);
                 rid[vals[k]] = (int)r;
             }
             const int cnt = e - k0 < 32 ? e - k0 : 32;
-            for (int t = 0; t < cnt; ++t) {
-                const float vt = __shfl_sync(0xffffffffu, v, t), mt = __shfl_sync(0xffffffffu, m, t);
-                vc = __fadd_rn(vc, __fmul_rn(vt, mt));
-                sd = __fadd_rn(sd, mt);
+            for (int t0 = 0; t0 < cnt; t0 += 8) {   // lanes past the end hold zeros, which change neither sum
+#pragma unroll
+                for (int t = 0; t < 8; ++t) {
+                    vc = __fadd_rn(vc, __shfl_sync(0xffffffffu, vm, t0 + t));
+                    sd = __fadd_rn(sd, __shfl_sync(0xffffffffu, m, t0 + t));
+                }
             }
         }
         if (sd != 0.f) vc = __fdiv_rn(vc, sd);
@@ -506,7 +519,9 @@ __global__ void pr_cells_kernel(int ncell, int64_t nm, const int *__restrict__ r
                 d2 = __fmul_rn(d, d);
             }
             const int cnt = e - k0 < 32 ? e - k0 : 32;
-            for (int t = 0; t < cnt; ++t) s2 = __fadd_rn(s2, __shfl_sync(0xffffffffu, d2, t));
+            for (int t0 = 0; t0 < cnt; t0 += 8)
+#pragma unroll
+                for (int t = 0; t < 8; ++t) s2 = __fadd_rn(s2, __shfl_sync(0xffffffffu, d2, t0 + t));
         }
         if (lane == 0) {
             cellv[r] = make_float4(sd, vc, __fsqrt_rn(__fdiv_rn(s2, (float)(e - b))), 0.f);
@@ -560,13 +575,21 @@ __global__ void __launch_bounds__(256) pr_proj_kernel(int G, int64_t nm, const i
                 for (int a = 0; a < 3; ++a)
                     term[a][q] = __fsqrt_rn(d2[a]) < r05[a] ? cellv[rid[a * nm + k]].z : -1.f;
             }
+            if (t < 8 && nt + t < ((nt + 7) & ~7)) term[0][nt + t] = term[1][nt + t] = term[2][nt + t] = -1.f;
             __syncthreads();
-            if (t < 3)
-                for (int q = 0; q < nt; ++q)
-                    if (term[t][q] >= 0.f) {
-                        s05 = __fadd_rn(s05, term[t][q]);
-                        cnt += 1;
+            if (t < 3)   // eight loads ahead of their additions; an excluded term adds +0, which changes nothing
+                for (int q = 0; q < nt; q += 8) {
+                    float p[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        p[u] = term[t][q + u];
+                        const bool in = p[u] >= 0.f;
+                        p[u] = in ? p[u] : 0.f;
+                        cnt += in ? 1 : 0;
                     }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) s05 = __fadd_rn(s05, p[u]);
+                }
             __syncthreads();
         }
         if (t < 3) red[t] = cnt > 0 ? __fdiv_rn(s05, (float)cnt) : s05;
@@ -611,10 +634,16 @@ __global__ void __launch_bounds__(256) pr_proj_kernel(int G, int64_t nm, const i
                     term[3][q] = __fmul_rn(__fmul_rn(cv.x, rbin),
                                            __fsqrt_rn(__fadd_rn(__fmul_rn(cv.y, cv.y), __fmul_rn(cv.z, cv.z))));
                 }
+                if (t < 8 && nt + t < ((nt + 7) & ~7)) term[0][nt + t] = -1.f;
                 __syncthreads();
                 if (t < 4)
-                    for (int q = 0; q < nt; ++q)
-                        if (term[0][q] >= 0.f) sum = __fadd_rn(sum, term[t][q]);
+                    for (int q = 0; q < nt; q += 8) {
+                        float p[8];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) p[u] = term[0][q + u] >= 0.f ? term[t][q + u] : 0.f;
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) sum = __fadd_rn(sum, p[u]);
+                    }
                 __syncthreads();
             }
             if (t < 4) red[3 + t] = sum;
@@ -664,6 +693,19 @@ __global__ void pr_proj_out_kernel(int G, const float *__restrict__ res, double 
     }
 }
 
+// A small array of the caller's on the host; host memory without a call to the driver.
+int to_host(void *dst, const void *src, size_t bytes) {
+    if (is_device_pointer(src)) HALMA_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost));
+    else memcpy(dst, src, bytes);
+    return HALMA_OK;
+}
+
+// off4[s * G + h] = s * nm + off[h] for four sets of the same members.
+__global__ void pr_off4_kernel(int G, int64_t nm, const int64_t *__restrict__ off, int64_t *__restrict__ off4) {
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k <= 4ll * G; k += (int64_t)gridDim.x * blockDim.x)
+        off4[k] = k == 4ll * G ? 4 * nm : (k / G) * nm + off[k % G];
+}
+
 int nbits(uint64_t v) {
     int b = 0;
     while (b < 64 && (v >> b) != 0) ++b;
@@ -690,14 +732,14 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
     if (n_groups == 0) return HALMA_OK;
     const int G = (int)n_groups;
     std::vector<int64_t> h_off(G + 1);
-    HALMA_CUDA(cudaMemcpy(h_off.data(), group_offsets, 8ull * (G + 1), cudaMemcpyDefault));
+    HALMA_TRY(to_host(h_off.data(), group_offsets, 8ull * (G + 1)));
     if (h_off[0] != 0) return fail(HALMA_ERR_INVALID, "group offsets must start at 0");
     for (int h = 0; h < G; ++h)
         if (h_off[h + 1] < h_off[h]) return fail(HALMA_ERR_INVALID, "group offsets must not decrease");
     const int64_t N0 = h_off[G];
     if (3 * N0 >= INT32_MAX) return fail(HALMA_ERR_CAPACITY, "at most (2^31-2)/3 members");
     std::vector<double> hc(5ull * G);
-    HALMA_CUDA(cudaMemcpy(hc.data(), centre, 40ull * G, cudaMemcpyDefault));
+    HALMA_TRY(to_host(hc.data(), centre, 40ull * G));
     double rmax = 0.0;
     for (int h = 0; h < G; ++h) {
         for (int q = 0; q < 5; ++q)
@@ -730,8 +772,11 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
     sg.add(centre, 5 * n_groups, true, false, &dcen);
     sg.add((const double *)out, n_groups * HALMA_PROP_NFIELDS, false, true, &dout);
     const int64_t NM = std::max<int64_t>(N0, 1), N3 = 3 * NM;
+    // the four half-mass reductions in one run, up to 2^25 members (5 GB of scratch), else one after another
+    const bool sets = N0 > 0 && N0 <= (1 << 25) && G <= (1 << 25);
     Layout L;
     sg.plan(L);
+    const size_t o_off4 = L.add(sets ? 8ull * (4ull * G + 1) : 8);
     const size_t o_g = L.add(64ull * NM), o_ab = L.add(8ull * 4 * G * HALMA_ABOUT_NFIELDS);
     const size_t o_red = L.add(8ull * 4 * G * HALMA_RED_NFIELDS), o_own = L.add(4ull * NM);
     const size_t o_kin = L.add(8ull * N3), o_kout = L.add(8ull * N3), o_vin = L.add(4ull * (N3 + 1)),
@@ -768,8 +813,9 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
             HALMA_CUDA(cudaMemcpy(hm.data(), group_members, 4ull * N0, cudaMemcpyDeviceToHost));
             mp = hm.data();
         }
-        for (int64_t k = 0; k < N0; ++k)
-            if (mp[k] < 0 || mp[k] >= n) return fail(HALMA_ERR_INVALID, "group member outside [0, n)");
+        bool outside = false;   // no early way out: the loop is a vector loop
+        for (int64_t k = 0; k < N0; ++k) outside |= (uint32_t)mp[k] >= (uint32_t)n;
+        if (outside) return fail(HALMA_ERR_INVALID, "group member outside [0, n)");
     }
     HALMA_CUDA(cudaMemsetAsync(dout, 0, 8ull * G * HALMA_PROP_NFIELDS, st));
     HALMA_LAUNCH(pr_gather_kernel, gN, 256, 0, st, N0, dmem, dx, dy, dz, dvx, dvy, dvz, dm, gbuf);
@@ -779,10 +825,16 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
     const double *gx = gbuf, *gy = gbuf + NM, *gz = gbuf + 2 * NM, *gvx = gbuf + 3 * NM, *gvy = gbuf + 4 * NM,
                  *gvz = gbuf + 5 * NM, *gm = gbuf + 6 * NM, *g0 = gbuf + 7 * NM;
     const double *pos[4][3] = {{gx, gy, gz}, {gy, gz, g0}, {gx, gz, g0}, {gx, gy, g0}};
-    for (int r = 0; r < 4; ++r)
-        HALMA_TRY(reductions_device(N0, G, doff, pos[r][0], pos[r][1], pos[r][2], gvx, gvy, gvz, gm, nullptr,
-                                    about + (int64_t)r * G * HALMA_ABOUT_NFIELDS,
-                                    red + (int64_t)r * G * HALMA_RED_NFIELDS, st));
+    if (sets) {
+        int64_t *off4 = at<int64_t>(base, o_off4);
+        HALMA_LAUNCH(pr_off4_kernel, grid_for(4ll * G + 1, 256, sms * 8), 256, 0, st, G, N0, doff, off4);
+        HALMA_TRY(reductions_sets_device(N0, G, off4, pos, gvx, gvy, gvz, gm, about, red, st));
+    } else {
+        for (int r = 0; r < 4; ++r)
+            HALMA_TRY(reductions_device(N0, G, doff, pos[r][0], pos[r][1], pos[r][2], gvx, gvy, gvz, gm, nullptr,
+                                        about + (int64_t)r * G * HALMA_ABOUT_NFIELDS,
+                                        red + (int64_t)r * G * HALMA_RED_NFIELDS, st));
+    }
     HALMA_LAUNCH(pr_r05_kernel, gH, 128, 0, st, G, red, dout, res);
     HALMA_CUDA(cudaMemsetAsync(kctr, 0, 4ull * G, st));
     HALMA_LAUNCH(pr_kin1_kernel, G * S, 256, 0, st, G, S, doff, gbuf, NM, dcen, dout, kpart, kctr, jvec);
