@@ -22,6 +22,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <map>
 #include <vector>
 
 #include "common.cuh"
@@ -192,30 +193,39 @@ constexpr int kTile = 1024;
 __global__ void __launch_bounds__(256) pr_shape_kernel(int G, const int64_t *__restrict__ off,
                                                        const double *__restrict__ g, int64_t nm,
                                                        const double *__restrict__ cen, double *__restrict__ out) {
-    __shared__ __align__(16) float sr[4][kTile];   // x, y, z relative to the centre (FP32), mass
+    constexpr int kRow = kTile + 8;   // rows start in different banks
+    __shared__ float sr[2][4][kRow];  // x, y, z relative to the centre (FP32), mass; one tile filled while the other is added
     __shared__ float acc[10];
     for (int h = blockIdx.x; h < G; h += gridDim.x) {
         const double *c = cen + (int64_t)h * kCenFields;
         const int t = threadIdx.x;
         float a = 0.f;   // thread t < 9: it[t % 3][t / 3]; thread 9: mass
-        for (int64_t b = off[h]; b < off[h + 1]; b += kTile) {
+        auto fill = [&](int64_t b, float (*to)[kRow], int first, int step) {
             const int cnt = (off[h + 1] - b < kTile ? (int)(off[h + 1] - b) : kTile);
-            for (int q = t; q < cnt; q += blockDim.x) {
+            for (int q = first; q < ((cnt + 7) & ~7); q += step) {
                 const int64_t k = b + q;
-                sr[0][q] = (float)__dsub_rn(g[k], c[0]);
-                sr[1][q] = (float)__dsub_rn(g[nm + k], c[1]);
-                sr[2][q] = (float)__dsub_rn(g[2 * nm + k], c[2]);
-                sr[3][q] = (float)g[6 * nm + k];
+                const bool in = q < cnt;
+                to[0][q] = in ? (float)__dsub_rn(g[k], c[0]) : 0.f;
+                to[1][q] = in ? (float)__dsub_rn(g[nm + k], c[1]) : 0.f;
+                to[2][q] = in ? (float)__dsub_rn(g[2 * nm + k], c[2]) : 0.f;
+                to[3][q] = in ? (float)g[6 * nm + k] : 0.f;
             }
-            if (t < 8 && cnt + t < ((cnt + 7) & ~7)) sr[0][cnt + t] = sr[1][cnt + t] = sr[2][cnt + t] = sr[3][cnt + t] = 0.f;
-            __syncthreads();
-            if (t < 10) {
-                const float *ri = sr[t % 3], *rj = sr[(t / 3) % 3];
+        };
+        fill(off[h], sr[0], t, blockDim.x);
+        __syncthreads();
+        int cur = 0;
+        for (int64_t b = off[h]; b < off[h + 1]; b += kTile, cur ^= 1) {
+            const int cnt = (off[h + 1] - b < kTile ? (int)(off[h + 1] - b) : kTile);
+            if (t >= 32) {
+                if (b + kTile < off[h + 1]) fill(b + kTile, sr[cur ^ 1], t - 32, blockDim.x - 32);
+            } else if (t < 10) {
+                // thread 9 adds m * 1 * 1
+                const float *rm = sr[cur][3], *ri = sr[cur][t % 3], *rj = sr[cur][(t / 3) % 3];
                 for (int q = 0; q < cnt; q += 8) {
                     float p[8];
 #pragma unroll
                     for (int u = 0; u < 8; ++u)
-                        p[u] = t < 9 ? __fmul_rn(__fmul_rn(sr[3][q + u], ri[q + u]), rj[q + u]) : sr[3][q + u];
+                        p[u] = __fmul_rn(__fmul_rn(rm[q + u], t < 9 ? ri[q + u] : 1.f), t < 9 ? rj[q + u] : 1.f);
 #pragma unroll
                     for (int u = 0; u < 8; ++u) a = __fadd_rn(a, p[u]);
                 }
@@ -256,9 +266,9 @@ __global__ void __launch_bounds__(256) pr_shape_kernel(int G, const int64_t *__r
 // Tully-Fisher velocity about it.
 // A group's members are split over up to S blocks of at least kKinMin (the FP64 work per member
 // is heavy and GB300's FP64 pipe is narrow, so one block per group would leave the biggest
-// group's SM as the critical path); each block writes partial sums and the last block of the
+// group's SM as the critical path; parts of 2,048 still left two blocks on some SMs and one on others); each block writes partial sums and the last block of the
 // group to finish (a per-group counter, no waiting) adds them in block order.
-constexpr int kKinMin = 2048;
+constexpr int kKinMin = 512;
 
 __device__ __forceinline__ bool kin_part_of(int bid, int S, int G, const int64_t *__restrict__ off, int &h, int &sh,
                                             int64_t &b, int64_t &e) {
@@ -346,33 +356,57 @@ __global__ void __launch_bounds__(256) pr_kin2_kernel(int G, int S, const int64_
     const double ex = jv[4], ey = jv[5], ez = jv[6];
     const double shell_lo = 0.81 * (1.0 - 1e-12) * r05 * r05, shell_hi = 1.21 * (1.0 + 1e-12) * r05 * r05;
     double s[4] = {0, 0, 0, 0};   // kin_corot, kin_total, v_TF, mass in the shell
-    for (int64_t k = b + threadIdx.x; k < e; k += blockDim.x) {
+    __shared__ int64_t list[8][64];   // per warp: members that may lie in the shell
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // v_rot of one member of the shell 0.9..1.1 R05
+    auto shell = [&](int64_t k) {
         const double rx = g[k] - c[0], ry = g[nm + k] - c[1], rz = g[2 * nm + k] - c[2];
+        const double dist = sqrt(rx * rx + ry * ry + rz * rz);
+        if (!(0.9 * r05 < dist && dist < 1.1 * r05)) return;
         const double vvx = g[3 * nm + k] - ux, vvy = g[4 * nm + k] - uy, vvz = g[5 * nm + k] - uz;
         const double mk = g[6 * nm + k];
-        const double llx = mk * (ry * vvz - rz * vvy), lly = mk * (rz * vvx - rx * vvz),
-                     llz = mk * (rx * vvy - ry * vvx);
-        const double lz = llx * ex + lly * ey + llz * ez;
         const double zi = rx * ex + ry * ey + rz * ez;
-        const double r2 = rx * rx + ry * ry + rz * rz;
-        const double R2 = r2 - zi * zi;
-        s[1] += 0.5 * mk * (vvx * vvx + vvy * vvy + vvz * vvz);
-        // 1/2 m (lz / (m R))^2 without the root (NaN, as there, where rounding leaves R^2 negative)
-        if (lz > 0.0) s[0] += R2 < 0.0 ? NAN : 0.5 * (lz * lz) / (mk * R2);
-        // the shell's bounds on squares, with a margin that the roots then decide
-        if (!(r2 > shell_lo && r2 < shell_hi)) continue;
-        const double dist = sqrt(r2);
-        if (0.9 * r05 < dist && dist < 1.1 * r05) {
-            // R_ip = r - (r.u)u, u_R = R_ip/|R_ip|, v_rot = v - (v.u)u - (v.u_R)u_R
-            const double Rx = rx - zi * ex, Ry = ry - zi * ey, Rz = rz - zi * ez;
-            const double Rn = sqrt(Rx * Rx + Ry * Ry + Rz * Rz);
-            const double qx = Rx / Rn, qy = Ry / Rn, qz = Rz / Rn;
-            const double vu = vvx * ex + vvy * ey + vvz * ez, vq = vvx * qx + vvy * qy + vvz * qz;
-            const double wx = vvx - vu * ex - vq * qx, wy = vvy - vu * ey - vq * qy, wz = vvz - vu * ez - vq * qz;
-            s[2] += sqrt(wx * wx + wy * wy + wz * wz) * mk;
-            s[3] += mk;
+        // R_ip = r - (r.u)u, u_R = R_ip/|R_ip|, v_rot = v - (v.u)u - (v.u_R)u_R
+        const double Rx = rx - zi * ex, Ry = ry - zi * ey, Rz = rz - zi * ez;
+        const double Rn = sqrt(Rx * Rx + Ry * Ry + Rz * Rz);
+        const double qx = Rx / Rn, qy = Ry / Rn, qz = Rz / Rn;
+        const double vu = vvx * ex + vvy * ey + vvz * ez, vq = vvx * qx + vvy * qy + vvz * qz;
+        const double wx = vvx - vu * ex - vq * qx, wy = vvy - vu * ey - vq * qy, wz = vvz - vu * ez - vq * qz;
+        s[2] += sqrt(wx * wx + wy * wy + wz * wz) * mk;
+        s[3] += mk;
+    };
+    int held = 0;
+    for (int64_t k0 = b + w * 32; k0 < e; k0 += blockDim.x) {
+        const int64_t k = k0 + lane;
+        bool cand = false;
+        if (k < e) {
+            const double rx = g[k] - c[0], ry = g[nm + k] - c[1], rz = g[2 * nm + k] - c[2];
+            const double vvx = g[3 * nm + k] - ux, vvy = g[4 * nm + k] - uy, vvz = g[5 * nm + k] - uz;
+            const double mk = g[6 * nm + k];
+            const double llx = mk * (ry * vvz - rz * vvy), lly = mk * (rz * vvx - rx * vvz),
+                         llz = mk * (rx * vvy - ry * vvx);
+            const double lz = llx * ex + lly * ey + llz * ez;
+            const double zi = rx * ex + ry * ey + rz * ez;
+            const double r2 = rx * rx + ry * ry + rz * rz;
+            const double R2 = r2 - zi * zi;
+            s[1] += 0.5 * mk * (vvx * vvx + vvy * vvy + vvz * vvz);
+            // 1/2 m (lz / (m R))^2 without the root (NaN, as there, where rounding leaves R^2 negative)
+            if (lz > 0.0) s[0] += R2 < 0.0 ? NAN : 0.5 * (lz * lz) / (mk * R2);
+            // the shell's bounds on squares, with a margin that the roots then decide
+            cand = r2 > shell_lo && r2 < shell_hi;
+        }
+        // a few members a warp: gathered, and worked through 32 at a time
+        const unsigned bal = __ballot_sync(0xffffffffu, cand);
+        if (cand) list[w][held + __popc(bal & ((1u << lane) - 1u))] = k;
+        held += __popc(bal);
+        __syncwarp();
+        if (held >= 32) {
+            held -= 32;
+            shell(list[w][held + lane]);
+            __syncwarp();
         }
     }
+    if (lane < held) shell(list[w][lane]);
     block_sums<4>(s, sm);
     if (threadIdx.x == 0) {
         const int sb = blockIdx.x % S;
@@ -473,59 +507,91 @@ __global__ void pr_runstart_kernel(int64_t n3, const int *__restrict__ head, con
     }
 }
 
-// One warp per cell: FP32 mass SD, mass-weighted velocity VCM (then / SD), count, and
-// sigma = sqrt(sum (v - VCM)^2 / count), members in order: the lanes load 32 members at a
-// time and every lane adds them one by one (shuffles), so the sums are the sequential ones;
-// rid[member entry] = cell.
-__global__ void pr_cells_kernel(int ncell, int64_t nm, const int *__restrict__ runstart,
+// Per cell: FP32 mass SD, mass-weighted velocity VCM (then / SD), count, and
+// sigma = sqrt(sum (v - VCM)^2 / count), members in order; rid[member entry] = cell.  Cells of at most kLaneCell
+// members take a lane each (most cells hold one or two members: a warp per cell waited on its few gathers with
+// 31 lanes idle), the others, neighbours mostly, a warp each in a second loop: 32 members loaded at a
+// time, every lane adding them one by one (shuffles), so that the sums are the sequential ones.
+constexpr int kLaneCell = 8;
+
+__global__ void __launch_bounds__(256) pr_cells_kernel(int ncell, int64_t nm, const int *__restrict__ runstart,
                                 const uint64_t *__restrict__ keys, const int *__restrict__ vals,
                                 const int *__restrict__ owner, const double *__restrict__ g,
                                 const double *__restrict__ out, float4 *__restrict__ cellv,
                                 uint64_t *__restrict__ cellkey, int *__restrict__ rid) {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < ncell; r += warps) {
+    // member entry k of projection a: velocity relative to the group's, and mass
+    auto member = [&](int k, int a, int64_t r, float &v, float &m) {
+        const int mk = vals[k] - a * (int)nm;
+        v = (float)__dsub_rn(g[(3 + a) * nm + mk], out[(int64_t)owner[mk] * HALMA_PROP_NFIELDS + HALMA_PROP_VX + a]);
+        m = (float)g[6 * nm + mk];
+        rid[vals[k]] = (int)r;
+    };
+    const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    for (int64_t r = w0 * 32 + lane; r < ncell; r += warps * 32) {
         const int b = runstart[r], e = runstart[r + 1];
+        if (e - b > kLaneCell) continue;
         const int a = vals[b] / (int)nm;   // projection of the cell
-        float sd = 0.f, vc = 0.f;
-        for (int k0 = b; k0 < e; k0 += 32) {
-            const int k = k0 + lane;
-            float vm = 0.f, m = 0.f;
-            if (k < e) {
-                const int mk = vals[k] - a * (int)nm;
-                const double *o = out + (int64_t)owner[mk] * HALMA_PROP_NFIELDS;
-                m = (float)g[6 * nm + mk];
-                vm = __fmul_rn((float)__dsub_rn(g[(3 + a) * nm + mk], o[HALMA_PROP_VX + a]), m);
-                rid[vals[k]] = (int)r;
-            }
-            const int cnt = e - k0 < 32 ? e - k0 : 32;
-            for (int t0 = 0; t0 < cnt; t0 += 8) {   // lanes past the end hold zeros, which change neither sum
+        float v[kLaneCell], sd = 0.f, vc = 0.f, s2 = 0.f;
 #pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    vc = __fadd_rn(vc, __shfl_sync(0xffffffffu, vm, t0 + t));
-                    sd = __fadd_rn(sd, __shfl_sync(0xffffffffu, m, t0 + t));
-                }
-            }
+        for (int k = 0; k < kLaneCell; ++k) {
+            if (b + k >= e) break;
+            float m;
+            member(b + k, a, r, v[k], m);
+            vc = __fadd_rn(vc, __fmul_rn(v[k], m));
+            sd = __fadd_rn(sd, m);
         }
         if (sd != 0.f) vc = __fdiv_rn(vc, sd);
-        float s2 = 0.f;
-        for (int k0 = b; k0 < e; k0 += 32) {
-            const int k = k0 + lane;
-            float d2 = 0.f;
-            if (k < e) {
-                const int mk = vals[k] - a * (int)nm;
-                const double *o = out + (int64_t)owner[mk] * HALMA_PROP_NFIELDS;
-                const float d = __fsub_rn((float)__dsub_rn(g[(3 + a) * nm + mk], o[HALMA_PROP_VX + a]), vc);
-                d2 = __fmul_rn(d, d);
-            }
-            const int cnt = e - k0 < 32 ? e - k0 : 32;
-            for (int t0 = 0; t0 < cnt; t0 += 8)
 #pragma unroll
-                for (int t = 0; t < 8; ++t) s2 = __fadd_rn(s2, __shfl_sync(0xffffffffu, d2, t0 + t));
+        for (int k = 0; k < kLaneCell; ++k) {
+            if (b + k >= e) break;
+            const float d = __fsub_rn(v[k], vc);
+            s2 = __fadd_rn(s2, __fmul_rn(d, d));
         }
-        if (lane == 0) {
-            cellv[r] = make_float4(sd, vc, __fsqrt_rn(__fdiv_rn(s2, (float)(e - b))), 0.f);
-            cellkey[r] = keys[b];
+        cellv[r] = make_float4(sd, vc, __fsqrt_rn(__fdiv_rn(s2, (float)(e - b))), 0.f);
+        cellkey[r] = keys[b];
+    }
+    for (int64_t r0 = w0; r0 < ncell; r0 += warps * 32) {   // 32 cells far apart looked at together
+        const int64_t mine = r0 + warps * lane;
+        const int b = mine < ncell ? runstart[mine] : 0, e = mine < ncell ? runstart[mine + 1] : 0;
+        for (unsigned todo = __ballot_sync(0xffffffffu, e - b > kLaneCell); todo; todo &= todo - 1) {
+            const int l = __ffs(todo) - 1;
+            const int64_t rr = r0 + warps * l;
+            const int bb = __shfl_sync(0xffffffffu, b, l), ee = __shfl_sync(0xffffffffu, e, l);
+            const int aa = vals[bb] / (int)nm;   // projection of the cell
+            float sd = 0.f, vc = 0.f, s2 = 0.f;
+            for (int k0 = bb; k0 < ee; k0 += 32) {
+                float v = 0.f, m = 0.f;
+                if (k0 + lane < ee) member(k0 + lane, aa, rr, v, m);
+                const float vm = __fmul_rn(v, m);
+                const int cnt = ee - k0 < 32 ? ee - k0 : 32;
+                for (int t0 = 0; t0 < cnt; t0 += 8) {   // lanes past the end hold zeros, which change neither sum
+#pragma unroll
+                    for (int t = 0; t < 8; ++t) {
+                        vc = __fadd_rn(vc, __shfl_sync(0xffffffffu, vm, t0 + t));
+                        sd = __fadd_rn(sd, __shfl_sync(0xffffffffu, m, t0 + t));
+                    }
+                }
+            }
+            if (sd != 0.f) vc = __fdiv_rn(vc, sd);
+            for (int k0 = bb; k0 < ee; k0 += 32) {
+                float d2 = 0.f;
+                if (k0 + lane < ee) {
+                    float v, m;
+                    member(k0 + lane, aa, rr, v, m);
+                    const float d = __fsub_rn(v, vc);
+                    d2 = __fmul_rn(d, d);
+                }
+                const int cnt = ee - k0 < 32 ? ee - k0 : 32;
+                for (int t0 = 0; t0 < cnt; t0 += 8)
+#pragma unroll
+                    for (int t = 0; t < 8; ++t) s2 = __fadd_rn(s2, __shfl_sync(0xffffffffu, d2, t0 + t));
+            }
+            if (lane == 0) {
+                cellv[rr] = make_float4(sd, vc, __fsqrt_rn(__fdiv_rn(s2, (float)(ee - bb))), 0.f);
+                cellkey[rr] = keys[bb];
+            }
         }
     }
 }
@@ -551,7 +617,9 @@ __global__ void __launch_bounds__(256) pr_proj_kernel(int G, int64_t nm, const i
                                                       const float4 *__restrict__ cellv,
                                                       const uint64_t *__restrict__ cellkey, int ncell,
                                                       float *__restrict__ res /* G x 3 x 3 */) {
-    __shared__ float term[4][kTile];
+    constexpr int kRow = kTile + 8;       // rows start in different banks
+    __shared__ float terms[2][4][kRow];   // one tile filled while the other is added
+    float (*const term)[kRow] = terms[0];
     __shared__ float red[12];
     const int t = threadIdx.x;
     for (int h = blockIdx.x; h < G; h += gridDim.x) {
@@ -563,26 +631,37 @@ __global__ void __launch_bounds__(256) pr_proj_kernel(int G, int64_t nm, const i
         // mean cell sigma inside R05: term[a] = the member's cell sigma (or -1 outside)
         float s05 = 0.f;
         int cnt = 0;
-        for (int64_t b = off[h]; b < off[h + 1]; b += kTile) {
+        auto fill = [&](int64_t b, float (*to)[kRow], int first, int step) {
             const int nt = (off[h + 1] - b < kTile ? (int)(off[h + 1] - b) : kTile);
-            for (int q = t; q < nt; q += blockDim.x) {
+#pragma unroll 2
+            for (int q = first; q < ((nt + 7) & ~7); q += step) {
                 const int64_t k = b + q;
+                if (q >= nt) {
+                    to[0][q] = to[1][q] = to[2][q] = -1.f;
+                    continue;
+                }
                 const float dx = __fsub_rn((float)g[k], cx), dy = __fsub_rn((float)g[nm + k], cy),
                             dz = __fsub_rn((float)g[2 * nm + k], cz);
                 const float d2[3] = {__fadd_rn(__fmul_rn(dy, dy), __fmul_rn(dz, dz)),
                                      __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dz, dz)),
                                      __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy))};
                 for (int a = 0; a < 3; ++a)
-                    term[a][q] = __fsqrt_rn(d2[a]) < r05[a] ? cellv[rid[a * nm + k]].z : -1.f;
+                    to[a][q] = __fsqrt_rn(d2[a]) < r05[a] ? cellv[rid[a * nm + k]].z : -1.f;
             }
-            if (t < 8 && nt + t < ((nt + 7) & ~7)) term[0][nt + t] = term[1][nt + t] = term[2][nt + t] = -1.f;
-            __syncthreads();
-            if (t < 3)   // eight loads ahead of their additions; an excluded term adds +0, which changes nothing
+        };
+        fill(off[h], terms[0], t, blockDim.x);
+        __syncthreads();
+        int cur = 0;
+        for (int64_t b = off[h]; b < off[h + 1]; b += kTile, cur ^= 1) {
+            const int nt = (off[h + 1] - b < kTile ? (int)(off[h + 1] - b) : kTile);
+            if (t >= 32) {
+                if (b + kTile < off[h + 1]) fill(b + kTile, terms[cur ^ 1], t - 32, blockDim.x - 32);
+            } else if (t < 3) {   // eight loads ahead of their additions; an excluded term adds +0, which changes nothing
                 for (int q = 0; q < nt; q += 8) {
                     float p[8];
 #pragma unroll
                     for (int u = 0; u < 8; ++u) {
-                        p[u] = term[t][q + u];
+                        p[u] = terms[cur][t][q + u];
                         const bool in = p[u] >= 0.f;
                         p[u] = in ? p[u] : 0.f;
                         cnt += in ? 1 : 0;
@@ -590,6 +669,7 @@ __global__ void __launch_bounds__(256) pr_proj_kernel(int G, int64_t nm, const i
 #pragma unroll
                     for (int u = 0; u < 8; ++u) s05 = __fadd_rn(s05, p[u]);
                 }
+            }
             __syncthreads();
         }
         if (t < 3) red[t] = cnt > 0 ? __fdiv_rn(s05, (float)cnt) : s05;
@@ -693,6 +773,31 @@ __global__ void pr_proj_out_kernel(int G, const float *__restrict__ res, double 
     }
 }
 
+// A second stream per device for the sums that need nothing of the half-mass radii (inertia tensor, angular momentum): a
+// few blocks with long chains, beside the sorts and walks of the main stream.
+struct PropSide {
+    cudaStream_t s = nullptr;
+    cudaEvent_t ready = nullptr, done = nullptr;
+};
+
+int prop_side(PropSide **out) {
+    static std::map<int, PropSide> m;   // under api_mutex()
+    PropSide &ps = m[current_device()];
+    if (!ps.s) {
+        HALMA_CUDA(cudaStreamCreateWithFlags(&ps.s, cudaStreamNonBlocking));
+        HALMA_CUDA(cudaEventCreateWithFlags(&ps.ready, cudaEventDisableTiming));
+        HALMA_CUDA(cudaEventCreateWithFlags(&ps.done, cudaEventDisableTiming));
+    }
+    *out = &ps;
+    return HALMA_OK;
+}
+
+// The side stream is idle again on every way out: its kernels use the call's workspace and the caller's arrays.
+struct SideIdle {
+    cudaStream_t s;
+    ~SideIdle() { cudaStreamSynchronize(s); }
+};
+
 // A small array of the caller's on the host; host memory without a call to the driver.
 int to_host(void *dst, const void *src, size_t bytes) {
     if (is_device_pointer(src)) HALMA_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost));
@@ -783,7 +888,7 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
                  o_vout = L.add(4ull * N3);
     const size_t o_head = L.add(4ull * N3), o_rpos = L.add(4ull * N3), o_rid = L.add(4ull * N3);
     const size_t o_cv = L.add(16ull * N3), o_ck = L.add(8ull * N3), o_res = L.add(4ull * 9 * G), o_cnt = L.add(64);
-    const int S = G >= 8192 ? 1 : 16;   // blocks per group for the angular-momentum kernels
+    const int S = G >= 8192 ? 1 : (G >= 1024 ? 16 : 64);   // blocks per group at most for the angular-momentum kernels
     const size_t o_kp = L.add(32ull * S * G), o_kctr = L.add(4ull * G), o_jv = L.add(64ull * G);
     const size_t sort_b = sort_pairs_u64_i32_bytes((int)N3, 64), scan_b = exclusive_sum_i32_bytes((int)N3);
     const size_t o_tmp = L.add(std::max(sort_b, scan_b));
@@ -821,6 +926,15 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
     HALMA_LAUNCH(pr_gather_kernel, gN, 256, 0, st, N0, dmem, dx, dy, dz, dvx, dvy, dvz, dm, gbuf);
     HALMA_LAUNCH(pr_fill_kernel, gG, 256, 0, st, G, doff, own);
     HALMA_LAUNCH(pr_bulk_kernel, gG, 256, 0, st, G, doff, gbuf, NM, dcen, dout, about);
+    PropSide *side = nullptr;
+    HALMA_TRY(prop_side(&side));
+    SideIdle side_idle{side->s};
+    HALMA_CUDA(cudaMemsetAsync(kctr, 0, 4ull * G, st));
+    HALMA_CUDA(cudaEventRecord(side->ready, st));
+    HALMA_CUDA(cudaStreamWaitEvent(side->s, side->ready, 0));
+    HALMA_LAUNCH(pr_shape_kernel, gG, 256, 0, side->s, G, doff, gbuf, NM, dcen, dout);
+    HALMA_LAUNCH(pr_kin1_kernel, G * S, 256, 0, side->s, G, S, doff, gbuf, NM, dcen, dout, kpart, kctr, jvec);
+    HALMA_CUDA(cudaEventRecord(side->done, side->s));
     // half-mass radii (3-D with sigma_effective, then x, y, z projections) by the reductions
     const double *gx = gbuf, *gy = gbuf + NM, *gz = gbuf + 2 * NM, *gvx = gbuf + 3 * NM, *gvy = gbuf + 4 * NM,
                  *gvz = gbuf + 5 * NM, *gm = gbuf + 6 * NM, *g0 = gbuf + 7 * NM;
@@ -836,10 +950,8 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
                                         red + (int64_t)r * G * HALMA_RED_NFIELDS, st));
     }
     HALMA_LAUNCH(pr_r05_kernel, gH, 128, 0, st, G, red, dout, res);
-    HALMA_CUDA(cudaMemsetAsync(kctr, 0, 4ull * G, st));
-    HALMA_LAUNCH(pr_kin1_kernel, G * S, 256, 0, st, G, S, doff, gbuf, NM, dcen, dout, kpart, kctr, jvec);
+    HALMA_CUDA(cudaStreamWaitEvent(st, side->done, 0));
     HALMA_LAUNCH(pr_kin2_kernel, G * S, 256, 0, st, G, S, doff, gbuf, NM, dcen, dout, kpart, kctr, jvec);
-    HALMA_LAUNCH(pr_shape_kernel, gG, 256, 0, st, G, doff, gbuf, NM, dcen, dout);
     if (N0 > 0) {
         HALMA_LAUNCH(pr_pkeys_kernel, gN, 256, 0, st, N0, G, doff, own, gbuf, dcen, linking_length, cbits, kin, vin);
         const int n3 = (int)(3 * N0);
