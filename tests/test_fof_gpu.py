@@ -211,3 +211,75 @@ def test_particles_as_nodes(cuda, ll, box, n):
     p = p[rng.permutation(len(p))]
     x, y, z = (np.ascontiguousarray(c) for c in p.T)
     assert np.array_equal(fof.fof_labels(x, y, z, ll), oracle.fof_labels(x, y, z, ll))
+
+
+def _filled(x, y, z, ll, total):
+    """The points followed by isolated ones beyond them, `total` in all: past the limit of the small path."""
+    k = total - len(x)
+    step = 4.0 * ll if ll > 0 else 1.0
+    fx = (x.max() if len(x) else 0.0) + step * (1.0 + np.arange(k))
+    f = lambda a, b: np.ascontiguousarray(np.concatenate([a, b]))
+    return f(x, fx), f(y, np.zeros(k)), f(z, np.zeros(k))
+
+
+@pytest.mark.parametrize("total", [8192, 8193])
+def test_both_sides_of_the_small_path(golden, cuda, total):
+    """The reference's own cases on the all-pairs path and, filled up past its limit, on the cell path."""
+    d = golden("fof_cases.npz")
+    for name in _cases(d):
+        x, y, z = (np.ascontiguousarray(c) for c in d[f"{name}__xyz"].astype(np.float64).T)
+        ll = float(d[f"{name}__ll"])
+        if len(x) > total:
+            continue
+        want = oracle.fof_labels(x, y, z, ll)
+        fx, fy, fz = _filled(x, y, z, ll, total)
+        lab = fof.fof_labels(fx, fy, fz, ll)
+        assert np.array_equal(lab[:len(x)], want), name
+        assert (lab[len(x):] == -1).all(), name
+        off, mem = fof.fof_groups(lab, 2)
+        woff, wmem = fof.fof_groups(want, 2)
+        assert np.array_equal(off, woff) and np.array_equal(mem, wmem), name
+
+
+@pytest.mark.parametrize("far,ll", [(0.0, 1.5e-3), (3e5, 1.5e-3), (1e300, 1e290), (5.0, 1e-310)])
+def test_small_path_on_far_coordinates(cuda, far, ll):
+    """Coordinates beyond 2^24 linking lengths of the first particle are tested in FP64."""
+    rng = np.random.default_rng(4)
+    s = min(ll, 1e290) if ll > 1e-300 else 1e-310
+    p = rng.uniform(0.0, 12.0, (1500, 3)) * s
+    p[700:] += far
+    x, y, z = (np.ascontiguousarray(c) for c in p.T)
+    assert np.array_equal(fof.fof_labels(x, y, z, ll), _brute(p, ll))
+
+
+def _brute(p, ll):
+    n = len(p)
+    lab = np.arange(n)
+    with np.errstate(all="ignore"):
+        adj = [np.nonzero(((p[i, 0] - p[:, 0]) ** 2 + (p[i, 1] - p[:, 1]) ** 2) + (p[i, 2] - p[:, 2]) ** 2 <= ll * ll)[0]
+               for i in range(n)]
+    while True:
+        new = np.array([lab[a].min() if len(a) else lab[i] for i, a in enumerate(adj)])
+        if np.array_equal(new, lab):
+            break
+        lab = new
+    alone = np.array([len(a) <= 1 for a in adj])
+    return np.where(alone, -1, lab)
+
+
+@pytest.mark.parametrize("n", [1, 31, 1023, 1025, 5000, 8192, 8193, 30000])
+def test_groups_of_given_labels(cuda, n):
+    """Groups from labels alone, in the order of their smallest members, on both sides of the one-block path."""
+    rng = np.random.default_rng(n)
+    head = np.minimum(np.arange(n), (rng.uniform(0, 1, n) ** 3 * n).astype(np.int64))
+    while not np.array_equal(head, head[head]):
+        head = head[head]
+    lab = np.where(rng.random(n) < 0.1, -1, head).astype(np.int32)
+    lab[np.unique(lab[lab >= 0])] = np.unique(lab[lab >= 0])
+    for minp in (1, 2, 7):
+        off, mem = fof.fof_groups(lab, minp)
+        heads, count = np.unique(lab[lab >= 0], return_counts=True)
+        heads = heads[count >= minp]
+        assert len(off) == len(heads) + 1
+        for g, h in enumerate(heads):
+            assert np.array_equal(mem[off[g]:off[g + 1]], np.nonzero(lab == h)[0])
