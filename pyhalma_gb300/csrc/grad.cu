@@ -81,8 +81,8 @@ __device__ __forceinline__ void fold2(float &s, float &c, f2x v) {
 //
 // Bound: the FP32 pipe (12 or 13 lane-operations a pair, 10 pairs per SM-cycle).  The partners are sliced so
 // that several items wait for every warp slot (choose_slices): one item per tile left 94 warps for 3,000
-// cells (150 us a sweep, now 15) and 2.06 blocks an SM, the third round nearly empty, for 160,000
-// (19.6 ms, now 11.5).
+// cells (150 us a sweep, now 11) and 2.06 blocks an SM, the third round nearly empty, for 160,000
+// (19.6 ms, now 13.3).
 template <int T, bool WANT_S>
 __global__ void __launch_bounds__(32 * kGWarps) adjoint_kernel(
     const float *__restrict__ bx, const float *__restrict__ by, const float *__restrict__ bz,
@@ -198,6 +198,239 @@ void choose_slices(int64_t na, int64_t nb, int T, int nv, int *n_split, int64_t 
     *split_len = len;
 }
 
+// ---- both sides of a pair at once -----------------------------------------------------------
+// When the gradients of targets and sources are both wanted and there are enough pairs, one sweep gives them: distance,
+// rsqrt and r^-3 of a pair are formed once, 17 lane-operations instead of 12 + 13, and the sources' four
+// sums (r^-1 and the vector) are reduced over the warp's lanes (1 lane-operation a pair, 4 instructions).
+// A block of four warps holds 512 targets, four a lane, and stages 512 sources; an item is one block of sources against
+// `tblocks` blocks of targets, the sources' sums kept in shared memory (compensated) over them.  Per item and
+// target, or source, one partial sum is written; they are added in order in FP64.
+// Bound: the FP32 pipe (18.7 lane-operations and a rsqrt a pair).  160,000 targets x 200,000 sources: 27.5 ms in two
+// sweeps, 23.5 in one.
+constexpr int kBothT = 4, kBothTargets = 128 * kBothT, kBothSources = 512, kBothChunks = kBothSources / 32;
+
+struct BothShared {
+    float4 src[kBothSources];               // 32-source chunks as pairs: 16 x {x, x, y, y}, 16 x {z, z, m, m}
+    float part[4][kBothSources][4];         // per warp: the sources' sums over the warp's targets of one block
+    float sum[kBothSources][4], comp[kBothSources][4];
+};
+
+template <bool SELF>
+__device__ __forceinline__ void both_chunk(const float4 *sa, const float4 *sb, const f2x (&px)[kBothT],
+                                           const f2x (&py)[kBothT], const f2x (&pz)[kBothT], const f2x (&g)[kBothT],
+                                           f2x e2, int j0, const int (&self)[kBothT], f2x (&vx)[kBothT],
+                                           f2x (&vy)[kBothT], f2x (&vz)[kBothT], float *out, int lane) {
+#pragma unroll 1
+    for (int k0 = 0; k0 < 16; k0 += 2) {
+        float v[16];   // sums of 4 sources: s, x, y, z of each pair of sources
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int kp = k0 + k;
+            const float4 a = sa[kp], b = sb[kp];
+            const f2x X = pack2(a.x, a.y), Y = pack2(a.z, a.w), Z = pack2(b.x, b.y), W = pack2(b.z, b.w);
+            f2x s0 = pack2(0.f, 0.f), s1 = s0, s2 = s0, s3 = s0;
+#pragma unroll
+            for (int t = 0; t < kBothT; ++t) {
+                const f2x dx = sub2(X, px[t]), dy = sub2(Y, py[t]), dz = sub2(Z, pz[t]);
+                f2x r2 = fma2(dz, dz, e2);
+                r2 = fma2(dy, dy, r2);
+                r2 = fma2(dx, dx, r2);
+                float r0, r1;
+                unpack2(r2, r0, r1);
+                float i0 = rsqrt_ftz(r0), i1 = rsqrt_ftz(r1);
+                if (SELF) {
+                    if (j0 + 2 * kp == self[t]) i0 = 0.f;
+                    if (j0 + 2 * kp + 1 == self[t]) i1 = 0.f;
+                }
+                const f2x ri = pack2(i0, i1);
+                const f2x ri2 = mul2(ri, ri);
+                const f2x wr = mul2(mul2(W, ri), ri2);
+                vx[t] = fma2(wr, dx, vx[t]);
+                vy[t] = fma2(wr, dy, vy[t]);
+                vz[t] = fma2(wr, dz, vz[t]);
+                const f2x gr = mul2(g[t], ri);
+                const f2x gr3 = mul2(gr, ri2);
+                s0 = add2(s0, gr);
+                s1 = fma2(gr3, dx, s1);
+                s2 = fma2(gr3, dy, s2);
+                s3 = fma2(gr3, dz, s3);
+            }
+            unpack2(s0, v[8 * k + 0], v[8 * k + 4]);
+            unpack2(s1, v[8 * k + 1], v[8 * k + 5]);
+            unpack2(s2, v[8 * k + 2], v[8 * k + 6]);
+            unpack2(s3, v[8 * k + 3], v[8 * k + 7]);
+        }
+        // lane l and l ^ 1 get value l >> 1: source (l >> 3) of the four, component (l >> 1) & 3
+        const float r = warp_reduce_scatter16(v, lane);
+        if ((lane & 1) == 0) out[k0 * 8 + (lane >> 1)] = r;
+    }
+}
+
+// part_t[(sb - sb0) * nt + i][3]: target i's vector over source block sb; part_s[tsb * nsrc + j - j0][4]: source j's sums
+// over the targets of item column tsb (nsrc sources from j0 = sb0 * kBothSources on).
+__global__ void __launch_bounds__(128, 4) adjoint_both_kernel(
+    const float *__restrict__ sx, const float *__restrict__ sy, const float *__restrict__ sz,
+    const float *__restrict__ sm, int64_t ns, const float *__restrict__ tx, const float *__restrict__ ty,
+    const float *__restrict__ tz, const float *__restrict__ tg, int64_t nt, float eps2, int self_mask, int64_t self_off,
+    int sb0, int nsb, int tblocks, double *__restrict__ part_t, double *__restrict__ part_s) {
+    extern __shared__ __align__(16) unsigned char both_raw[];
+    BothShared &sh = *reinterpret_cast<BothShared *>(both_raw);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int sbl = blockIdx.x % nsb;   // consecutive items share their targets
+    const int tsb = blockIdx.x / nsb;
+    const int64_t j0 = (int64_t)(sb0 + sbl) * kBothSources;
+    const f2x e2 = pack2(eps2, eps2);
+    for (int k = threadIdx.x; k < kBothSources; k += 128) {
+        const float4 q = load_b(sx, sy, sz, sm, j0 + k, ns);
+        float *c = reinterpret_cast<float *>(sh.src + (k >> 5) * 32);
+        const int kp = (k & 31) >> 1, hf = k & 1;
+        c[kp * 4 + hf] = q.x;
+        c[kp * 4 + 2 + hf] = q.y;
+        c[64 + kp * 4 + hf] = q.z;
+        c[64 + kp * 4 + 2 + hf] = q.w;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) sh.sum[k][v] = sh.comp[k][v] = 0.f;
+    }
+    __syncthreads();
+    for (int tb = 0; tb < tblocks; ++tb) {
+        const int64_t i0 = ((int64_t)tsb * tblocks + tb) * kBothTargets;
+        if (i0 >= nt) break;   // the same for the block
+        const int64_t iw = i0 + w * 32 * kBothT;
+        f2x px[kBothT], py[kBothT], pz[kBothT], g[kBothT];
+        float vs[kBothT][3], vc[kBothT][3];
+        int self[kBothT];
+#pragma unroll
+        for (int t = 0; t < kBothT; ++t) {
+            const int64_t i = iw + t * 32 + lane;
+            const bool in = i < nt;   // far and with zero weight otherwise
+            const float4 p = in ? make_float4(tx[i], ty[i], tz[i], tg[i]) : make_float4(-kFarG, -kFarG, -kFarG, 0.f);
+            px[t] = pack2(p.x, p.x);
+            py[t] = pack2(p.y, p.y);
+            pz[t] = pack2(p.z, p.z);
+            g[t] = pack2(p.w, p.w);
+            const int64_t sj = i + self_off - j0;   // the self pair's source in the block
+            self[t] = in && self_mask && sj >= 0 && sj < kBothSources ? (int)sj : -1;
+#pragma unroll
+            for (int v = 0; v < 3; ++v) vs[t][v] = vc[t][v] = 0.f;
+        }
+        const int64_t lo = iw + self_off - j0;   // self pairs: sources lo .. lo + 32 T - 1 of the block
+        for (int c = 0; c < kBothChunks; ++c) {
+            f2x vx[kBothT], vy[kBothT], vz[kBothT];
+#pragma unroll
+            for (int t = 0; t < kBothT; ++t) vx[t] = vy[t] = vz[t] = pack2(0.f, 0.f);
+            const float4 *buf = sh.src + c * 32;
+            float *out = &sh.part[w][c * 32][0];
+            if (self_mask && lo < c * 32 + 32 && lo + 32 * kBothT > c * 32)
+                both_chunk<true>(buf, buf + 16, px, py, pz, g, e2, c * 32, self, vx, vy, vz, out, lane);
+            else
+                both_chunk<false>(buf, buf + 16, px, py, pz, g, e2, c * 32, self, vx, vy, vz, out, lane);
+#pragma unroll
+            for (int t = 0; t < kBothT; ++t) {
+                fold2(vs[t][0], vc[t][0], vx[t]);
+                fold2(vs[t][1], vc[t][1], vy[t]);
+                fold2(vs[t][2], vc[t][2], vz[t]);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < kBothT; ++t) {
+            const int64_t i = iw + t * 32 + lane;
+            if (i >= nt) continue;
+            double *p = part_t + ((int64_t)sbl * nt + i) * 3;
+#pragma unroll
+            for (int v = 0; v < 3; ++v) p[v] = (double)vs[t][v] + (double)vc[t][v];
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < kBothSources * 4; k += 128) {   // the warps in order, compensated
+            float *sum = &sh.sum[0][0] + k, *comp = &sh.comp[0][0] + k;
+            float s = *sum, e = *comp;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) two_sum_acc(s, e, (&sh.part[q][0][0])[k]);
+            *sum = s;
+            *comp = e;
+        }
+        __syncthreads();
+    }
+    for (int k = threadIdx.x; k < kBothSources * 4; k += 128)
+        part_s[((int64_t)tsb * nsb + sbl) * kBothSources * 4 + k] =
+            (double)(&sh.sum[0][0])[k] + (double)(&sh.comp[0][0])[k];
+}
+
+// After a band of source blocks: the targets' vectors over the band added to tot (first: set), and, after the last
+// band, the gradients; the band's sources' sums over the item columns in order, and their gradients.
+__global__ void __launch_bounds__(256) both_targets_kernel(const double *__restrict__ part_t, int nsb, int64_t nt,
+                                                           int first, int last, double *__restrict__ tot,
+                                                           const float *__restrict__ scale, float *__restrict__ out) {
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < 3 * nt; k += (int64_t)gridDim.x * blockDim.x) {
+        double acc = first ? 0.0 : tot[k];
+#pragma unroll 8
+        for (int s = 0; s < nsb; ++s) acc += part_t[(int64_t)s * 3 * nt + k];
+        if (last) out[k] = scale[k / 3] * (float)acc;
+        else tot[k] = acc;
+    }
+}
+
+__global__ void __launch_bounds__(256) both_sources_kernel(const double *__restrict__ part_s, int ntsb, int64_t nsrc,
+                                                           int64_t j0, int64_t ns, const float *__restrict__ m,
+                                                           float *__restrict__ gm, float *__restrict__ gs) {
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < 4 * nsrc; k += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t j = j0 + k / 4;
+        const int v = (int)(k & 3);
+        if (j >= ns) continue;
+        double acc = 0.0;
+#pragma unroll 8
+        for (int s = 0; s < ntsb; ++s) acc += part_s[(int64_t)s * nsrc * 4 + k];
+        // the vector was summed as (source - target): the source's gradient points the other way
+        if (v == 0) {
+            if (gm) gm[j] = (float)acc;
+        } else if (gs) {
+            gs[3 * j + v - 1] = m[j] * -(float)acc;
+        }
+    }
+}
+
+// Scratch: the targets' partial sums of one band within kBothBand bytes (one source block at least).
+constexpr int64_t kBothBand = 256ll << 20;
+// Below kBothPairs pairs its blocks, 512 x 512 pairs for an item of four warps, are too few for the GPU: 4.8e7
+// pairs take 89 us against 80 in two sweeps, 1.2e8 146 against 150, 5e8 405 against 479.
+constexpr double kBothPairs = 1e8;
+
+struct BothPlan {
+    int64_t nsb = 0, band = 0, ntsb = 0;   // source blocks, source blocks of a band, item columns
+    int tblocks = 0;
+    BothPlan(int64_t ns, int64_t nt) {
+        nsb = (ns + kBothSources - 1) / kBothSources;
+        band = std::min(nsb, std::max<int64_t>(1, kBothBand / (24 * nt)));
+        const int64_t tb = (nt + kBothTargets - 1) / kBothTargets;
+        // about eight items for every block that fits on the GPU (four an SM)
+        const int64_t columns = std::min(tb, std::max<int64_t>(1, ((int64_t)device_sm_count() * 32 + band - 1) / band));
+        tblocks = (int)((tb + columns - 1) / columns);
+        ntsb = (tb + tblocks - 1) / tblocks;
+    }
+    size_t bytes(int64_t nt) const {
+        return 8 * (size_t)(3 * nt * (band + 1) + ntsb * band * kBothSources * 4);
+    }
+};
+
+int launch_both(const BothPlan &P, const float *sx, const float *sy, const float *sz, const float *m, int64_t ns,
+                const float *tx, const float *ty, const float *tz, const float *g, int64_t nt, float eps2, int self,
+                int64_t self_off, float *gm, float *gs, float *gt, double *scratch, cudaStream_t st) {
+    double *part_t = scratch, *tot = part_t + 3 * nt * P.band, *part_s = tot + 3 * nt;
+    const int smem = (int)sizeof(BothShared), cap = device_sm_count() * 8;
+    HALMA_CUDA(cudaFuncSetAttribute(adjoint_both_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    for (int64_t sb0 = 0; sb0 < P.nsb; sb0 += P.band) {
+        const int nsb = (int)std::min(P.band, P.nsb - sb0);
+        const int64_t j0 = sb0 * kBothSources, nsrc = (int64_t)nsb * kBothSources;
+        HALMA_LAUNCH(adjoint_both_kernel, (unsigned)(nsb * P.ntsb), 128, smem, st, sx, sy, sz, m, ns, tx, ty, tz, g, nt,
+                     eps2, self, self_off, (int)sb0, nsb, P.tblocks, part_t, part_s);
+        HALMA_LAUNCH(both_targets_kernel, grid_for(3 * nt, 256, cap), 256, 0, st, part_t, nsb, nt, sb0 == 0,
+                     sb0 + nsb >= P.nsb, tot, g, gt);
+        if (gm || gs)
+            HALMA_LAUNCH(both_sources_kernel, grid_for(4 * nsrc, 256, cap), 256, 0, st, part_s, (int)P.ntsb, nsrc, j0, ns,
+                         m, gm, gs);
+    }
+    return HALMA_OK;
+}
+
 template <bool WANT_S>
 int launch_adjoint(const float *bx, const float *by, const float *bz, const float *bw, int64_t nb, const float *ax,
                    const float *ay, const float *az, int64_t na, float eps2, int self_mask, int64_t self_off,
@@ -263,14 +496,25 @@ extern "C" int halma_potential_grad_f32(int64_t ns, const float *m_, const float
     int64_t len_t = ns, len_s = nt;
     if (grad_tgt) choose_slices(nt, ns, kGT, 3, &split_t, &len_t);
     if (grad_m || grad_src) choose_slices(ns, nt, kGT, 4, &split_s, &len_s);
+    // both sides in one sweep from kBothPairs pairs on, and with a softening that keeps r^-2 finite
+    const bool both = grad_tgt && (grad_m || grad_src) && (double)ns * (double)nt >= kBothPairs &&
+                      (float)eps2 >= 0x1p-126f;
+    const BothPlan plan(ns, nt);
     Layout L;
     sg.plan(L);
-    const size_t o_part = L.add(8 * (size_t)std::max(split_t > 1 ? 3 * nt * split_t : 0, split_s > 1 ? 4 * ns * split_s : 0));
+    const size_t o_part =
+        L.add(both ? plan.bytes(nt)
+                   : 8 * (size_t)std::max(split_t > 1 ? 3 * nt * split_t : 0, split_s > 1 ? 4 * ns * split_s : 0));
     void *base = nullptr;
     HALMA_TRY(workspace(L.total, &base, st));
     HALMA_TRY(sg.bind_and_upload(base, st));
     double *part = at<double>(base, o_part);
     const int self = mask == HALMA_MASK_SELF;
+    if (both) {
+        HALMA_TRY(launch_both(plan, sx, sy, sz, m, ns, tx, ty, tz, g, nt, (float)eps2, self, self_offset, gm, gs, gt, part,
+                              st));
+        return sg.download(st);
+    }
     if (gt)
         HALMA_TRY(launch_adjoint<false>(sx, sy, sz, m, ns, tx, ty, tz, nt, (float)eps2, self, self_offset, split_t, len_t,
                                         g, nullptr, gt, part, st));

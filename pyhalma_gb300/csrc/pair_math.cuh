@@ -86,6 +86,41 @@ __device__ __forceinline__ float2 df_from_acc(float s, float c) { return df_fast
 
 __device__ __forceinline__ double df_to_double(float2 a) { return (double)a.x + (double)a.y; }
 
+// Reduce-scatter of 16 per-lane values across the warp: lanes l and l^1 end with the warp's
+// total of value (l >> 1) & 15 (fixed association: halving steps over lane bits 4..1, then
+// the pair l, l^1).
+__device__ __forceinline__ float warp_reduce_scatter16(float (&v)[16], int lane) {
+    float a[8], b[4], c[2];
+    {
+        const bool up = lane & 16;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const float send = up ? v[k] : v[k + 8], keep = up ? v[k + 8] : v[k];
+            a[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+        }
+    }
+    {
+        const bool up = lane & 8;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float send = up ? a[k] : a[k + 4], keep = up ? a[k + 4] : a[k];
+            b[k] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+        }
+    }
+    {
+        const bool up = lane & 4;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const float send = up ? b[k] : b[k + 2], keep = up ? b[k + 2] : b[k];
+            c[k] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+        }
+    }
+    const bool up = lane & 2;
+    const float send = up ? c[0] : c[1], keep = up ? c[1] : c[0];
+    const float d = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+    return d + __shfl_xor_sync(0xffffffffu, d, 1);
+}
+
 // The reference's float32 term, each operation rounded on its own (no FMA):
 //   r = sqrt((xj-xi)**2 + (yj-yi)**2 + (zj-zi)**2); phi = phi + m / r
 // (particle_subroutines.f90:502-505); +0, which leaves the sum as it is, where the mask of

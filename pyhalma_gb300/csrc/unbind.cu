@@ -487,41 +487,6 @@ __global__ void __launch_bounds__(256) ub_pair_kernel(const float4 *__restrict__
     }
 }
 
-// Reduce-scatter of 16 per-lane values across the warp: lanes l and l^1 end with the warp's
-// total of value (l >> 1) & 15 (fixed association: halving steps over lane bits 4..1, then
-// the pair l, l^1).
-__device__ __forceinline__ float warp_reduce_scatter16(float (&v)[16], int lane) {
-    float a[8], b[4], c[2];
-    {
-        const bool up = lane & 16;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const float send = up ? v[k] : v[k + 8], keep = up ? v[k + 8] : v[k];
-            a[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-        }
-    }
-    {
-        const bool up = lane & 8;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float send = up ? a[k] : a[k + 4], keep = up ? a[k + 4] : a[k];
-            b[k] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-        }
-    }
-    {
-        const bool up = lane & 4;
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const float send = up ? b[k] : b[k + 2], keep = up ? b[k + 2] : b[k];
-            c[k] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-        }
-    }
-    const bool up = lane & 2;
-    const float send = up ? c[0] : c[1], keep = up ? c[1] : c[0];
-    const float d = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-    return d + __shfl_xor_sync(0xffffffffu, d, 1);
-}
-
 // Symmetric form of chunk_pairs: every pair term 1/r is used twice, m_source / r for the
 // lane's targets (acc, as in chunk_pairs) and m_target / r for the chunk's sources.  The
 // source side is summed over the lane's T targets, then over the warp (reduce-scatter), and

@@ -130,3 +130,34 @@ def test_gas_halo_adjoint_at_full_scale(cuda):
         dm = 1e-3 * M64[j]
         fdm = (l_source(j, S64[j], M64[j] + dm) - l_source(j, S64[j], M64[j] - dm)) / (2 * dm)
         assert abs(gm_gpu[j] - fdm) <= 1e-5 * abs(fdm), j
+
+
+@pytest.mark.parametrize("ns,nt,self_offset", [
+    (10_001, 10_007, None), (512 * 40, 512 * 10, 0), (512 * 40 + 1, 512 * 10 + 1, 7), (511, 200_003, 0),
+    (200_003, 513, -300), (300_000, 1, None), (1, 120_000_000 // 200, None), (4_097, 40_001, 4_000)])
+def test_both_gradients_in_one_sweep(cuda, ns, nt, self_offset):
+    """Enough pairs for the kernel that gives both ends' gradients at once (and shapes short of it), at the edges of
+    its blocks of 512, with and without a skipped pair, against the FP64 gradient."""
+    import torch
+    from pyhalma_gb300.autograd import softened_potential
+    rng = np.random.default_rng(8)
+    f = lambda a: np.ascontiguousarray(a, dtype=np.float32)
+    s, t = f(rng.normal(0, 0.02, (ns, 3))), f(rng.normal(0, 0.02, (nt, 3)))
+    m, g = f(np.exp(rng.normal(np.log(1e5), 1.0, ns))), f(rng.normal(size=nt))
+    if self_offset is not None:   # the skipped pair is a coincident one
+        i = np.arange(nt)
+        ok = (i + self_offset >= 0) & (i + self_offset < ns)
+        t[i[ok]] = s[i[ok] + self_offset]
+    eps = 1e-4
+    S, T = ([torch.tensor(f(a[:, k]), device=cuda, requires_grad=True) for k in range(3)] for a in (s, t))
+    M = torch.tensor(m, device=cuda, requires_grad=True)
+    phi = softened_potential(*S, M, *T, eps, self_offset=self_offset)
+    phi.backward(torch.tensor(g, device=cuda))
+    d = lambda a: a.astype(np.float64)
+    mask = oracle.MASK_NONE if self_offset is None else oracle.MASK_SELF
+    kw = {} if self_offset is None else {"self_offset": self_offset}
+    gm, gs, gt = oracle.potential_grad_f64(d(m), *d(s).T, *d(t).T, d(g), eps2=eps * eps, mask=mask, **kw)
+    rel = lambda a, b: np.linalg.norm(a - b) / np.linalg.norm(b)
+    assert rel(M.grad.cpu().numpy(), gm) < 1e-5
+    assert rel(np.stack([a.grad.cpu().numpy() for a in S], 1), gs) < 1e-5
+    assert rel(np.stack([a.grad.cpu().numpy() for a in T], 1), gt) < 1e-5
