@@ -60,9 +60,10 @@ class SoftenedPotential(torch.autograd.Function):
         need_m = ctx.needs_input_grad[3]
         need_s = any(ctx.needs_input_grad[0:3])
         need_t = any(ctx.needs_input_grad[4:7])
-        gm = torch.zeros(ns, dtype=torch.float32, device=sx.device) if need_m else None
-        gs = torch.zeros(ns, 3, dtype=torch.float32, device=sx.device) if need_s else None
-        gt = torch.zeros(nt, 3, dtype=torch.float32, device=sx.device) if need_t else None
+        # the call writes every element, zeros where the other side is empty
+        gm = torch.empty(ns, dtype=torch.float32, device=sx.device) if need_m else None
+        gs = torch.empty(ns, 3, dtype=torch.float32, device=sx.device) if need_s else None
+        gt = torch.empty(nt, 3, dtype=torch.float32, device=sx.device) if need_t else None
         mask = _lib.MASK_NONE if ctx.self_offset is None else _lib.MASK_SELF
         st = _lib.lib().halma_potential_grad_f32(ns, *_ptrs(m, sx, sy, sz), nt, *_ptrs(tx, ty, tz, g),
                                                  ctx.eps ** 2, mask, int(ctx.self_offset or 0), _lib.ptr(gm),
