@@ -276,80 +276,167 @@ __device__ __forceinline__ int warp_incl_scan(int v, int lane) {
 constexpr int kSymWarps = 4, kSymT = 8;
 constexpr int kSymBlock = kSymWarps * 32 * kSymT;   // 1024 slots
 
-// The pass's work list, built in three steps over the haloes in size order (q):
+// The pass's work list over the haloes in size order (q):
 //   count - per halo q: its halo h, tile shape, source slices, and three counts: warp items
 //           (tiles x slices), energy segments, symmetric block-pair items (0 unless active);
-//   scan  - exclusive prefix sums of the three counts (CUB);
+//   scan  - exclusive prefix sums of the three counts;
 //   fill  - the prefix sums become istart / sstart / ystart, every segment records its owner
 //           (sown), and the totals go to cnt[] (warp items, energy segments, block-pair items,
 //           their counters reset) and to the last entries of the start arrays.
 // With pairs_out (profiling), the pass's pair terms (nb x sources, all haloes) and those of the
 // haloes on the symmetric block kernel are summed into pairs_out[0..1] (zeroed beforehand).
+// For up to kItemsBlock haloes one block does all three (items_block), for the next pass beside the last one's
+// compaction.  As a count, a scan and a fill, four launches with nothing beside them, it took 8.7 us of every pass.
+// A block takes 6.9 us for 260 haloes and 32 for 2,000, most of it hidden: haloes of 1,100 to 1,500 members, all
+// passes, 260 of them 977 -> 871 us, 1,000 1,974 -> 1,808, 2,000 3,012 -> 2,966.  More haloes take the three steps,
+// spread over the GPU.
+constexpr int kItemsBlock = 2048;
+
+struct WorkList {
+    int4 *idesc;
+    int *istart, *ystart, *sstart, *sown, *cnt;
+};
+
+struct ItemRule {
+    TileTable tab;
+    int slice_len, inc, sym_ok;
+};
+
+// Counts of halo h (x warp items, y energy segments, z block pairs), its description and its pair terms.
+__device__ __forceinline__ int3 halo_items(const HaloState &s, int h, const ItemRule &rule, int4 &desc,
+                                           unsigned long long &pairs, unsigned long long &spairs) {
+    int n = 0, T = 4, nsl = 1, nseg = 0, ny = 0, nsl_e = 0;
+    if (s.active) {
+        const int nb = s.nb;
+        const int ns = rule.inc ? s.nrem : nb;   // sources: removed particles or the halo itself
+        T = tile_t_for(rule.tab, nb);
+        nsl = (int)(((int64_t)ns + rule.slice_len - 1) / rule.slice_len);
+        if (!rule.inc && rule.sym_ok && nb > kSymBlock && nb <= 65535 * kSymBlock) {
+            const int B = (nb + kSymBlock - 1) / kSymBlock;   // B <= 65535: B(B+1)/2 < 2^31
+            ny = (int)((int64_t)B * (B + 1) / 2);
+            nsl_e = B;
+            spairs = (unsigned long long)nb * (unsigned long long)nb;
+        } else {
+            n = ns > 0 ? ((nb + 32 * T - 1) / (32 * T)) * nsl : 0;
+            nsl_e = nsl;
+        }
+        nseg = max(1, (nb + kSeg - 1) / kSeg);
+        pairs = (unsigned long long)nb * (unsigned long long)ns;
+    }
+    desc = make_int4(h, T, max(nsl, 1), nsl_e);
+    return make_int3(n, nseg, ny);
+}
+
+__device__ __forceinline__ void add_pairs(unsigned long long *pairs_out, unsigned long long pairs,
+                                          unsigned long long spairs, int lane) {
+    if (!pairs_out) return;
+    for (int o = 16; o > 0; o >>= 1) {
+        pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+        spairs += __shfl_xor_sync(0xffffffffu, spairs, o);
+    }
+    if (lane == 0 && (pairs | spairs)) {   // one atomic per warp
+        atomicAdd(pairs_out, pairs);
+        atomicAdd(pairs_out + 1, spairs);
+    }
+}
+
+__device__ __forceinline__ void items_total(const WorkList &wl, int nh, int3 t) {
+    wl.istart[nh] = t.x;
+    wl.sstart[nh] = t.y;
+    wl.ystart[nh] = t.z;
+    wl.cnt[0] = t.x;   // warp items
+    wl.cnt[1] = 0;     // their counter
+    wl.cnt[2] = t.y;   // energy segments
+    wl.cnt[3] = t.z;   // symmetric block items
+    wl.cnt[4] = 0;     // their counter
+}
+
+// The whole list by one block of kSegThreads threads.
+__device__ __forceinline__ void items_block(int nh, const int *__restrict__ order, const HaloState *hs,
+                                            const ItemRule &rule, const WorkList &wl, unsigned long long *pairs_out) {
+    constexpr int kWarps = kSegThreads / 32;
+    __shared__ int3 tot[2][kWarps];   // of two rounds in turn: one barrier a round
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int3 run = make_int3(0, 0, 0);
+    int par = 0;
+    for (int q0 = 0; q0 < nh; q0 += kSegThreads, par ^= 1) {
+        const int q = q0 + threadIdx.x;
+        int3 c = make_int3(0, 0, 0);
+        unsigned long long pairs = 0, spairs = 0;
+        if (q < nh) {
+            int4 desc;
+            const int h = order[q];
+            c = halo_items(hs[h], h, rule, desc, pairs, spairs);
+            wl.idesc[q] = desc;
+        }
+        add_pairs(pairs_out, pairs, spairs, lane);
+        const int3 i = make_int3(warp_incl_scan(c.x, lane), warp_incl_scan(c.y, lane), warp_incl_scan(c.z, lane));
+        if (lane == 31) tot[par][w] = i;
+        __syncthreads();
+        int3 p = make_int3(run.x + i.x - c.x, run.y + i.y - c.y, run.z + i.z - c.z);
+#pragma unroll
+        for (int k = 0; k < kWarps; ++k) {
+            const int3 t = tot[par][k];
+            if (k < w) {
+                p.x += t.x;
+                p.y += t.y;
+                p.z += t.z;
+            }
+            run.x += t.x;
+            run.y += t.y;
+            run.z += t.z;
+        }
+        if (q < nh) {
+            wl.istart[q] = p.x;
+            wl.sstart[q] = p.y;
+            wl.ystart[q] = p.z;
+        }
+        // a halo's segments: a few by its thread, many by the warp
+        const bool many = c.y > 4;
+        if (!many)
+            for (int sg = 0; sg < c.y; ++sg) wl.sown[p.y + sg] = q;
+        for (unsigned todo = __ballot_sync(0xffffffffu, many); todo; todo &= todo - 1) {
+            const int l = __ffs(todo) - 1;
+            const int first = __shfl_sync(0xffffffffu, p.y, l), count = __shfl_sync(0xffffffffu, c.y, l);
+            for (int sg = lane; sg < count; sg += 32) wl.sown[first + sg] = q0 + w * 32 + l;
+        }
+    }
+    if (threadIdx.x == 0) items_total(wl, nh, run);
+}
+
+__global__ void __launch_bounds__(kSegThreads) ub_items_kernel(int nh, const int *__restrict__ order,
+                                                               const HaloState *hs, ItemRule rule, WorkList wl,
+                                                               unsigned long long *__restrict__ pairs_out) {
+    items_block(nh, order, hs, rule, wl, pairs_out);
+}
+
 __global__ void __launch_bounds__(256) ub_items_count_kernel(int nh, const int *__restrict__ order,
-                                                             const HaloState *hs, TileTable tab, int slice_len,
-                                                             int inc, int sym_ok, int4 *__restrict__ counts,
-                                                             int4 *__restrict__ idesc,
+                                                             const HaloState *hs, ItemRule rule,
+                                                             int4 *__restrict__ counts, int4 *__restrict__ idesc,
                                                              unsigned long long *__restrict__ pairs_out) {
-    const int lane = threadIdx.x & 31;
     for (int q0 = blockIdx.x * blockDim.x; q0 < nh; q0 += gridDim.x * blockDim.x) {
         const int q = q0 + threadIdx.x;
-        int h = -1, n = 0, T = 4, nsl = 1, nseg = 0, ny = 0, nsl_e = 0;
-        unsigned long long my_pairs = 0, my_spairs = 0;
+        unsigned long long pairs = 0, spairs = 0;
         if (q < nh) {
-            h = order[q];
-            if (hs[h].active) {
-                const int nb = hs[h].nb;
-                const int ns = inc ? hs[h].nrem : nb;   // sources: removed particles or the halo itself
-                T = tile_t_for(tab, nb);
-                nsl = (int)(((int64_t)ns + slice_len - 1) / slice_len);
-                if (!inc && sym_ok && nb > kSymBlock && nb <= 65535 * kSymBlock) {
-                    const int B = (nb + kSymBlock - 1) / kSymBlock;   // B <= 65535: B(B+1)/2 < 2^31
-                    ny = (int)((int64_t)B * (B + 1) / 2);
-                    nsl_e = B;
-                    my_spairs = (unsigned long long)nb * (unsigned long long)nb;
-                } else {
-                    n = ns > 0 ? ((nb + 32 * T - 1) / (32 * T)) * nsl : 0;
-                    nsl_e = nsl;
-                }
-                nseg = max(1, (nb + kSeg - 1) / kSeg);
-                my_pairs = (unsigned long long)nb * (unsigned long long)ns;
-            }
-            counts[q] = make_int4(n, nseg, ny, 0);
-            idesc[q] = make_int4(h, T, max(nsl, 1), nsl_e);
+            int4 desc;
+            const int h = order[q];
+            const int3 c = halo_items(hs[h], h, rule, desc, pairs, spairs);
+            counts[q] = make_int4(c.x, c.y, c.z, 0);
+            idesc[q] = desc;
         }
-        if (pairs_out) {   // one atomic per warp
-            for (int o = 16; o > 0; o >>= 1) {
-                my_pairs += __shfl_xor_sync(0xffffffffu, my_pairs, o);
-                my_spairs += __shfl_xor_sync(0xffffffffu, my_spairs, o);
-            }
-            if (lane == 0 && (my_pairs | my_spairs)) {
-                atomicAdd(pairs_out, my_pairs);
-                atomicAdd(pairs_out + 1, my_spairs);
-            }
-        }
+        add_pairs(pairs_out, pairs, spairs, threadIdx.x & 31);
     }
 }
 
 __global__ void __launch_bounds__(256) ub_items_fill_kernel(int nh, const int4 *__restrict__ counts,
-                                                            const int4 *__restrict__ pre, int *__restrict__ istart,
-                                                            int *__restrict__ ystart, int *__restrict__ sstart,
-                                                            int *__restrict__ sown, int *__restrict__ cnt) {
+                                                            const int4 *__restrict__ pre, WorkList wl) {
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nh; q += gridDim.x * blockDim.x) {
         const int4 c = counts[q], p = pre[q];
-        istart[q] = p.x;
-        sstart[q] = p.y;
-        ystart[q] = p.z;
-        for (int sg = 0; sg < c.y; ++sg) sown[p.y + sg] = q;
-        if (q == nh - 1) {
-            istart[nh] = p.x + c.x;
-            sstart[nh] = p.y + c.y;
-            ystart[nh] = p.z + c.z;
-            cnt[0] = p.x + c.x;   // warp items
-            cnt[1] = 0;           // their counter
-            cnt[2] = p.y + c.y;   // energy segments
-            cnt[3] = p.z + c.z;   // symmetric block items
-            cnt[4] = 0;           // their counter
-        }
+        wl.istart[q] = p.x;
+        wl.sstart[q] = p.y;
+        wl.ystart[q] = p.z;
+        for (int sg = 0; sg < c.y; ++sg) wl.sown[p.y + sg] = q;
+        if (q == nh - 1) items_total(wl, nh, make_int3(p.x + c.x, p.y + c.y, p.z + c.z));
     }
 }
 
@@ -1180,16 +1267,24 @@ __global__ void ub_finalize_df_kernel(int nh, const int *__restrict__ order, con
 // Per segment of a halo that stays active (FP32 path): survivors' packed position, velocity
 // offset, index and potential copied in order into the other buffers, removed particles'
 // packed positions into the next pass's source list; the halo's last segment pads both.
+// With next.idesc, block 0 writes the next pass's work list meanwhile (another one than this pass's).
+// Bound: memory traffic (90 bytes a slot) for large catalogues.
 __global__ void __launch_bounds__(kSegThreads) ub_compact_df_kernel(
     const int *__restrict__ sstart, const int *__restrict__ sown, const int4 *__restrict__ idesc,
     const int *__restrict__ nsegs, const int64_t *__restrict__ poff, const HaloState *__restrict__ hs,
     const unsigned char *__restrict__ keepf, const int2 *__restrict__ seg_pre, const float4 *__restrict__ pk_in,
     const float4 *__restrict__ pv_in, const int *__restrict__ pidx_in, const float2 *__restrict__ phi_cur,
     float4 *__restrict__ pk_out, float4 *__restrict__ pv_out, int *__restrict__ pidx_out,
-    float2 *__restrict__ phi_next, float4 *__restrict__ removed) {
+    float2 *__restrict__ phi_next, float4 *__restrict__ removed, int nh, const int *__restrict__ order, ItemRule rule,
+    WorkList next, unsigned long long *__restrict__ next_pairs) {
     __shared__ int wcount[kSegThreads / 32], wrem[kSegThreads / 32];
+    const int lists = next.idesc ? 1 : 0;
+    if ((int)blockIdx.x < lists) {
+        items_block(nh, order, hs, rule, next, next_pairs);
+        return;
+    }
     const int nseg_all = *nsegs;
-    for (int seg = blockIdx.x; seg < nseg_all; seg += gridDim.x) {
+    for (int seg = blockIdx.x - lists; seg < nseg_all; seg += gridDim.x - lists) {
         const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
         const int q = sown[seg];
         const int h = idesc[q].x;
@@ -1796,17 +1891,20 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
     const size_t o_rk = L.add(vsz * P);                               // removed particles' slots
     const size_t o_phic = L.add(sizeof(double) * P), o_phin = L.add(sizeof(double) * P);
     const size_t o_phi = L.add(sizeof(double) * Q);
-    const size_t o_istart = L.add(sizeof(int) * (nh + 1));
-    const size_t o_sstart = L.add(sizeof(int) * (nh + 1));
-    const size_t o_idesc = L.add(sizeof(int4) * std::max(nh, 1));
     const size_t o_ssum = L.add(std::max(sizeof(double) * kSegSums, sizeof(SegDF)) * segcap);
     const size_t o_pv = L.add(f64 ? 0 : sizeof(float4) * P), o_pv2 = L.add(f64 ? 0 : sizeof(float4) * P);
-    const size_t o_sown = L.add(sizeof(int) * segcap);
     const size_t o_spre = L.add(sizeof(int2) * segcap);
     const size_t o_rpart = L.add(sizeof(double) * kRedSums * std::max(nchunks, 1));
     const size_t o_cnt = L.add(64);
+    // the work lists of a pass and of the next one
+    size_t o_list[2][6];
+    for (auto &o : o_list) {
+        o[0] = L.add(sizeof(int4) * std::max(nh, 1));
+        for (int k = 1; k < 4; ++k) o[k] = L.add(sizeof(int) * (nh + 1));
+        o[4] = L.add(sizeof(int) * segcap);
+        o[5] = L.add(64);
+    }
     const size_t o_pairs = L.add(sizeof(unsigned long long) * 2 * p.max_iter);
-    const size_t o_ystart = L.add(sizeof(int) * (nh + 1));
     const size_t o_off = d_off ? 0 : L.add(sizeof(int64_t) * (nh + 1));
     const size_t o_icnt = L.add(sizeof(int4) * std::max(nh, 1)), o_ipre = L.add(sizeof(int4) * std::max(nh, 1));
     const size_t iscan_bytes = exclusive_sum_int3_bytes(std::max(nb_, 1));
@@ -1821,19 +1919,18 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
     auto *keepf = at<unsigned char>(base, o_keep);
     auto *phic = at<double>(base, o_phic), *phin = at<double>(base, o_phin);
     auto *phi = at<double>(base, o_phi);
-    auto *istart = at<int>(base, o_istart);
-    auto *sstart = at<int>(base, o_sstart);
-    auto *idesc = at<int4>(base, o_idesc);
     auto *ssum = at<double>(base, o_ssum);
-    auto *sown = at<int>(base, o_sown);
     auto *segpre = at<int2>(base, o_spre);
     auto *dcst = at<int>(base, o_plan + pl_cst);
     auto *dchh = at<int>(base, o_plan + pl_chh);
     auto *rpart = at<double>(base, o_rpart);
-    int *cnt = at<int>(base, o_cnt);   // [0] nitems [1] counter [2] energy segments
+    int *nactive = at<int>(base, o_cnt);   // haloes left after a chunk of passes
+    WorkList list[2];
+    for (int k = 0; k < 2; ++k)
+        list[k] = {at<int4>(base, o_list[k][0]), at<int>(base, o_list[k][1]), at<int>(base, o_list[k][2]),
+                   at<int>(base, o_list[k][3]),  at<int>(base, o_list[k][4]), at<int>(base, o_list[k][5])};
     const int sgrid = (int)segcap;
     auto *dpairs = at<unsigned long long>(base, o_pairs);
-    auto *ystart = at<int>(base, o_ystart);
     Profile &prof = profile();
     const bool profiling = prof.enabled;
     if (profiling) {
@@ -1856,16 +1953,21 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
         HALMA_CUDA(cudaMemcpyAsync(dpoff, plan.data(), pl_bytes, cudaMemcpyHostToDevice, st));
     }
     const int fgrid = grid_for((int64_t)nb_ * 32, 256);   // one warp per halo
-    // the pass's work list (count, scan, fill; see ub_items_count_kernel)
+    // the pass's work list (see kItemsBlock)
     auto *icount = at<int4>(base, o_icnt), *ipre = at<int4>(base, o_ipre);
     void *iscan_tmp = at<void>(base, o_iscan);
     const int igrid = std::min(grid_for(nb_, 256), device_sm_count() * 4);
-    auto items = [&](cudaStream_t rs, int inc, int sym_ok, unsigned long long *pairs) -> int {
+    const bool one_block = nb_ <= kItemsBlock;
+    auto items = [&](cudaStream_t rs, const WorkList &wl, int inc, int sym_ok, unsigned long long *pairs) -> int {
+        const ItemRule rule{tab, slice_len, inc, sym_ok};
         if (pairs) HALMA_CUDA(cudaMemsetAsync(pairs, 0, 2 * sizeof(unsigned long long), rs));
-        HALMA_LAUNCH(ub_items_count_kernel, igrid, 256, 0, rs, nb_, dorder, hs, tab, slice_len, inc, sym_ok, icount,
-                     idesc, pairs);
+        if (one_block) {
+            HALMA_LAUNCH(ub_items_kernel, 1, kSegThreads, 0, rs, nb_, dorder, hs, rule, wl, pairs);
+            return HALMA_OK;
+        }
+        HALMA_LAUNCH(ub_items_count_kernel, igrid, 256, 0, rs, nb_, dorder, hs, rule, icount, wl.idesc, pairs);
         HALMA_TRY(exclusive_sum_int3(iscan_tmp, iscan_bytes, icount, ipre, nb_, rs));
-        HALMA_LAUNCH(ub_items_fill_kernel, igrid, 256, 0, rs, nb_, icount, ipre, istart, ystart, sstart, sown, cnt);
+        HALMA_LAUNCH(ub_items_fill_kernel, igrid, 256, 0, rs, nb_, icount, ipre, wl);
         return HALMA_OK;
     };
     // FP64 bound mass, centre and bulk velocity per halo (active ones, or all with force);
@@ -1939,17 +2041,19 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
             for (int it = it0; it < it1; ++it) {
                 const int a = it & 1, b = a ^ 1;
                 const int inc = (it > 0 && incremental) ? 1 : 0;
-                HALMA_TRY(items(rs, inc, 1, profiling ? dpairs + 2 * it : nullptr));
+                const WorkList &wl = list[a];
+                // from the second pass on the last compaction may have written it
+                if (it == 0 || !one_block) HALMA_TRY(items(rs, wl, inc, 1, profiling ? dpairs + 2 * it : nullptr));
                 // External: captured as an event-record node, so the replay records it
                 if (profiling) HALMA_CUDA(cudaEventRecordWithFlags(prof.ev0[it], rs, cudaEventRecordExternal));
                 // full passes: the big haloes' block pairs first (the longest items), then the
                 // tiles of the small ones; incremental passes have only tiles
                 if (!inc)
-                    HALMA_LAUNCH(ub_pair_sym_kernel, ygrid, 128, kSymSmem, rs, pkb[a], dpoff, dqoff, hs, nb_, ystart,
-                                 idesc, cnt, cnt + 4, eps2, part2);
+                    HALMA_LAUNCH(ub_pair_sym_kernel, ygrid, 128, kSymSmem, rs, pkb[a], dpoff, dqoff, hs, nb_,
+                                 wl.ystart, wl.idesc, wl.cnt, wl.cnt + 4, eps2, part2);
                 if (profiling) HALMA_CUDA(cudaEventRecordWithFlags(prof.evm[it], rs, cudaEventRecordExternal));
-                HALMA_LAUNCH(ub_pair_kernel, pgrid, 256, 0, rs, pkb[a], rk, inc, dpoff, dqoff, hs, nb_, istart, idesc,
-                             cnt, cnt + 1, eps2, slice_len / 32, part2);
+                HALMA_LAUNCH(ub_pair_kernel, pgrid, 256, 0, rs, pkb[a], rk, inc, dpoff, dqoff, hs, nb_, wl.istart,
+                             wl.idesc, wl.cnt, wl.cnt + 1, eps2, slice_len / 32, part2);
                 if (profiling) HALMA_CUDA(cudaEventRecordWithFlags(prof.ev1[it], rs, cudaEventRecordExternal));
                 if (it == 0 && vel_ready) {
                     HALMA_CUDA(cudaStreamWaitEvent(rs, vel_ready, cudaEventWaitExternal));
@@ -1958,15 +2062,18 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                         HALMA_LAUNCH(ub_pack_kernel<float4>, nchunks, kSegThreads, 0, rs, off, dpoff, dcst, dchh, x, y,
                                      z, m, vx, vy, vz, hs, (float4 *)nullptr, pvb[0], (int *)nullptr);
                 }
-                HALMA_LAUNCH(ub_energy_df_kernel, egrid, kSegThreads, 0, rs, sstart, sown, idesc, cnt + 2, dpoff, dqoff,
-                             inc, pidxb[a], pvb[a], part2, phin2, phic2, x, y, z, vx, vy, vz, m, gfac_f, hs, bound,
-                             phi_out, keepf, sdf);
-                HALMA_LAUNCH(ub_finalize_df_kernel, fgrid, 256, 0, rs, nb_, dorder, sstart, sdf, gfac, hs, segpre);
-                HALMA_LAUNCH(ub_compact_df_kernel, cgrid, kSegThreads, 0, rs, sstart, sown, idesc, cnt + 2, dpoff, hs,
-                             keepf, segpre, pkb[a], pvb[a], pidxb[a], phic2, pkb[b], pvb[b], pidxb[b], phin2, rk);
+                HALMA_LAUNCH(ub_energy_df_kernel, egrid, kSegThreads, 0, rs, wl.sstart, wl.sown, wl.idesc, wl.cnt + 2,
+                             dpoff, dqoff, inc, pidxb[a], pvb[a], part2, phin2, phic2, x, y, z, vx, vy, vz, m, gfac_f,
+                             hs, bound, phi_out, keepf, sdf);
+                HALMA_LAUNCH(ub_finalize_df_kernel, fgrid, 256, 0, rs, nb_, dorder, wl.sstart, sdf, gfac, hs, segpre);
+                HALMA_LAUNCH(ub_compact_df_kernel, cgrid + one_block, kSegThreads, 0, rs, wl.sstart, wl.sown, wl.idesc,
+                             wl.cnt + 2, dpoff, hs, keepf, segpre, pkb[a], pvb[a], pidxb[a], phic2, pkb[b], pvb[b],
+                             pidxb[b], phin2, rk, nb_, dorder, ItemRule{tab, slice_len, incremental ? 1 : 0, 1},
+                             one_block ? list[b] : WorkList{},
+                             profiling && it + 1 < p.max_iter ? dpairs + 2 * (it + 1) : nullptr);
             }
-            HALMA_CUDA(cudaMemsetAsync(cnt + 6, 0, sizeof(int), rs));
-            HALMA_LAUNCH(ub_active_kernel, std::min(grid_for(nb_, 256), 64), 256, 0, rs, nb_, dorder, hs, cnt + 6);
+            HALMA_CUDA(cudaMemsetAsync(nactive, 0, sizeof(int), rs));
+            HALMA_LAUNCH(ub_active_kernel, std::min(grid_for(nb_, 256), 64), 256, 0, rs, nb_, dorder, hs, nactive);
             return HALMA_OK;
         };
         int passes_run = p.max_iter;
@@ -2034,7 +2141,7 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                 passes_run = it1;
                 if (it1 >= p.max_iter) break;
                 int active = 0;
-                HALMA_CUDA(cudaMemcpyAsync(&active, cnt + 6, sizeof(int), cudaMemcpyDeviceToHost, st));
+                HALMA_CUDA(cudaMemcpyAsync(&active, nactive, sizeof(int), cudaMemcpyDeviceToHost, st));
                 HALMA_CUDA(cudaStreamSynchronize(st));
                 if (active == 0) break;
             }
@@ -2068,7 +2175,8 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
         double4 *rk = at<double4>(base, o_rk);
         for (int it = 0; it < p.max_iter; ++it) {
             const int a = it & 1, b = a ^ 1;
-            HALMA_TRY(items(st, 0, 0, nullptr));
+            const WorkList &wl = list[0];
+            HALMA_TRY(items(st, wl, 0, 0, nullptr));
             HALMA_CUDA(cudaMemcpyAsync(hh.data(), hs, sizeof(HaloState) * nh, cudaMemcpyDeviceToHost, st));
             HALMA_CUDA(cudaStreamSynchronize(st));
             int any = 0;
@@ -2079,12 +2187,12 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                              p.eps * p.eps, phi + poff[h]);
             }
             if (!any) break;
-            HALMA_LAUNCH(ub_energy_seg_kernel<double4>, sgrid, kSegThreads, 0, st, sstart, sown, idesc, cnt + 2, dpoff,
-                         dqoff, 0, pidxb[a], phi, phin, phic, vx, vy, vz, m, gfac, hs, bound, phi_out, keepf,
+            HALMA_LAUNCH(ub_energy_seg_kernel<double4>, sgrid, kSegThreads, 0, st, wl.sstart, wl.sown, wl.idesc,
+                         wl.cnt + 2, dpoff, dqoff, 0, pidxb[a], phi, phin, phic, vx, vy, vz, m, gfac, hs, bound, phi_out, keepf,
                          ssum);
-            HALMA_LAUNCH(ub_finalize_kernel, fgrid, 256, 0, st, nh, dorder, sstart, ssum, gfac, hs, segpre);
-            HALMA_LAUNCH(ub_compact_seg_kernel<double4>, sgrid, kSegThreads, 0, st, sstart, sown, idesc, cnt + 2, dpoff,
-                         hs, keepf, segpre, pkb[a], pidxb[a], phic, pkb[b], pidxb[b], phin, rk);
+            HALMA_LAUNCH(ub_finalize_kernel, fgrid, 256, 0, st, nh, dorder, wl.sstart, ssum, gfac, hs, segpre);
+            HALMA_LAUNCH(ub_compact_seg_kernel<double4>, sgrid, kSegThreads, 0, st, wl.sstart, wl.sown, wl.idesc,
+                         wl.cnt + 2, dpoff, hs, keepf, segpre, pkb[a], pidxb[a], phic, pkb[b], pidxb[b], phin, rk);
         }
         HALMA_TRY(reduce(st, 1));
     }

@@ -218,3 +218,28 @@ def test_small_haloes_equal_the_pass_kernels(cuda):
             np.testing.assert_array_equal(g, w)
         if max_iter == 30:
             assert len(set(got[1][:, 8])) > 3   # haloes of one, two, .. passes
+
+
+@pytest.mark.parametrize("count", [1, 255, 256, 257, 2048, 2049])
+def test_work_list_of_many_haloes(cuda, count):
+    """The pass kernels' work list at its rounds of 256 haloes and on both sides of the one-block limit (2,048
+    haloes): bit for bit what the haloes that run in one block each give."""
+    from pyhalma_gb300 import autotune
+    rng = np.random.default_rng(count)
+    sizes = rng.integers(1, 60, count)
+    sizes[count // 2] = 970
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    n = int(off[-1])
+    cols = [rng.normal(0.0, 0.01, n) for _ in range(3)] + [rng.normal(0.0, 40.0, n) for _ in range(3)]
+    cols.append(rng.uniform(0.5, 2.0, n) * 1e7)
+    opt = UnbindOptions(eps=EPS)
+    upper, t, slice_len = autotune.get_table()
+    assert slice_len >= 1024
+    got = unbind_batched(off, *cols, opt, want_phi=True)
+    try:
+        autotune.set_table(upper, t, 992)
+        want = unbind_batched(off, *cols, opt, want_phi=True)
+    finally:
+        autotune.set_table(upper, t, slice_len)
+    for g, w in zip(got, want):
+        np.testing.assert_array_equal(g, w)
