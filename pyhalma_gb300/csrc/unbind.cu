@@ -1691,15 +1691,20 @@ __global__ void ub_output_kernel(int nh, const HaloState *__restrict__ hs, doubl
     }
 }
 
-// The passes are captured in chunks of kPassChunk (the first chunk also holds the reduction
-// and packing); one graph per chunk start, all cached for the same problem shape.
+// The passes run in chunks: the first pass (with the reduction and packing) alone, then kPassChunk at a time, after
+// which the host asks whether any halo is left.  A call with the buffers, sizes and options of the one before replays
+// one graph per chunk, the first two in one.  Another call launches the first pass as it is and captures the others
+// while it runs, if its pairs keep the GPU busy for longer than a capture takes (100 us; kCapturePairs take 140);
+// otherwise all its passes are launched as they are.  500 haloes of 50 to 200,000 members, other buffers on each
+// call: 8,815 us with every chunk captured before its launch, 8,738 so; five of 1,500 to 5,000: 866 and 715.
 constexpr int kPassChunk = 8;
+constexpr double kCapturePairs = 1e9;
 struct GraphCache {
     struct Entry {
         cudaGraphExec_t exec = nullptr;
         int64_t nodes = 0;
     };
-    std::vector<Entry> chunks;   // by chunk start / kPassChunk
+    std::vector<Entry> chunks;
     std::vector<uintptr_t> key;
     cudaStream_t capture_stream = nullptr;
     int capture_device = -1;
@@ -2024,13 +2029,14 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
         const int egrid = std::min(sgrid, device_sm_count() * std::max(bps, 1));
         HALMA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, ub_compact_df_kernel, kSegThreads, 0));
         const int cgrid = std::min(sgrid, device_sm_count() * std::max(bps, 1));
-        auto record = [&](cudaStream_t rs, int it0, int it1) -> int {
+        auto record = [&](cudaStream_t rs, int it0, int it1, bool capturing) -> int {
+            // external: captured as event nodes, so that the replay records and waits for them
+            const unsigned rec = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
             // first pass: centre of mass and packing into buffer 0; every pass then compacts
             // its survivors into the other buffer and sets the next pass's halo state
             // With vel_ready, the velocities may still be arriving: the first pass's pair
             // kernels start from the positions and masses, and the velocity sums and packed
-            // velocities follow once vel_ready has fired (an external wait: a node of the
-            // captured graph), before the first energy kernel.
+            // velocities follow once vel_ready has fired, before the first energy kernel.
             if (it0 == 0) {
                 HALMA_TRY(reduce(rs, 0, vel_ready ? 1 : 0));
                 if (nchunks > 0)
@@ -2044,19 +2050,18 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                 const WorkList &wl = list[a];
                 // from the second pass on the last compaction may have written it
                 if (it == 0 || !one_block) HALMA_TRY(items(rs, wl, inc, 1, profiling ? dpairs + 2 * it : nullptr));
-                // External: captured as an event-record node, so the replay records it
-                if (profiling) HALMA_CUDA(cudaEventRecordWithFlags(prof.ev0[it], rs, cudaEventRecordExternal));
+                if (profiling) HALMA_CUDA(cudaEventRecordWithFlags(prof.ev0[it], rs, rec));
                 // full passes: the big haloes' block pairs first (the longest items), then the
                 // tiles of the small ones; incremental passes have only tiles
                 if (!inc)
                     HALMA_LAUNCH(ub_pair_sym_kernel, ygrid, 128, kSymSmem, rs, pkb[a], dpoff, dqoff, hs, nb_,
                                  wl.ystart, wl.idesc, wl.cnt, wl.cnt + 4, eps2, part2);
-                if (profiling) HALMA_CUDA(cudaEventRecordWithFlags(prof.evm[it], rs, cudaEventRecordExternal));
+                if (profiling) HALMA_CUDA(cudaEventRecordWithFlags(prof.evm[it], rs, rec));
                 HALMA_LAUNCH(ub_pair_kernel, pgrid, 256, 0, rs, pkb[a], rk, inc, dpoff, dqoff, hs, nb_, wl.istart,
                              wl.idesc, wl.cnt, wl.cnt + 1, eps2, slice_len / 32, part2);
-                if (profiling) HALMA_CUDA(cudaEventRecordWithFlags(prof.ev1[it], rs, cudaEventRecordExternal));
+                if (profiling) HALMA_CUDA(cudaEventRecordWithFlags(prof.ev1[it], rs, rec));
                 if (it == 0 && vel_ready) {
-                    HALMA_CUDA(cudaStreamWaitEvent(rs, vel_ready, cudaEventWaitExternal));
+                    HALMA_CUDA(cudaStreamWaitEvent(rs, vel_ready, capturing ? cudaEventWaitExternal : cudaEventWaitDefault));
                     HALMA_TRY(reduce(rs, 0, 2));
                     if (nchunks > 0)
                         HALMA_LAUNCH(ub_pack_kernel<float4>, nchunks, kSegThreads, 0, rs, off, dpoff, dcst, dchh, x, y,
@@ -2072,6 +2077,7 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                              one_block ? list[b] : WorkList{},
                              profiling && it + 1 < p.max_iter ? dpairs + 2 * (it + 1) : nullptr);
             }
+            if (it1 == 1) return HALMA_OK;
             HALMA_CUDA(cudaMemsetAsync(nactive, 0, sizeof(int), rs));
             HALMA_LAUNCH(ub_active_kernel, std::min(grid_for(nb_, 256), 64), 256, 0, rs, nb_, dorder, hs, nactive);
             return HALMA_OK;
@@ -2102,7 +2108,8 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                 key.push_back((uintptr_t)tab.t[c]);
             }
             GraphCache &gc = graph_cache();
-            if (gc.key != key) {
+            const bool again = gc.key == key;
+            if (!again) {
                 for (auto &e : gc.chunks)
                     if (e.exec) cudaGraphExecDestroy(e.exec);
                 gc.chunks.clear();
@@ -2113,40 +2120,58 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                 HALMA_CUDA(cudaStreamCreateWithFlags(&gc.capture_stream, cudaStreamNonBlocking));
                 gc.capture_device = current_device();
             }
-            const int nchunk = (p.max_iter + kPassChunk - 1) / kPassChunk;
+            const int nchunk = 1 + (p.max_iter - 1 + kPassChunk - 1) / kPassChunk;
+            auto chunk_start = [&](int ci) { return ci == 0 ? 0 : std::min(p.max_iter, 1 + (ci - 1) * kPassChunk); };
+            // replayed, the first chunk is one graph with the second
+            auto next_chunk = [&](int ci) { return again && ci == 0 ? 2 : ci + 1; };
             gc.chunks.resize(nchunk);
-            passes_run = 0;
-            for (int ci = 0; ci < nchunk; ++ci) {
-                const int it0 = ci * kPassChunk, it1 = std::min(p.max_iter, it0 + kPassChunk);
+            double pairs = 0.0;
+            for (int q = 0; q < nb_; ++q) {
+                const double c = (double)(h_off[order[q] + 1] - h_off[order[q]]);
+                pairs += c * c;
+            }
+            // chunks from here on are graphs, those before are launched one by one
+            const int first_graph = again ? 0 : pairs >= kCapturePairs ? 1 : nchunk;
+            auto capture = [&](int ci) -> int {
+                if (ci < first_graph || ci >= nchunk || gc.chunks[ci].exec) return HALMA_OK;
                 GraphCache::Entry &ge = gc.chunks[ci];
-                if (!ge.exec) {
-                    cudaGraph_t graph = nullptr;
-                    HALMA_CUDA(cudaStreamBeginCapture(gc.capture_stream, cudaStreamCaptureModeThreadLocal));
-                    const int64_t before = halma_kernel_launch_count();
-                    int s = record(gc.capture_stream, it0, it1);
-                    cudaError_t ce = cudaStreamEndCapture(gc.capture_stream, &graph);
-                    if (s != HALMA_OK) {
-                        if (graph) cudaGraphDestroy(graph);
-                        return s;
-                    }
-                    HALMA_CUDA(ce);
-                    cudaError_t ie = cudaGraphInstantiate(&ge.exec, graph, 0);
-                    cudaGraphDestroy(graph);
-                    HALMA_CUDA(ie);
-                    ge.nodes = halma_kernel_launch_count() - before;
-                    add_launches(-ge.nodes);   // counted again at every replay below
+                cudaGraph_t graph = nullptr;
+                HALMA_CUDA(cudaStreamBeginCapture(gc.capture_stream, cudaStreamCaptureModeThreadLocal));
+                const int64_t before = halma_kernel_launch_count();
+                int s = record(gc.capture_stream, chunk_start(ci), chunk_start(next_chunk(ci)), true);
+                cudaError_t ce = cudaStreamEndCapture(gc.capture_stream, &graph);
+                if (s != HALMA_OK) {
+                    if (graph) cudaGraphDestroy(graph);
+                    return s;
                 }
-                HALMA_CUDA(cudaGraphLaunch(ge.exec, st));
-                add_launches(ge.nodes);
-                passes_run = it1;
-                if (it1 >= p.max_iter) break;
+                HALMA_CUDA(ce);
+                cudaError_t ie = cudaGraphInstantiate(&ge.exec, graph, 0);
+                cudaGraphDestroy(graph);
+                HALMA_CUDA(ie);
+                ge.nodes = halma_kernel_launch_count() - before;
+                add_launches(-ge.nodes);   // counted again at every replay below
+                return HALMA_OK;
+            };
+            passes_run = 0;
+            for (int ci = 0; ci < nchunk; ci = next_chunk(ci)) {
+                HALMA_TRY(capture(ci));
+                if (ci >= first_graph) {
+                    HALMA_CUDA(cudaGraphLaunch(gc.chunks[ci].exec, st));
+                    add_launches(gc.chunks[ci].nodes);
+                } else {
+                    HALMA_TRY(record(st, chunk_start(ci), chunk_start(next_chunk(ci)), false));
+                }
+                passes_run = chunk_start(next_chunk(ci));
+                if (passes_run >= p.max_iter) break;
+                HALMA_TRY(capture(next_chunk(ci)));   // while this one runs
+                if (passes_run == 1) continue;
                 int active = 0;
                 HALMA_CUDA(cudaMemcpyAsync(&active, nactive, sizeof(int), cudaMemcpyDeviceToHost, st));
                 HALMA_CUDA(cudaStreamSynchronize(st));
                 if (active == 0) break;
             }
         } else {
-            HALMA_TRY(record(st, 0, p.max_iter));
+            HALMA_TRY(record(st, 0, p.max_iter, false));
         }
         // the halo state already holds the final bound set's mass, centre and bulk velocity
         if (profiling) {
