@@ -72,6 +72,9 @@ typedef void *halma_stream_t;        /* cudaStream_t */
 int         halma_abi_version(void);
 const char *halma_status_string(int status);
 const char *halma_last_error(void);
+/* Members of all groups together (offsets[*n_groups]) that the calling thread's last successful halma_fof_groups or
+ * halma_find_haloes stored, without a copy from the device. */
+int64_t     halma_last_group_members(void);
 int         halma_release_workspace(void);
 /* Number of kernels this library launched since load (all entry points, all devices). */
 int64_t     halma_kernel_launch_count(void);

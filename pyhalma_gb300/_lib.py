@@ -82,6 +82,7 @@ SIGNATURES = {
     "halma_abi_version": ([], ctypes.c_int),
     "halma_status_string": ([ctypes.c_int], ctypes.c_char_p),
     "halma_last_error": ([], ctypes.c_char_p),
+    "halma_last_group_members": ([], ctypes.c_int64),
     "halma_release_workspace": ([], ctypes.c_int),
     "halma_kernel_launch_count": ([], ctypes.c_int64),
     "halma_set_profiling": ([_I32], ctypes.c_int),
@@ -123,6 +124,8 @@ SIGNATURES = {
 def lib():
     """The loaded library; raises ImportError if it has not been built."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is None:
             if not os.path.exists(LIB_PATH):
@@ -248,17 +251,21 @@ def check_arrays(dtype, n, **arrays):
     CUDA device must also be on the current device.  The library reads n elements of that
     type through each raw pointer, so an array of another dtype or length would be read
     past its end."""
+    want = current = None   # the torch type and device, looked up once
     for name, a in arrays.items():
         if a is None:
             continue
         if _is_torch(a):
-            import torch
-            want = getattr(torch, _TORCH_DTYPE_NAMES[np.dtype(dtype).type])
+            if want is None:
+                import torch
+                want = getattr(torch, _TORCH_DTYPE_NAMES[np.dtype(dtype).type])
             if a.dtype != want:
                 raise ValueError(f"{name} must be a {want} tensor, got {a.dtype}")
-            if a.is_cuda and a.device.index != torch.cuda.current_device():
-                raise ValueError(f"{name} is on {a.device}, not on the current device "
-                                 f"cuda:{torch.cuda.current_device()}")
+            if a.is_cuda:
+                if current is None:
+                    current = torch.cuda.current_device()
+                if a.device.index != current:
+                    raise ValueError(f"{name} is on {a.device}, not on the current device cuda:{current}")
         elif not isinstance(a, np.ndarray) or a.dtype != np.dtype(dtype):
             raise ValueError(f"{name} must be a {np.dtype(dtype).name} array or tensor")
         shape = tuple(a.shape)

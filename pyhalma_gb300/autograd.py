@@ -69,8 +69,8 @@ class SoftenedPotential(torch.autograd.Function):
                                                  ctx.eps ** 2, mask, int(ctx.self_offset or 0), _lib.ptr(gm),
                                                  _lib.ptr(gs), _lib.ptr(gt), _lib.stream_of(sx))
         _lib.check(st, "halma_potential_grad_f32")
-        out_s = (gs[:, 0], gs[:, 1], gs[:, 2]) if need_s else (None, None, None)
-        out_t = (gt[:, 0], gt[:, 1], gt[:, 2]) if need_t else (None, None, None)
+        out_s = gs.unbind(1) if need_s else (None, None, None)
+        out_t = gt.unbind(1) if need_t else (None, None, None)
         return (*out_s, gm, *out_t, None, None)
 
 

@@ -10,6 +10,9 @@
 namespace halma {
 
 static thread_local char g_last_error[512] = "";
+static thread_local int64_t g_group_members = 0;
+
+void set_group_members(int64_t n) { g_group_members = n; }
 static std::atomic<int64_t> g_launches{0};
 
 int fail(int status, const char *fmt, ...) {
@@ -124,6 +127,8 @@ const char *halma_status_string(int s) {
 }
 
 const char *halma_last_error(void) { return halma::g_last_error; }
+
+int64_t halma_last_group_members(void) { return halma::g_group_members; }
 
 int64_t halma_kernel_launch_count(void) { return halma::g_launches.load(); }
 

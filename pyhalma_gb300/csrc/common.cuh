@@ -43,6 +43,7 @@ void add_launches(int64_t k);   // graph replays: one count per captured kernel 
 
 int device_sm_count();          // SMs of the current device (cached per device)
 int current_device();
+void set_group_members(int64_t n);   // what halma_last_group_members() returns on this thread
 
 // One process-wide lock serialises the entry points that use the cached workspace.
 std::mutex &api_mutex();

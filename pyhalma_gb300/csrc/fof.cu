@@ -1811,5 +1811,6 @@ extern "C" int halma_fof_groups(int64_t n, const int32_t *labels, int32_t min_me
     }
     if (stage) cudaFreeAsync(stage, st);
     cudaStreamSynchronize(st);
+    set_group_members(nm);
     return s;
 }

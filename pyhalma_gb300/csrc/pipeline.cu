@@ -74,19 +74,32 @@ struct OutCopy {
     size_t bytes;
 };
 
-// The labels and the groups to the caller's buffers (host or device) on the side stream once
-// `groups` has fired, waiting for the copies to end.  Runs on a helper thread while the
+// The copies on the side stream, once `groups` has fired.
+int issue_groups_out(SideStream *side, const OutCopy *outs, int nout) {
+    HALMA_CUDA(cudaStreamWaitEvent(side->s, side->groups, 0));
+    for (int k = 0; k < nout; ++k)
+        if (outs[k].user && outs[k].bytes)
+            HALMA_CUDA(cudaMemcpyAsync(outs[k].user, outs[k].dev, outs[k].bytes, cudaMemcpyDefault, side->s));
+    return HALMA_OK;
+}
+
+// The labels and the groups to the caller's buffers (host or device) on the side stream,
+// waiting for the copies to end.  Runs on a helper thread while the
 // calling thread drives the unbinding: a copy to pageable host memory returns only when it is
 // complete.  (Staging them through pinned memory and a CPU memcpy measured far slower: the
 // CUDA driver's own pageable path writes fresh pages much faster than a memcpy that faults them in.)
 int copy_groups_out(int dev, SideStream *side, const OutCopy *outs, int nout) {
     HALMA_CUDA(cudaSetDevice(dev));
-    HALMA_CUDA(cudaStreamWaitEvent(side->s, side->groups, 0));
-    for (int k = 0; k < nout; ++k)
-        if (outs[k].user && outs[k].bytes)
-            HALMA_CUDA(cudaMemcpyAsync(outs[k].user, outs[k].dev, outs[k].bytes, cudaMemcpyDefault, side->s));
+    HALMA_TRY(issue_groups_out(side, outs, nout));
     HALMA_CUDA(cudaStreamSynchronize(side->s));
     return HALMA_OK;
+}
+
+// Whether every copy that is wanted goes to device memory.
+bool copies_on_device(const OutCopy *outs, int nout) {
+    for (int k = 0; k < nout; ++k)
+        if (outs[k].user && outs[k].bytes && !is_device_pointer(outs[k].user)) return false;
+    return true;
 }
 
 // Joins a helper thread on every way out of the scope that started it.
@@ -193,6 +206,13 @@ extern "C" int halma_find_haloes(int64_t n, const double *x, const double *y, co
     std::thread early;
     JoinOnExit join_early{early};
     const OutCopy outs[3] = {{labels, dlab, 4ull * n}, {halo_offsets, doff, 8ull * (ng + 1)}, {members, dmem, 4ull * nm}};
+    // the offsets are read before anything else is issued, which then runs while the host plans
+    std::vector<int64_t> h_off(ng + 1);
+    if (ng > 0) {
+        HALMA_CUDA(cudaMemcpyAsync(h_off.data(), doff, 8ull * (ng + 1), cudaMemcpyDeviceToHost, st));
+        HALMA_CUDA(cudaStreamSynchronize(st));
+    }
+    HALMA_CUDA(cudaEventRecord(side->groups, st));
     HALMA_CUDA(cudaMemsetAsync(dbnd, 0, n, st));
     // Velocities copied from host memory are waited for only by the first pass's energy
     // kernel (FP32C path): on a slow host link their upload then overlaps the first pass's
@@ -201,7 +221,6 @@ extern "C" int halma_find_haloes(int64_t n, const double *x, const double *y, co
                            (!is_device_pointer(vx) || !is_device_pointer(vy) || !is_device_pointer(vz));
     HALMA_CUDA(cudaStreamWaitEvent(st, defer_vel ? side->mass : side->done, 0));
     const int g = std::min(device_sm_count() * 8, grid_for(std::max<int64_t>(nm, 1), 256));
-    std::vector<int64_t> h_off(ng + 1);
     if (ng > 0) {
         if (defer_vel) {
             HALMA_LAUNCH(gather_kernel<4>, g, 256, 0, st, nm, dmem, (GatherSrc<4>{{dx, dy, dz, dm}, {0, 1, 2, 6}}), g7);
@@ -214,13 +233,13 @@ extern "C" int halma_find_haloes(int64_t n, const double *x, const double *y, co
             HALMA_LAUNCH(gather_kernel<7>, g, 256, 0, st, nm, dmem,
                          (GatherSrc<7>{{dx, dy, dz, dvx, dvy, dvz, dm}, {0, 1, 2, 3, 4, 5, 6}}), g7);
         }
-        HALMA_CUDA(cudaMemcpyAsync(h_off.data(), doff, 8ull * (ng + 1), cudaMemcpyDeviceToHost, st));
-        HALMA_CUDA(cudaStreamSynchronize(st));
     }
-    // started only now, so that the halo offsets above did not queue behind them on the
-    // device-to-host copy engine
-    if (fits) {
-        HALMA_CUDA(cudaEventRecord(side->groups, st));
+    // Started only now, so that the halo offsets above did not queue behind them on the
+    // device-to-host copy engine.  Copies within the device do not wait for one another on the host and
+    // need no thread, which takes 30 us to start.
+    if (fits && copies_on_device(outs, 3)) {
+        HALMA_TRY(issue_groups_out(side, outs, 3));
+    } else if (fits) {
         const int dev = current_device();
         early = std::thread([&, dev]() {
             early_status = copy_groups_out(dev, side, outs, 3);
@@ -262,7 +281,9 @@ extern "C" int halma_find_haloes(int64_t n, const double *x, const double *y, co
     }
     HALMA_TRY(put(halo_out, dhalo, 8ull * HALMA_UB_NFIELDS * ng));
     HALMA_CUDA(cudaStreamSynchronize(st));
-    early.join();
+    if (early.joinable()) early.join();
+    else HALMA_CUDA(cudaStreamSynchronize(side->s));
+    set_group_members(nm);
     if (early_status != HALMA_OK) return fail(early_status, "%s", early_msg.c_str());
     return HALMA_OK;
 }

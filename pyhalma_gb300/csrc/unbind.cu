@@ -1705,6 +1705,7 @@ struct GraphCache {
         int64_t nodes = 0;
     };
     std::vector<Entry> chunks;
+    std::vector<cudaGraphExec_t> old;   // of the key before, destroyed once the first chunk has been launched
     std::vector<uintptr_t> key;
     cudaStream_t capture_stream = nullptr;
     int capture_device = -1;
@@ -2111,7 +2112,7 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
             const bool again = gc.key == key;
             if (!again) {
                 for (auto &e : gc.chunks)
-                    if (e.exec) cudaGraphExecDestroy(e.exec);
+                    if (e.exec) gc.old.push_back(e.exec);
                 gc.chunks.clear();
                 gc.key = key;
             }
@@ -2161,6 +2162,8 @@ int unbind_device(int64_t n, int nh, const int64_t *d_off, const int64_t *h_off,
                 } else {
                     HALMA_TRY(record(st, chunk_start(ci), chunk_start(next_chunk(ci)), false));
                 }
+                for (cudaGraphExec_t e : gc.old) cudaGraphExecDestroy(e);   // 100 us of the host's time
+                gc.old.clear();
                 passes_run = chunk_start(next_chunk(ci));
                 if (passes_run >= p.max_iter) break;
                 HALMA_TRY(capture(next_chunk(ci)));   // while this one runs

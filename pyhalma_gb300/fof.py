@@ -79,7 +79,7 @@ def fof_groups(labels, min_members=2):
     _lib.check(st, "halma_fof_groups")
     g = int(ng.value)
     offsets = offsets[: g + 1]
-    return offsets, members[: int(offsets[-1])] if g > 0 else members[:0]
+    return offsets, members[: _lib.lib().halma_last_group_members()] if g > 0 else members[:0]
 
 
 def _split(offsets, members):

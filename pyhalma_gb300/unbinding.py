@@ -128,5 +128,5 @@ def find_haloes(st_x, st_y, st_z, st_vx, st_vy, st_vz, st_mass, linking_length, 
     _lib.check(st, "halma_find_haloes")
     g = int(nh.value)
     offsets = offsets[: g + 1]
-    nm = int(offsets[-1]) if g > 0 else 0
+    nm = _lib.lib().halma_last_group_members() if g > 0 else 0
     return HaloCatalogue(labels, bound, offsets, members[:nm], haloes[:g])
