@@ -433,6 +433,7 @@ __global__ void __launch_bounds__(256) pr_kin2_kernel(int G, int S, const int64_
 // --- projected dispersion, V/sigma and lambda (f90:217-461), FP32 -----------------------
 struct ProjGrid {
     double start, next, delta, step;
+    double inv;   // 1 / step, 0 for grids whose FP32 values may coincide (minloc32 then divides)
     long long n;
 };
 
@@ -446,6 +447,7 @@ __device__ __forceinline__ ProjGrid proj_grid(double rmax, double ll) {
     p.delta = __dsub_rn(p.next, p.start);
     p.n = (long long)ceil(__ddiv_rn(__dsub_rn(stop, p.start), p.step));
     if (p.n < 1) p.n = 1;
+    p.inv = p.n < (1 << 20) && p.step > 1e-300 ? 1.0 / p.step : 0.0;
     return p;
 }
 
@@ -456,7 +458,9 @@ __device__ __forceinline__ float grid32(const ProjGrid &p, long long i) {
 
 // minloc(abs(grid - v)): first index of the smallest |grid(i) - v| in FP32
 __device__ __forceinline__ int minloc32(const ProjGrid &p, float v) {
-    long long k = (long long)floor(((double)v - p.start) / p.step + 0.5);
+    // either rounding of the quotient leaves the nearest value among the three looked at
+    const double q0 = (double)v - p.start;
+    long long k = (long long)floor((p.inv != 0.0 ? q0 * p.inv : q0 / p.step) + 0.5);
     k = k < 0 ? 0 : (k > p.n - 1 ? p.n - 1 : k);
     long long best = k;
     float bd = fabsf(__fsub_rn(grid32(p, k), v));
@@ -471,16 +475,27 @@ __device__ __forceinline__ int minloc32(const ProjGrid &p, float v) {
     return (int)best;
 }
 
+// Results of a group's projection.
+constexpr int kResSig05 = 0, kResVsigma = 1, kResLambda = 2, kResR05 = 3, kRes = 4;
+
+// A group's grid, formed once (with its division per member, and one per coordinate in minloc32,
+// pr_pkeys_kernel took 76 us for 4e5 members, without 47).
+__global__ void pr_grid_kernel(int G, const double *__restrict__ cen, double ll, ProjGrid *__restrict__ grid) {
+    for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < G; h += gridDim.x * blockDim.x)
+        grid[h] = proj_grid(cen[(int64_t)h * kCenFields + 4], ll);
+}
+
 // Per member and projection: the cell (inner + outer * n, inner running fastest as in the
 // Fortran loops of the V/sigma sums) and the sort key (group, projection, cell).
 //   projection 0 (x, plane YZ): cell (iy, iz);  1 (y, XZ): (ix, iz);  2 (z, XY): (ix, iy)
 __global__ void pr_pkeys_kernel(int64_t nm, int G, const int64_t *__restrict__ off, const int *__restrict__ owner,
-                                const double *__restrict__ g, const double *__restrict__ cen, double ll, int cbits,
-                                uint64_t *__restrict__ keys, int *__restrict__ vals) {
+                                const double *__restrict__ g, const double *__restrict__ cen,
+                                const ProjGrid *__restrict__ grid, int cbits, uint64_t *__restrict__ keys,
+                                int *__restrict__ vals) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nm; k += (int64_t)gridDim.x * blockDim.x) {
         const int h = owner[k];
         const double *c = cen + (int64_t)h * kCenFields;
-        const ProjGrid p = proj_grid(c[4], ll);
+        const ProjGrid p = grid[h];
         const int ix = minloc32(p, __fsub_rn((float)g[k], (float)c[0]));
         const int iy = minloc32(p, __fsub_rn((float)g[nm + k], (float)c[1]));
         const int iz = minloc32(p, __fsub_rn((float)g[2 * nm + k], (float)c[2]));
@@ -498,49 +513,60 @@ __global__ void pr_head_kernel(int64_t n, const uint64_t *__restrict__ keys, int
         head[k] = (k == 0 || keys[k] != keys[k - 1]) ? 1 : 0;
 }
 
-// Cell starts: runstart[r] = first sorted entry of cell r, runstart[ncell] = n3.
-__global__ void pr_runstart_kernel(int64_t n3, const int *__restrict__ head, const int *__restrict__ rpos,
-                                   int *__restrict__ runstart) {
+// Per sorted entry: cell starts (runstart[r] = first entry of cell r, runstart[cells] = n3; the number of cells in
+// *ncell), the cell of every member entry (rid), and what the cell's sums need, velocity relative to the group's
+// and mass in FP32, in the order of the cells.
+// The scattered reads are all here, an entry a lane: read by the warps that add up a cell, 32 members after 32,
+// they kept the cells of a halo's centre (2,000 members) waiting for 63 round trips, twice.
+__global__ void pr_entries_kernel(int64_t n3, int64_t nm, int cbits, const uint64_t *__restrict__ keys,
+                                  const int *__restrict__ vals, const int *__restrict__ head,
+                                  const int *__restrict__ rpos, const double *__restrict__ g,
+                                  const double *__restrict__ out, int *__restrict__ runstart, int *__restrict__ rid,
+                                  float2 *__restrict__ entry, int *__restrict__ ncell) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n3; k += (int64_t)gridDim.x * blockDim.x) {
-        if (head[k]) runstart[rpos[k]] = (int)k;
-        if (k == n3 - 1) runstart[rpos[k] + head[k]] = (int)n3;
+        const int r = rpos[k] + head[k] - 1;
+        if (head[k]) runstart[r] = (int)k;
+        if (k == n3 - 1) {
+            runstart[r + 1] = (int)n3;
+            *ncell = r + 1;
+        }
+        const unsigned set = (unsigned)(keys[k] >> cbits), h = set / 3, a = set - 3 * h;
+        const int v = vals[k], mk = v - (int)(a * nm);
+        entry[k] = make_float2((float)__dsub_rn(g[(3 + a) * nm + mk],
+                                                out[(int64_t)h * HALMA_PROP_NFIELDS + HALMA_PROP_VX + a]),
+                               (float)g[6 * nm + mk]);
+        rid[v] = r;
     }
 }
 
 // Per cell: FP32 mass SD, mass-weighted velocity VCM (then / SD), count, and
-// sigma = sqrt(sum (v - VCM)^2 / count), members in order; rid[member entry] = cell.  Cells of at most kLaneCell
-// members take a lane each (most cells hold one or two members: a warp per cell waited on its few gathers with
-// 31 lanes idle), the others, neighbours mostly, a warp each in a second loop: 32 members loaded at a
-// time, every lane adding them one by one (shuffles), so that the sums are the sequential ones.
+// sigma = sqrt(sum (v - VCM)^2 / count), members in order.  Cells of at most kLaneCell members take a lane
+// each (most cells hold one or two members: a warp per cell waited with 31 lanes idle), the others, neighbours
+// mostly, a warp each in a second loop: 32 members loaded at a time, every lane adding them one by one (shuffles), so
+// that the sums are the sequential ones.  With the entries in order (pr_entries_kernel) 4e5 members take
+// 61 us and the entries 13; gathering them here took 141.
 constexpr int kLaneCell = 8;
 
-__global__ void __launch_bounds__(256) pr_cells_kernel(int ncell, int64_t nm, const int *__restrict__ runstart,
-                                const uint64_t *__restrict__ keys, const int *__restrict__ vals,
-                                const int *__restrict__ owner, const double *__restrict__ g,
-                                const double *__restrict__ out, float4 *__restrict__ cellv,
-                                uint64_t *__restrict__ cellkey, int *__restrict__ rid) {
+__global__ void __launch_bounds__(256) pr_cells_kernel(const int *__restrict__ ncell_p,
+                                                       const int *__restrict__ runstart,
+                                                       const uint64_t *__restrict__ keys,
+                                                       const float2 *__restrict__ entry, float4 *__restrict__ cellv,
+                                                       uint64_t *__restrict__ cellkey) {
     const int lane = threadIdx.x & 31;
+    const int ncell = *ncell_p;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    // member entry k of projection a: velocity relative to the group's, and mass
-    auto member = [&](int k, int a, int64_t r, float &v, float &m) {
-        const int mk = vals[k] - a * (int)nm;
-        v = (float)__dsub_rn(g[(3 + a) * nm + mk], out[(int64_t)owner[mk] * HALMA_PROP_NFIELDS + HALMA_PROP_VX + a]);
-        m = (float)g[6 * nm + mk];
-        rid[vals[k]] = (int)r;
-    };
     const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     for (int64_t r = w0 * 32 + lane; r < ncell; r += warps * 32) {
         const int b = runstart[r], e = runstart[r + 1];
         if (e - b > kLaneCell) continue;
-        const int a = vals[b] / (int)nm;   // projection of the cell
         float v[kLaneCell], sd = 0.f, vc = 0.f, s2 = 0.f;
 #pragma unroll
         for (int k = 0; k < kLaneCell; ++k) {
             if (b + k >= e) break;
-            float m;
-            member(b + k, a, r, v[k], m);
-            vc = __fadd_rn(vc, __fmul_rn(v[k], m));
-            sd = __fadd_rn(sd, m);
+            const float2 q = entry[b + k];
+            v[k] = q.x;
+            vc = __fadd_rn(vc, __fmul_rn(q.x, q.y));
+            sd = __fadd_rn(sd, q.y);
         }
         if (sd != 0.f) vc = __fdiv_rn(vc, sd);
 #pragma unroll
@@ -559,12 +585,12 @@ __global__ void __launch_bounds__(256) pr_cells_kernel(int ncell, int64_t nm, co
             const int l = __ffs(todo) - 1;
             const int64_t rr = r0 + warps * l;
             const int bb = __shfl_sync(0xffffffffu, b, l), ee = __shfl_sync(0xffffffffu, e, l);
-            const int aa = vals[bb] / (int)nm;   // projection of the cell
+            auto load = [&](int k) { return k < ee ? entry[k] : make_float2(0.f, 0.f); };
             float sd = 0.f, vc = 0.f, s2 = 0.f;
+            float2 next = load(bb + lane);
             for (int k0 = bb; k0 < ee; k0 += 32) {
-                float v = 0.f, m = 0.f;
-                if (k0 + lane < ee) member(k0 + lane, aa, rr, v, m);
-                const float vm = __fmul_rn(v, m);
+                const float vm = __fmul_rn(next.x, next.y), m = next.y;
+                next = load(k0 + 32 + lane);
                 const int cnt = ee - k0 < 32 ? ee - k0 : 32;
                 for (int t0 = 0; t0 < cnt; t0 += 8) {   // lanes past the end hold zeros, which change neither sum
 #pragma unroll
@@ -575,14 +601,11 @@ __global__ void __launch_bounds__(256) pr_cells_kernel(int ncell, int64_t nm, co
                 }
             }
             if (sd != 0.f) vc = __fdiv_rn(vc, sd);
+            next = load(bb + lane);
             for (int k0 = bb; k0 < ee; k0 += 32) {
-                float d2 = 0.f;
-                if (k0 + lane < ee) {
-                    float v, m;
-                    member(k0 + lane, aa, rr, v, m);
-                    const float d = __fsub_rn(v, vc);
-                    d2 = __fmul_rn(d, d);
-                }
+                const float d = __fsub_rn(next.x, vc);
+                const float d2 = k0 + lane < ee ? __fmul_rn(d, d) : 0.f;
+                next = load(k0 + 32 + lane);
                 const int cnt = ee - k0 < 32 ? ee - k0 : 32;
                 for (int t0 = 0; t0 < cnt; t0 += 8)
 #pragma unroll
@@ -596,146 +619,153 @@ __global__ void __launch_bounds__(256) pr_cells_kernel(int ncell, int64_t nm, co
     }
 }
 
-__device__ __forceinline__ int lower_bound_key(const uint64_t *__restrict__ keys, int n, uint64_t k) {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (keys[mid] < k) lo = mid + 1;
-        else hi = mid;
+// First position of keys[0..n) that is not below k, by a warp: 32 probes at a time.
+__device__ __forceinline__ int warp_lower_bound(const uint64_t *__restrict__ keys, int n, uint64_t k, int lane) {
+    int lo = 0, hi = n;   // keys before lo are below k, those from hi on are not
+    while (hi > lo) {
+        const int step = (hi - lo + 31) / 32;
+        const int64_t at = lo + (int64_t)(lane + 1) * step - 1;
+        const int below = __popc(__ballot_sync(0xffffffffu, at < hi && keys[at < hi ? at : lo] < k));
+        const int64_t first = lo + (int64_t)below * step;   // the next probe, or the end, is not below k
+        hi = (int)std::min<int64_t>(hi, first + step - 1);
+        lo = (int)std::min<int64_t>(first, hi);
     }
     return lo;
 }
 
-// Block per group: per projection the mean cell sigma over the members inside the projected
-// half-mass radius (members in order), and the V/sigma and lambda sums over the group's cells
-// with R_cell < R05 + 2 ll in the Fortran's loop order.  Tiles of members (then of cells) are
-// staged in shared memory by the whole block; each sum is then added in order by one thread
-// (three for the sigma sums, four per projection for the V/sigma and lambda sums).
+// The projections' sums: sig05, the mean cell sigma over the members inside the projected half-mass radius (members
+// in order), and the V/sigma and lambda sums over the group's cells with R_cell < R05 + 2 ll in the Fortran's
+// loop order.  Tiles of members (or of cells) are staged in shared memory by seven warps while the first adds the tile
+// before, each sum in order by one thread (sig05 one; four for V/sigma and lambda).
+// Bound: the longest group's chains of additions (4 cycles each).  Every group has six blocks, one for either kind of sum and
+// each projection: as one block, sig05 first and the projections after one another, the group of 19,500
+// members took 198 us, so 101.
 __global__ void __launch_bounds__(256) pr_proj_kernel(int G, int64_t nm, const int64_t *__restrict__ off,
                                                       const double *__restrict__ g, const double *__restrict__ cen,
-                                                      double ll, int cbits, const int *__restrict__ rid,
-                                                      const float4 *__restrict__ cellv,
-                                                      const uint64_t *__restrict__ cellkey, int ncell,
-                                                      float *__restrict__ res /* G x 3 x 3 */) {
+                                                      const ProjGrid *__restrict__ grid, double ll, int cbits,
+                                                      const int *__restrict__ rid, const float4 *__restrict__ cellv,
+                                                      const uint64_t *__restrict__ cellkey,
+                                                      const int *__restrict__ ncell,
+                                                      float *__restrict__ res /* G x 3 x kRes */) {
     constexpr int kRow = kTile + 8;       // rows start in different banks
-    __shared__ float terms[2][4][kRow];   // one tile filled while the other is added
-    float (*const term)[kRow] = terms[0];
-    __shared__ float red[12];
+    __shared__ float term[2][4][kRow];    // one tile filled while the other is added
+    __shared__ float red[4];
+    __shared__ int range[2];
     const int t = threadIdx.x;
-    for (int h = blockIdx.x; h < G; h += gridDim.x) {
-        const double *c = cen + (int64_t)h * kCenFields;
-        const ProjGrid p = proj_grid(c[4], ll);
-        const float cx = (float)c[0], cy = (float)c[1], cz = (float)c[2];
-        float r05[3];
-        for (int a = 0; a < 3; ++a) r05[a] = res[((int64_t)h * 3 + a) * 3];
-        // mean cell sigma inside R05: term[a] = the member's cell sigma (or -1 outside)
-        float s05 = 0.f;
-        int cnt = 0;
-        auto fill = [&](int64_t b, float (*to)[kRow], int first, int step) {
-            const int nt = (off[h + 1] - b < kTile ? (int)(off[h + 1] - b) : kTile);
-#pragma unroll 2
-            for (int q = first; q < ((nt + 7) & ~7); q += step) {
-                const int64_t k = b + q;
-                if (q >= nt) {
-                    to[0][q] = to[1][q] = to[2][q] = -1.f;
-                    continue;
-                }
-                const float dx = __fsub_rn((float)g[k], cx), dy = __fsub_rn((float)g[nm + k], cy),
-                            dz = __fsub_rn((float)g[2 * nm + k], cz);
-                const float d2[3] = {__fadd_rn(__fmul_rn(dy, dy), __fmul_rn(dz, dz)),
-                                     __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dz, dz)),
-                                     __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy))};
-                for (int a = 0; a < 3; ++a)
-                    to[a][q] = __fsqrt_rn(d2[a]) < r05[a] ? cellv[rid[a * nm + k]].z : -1.f;
-            }
-        };
-        fill(off[h], terms[0], t, blockDim.x);
-        __syncthreads();
-        int cur = 0;
-        for (int64_t b = off[h]; b < off[h + 1]; b += kTile, cur ^= 1) {
-            const int nt = (off[h + 1] - b < kTile ? (int)(off[h + 1] - b) : kTile);
-            if (t >= 32) {
-                if (b + kTile < off[h + 1]) fill(b + kTile, terms[cur ^ 1], t - 32, blockDim.x - 32);
-            } else if (t < 3) {   // eight loads ahead of their additions; an excluded term adds +0, which changes nothing
-                for (int q = 0; q < nt; q += 8) {
-                    float p[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        p[u] = terms[cur][t][q + u];
-                        const bool in = p[u] >= 0.f;
-                        p[u] = in ? p[u] : 0.f;
-                        cnt += in ? 1 : 0;
+    for (int64_t item = blockIdx.x; item < 6ll * G; item += gridDim.x) {
+        const int h = (int)(item / 6), a = (int)(item % 6) >> 1;
+        float *o = res + ((int64_t)h * 3 + a) * kRes;
+        const float r05 = o[kResR05];
+        if (item & 1) {   // sig05: term 0 = the member's cell sigma, or -1 outside
+            const double *c = cen + (int64_t)h * kCenFields;
+            const int u = a == 0 ? 1 : 0, v = a == 2 ? 1 : 2;   // the projection's two coordinates
+            const float cu = (float)c[u], cv = (float)c[v];
+            auto fill = [&](int64_t b, float *to, int first, int step) {
+                const int nt = (off[h + 1] - b < kTile ? (int)(off[h + 1] - b) : kTile);
+#pragma unroll 4
+                for (int q = first; q < ((nt + 7) & ~7); q += step) {
+                    const int64_t k = b + q;
+                    if (q >= nt) {
+                        to[q] = -1.f;
+                        continue;
                     }
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) s05 = __fadd_rn(s05, p[u]);
+                    const float du = __fsub_rn((float)g[u * nm + k], cu), dv = __fsub_rn((float)g[v * nm + k], cv);
+                    const float d2 = __fadd_rn(__fmul_rn(du, du), __fmul_rn(dv, dv));
+                    to[q] = __fsqrt_rn(d2) < r05 ? cellv[rid[a * nm + k]].z : -1.f;
                 }
-            }
+            };
+            float s05 = 0.f;
+            int cnt = 0;
+            fill(off[h], term[0][0], t, blockDim.x);
             __syncthreads();
-        }
-        if (t < 3) red[t] = cnt > 0 ? __fdiv_rn(s05, (float)cnt) : s05;
-        __syncthreads();
-        // V/sigma and lambda per projection: term[q] of every cell of the tile (0 outside)
-        for (int a = 0; a < 3; ++a) {
-            const float lim = __fadd_rn(r05[a], __fmul_rn(2.f, (float)ll));
-            const uint64_t k0 = (uint64_t)(3 * (int64_t)h + a) << cbits, k1 = (uint64_t)(3 * (int64_t)h + a + 1) << cbits;
-            __shared__ int range[2];
-            if (t == 0) {
-                int lo = 0, hi = ncell;
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (cellkey[mid] < k0) lo = mid + 1;
-                    else hi = mid;
-                }
-                int e = lo, hi2 = ncell;
-                while (e < hi2) {
-                    const int mid = (e + hi2) >> 1;
-                    if (cellkey[mid] < k1) e = mid + 1;
-                    else hi2 = mid;
-                }
-                range[0] = lo;
-                range[1] = e;
-            }
-            __syncthreads();
-            const int r0 = range[0], r1 = range[1];
-            float sum = 0.f;   // thread q < 4: sumV, sumSigma, sumUp, sumDown
-            for (int b = r0; b < r1; b += kTile) {
-                const int nt = min(kTile, r1 - b);
-                for (int q = t; q < nt; q += blockDim.x) {
-                    const int r = b + q;
-                    const uint64_t cell = cellkey[r] - k0;
-                    const float gi = grid32(p, (long long)(cell % (uint64_t)p.n)),
-                                go = grid32(p, (long long)(cell / (uint64_t)p.n));
-                    const float rbin = __fsqrt_rn(__fadd_rn(__fmul_rn(gi, gi), __fmul_rn(go, go)));
-                    const float4 cv = cellv[r];   // (SD, VCM, SIG)
-                    const bool in = rbin < lim;
-                    term[0][q] = in ? __fmul_rn(__fmul_rn(cv.y, cv.y), cv.x) : -1.f;
-                    term[1][q] = __fmul_rn(__fmul_rn(cv.z, cv.z), cv.x);
-                    term[2][q] = __fmul_rn(__fmul_rn(cv.x, rbin), fabsf(cv.y));
-                    term[3][q] = __fmul_rn(__fmul_rn(cv.x, rbin),
-                                           __fsqrt_rn(__fadd_rn(__fmul_rn(cv.y, cv.y), __fmul_rn(cv.z, cv.z))));
-                }
-                if (t < 8 && nt + t < ((nt + 7) & ~7)) term[0][nt + t] = -1.f;
-                __syncthreads();
-                if (t < 4)
+            int cur = 0;
+            for (int64_t b = off[h]; b < off[h + 1]; b += kTile, cur ^= 1) {
+                const int nt = (off[h + 1] - b < kTile ? (int)(off[h + 1] - b) : kTile);
+                if (t >= 32) {
+                    if (b + kTile < off[h + 1]) fill(b + kTile, term[cur ^ 1][0], t - 32, blockDim.x - 32);
+                } else if (t == 0) {   // eight loads ahead of their additions; an excluded term adds +0, which changes nothing
                     for (int q = 0; q < nt; q += 8) {
                         float p[8];
 #pragma unroll
-                        for (int u = 0; u < 8; ++u) p[u] = term[0][q + u] >= 0.f ? term[t][q + u] : 0.f;
+                        for (int w = 0; w < 8; ++w) {
+                            p[w] = term[cur][0][q + w];
+                            const bool in = p[w] >= 0.f;
+                            p[w] = in ? p[w] : 0.f;
+                            cnt += in ? 1 : 0;
+                        }
 #pragma unroll
-                        for (int u = 0; u < 8; ++u) sum = __fadd_rn(sum, p[u]);
+                        for (int w = 0; w < 8; ++w) s05 = __fadd_rn(s05, p[w]);
                     }
+                }
                 __syncthreads();
             }
-            if (t < 4) red[3 + t] = sum;
-            __syncthreads();
-            if (t == 0) {
-                float *o = res + ((int64_t)h * 3 + a) * 3;
-                o[0] = red[a];
-                o[1] = red[4] > 0.f ? __fsqrt_rn(__fdiv_rn(red[3], red[4])) : 0.f;
-                o[2] = red[6] > 0.f ? __fdiv_rn(red[5], red[6]) : 0.f;
+            if (t == 0) o[kResSig05] = cnt > 0 ? __fdiv_rn(s05, (float)cnt) : s05;
+        } else {   // V/sigma and lambda: term[q] of every cell of the tile (0 outside)
+            const ProjGrid p = grid[h];
+            const float lim = __fadd_rn(r05, __fmul_rn(2.f, (float)ll));
+            const uint64_t set = 3 * (uint64_t)h + a, k0 = set << cbits;
+            if (t < 64) {   // the set's cells
+                const int at = warp_lower_bound(cellkey, *ncell, (set + (t >> 5)) << cbits, t & 31);
+                if ((t & 31) == 0) range[t >> 5] = at;
             }
             __syncthreads();
+            const int r0 = range[0], r1 = range[1];
+            const bool narrow = p.n < 65536;   // cell < n^2: 32-bit division
+            auto fill = [&](int b, float (*to)[kRow], int first, int step) {
+                const int nt = min(kTile, r1 - b);
+                for (int q = first; q < ((nt + 7) & ~7); q += step) {
+                    if (q >= nt) {
+                        to[0][q] = to[1][q] = to[2][q] = to[3][q] = 0.f;
+                        continue;
+                    }
+                    const uint64_t cell = cellkey[b + q] - k0;
+                    const float4 cv = cellv[b + q];   // (SD, VCM, SIG)
+                    long long in, io;
+                    if (narrow) {
+                        io = (unsigned)cell / (unsigned)p.n;
+                        in = (unsigned)cell - (unsigned)io * (unsigned)p.n;
+                    } else {
+                        io = (long long)(cell / (uint64_t)p.n);
+                        in = (long long)(cell % (uint64_t)p.n);
+                    }
+                    const float gi = grid32(p, in), go = grid32(p, io);
+                    const float rbin = __fsqrt_rn(__fadd_rn(__fmul_rn(gi, gi), __fmul_rn(go, go)));
+                    const bool inside = rbin < lim && __fmul_rn(__fmul_rn(cv.y, cv.y), cv.x) >= 0.f;
+                    to[0][q] = inside ? __fmul_rn(__fmul_rn(cv.y, cv.y), cv.x) : 0.f;
+                    to[1][q] = inside ? __fmul_rn(__fmul_rn(cv.z, cv.z), cv.x) : 0.f;
+                    to[2][q] = inside ? __fmul_rn(__fmul_rn(cv.x, rbin), fabsf(cv.y)) : 0.f;
+                    to[3][q] = inside ? __fmul_rn(__fmul_rn(cv.x, rbin),
+                                                  __fsqrt_rn(__fadd_rn(__fmul_rn(cv.y, cv.y), __fmul_rn(cv.z, cv.z))))
+                                      : 0.f;
+                }
+            };
+            float sum = 0.f;   // thread q < 4: sumV, sumSigma, sumUp, sumDown
+            if (r0 < r1) fill(r0, term[0], t, blockDim.x);
+            __syncthreads();
+            int cur = 0;
+            for (int b = r0; b < r1; b += kTile, cur ^= 1) {
+                const int nt = min(kTile, r1 - b);
+                if (t >= 32) {
+                    if (b + kTile < r1) fill(b + kTile, term[cur ^ 1], t - 32, blockDim.x - 32);
+                } else if (t < 4) {
+                    for (int q = 0; q < nt; q += 8) {
+                        float w[8];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) w[u] = term[cur][t][q + u];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) sum = __fadd_rn(sum, w[u]);
+                    }
+                }
+                __syncthreads();
+            }
+            if (t < 4) red[t] = sum;
+            __syncthreads();
+            if (t == 0) {
+                o[kResVsigma] = red[1] > 0.f ? __fsqrt_rn(__fdiv_rn(red[0], red[1])) : 0.f;
+                o[kResLambda] = red[3] > 0.f ? __fdiv_rn(red[2], red[3]) : 0.f;
+            }
         }
+        __syncthreads();   // the shared arrays are reused
     }
 }
 
@@ -755,7 +785,7 @@ __global__ void pr_r05_kernel(int G, const double *__restrict__ red /* 4 x G x N
         for (int a = 0; a < 3; ++a) {
             const double r = red[((int64_t)(a + 1) * G + h) * HALMA_RED_NFIELDS + HALMA_RED_R05];
             o[HALMA_PROP_R05X + a] = r;
-            res[((int64_t)h * 3 + a) * 3] = (float)r;
+            res[((int64_t)h * 3 + a) * kRes + kResR05] = (float)r;
         }
     }
 }
@@ -763,13 +793,14 @@ __global__ void pr_r05_kernel(int G, const double *__restrict__ red /* 4 x G x N
 __global__ void pr_proj_out_kernel(int G, const float *__restrict__ res, double *__restrict__ out) {
     for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < G; h += gridDim.x * blockDim.x) {
         double *o = out + (int64_t)h * HALMA_PROP_NFIELDS;
-        const float *r = res + (int64_t)h * 9;   // [projection][sig05, vsigma, lambda]
-        o[HALMA_PROP_SIG1DX] = r[0];
-        o[HALMA_PROP_SIG1DY] = r[3];
-        o[HALMA_PROP_SIG1DZ] = r[6];
+        const float *r = res + (int64_t)h * 3 * kRes;
+        o[HALMA_PROP_SIG1DX] = r[kResSig05];
+        o[HALMA_PROP_SIG1DY] = r[kRes + kResSig05];
+        o[HALMA_PROP_SIG1DZ] = r[2 * kRes + kResSig05];
         // (V_sigma_x + V_sigma_y + V_sigma_z) / 3. and the same for lambda (f90:456-457)
-        o[HALMA_PROP_VSIGMA] = __fdiv_rn(__fadd_rn(__fadd_rn(r[1], r[4]), r[7]), 3.f);
-        o[HALMA_PROP_LAMBDA] = __fdiv_rn(__fadd_rn(__fadd_rn(r[2], r[5]), r[8]), 3.f);
+        auto mean = [&](int f) { return __fdiv_rn(__fadd_rn(__fadd_rn(r[f], r[kRes + f]), r[2 * kRes + f]), 3.f); };
+        o[HALMA_PROP_VSIGMA] = mean(kResVsigma);
+        o[HALMA_PROP_LAMBDA] = mean(kResLambda);
     }
 }
 
@@ -887,8 +918,9 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
     const size_t o_kin = L.add(8ull * N3), o_kout = L.add(8ull * N3), o_vin = L.add(4ull * (N3 + 1)),
                  o_vout = L.add(4ull * N3);
     const size_t o_head = L.add(4ull * N3), o_rpos = L.add(4ull * N3), o_rid = L.add(4ull * N3);
-    const size_t o_cv = L.add(16ull * N3), o_ck = L.add(8ull * N3), o_res = L.add(4ull * 9 * G), o_cnt = L.add(64);
+    const size_t o_cv = L.add(16ull * N3), o_ck = L.add(8ull * N3), o_res = L.add(4ull * 3 * kRes * G), o_cnt = L.add(64);
     const int S = G >= 8192 ? 1 : (G >= 1024 ? 16 : 64);   // blocks per group at most for the angular-momentum kernels
+    const size_t o_grid = L.add(sizeof(ProjGrid) * G);
     const size_t o_kp = L.add(32ull * S * G), o_kctr = L.add(4ull * G), o_jv = L.add(64ull * G);
     const size_t sort_b = sort_pairs_u64_i32_bytes((int)N3, 64), scan_b = exclusive_sum_i32_bytes((int)N3);
     const size_t o_tmp = L.add(std::max(sort_b, scan_b));
@@ -904,6 +936,7 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
     auto *cellkey = at<uint64_t>(base, o_ck);
     float *res = at<float>(base, o_res);
     int *cnt = at<int>(base, o_cnt);
+    auto *grid = at<ProjGrid>(base, o_grid);
     double *kpart = at<double>(base, o_kp), *jvec = at<double>(base, o_jv);
     int *kctr = at<int>(base, o_kctr);
     void *tmp = at<void>(base, o_tmp);
@@ -953,27 +986,24 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
     HALMA_CUDA(cudaStreamWaitEvent(st, side->done, 0));
     HALMA_LAUNCH(pr_kin2_kernel, G * S, 256, 0, st, G, S, doff, gbuf, NM, dcen, dout, kpart, kctr, jvec);
     if (N0 > 0) {
-        HALMA_LAUNCH(pr_pkeys_kernel, gN, 256, 0, st, N0, G, doff, own, gbuf, dcen, linking_length, cbits, kin, vin);
+        HALMA_LAUNCH(pr_grid_kernel, gH, 128, 0, st, G, dcen, linking_length, grid);
+        HALMA_LAUNCH(pr_pkeys_kernel, gN, 256, 0, st, N0, G, doff, own, gbuf, dcen, grid, cbits, kin, vin);
         const int n3 = (int)(3 * N0);
         const int g3 = std::min(sms * 8, grid_for(n3, 256));
         // keys hold (3 group + projection) above cbits of cell index: sort only those bits
         HALMA_TRY(sort_pairs_u64_i32(tmp, sort_b, kin, kout, vin, vout, n3, cbits + nbits((uint64_t)3 * G), st));
         HALMA_LAUNCH(pr_head_kernel, g3, 256, 0, st, n3, kout, head);
         HALMA_TRY(exclusive_sum_i32(tmp, scan_b, head, rpos, n3, st));
-        int last[2];
-        HALMA_CUDA(cudaMemcpyAsync(&last[0], rpos + n3 - 1, 4, cudaMemcpyDeviceToHost, st));
-        HALMA_CUDA(cudaMemcpyAsync(&last[1], head + n3 - 1, 4, cudaMemcpyDeviceToHost, st));
-        HALMA_CUDA(cudaStreamSynchronize(st));
-        const int ncell = last[0] + last[1];
-        int *runstart = vin;   // the sort's input values are no longer needed
-        HALMA_LAUNCH(pr_runstart_kernel, g3, 256, 0, st, n3, head, rpos, runstart);
-        HALMA_LAUNCH(pr_cells_kernel, sms * 16, 256, 0, st, ncell, N0, runstart, kout, vout, own, gbuf, dout, cellv,
-                     cellkey, rid);
-        HALMA_LAUNCH(pr_proj_kernel, gG, 256, 0, st, G, N0, doff, gbuf, dcen, linking_length, cbits, rid, cellv,
-                     cellkey, ncell, res);
+        // the sort's input is no longer needed
+        int *runstart = vin;
+        auto *entry = reinterpret_cast<float2 *>(kin);
+        HALMA_LAUNCH(pr_entries_kernel, g3, 256, 0, st, n3, N0, cbits, kout, vout, head, rpos, gbuf, dout, runstart, rid,
+                     entry, cnt);
+        HALMA_LAUNCH(pr_cells_kernel, sms * 16, 256, 0, st, cnt, runstart, kout, entry, cellv, cellkey);
+        HALMA_LAUNCH(pr_proj_kernel, (int)std::min<int64_t>(6ll * G, sms * 16), 256, 0, st, G, N0, doff, gbuf, dcen, grid,
+                     linking_length, cbits, rid, cellv, cellkey, cnt, res);
         HALMA_LAUNCH(pr_proj_out_kernel, gH, 128, 0, st, G, res, dout);
     }
-    (void)cnt;
     HALMA_TRY(sg.download(st));
     HALMA_CUDA(cudaStreamSynchronize(st));
     return HALMA_OK;

@@ -144,3 +144,35 @@ def test_tiny_groups(cuda):
                                           0.0015)
         assert _same(tuple(t[h, F[k]] for k in ("sig_1d_x", "sig_1d_y", "sig_1d_z", "v_sigma", "lambda")), sp)
     assert np.isnan(t[0, F["v_tf"]])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ll", [0.0004, 0.02])
+def test_projections_at_cell_and_tile_edges(cuda, ll):
+    """The projections' sums with cells of one member up to all of them (small cells are a lane's, others a warp's) and
+    groups at the edges of the 1,024-entry tiles: exactly the oracle's."""
+    from pyhalma_gb300 import _lib, halo_properties
+    rng = np.random.default_rng(7)
+    sizes = [8, 9, 32, 33, 1023, 1024, 1025, 2049]
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    n = int(off[-1])
+    mem = rng.permutation(n).astype(np.int32)
+    x, y, z = rng.normal(0.0, 0.01, (3, n))
+    vx, vy, vz = rng.normal(0.0, 100.0, (3, n))
+    m = rng.uniform(0.5, 2.0, n)
+    cen = []
+    for h in range(len(sizes)):
+        g = mem[off[h]:off[h + 1]]
+        M = m[g].sum()
+        c = [(m[g] * a[g]).sum() / M for a in (x, y, z)]
+        cen.append(c + [M, np.sqrt((c[0] - x[g]) ** 2 + (c[1] - y[g]) ** 2 + (c[2] - z[g]) ** 2).max()])
+    t = halo_properties.halo_property_table(off, mem, x, y, z, vx, vy, vz, m, np.array(cen), ll)
+    F = {k: i for i, k in enumerate(_lib.PROP_FIELDS)}
+    for h in range(len(sizes)):
+        g = mem[off[h]:off[h + 1]]
+        cx, cy, cz, M, rmax = cen[h]
+        rp = tuple(t[h, F[k]] for k in ("r05x", "r05y", "r05z"))
+        ux, uy, uz = (t[h, F[k]] for k in ("vx", "vy", "vz"))
+        grid = np.arange(-(rmax + ll), rmax + ll, 2 * ll)
+        sp = op.sigma_projections_fortran(grid, len(grid), g, x, y, z, vx, vy, vz, ux, uy, uz, m, cx, cy, cz, *rp, ll)
+        assert _same(tuple(t[h, F[k]] for k in ("sig_1d_x", "sig_1d_y", "sig_1d_z", "v_sigma", "lambda")), sp), sizes[h]
