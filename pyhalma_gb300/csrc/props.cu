@@ -34,13 +34,18 @@ namespace {
 
 constexpr int kCenFields = 5;   // cx, cy, cz, mass, rmax per group (the cleaning's outputs)
 
-__global__ void pr_gather_kernel(int64_t nm, const int *__restrict__ mem, const double *__restrict__ x,
+// An index outside [0, n) sets *bad (the call then fails) and reads particle 0.
+__global__ void pr_gather_kernel(int64_t nm, const int *__restrict__ mem, int64_t n, const double *__restrict__ x,
                                  const double *__restrict__ y, const double *__restrict__ z,
                                  const double *__restrict__ vx, const double *__restrict__ vy,
                                  const double *__restrict__ vz, const double *__restrict__ m,
-                                 double *__restrict__ g /* 8 x nm: x y z vx vy vz m 0 */) {
+                                 double *__restrict__ g /* 8 x nm: x y z vx vy vz m 0 */, int *__restrict__ bad) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nm; k += (int64_t)gridDim.x * blockDim.x) {
-        const int i = mem[k];
+        int i = mem[k];
+        if ((unsigned)i >= (unsigned)n) {
+            *bad = 1;
+            i = 0;
+        }
         g[k] = x[i];
         g[nm + k] = y[i];
         g[2 * nm + k] = z[i];
@@ -804,26 +809,27 @@ __global__ void pr_proj_out_kernel(int G, const float *__restrict__ res, double 
     }
 }
 
-// A second stream per device for the sums that need nothing of the half-mass radii (inertia tensor, angular momentum): a
-// few blocks with long chains, beside the sorts and walks of the main stream.
+// Two more streams per device, beside the half-mass radii (sorts and walks on the call's stream): the inertia tensor and
+// the angular momentum, and the projected cells, which need nothing of the radii; then what needs them.  All
+// are long chains, FP64 or small launches that leave most of the GPU idle alone.
 struct PropSide {
-    cudaStream_t s = nullptr;
-    cudaEvent_t ready = nullptr, done = nullptr;
+    cudaStream_t s = nullptr, cells = nullptr;
+    cudaEvent_t ready = nullptr, radii = nullptr, done = nullptr, cells_done = nullptr;
 };
 
 int prop_side(PropSide **out) {
     static std::map<int, PropSide> m;   // under api_mutex()
     PropSide &ps = m[current_device()];
     if (!ps.s) {
-        HALMA_CUDA(cudaStreamCreateWithFlags(&ps.s, cudaStreamNonBlocking));
-        HALMA_CUDA(cudaEventCreateWithFlags(&ps.ready, cudaEventDisableTiming));
-        HALMA_CUDA(cudaEventCreateWithFlags(&ps.done, cudaEventDisableTiming));
+        for (cudaStream_t *q : {&ps.s, &ps.cells}) HALMA_CUDA(cudaStreamCreateWithFlags(q, cudaStreamNonBlocking));
+        for (cudaEvent_t *e : {&ps.ready, &ps.radii, &ps.done, &ps.cells_done})
+            HALMA_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
     *out = &ps;
     return HALMA_OK;
 }
 
-// The side stream is idle again on every way out: its kernels use the call's workspace and the caller's arrays.
+// A side stream is idle again on every way out: its kernels use the call's workspace and the caller's arrays.
 struct SideIdle {
     cudaStream_t s;
     ~SideIdle() { cudaStreamSynchronize(s); }
@@ -873,6 +879,7 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
     for (int h = 0; h < G; ++h)
         if (h_off[h + 1] < h_off[h]) return fail(HALMA_ERR_INVALID, "group offsets must not decrease");
     const int64_t N0 = h_off[G];
+    if (n == 0 && N0 > 0) return fail(HALMA_ERR_INVALID, "group member outside [0, n)");
     if (3 * N0 >= INT32_MAX) return fail(HALMA_ERR_CAPACITY, "at most (2^31-2)/3 members");
     std::vector<double> hc(5ull * G);
     HALMA_TRY(to_host(hc.data(), centre, 40ull * G));
@@ -942,32 +949,19 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
     void *tmp = at<void>(base, o_tmp);
     const int sms = device_sm_count();
     const int gN = std::min(sms * 8, grid_for(NM, 256)), gG = std::min(G, sms * 16), gH = grid_for(G, 128);
-    // members in range (validated before any gather)
-    {
-        std::vector<int32_t> hm;
-        const int32_t *mp = group_members;
-        if (is_device_pointer(group_members)) {
-            hm.resize(N0);
-            HALMA_CUDA(cudaMemcpy(hm.data(), group_members, 4ull * N0, cudaMemcpyDeviceToHost));
-            mp = hm.data();
-        }
-        bool outside = false;   // no early way out: the loop is a vector loop
-        for (int64_t k = 0; k < N0; ++k) outside |= (uint32_t)mp[k] >= (uint32_t)n;
-        if (outside) return fail(HALMA_ERR_INVALID, "group member outside [0, n)");
-    }
+    HALMA_CUDA(cudaMemsetAsync(cnt, 0, 64, st));   // [0] cells, [1] a member index out of range
     HALMA_CUDA(cudaMemsetAsync(dout, 0, 8ull * G * HALMA_PROP_NFIELDS, st));
-    HALMA_LAUNCH(pr_gather_kernel, gN, 256, 0, st, N0, dmem, dx, dy, dz, dvx, dvy, dvz, dm, gbuf);
+    HALMA_LAUNCH(pr_gather_kernel, gN, 256, 0, st, N0, dmem, n, dx, dy, dz, dvx, dvy, dvz, dm, gbuf, cnt + 1);
     HALMA_LAUNCH(pr_fill_kernel, gG, 256, 0, st, G, doff, own);
     HALMA_LAUNCH(pr_bulk_kernel, gG, 256, 0, st, G, doff, gbuf, NM, dcen, dout, about);
     PropSide *side = nullptr;
     HALMA_TRY(prop_side(&side));
-    SideIdle side_idle{side->s};
+    SideIdle side_idle{side->s}, cells_idle{side->cells};
     HALMA_CUDA(cudaMemsetAsync(kctr, 0, 4ull * G, st));
     HALMA_CUDA(cudaEventRecord(side->ready, st));
     HALMA_CUDA(cudaStreamWaitEvent(side->s, side->ready, 0));
-    HALMA_LAUNCH(pr_shape_kernel, gG, 256, 0, side->s, G, doff, gbuf, NM, dcen, dout);
     HALMA_LAUNCH(pr_kin1_kernel, G * S, 256, 0, side->s, G, S, doff, gbuf, NM, dcen, dout, kpart, kctr, jvec);
-    HALMA_CUDA(cudaEventRecord(side->done, side->s));
+    HALMA_LAUNCH(pr_shape_kernel, gG, 256, 0, side->s, G, doff, gbuf, NM, dcen, dout);
     // half-mass radii (3-D with sigma_effective, then x, y, z projections) by the reductions
     const double *gx = gbuf, *gy = gbuf + NM, *gz = gbuf + 2 * NM, *gvx = gbuf + 3 * NM, *gvy = gbuf + 4 * NM,
                  *gvz = gbuf + 5 * NM, *gm = gbuf + 6 * NM, *g0 = gbuf + 7 * NM;
@@ -983,27 +977,38 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
                                         red + (int64_t)r * G * HALMA_RED_NFIELDS, st));
     }
     HALMA_LAUNCH(pr_r05_kernel, gH, 128, 0, st, G, red, dout, res);
-    HALMA_CUDA(cudaStreamWaitEvent(st, side->done, 0));
-    HALMA_LAUNCH(pr_kin2_kernel, G * S, 256, 0, st, G, S, doff, gbuf, NM, dcen, dout, kpart, kctr, jvec);
+    HALMA_CUDA(cudaEventRecord(side->radii, st));
+    HALMA_CUDA(cudaStreamWaitEvent(side->s, side->radii, 0));
+    HALMA_LAUNCH(pr_kin2_kernel, G * S, 256, 0, side->s, G, S, doff, gbuf, NM, dcen, dout, kpart, kctr, jvec);
+    HALMA_CUDA(cudaEventRecord(side->done, side->s));
     if (N0 > 0) {
-        HALMA_LAUNCH(pr_grid_kernel, gH, 128, 0, st, G, dcen, linking_length, grid);
-        HALMA_LAUNCH(pr_pkeys_kernel, gN, 256, 0, st, N0, G, doff, own, gbuf, dcen, grid, cbits, kin, vin);
+        cudaStream_t sc = side->cells;
         const int n3 = (int)(3 * N0);
         const int g3 = std::min(sms * 8, grid_for(n3, 256));
+        HALMA_CUDA(cudaStreamWaitEvent(sc, side->ready, 0));
+        HALMA_LAUNCH(pr_grid_kernel, gH, 128, 0, sc, G, dcen, linking_length, grid);
+        HALMA_LAUNCH(pr_pkeys_kernel, gN, 256, 0, sc, N0, G, doff, own, gbuf, dcen, grid, cbits, kin, vin);
         // keys hold (3 group + projection) above cbits of cell index: sort only those bits
-        HALMA_TRY(sort_pairs_u64_i32(tmp, sort_b, kin, kout, vin, vout, n3, cbits + nbits((uint64_t)3 * G), st));
-        HALMA_LAUNCH(pr_head_kernel, g3, 256, 0, st, n3, kout, head);
-        HALMA_TRY(exclusive_sum_i32(tmp, scan_b, head, rpos, n3, st));
+        HALMA_TRY(sort_pairs_u64_i32(tmp, sort_b, kin, kout, vin, vout, n3, cbits + nbits((uint64_t)3 * G), sc));
+        HALMA_LAUNCH(pr_head_kernel, g3, 256, 0, sc, n3, kout, head);
+        HALMA_TRY(exclusive_sum_i32(tmp, scan_b, head, rpos, n3, sc));
         // the sort's input is no longer needed
         int *runstart = vin;
         auto *entry = reinterpret_cast<float2 *>(kin);
-        HALMA_LAUNCH(pr_entries_kernel, g3, 256, 0, st, n3, N0, cbits, kout, vout, head, rpos, gbuf, dout, runstart, rid,
+        HALMA_LAUNCH(pr_entries_kernel, g3, 256, 0, sc, n3, N0, cbits, kout, vout, head, rpos, gbuf, dout, runstart, rid,
                      entry, cnt);
-        HALMA_LAUNCH(pr_cells_kernel, sms * 16, 256, 0, st, cnt, runstart, kout, entry, cellv, cellkey);
+        HALMA_LAUNCH(pr_cells_kernel, sms * 16, 256, 0, sc, cnt, runstart, kout, entry, cellv, cellkey);
+        HALMA_CUDA(cudaEventRecord(side->cells_done, sc));
+        HALMA_CUDA(cudaStreamWaitEvent(st, side->cells_done, 0));
         HALMA_LAUNCH(pr_proj_kernel, (int)std::min<int64_t>(6ll * G, sms * 16), 256, 0, st, G, N0, doff, gbuf, dcen, grid,
                      linking_length, cbits, rid, cellv, cellkey, cnt, res);
         HALMA_LAUNCH(pr_proj_out_kernel, gH, 128, 0, st, G, res, dout);
     }
+    HALMA_CUDA(cudaStreamWaitEvent(st, side->done, 0));
+    int bad = 0;
+    HALMA_CUDA(cudaMemcpyAsync(&bad, cnt + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    HALMA_CUDA(cudaStreamSynchronize(st));
+    if (bad) return fail(HALMA_ERR_INVALID, "group member outside [0, n)");
     HALMA_TRY(sg.download(st));
     HALMA_CUDA(cudaStreamSynchronize(st));
     return HALMA_OK;

@@ -176,3 +176,20 @@ def test_projections_at_cell_and_tile_edges(cuda, ll):
         grid = np.arange(-(rmax + ll), rmax + ll, 2 * ll)
         sp = op.sigma_projections_fortran(grid, len(grid), g, x, y, z, vx, vy, vz, ux, uy, uz, m, cx, cy, cz, *rp, ll)
         assert _same(tuple(t[h, F[k]] for k in ("sig_1d_x", "sig_1d_y", "sig_1d_z", "v_sigma", "lambda")), sp), sizes[h]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bad", [-1, 40, 2 ** 31 - 1])
+def test_member_index_out_of_range(cuda, bad):
+    from pyhalma_gb300 import halo_properties
+    rng = np.random.default_rng(3)
+    cols = rng.uniform(0.1, 1.0, (7, 40))
+    mem = np.arange(20, dtype=np.int32)
+    cen = np.array([[0.5, 0.5, 0.5, cols[6, :20].sum(), 1.0]])
+    off = np.array([0, 20])
+    good = halo_properties.halo_property_table(off, mem, *cols, cen, 0.1)
+    wrong = mem.copy()
+    wrong[7] = bad
+    with pytest.raises(ValueError, match="outside"):
+        halo_properties.halo_property_table(off, wrong, *cols, cen, 0.1)
+    assert _same(halo_properties.halo_property_table(off, mem, *cols, cen, 0.1), good)
