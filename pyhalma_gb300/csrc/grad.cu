@@ -201,36 +201,42 @@ void choose_slices(int64_t na, int64_t nb, int T, int nv, int *n_split, int64_t 
 // ---- both sides of a pair at once -----------------------------------------------------------
 // When the gradients of targets and sources are both wanted and there are enough pairs, one sweep gives them: distance,
 // rsqrt and r^-3 of a pair are formed once, 17 lane-operations instead of 12 + 13, and the sources' four
-// sums (r^-1 and the vector) are reduced over the warp's lanes (1 lane-operation a pair, 4 instructions).
-// A block of four warps holds 512 targets, four a lane, and stages 512 sources; an item is one block of sources against
+// sums (r^-1 and the vector) are reduced over the warp's lanes (1 lane-operation a pair).
+// A block of four warps holds 1,024 targets, eight a lane, and stages 512 sources; an item is one block of sources against
 // `tblocks` blocks of targets, the sources' sums kept in shared memory (compensated) over them.  Per item and
-// target, or source, one partial sum is written; they are added in order in FP64.
-// Bound: the FP32 pipe (18.7 lane-operations and a rsqrt a pair).  160,000 targets x 200,000 sources: 27.5 ms in two
-// sweeps, 23.5 in one.
-constexpr int kBothT = 4, kBothTargets = 128 * kBothT, kBothSources = 512, kBothChunks = kBothSources / 32;
+// target, or source, one partial sum is written; they are added in order.
+// Bound: the FP32 pipe (18 lane-operations and a rsqrt a pair; it is 75 % busy).  160,000 targets x 200,000 sources:
+// 27.5 ms in two sweeps, 22.0 in one (four targets a lane, two sources an instruction and r^-3 weighted twice: 23.5;
+// 256 sources, or ten or six targets a lane, 3 to 5 % more).
+constexpr int kBothT = 8, kBothTargets = 128 * kBothT, kBothSources = 512, kBothChunks = kBothSources / 32;
 
 struct BothShared {
-    float4 src[kBothSources];               // 32-source chunks as pairs: 16 x {x, x, y, y}, 16 x {z, z, m, m}
+    float4 src[kBothSources][2];            // {x, x, y, y}, {z, z, m, m}
     float part[4][kBothSources][4];         // per warp: the sources' sums over the warp's targets of one block
     float sum[kBothSources][4], comp[kBothSources][4];
 };
 
-template <bool SELF>
-__device__ __forceinline__ void both_chunk(const float4 *sa, const float4 *sb, const f2x (&px)[kBothT],
-                                           const f2x (&py)[kBothT], const f2x (&pz)[kBothT], const f2x (&g)[kBothT],
-                                           f2x e2, int j0, const int (&self)[kBothT], f2x (&vx)[kBothT],
-                                           f2x (&vy)[kBothT], f2x (&vz)[kBothT], float *out, int lane) {
+// 32 sources against the lane's targets, two targets a two-lane instruction.  r^-3 is formed once for both ends of a pair;
+// with WIDE each end multiplies its weight in between, where r^-3 by itself could leave the range of normal
+// numbers: softenings outside 2^-40 .. 2^40 or coordinates from 2^40 on.
+constexpr float kBothReach = 0x1p40f;
+
+template <bool SELF, bool WIDE>
+__device__ __forceinline__ void both_chunk(const float4 (*src)[2], const f2x (&px)[kBothT / 2],
+                                           const f2x (&py)[kBothT / 2], const f2x (&pz)[kBothT / 2],
+                                           const f2x (&g)[kBothT / 2], f2x e2, int j0, const int (&self)[kBothT],
+                                           f2x (&vx)[kBothT / 2], f2x (&vy)[kBothT / 2], f2x (&vz)[kBothT / 2],
+                                           float *out, int lane) {
 #pragma unroll 1
-    for (int k0 = 0; k0 < 16; k0 += 2) {
-        float v[16];   // sums of 4 sources: s, x, y, z of each pair of sources
+    for (int k0 = 0; k0 < 32; k0 += 4) {
+        float v[16];   // sums of 4 sources: s, x, y, z of each
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int kp = k0 + k;
-            const float4 a = sa[kp], b = sb[kp];
+        for (int k = 0; k < 4; ++k) {
+            const float4 a = src[k0 + k][0], b = src[k0 + k][1];
             const f2x X = pack2(a.x, a.y), Y = pack2(a.z, a.w), Z = pack2(b.x, b.y), W = pack2(b.z, b.w);
             f2x s0 = pack2(0.f, 0.f), s1 = s0, s2 = s0, s3 = s0;
 #pragma unroll
-            for (int t = 0; t < kBothT; ++t) {
+            for (int t = 0; t < kBothT / 2; ++t) {
                 const f2x dx = sub2(X, px[t]), dy = sub2(Y, py[t]), dz = sub2(Z, pz[t]);
                 f2x r2 = fma2(dz, dz, e2);
                 r2 = fma2(dy, dy, r2);
@@ -239,40 +245,45 @@ __device__ __forceinline__ void both_chunk(const float4 *sa, const float4 *sb, c
                 unpack2(r2, r0, r1);
                 float i0 = rsqrt_ftz(r0), i1 = rsqrt_ftz(r1);
                 if (SELF) {
-                    if (j0 + 2 * kp == self[t]) i0 = 0.f;
-                    if (j0 + 2 * kp + 1 == self[t]) i1 = 0.f;
+                    if (j0 + k0 + k == self[2 * t]) i0 = 0.f;
+                    if (j0 + k0 + k == self[2 * t + 1]) i1 = 0.f;
                 }
                 const f2x ri = pack2(i0, i1);
                 const f2x ri2 = mul2(ri, ri);
-                const f2x wr = mul2(mul2(W, ri), ri2);
+                const f2x ri3 = mul2(ri, ri2);
+                const f2x wr = WIDE ? mul2(mul2(W, ri), ri2) : mul2(W, ri3);
+                const f2x gr3 = WIDE ? mul2(mul2(g[t], ri), ri2) : mul2(g[t], ri3);
                 vx[t] = fma2(wr, dx, vx[t]);
                 vy[t] = fma2(wr, dy, vy[t]);
                 vz[t] = fma2(wr, dz, vz[t]);
-                const f2x gr = mul2(g[t], ri);
-                const f2x gr3 = mul2(gr, ri2);
-                s0 = add2(s0, gr);
+                s0 = fma2(g[t], ri, s0);
                 s1 = fma2(gr3, dx, s1);
                 s2 = fma2(gr3, dy, s2);
                 s3 = fma2(gr3, dz, s3);
             }
-            unpack2(s0, v[8 * k + 0], v[8 * k + 4]);
-            unpack2(s1, v[8 * k + 1], v[8 * k + 5]);
-            unpack2(s2, v[8 * k + 2], v[8 * k + 6]);
-            unpack2(s3, v[8 * k + 3], v[8 * k + 7]);
+            float lo, hi;
+            unpack2(s0, lo, hi);
+            v[4 * k + 0] = lo + hi;
+            unpack2(s1, lo, hi);
+            v[4 * k + 1] = lo + hi;
+            unpack2(s2, lo, hi);
+            v[4 * k + 2] = lo + hi;
+            unpack2(s3, lo, hi);
+            v[4 * k + 3] = lo + hi;
         }
         // lane l and l ^ 1 get value l >> 1: source (l >> 3) of the four, component (l >> 1) & 3
         const float r = warp_reduce_scatter16(v, lane);
-        if ((lane & 1) == 0) out[k0 * 8 + (lane >> 1)] = r;
+        if ((lane & 1) == 0) out[k0 * 4 + (lane >> 1)] = r;
     }
 }
 
 // part_t[(sb - sb0) * nt + i][3]: target i's vector over source block sb; part_s[tsb * nsrc + j - j0][4]: source j's sums
 // over the targets of item column tsb (nsrc sources from j0 = sb0 * kBothSources on).
-__global__ void __launch_bounds__(128, 4) adjoint_both_kernel(
+__global__ void __launch_bounds__(128, 3) adjoint_both_kernel(
     const float *__restrict__ sx, const float *__restrict__ sy, const float *__restrict__ sz,
     const float *__restrict__ sm, int64_t ns, const float *__restrict__ tx, const float *__restrict__ ty,
     const float *__restrict__ tz, const float *__restrict__ tg, int64_t nt, float eps2, int self_mask, int64_t self_off,
-    int sb0, int nsb, int tblocks, double *__restrict__ part_t, double *__restrict__ part_s) {
+    int sb0, int nsb, int tblocks, float2 *__restrict__ part_t, float2 *__restrict__ part_s) {
     extern __shared__ __align__(16) unsigned char both_raw[];
     BothShared &sh = *reinterpret_cast<BothShared *>(both_raw);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -280,64 +291,84 @@ __global__ void __launch_bounds__(128, 4) adjoint_both_kernel(
     const int tsb = blockIdx.x / nsb;
     const int64_t j0 = (int64_t)(sb0 + sbl) * kBothSources;
     const f2x e2 = pack2(eps2, eps2);
+    auto beyond = [](const float4 &q) {
+        return !(fmaxf(fabsf(q.x), fmaxf(fabsf(q.y), fabsf(q.z))) < kBothReach);
+    };
+    bool far = !(eps2 >= 0x1p-80f && eps2 <= 0x1p80f);
     for (int k = threadIdx.x; k < kBothSources; k += 128) {
         const float4 q = load_b(sx, sy, sz, sm, j0 + k, ns);
-        float *c = reinterpret_cast<float *>(sh.src + (k >> 5) * 32);
-        const int kp = (k & 31) >> 1, hf = k & 1;
-        c[kp * 4 + hf] = q.x;
-        c[kp * 4 + 2 + hf] = q.y;
-        c[64 + kp * 4 + hf] = q.z;
-        c[64 + kp * 4 + 2 + hf] = q.w;
+        far |= j0 + k < ns && beyond(q);
+        sh.src[k][0] = make_float4(q.x, q.x, q.y, q.y);
+        sh.src[k][1] = make_float4(q.z, q.z, q.w, q.w);
 #pragma unroll
         for (int v = 0; v < 4; ++v) sh.sum[k][v] = sh.comp[k][v] = 0.f;
     }
-    __syncthreads();
+    const bool far_sources = __syncthreads_or(far);
     for (int tb = 0; tb < tblocks; ++tb) {
         const int64_t i0 = ((int64_t)tsb * tblocks + tb) * kBothTargets;
         if (i0 >= nt) break;   // the same for the block
         const int64_t iw = i0 + w * 32 * kBothT;
-        f2x px[kBothT], py[kBothT], pz[kBothT], g[kBothT];
+        f2x px[kBothT / 2], py[kBothT / 2], pz[kBothT / 2], g[kBothT / 2];
         float vs[kBothT][3], vc[kBothT][3];
         int self[kBothT];
+        bool far_target = false;
+#pragma unroll
+        for (int t = 0; t < kBothT / 2; ++t) {
+            float4 p[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int64_t i = iw + (2 * t + u) * 32 + lane;   // far and with zero weight past the end
+                p[u] = i < nt ? make_float4(tx[i], ty[i], tz[i], tg[i]) : make_float4(-kFarG, -kFarG, -kFarG, 0.f);
+                far_target |= i < nt && beyond(p[u]);
+            }
+            px[t] = pack2(p[0].x, p[1].x);
+            py[t] = pack2(p[0].y, p[1].y);
+            pz[t] = pack2(p[0].z, p[1].z);
+            g[t] = pack2(p[0].w, p[1].w);
+        }
 #pragma unroll
         for (int t = 0; t < kBothT; ++t) {
             const int64_t i = iw + t * 32 + lane;
-            const bool in = i < nt;   // far and with zero weight otherwise
-            const float4 p = in ? make_float4(tx[i], ty[i], tz[i], tg[i]) : make_float4(-kFarG, -kFarG, -kFarG, 0.f);
-            px[t] = pack2(p.x, p.x);
-            py[t] = pack2(p.y, p.y);
-            pz[t] = pack2(p.z, p.z);
-            g[t] = pack2(p.w, p.w);
+            const bool in = i < nt;
             const int64_t sj = i + self_off - j0;   // the self pair's source in the block
             self[t] = in && self_mask && sj >= 0 && sj < kBothSources ? (int)sj : -1;
 #pragma unroll
             for (int v = 0; v < 3; ++v) vs[t][v] = vc[t][v] = 0.f;
         }
+        const bool wide = far_sources || __any_sync(0xffffffffu, far_target);
         const int64_t lo = iw + self_off - j0;   // self pairs: sources lo .. lo + 32 T - 1 of the block
         for (int c = 0; c < kBothChunks; ++c) {
-            f2x vx[kBothT], vy[kBothT], vz[kBothT];
+            f2x vx[kBothT / 2], vy[kBothT / 2], vz[kBothT / 2];
 #pragma unroll
-            for (int t = 0; t < kBothT; ++t) vx[t] = vy[t] = vz[t] = pack2(0.f, 0.f);
-            const float4 *buf = sh.src + c * 32;
+            for (int t = 0; t < kBothT / 2; ++t) vx[t] = vy[t] = vz[t] = pack2(0.f, 0.f);
+            const float4 (*buf)[2] = sh.src + c * 32;
             float *out = &sh.part[w][c * 32][0];
-            if (self_mask && lo < c * 32 + 32 && lo + 32 * kBothT > c * 32)
-                both_chunk<true>(buf, buf + 16, px, py, pz, g, e2, c * 32, self, vx, vy, vz, out, lane);
+            const bool own = self_mask && lo < c * 32 + 32 && lo + 32 * kBothT > c * 32;
+            if (wide)
+                both_chunk<true, true>(buf, px, py, pz, g, e2, c * 32, self, vx, vy, vz, out, lane);
+            else if (own)
+                both_chunk<true, false>(buf, px, py, pz, g, e2, c * 32, self, vx, vy, vz, out, lane);
             else
-                both_chunk<false>(buf, buf + 16, px, py, pz, g, e2, c * 32, self, vx, vy, vz, out, lane);
+                both_chunk<false, false>(buf, px, py, pz, g, e2, c * 32, self, vx, vy, vz, out, lane);
 #pragma unroll
-            for (int t = 0; t < kBothT; ++t) {
-                fold2(vs[t][0], vc[t][0], vx[t]);
-                fold2(vs[t][1], vc[t][1], vy[t]);
-                fold2(vs[t][2], vc[t][2], vz[t]);
+            for (int t = 0; t < kBothT; t += 2) {
+                const f2x q[3] = {vx[t / 2], vy[t / 2], vz[t / 2]};
+#pragma unroll
+                for (int v = 0; v < 3; ++v) {
+                    float a, b;
+                    unpack2(q[v], a, b);
+                    two_sum_acc(vs[t][v], vc[t][v], a);
+                    two_sum_acc(vs[t + 1][v], vc[t + 1][v], b);
+                }
             }
         }
 #pragma unroll
         for (int t = 0; t < kBothT; ++t) {
             const int64_t i = iw + t * 32 + lane;
             if (i >= nt) continue;
-            double *p = part_t + ((int64_t)sbl * nt + i) * 3;
+            float2 *p = part_t + ((int64_t)sbl * nt + i) * 3;
 #pragma unroll
-            for (int v = 0; v < 3; ++v) p[v] = (double)vs[t][v] + (double)vc[t][v];
+            for (int v = 0; v < 3; ++v) p[v] = make_float2(vs[t][v], vc[t][v]);
         }
         __syncthreads();
         for (int k = threadIdx.x; k < kBothSources * 4; k += 128) {   // the warps in order, compensated
@@ -352,46 +383,57 @@ __global__ void __launch_bounds__(128, 4) adjoint_both_kernel(
     }
     for (int k = threadIdx.x; k < kBothSources * 4; k += 128)
         part_s[((int64_t)tsb * nsb + sbl) * kBothSources * 4 + k] =
-            (double)(&sh.sum[0][0])[k] + (double)(&sh.comp[0][0])[k];
+            make_float2((&sh.sum[0][0])[k], (&sh.comp[0][0])[k]);
 }
 
 // After a band of source blocks: the targets' vectors over the band added to tot (first: set), and, after the last
-// band, the gradients; the band's sources' sums over the item columns in order, and their gradients.
-__global__ void __launch_bounds__(256) both_targets_kernel(const double *__restrict__ part_t, int nsb, int64_t nt,
-                                                           int first, int last, double *__restrict__ tot,
+// band, the gradients; the band's sources' sums over the item columns in order, and their gradients.  A partial sum is a
+// compensated FP32 sum and its errors; they are added up the same way (in FP64 that pipe was the bound: 452 and
+// 140 us of 160,000 targets x 200,000 sources, now 335 and 87).
+__global__ void __launch_bounds__(256) both_targets_kernel(const float2 *__restrict__ part_t, int nsb, int64_t nt,
+                                                           int first, int last, float2 *__restrict__ tot,
                                                            const float *__restrict__ scale, float *__restrict__ out) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < 3 * nt; k += (int64_t)gridDim.x * blockDim.x) {
-        double acc = first ? 0.0 : tot[k];
+        float2 acc = first ? make_float2(0.f, 0.f) : tot[k];
 #pragma unroll 8
-        for (int s = 0; s < nsb; ++s) acc += part_t[(int64_t)s * 3 * nt + k];
-        if (last) out[k] = scale[k / 3] * (float)acc;
+        for (int s = 0; s < nsb; ++s) {
+            const float2 v = part_t[(int64_t)s * 3 * nt + k];
+            two_sum_acc(acc.x, acc.y, v.x);
+            acc.y += v.y;
+        }
+        if (last) out[k] = scale[k / 3] * (acc.x + acc.y);
         else tot[k] = acc;
     }
 }
 
-__global__ void __launch_bounds__(256) both_sources_kernel(const double *__restrict__ part_s, int ntsb, int64_t nsrc,
+__global__ void __launch_bounds__(256) both_sources_kernel(const float2 *__restrict__ part_s, int ntsb, int64_t nsrc,
                                                            int64_t j0, int64_t ns, const float *__restrict__ m,
                                                            float *__restrict__ gm, float *__restrict__ gs) {
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < 4 * nsrc; k += (int64_t)gridDim.x * blockDim.x) {
         const int64_t j = j0 + k / 4;
         const int v = (int)(k & 3);
         if (j >= ns) continue;
-        double acc = 0.0;
+        float2 acc = make_float2(0.f, 0.f);
 #pragma unroll 8
-        for (int s = 0; s < ntsb; ++s) acc += part_s[(int64_t)s * nsrc * 4 + k];
+        for (int s = 0; s < ntsb; ++s) {
+            const float2 q = part_s[(int64_t)s * nsrc * 4 + k];
+            two_sum_acc(acc.x, acc.y, q.x);
+            acc.y += q.y;
+        }
+        const float sum = acc.x + acc.y;
         // the vector was summed as (source - target): the source's gradient points the other way
         if (v == 0) {
-            if (gm) gm[j] = (float)acc;
+            if (gm) gm[j] = sum;
         } else if (gs) {
-            gs[3 * j + v - 1] = m[j] * -(float)acc;
+            gs[3 * j + v - 1] = m[j] * -sum;
         }
     }
 }
 
 // Scratch: the targets' partial sums of one band within kBothBand bytes (one source block at least).
 constexpr int64_t kBothBand = 256ll << 20;
-// Below kBothPairs pairs its blocks, 512 x 512 pairs for an item of four warps, are too few for the GPU: 4.8e7
-// pairs take 89 us against 80 in two sweeps, 1.2e8 146 against 150, 5e8 405 against 479.
+// Below kBothPairs pairs its blocks, 1,024 x 512 pairs for an item of four warps, are too few for the GPU: 4.8e7
+// pairs take 89 us against 78 in two sweeps, 1.2e8 140 against 150, 5e8 407 against 479.
 constexpr double kBothPairs = 1e8;
 
 struct BothPlan {
@@ -401,20 +443,20 @@ struct BothPlan {
         nsb = (ns + kBothSources - 1) / kBothSources;
         band = std::min(nsb, std::max<int64_t>(1, kBothBand / (24 * nt)));
         const int64_t tb = (nt + kBothTargets - 1) / kBothTargets;
-        // about eight items for every block that fits on the GPU (four an SM)
-        const int64_t columns = std::min(tb, std::max<int64_t>(1, ((int64_t)device_sm_count() * 32 + band - 1) / band));
+        // about eight items for every block that fits on the GPU (three an SM)
+        const int64_t columns = std::min(tb, std::max<int64_t>(1, ((int64_t)device_sm_count() * 24 + band - 1) / band));
         tblocks = (int)((tb + columns - 1) / columns);
         ntsb = (tb + tblocks - 1) / tblocks;
     }
     size_t bytes(int64_t nt) const {
-        return 8 * (size_t)(3 * nt * (band + 1) + ntsb * band * kBothSources * 4);
+        return sizeof(float2) * (size_t)(3 * nt * (band + 1) + ntsb * band * kBothSources * 4);
     }
 };
 
 int launch_both(const BothPlan &P, const float *sx, const float *sy, const float *sz, const float *m, int64_t ns,
                 const float *tx, const float *ty, const float *tz, const float *g, int64_t nt, float eps2, int self,
-                int64_t self_off, float *gm, float *gs, float *gt, double *scratch, cudaStream_t st) {
-    double *part_t = scratch, *tot = part_t + 3 * nt * P.band, *part_s = tot + 3 * nt;
+                int64_t self_off, float *gm, float *gs, float *gt, float2 *scratch, cudaStream_t st) {
+    float2 *part_t = scratch, *tot = part_t + 3 * nt * P.band, *part_s = tot + 3 * nt;
     const int smem = (int)sizeof(BothShared), cap = device_sm_count() * 8;
     HALMA_CUDA(cudaFuncSetAttribute(adjoint_both_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     for (int64_t sb0 = 0; sb0 < P.nsb; sb0 += P.band) {
@@ -511,8 +553,8 @@ extern "C" int halma_potential_grad_f32(int64_t ns, const float *m_, const float
     double *part = at<double>(base, o_part);
     const int self = mask == HALMA_MASK_SELF;
     if (both) {
-        HALMA_TRY(launch_both(plan, sx, sy, sz, m, ns, tx, ty, tz, g, nt, (float)eps2, self, self_offset, gm, gs, gt, part,
-                              st));
+        HALMA_TRY(launch_both(plan, sx, sy, sz, m, ns, tx, ty, tz, g, nt, (float)eps2, self, self_offset, gm, gs, gt,
+                              reinterpret_cast<float2 *>(part), st));
         return sg.download(st);
     }
     if (gt)

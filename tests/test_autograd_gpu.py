@@ -137,7 +137,7 @@ def test_gas_halo_adjoint_at_full_scale(cuda):
     (200_003, 513, -300), (300_000, 1, None), (1, 120_000_000 // 200, None), (4_097, 40_001, 4_000)])
 def test_both_gradients_in_one_sweep(cuda, ns, nt, self_offset):
     """Enough pairs for the kernel that gives both ends' gradients at once (and shapes short of it), at the edges of
-    its blocks of 512, with and without a skipped pair, against the FP64 gradient."""
+    its blocks of 512 sources, with and without a skipped pair, against the FP64 gradient."""
     import torch
     from pyhalma_gb300.autograd import softened_potential
     rng = np.random.default_rng(8)
@@ -161,3 +161,24 @@ def test_both_gradients_in_one_sweep(cuda, ns, nt, self_offset):
     assert rel(M.grad.cpu().numpy(), gm) < 1e-5
     assert rel(np.stack([a.grad.cpu().numpy() for a in S], 1), gs) < 1e-5
     assert rel(np.stack([a.grad.cpu().numpy() for a in T], 1), gt) < 1e-5
+
+
+@pytest.mark.parametrize("shift", [45, -31])
+def test_both_gradients_in_other_units(cuda, shift):
+    """Lengths times 2^shift: softenings and coordinates past the range in which r^-3 is formed by itself.  The gradients
+    scale by exact powers of two, up to the order of the products (1e-5 as above).  (FP32 holds r^-3 down to
+    softenings of 1.5e-13: 2^-31 times 1e-3 is 4.7e-13.)"""
+    import torch
+    from pyhalma_gb300.autograd import softened_potential
+    rng = np.random.default_rng(9)
+    ns, nt, unit = 10_300, 10_100, 2.0 ** shift
+    s, t = rng.normal(0, 0.02, (3, ns)).astype(np.float32), rng.normal(0, 0.02, (3, nt)).astype(np.float32)
+    m, g = rng.uniform(1.0, 2.0, ns).astype(np.float32), torch.tensor(rng.normal(size=nt).astype(np.float32), device=cuda)
+
+    def gradients(u):
+        S, T = ([torch.tensor(a * np.float32(u), device=cuda, requires_grad=True) for a in c] for c in (s, t))
+        M = torch.tensor(m, device=cuda, requires_grad=True)
+        softened_potential(*S, M, *T, 1e-3 * u).backward(g)
+        return [M.grad.double() * u] + [a.grad.double() * u * u for a in S + T]
+    for a, b in zip(gradients(unit), gradients(1.0)):
+        assert float((a - b).norm() / b.norm()) < 1e-5
