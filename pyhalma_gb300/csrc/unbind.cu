@@ -998,55 +998,6 @@ __device__ __forceinline__ SlotEnergy slot_energy(float2 p, float4 u, float wx, 
     return s;
 }
 
-// FP64 sums (m, m x, m v) over the listed particles, one warp; lane 0 holds the totals.
-__device__ __forceinline__ void removed_sums(const int *list, int nrem, const double *__restrict__ x,
-                                             const double *__restrict__ y, const double *__restrict__ z,
-                                             const double *__restrict__ vx, const double *__restrict__ vy,
-                                             const double *__restrict__ vz, const double *__restrict__ m, int lane,
-                                             double (&a)[7]) {
-#pragma unroll
-    for (int k = 0; k < 7; ++k) a[k] = 0.0;
-    for (int k = lane; k < nrem; k += 32) {
-        const int i = list[k];
-        const double mi = m[i];
-        a[0] += mi;
-        a[1] += mi * x[i];
-        a[2] += mi * y[i];
-        a[3] += mi * z[i];
-        a[4] += mi * vx[i];
-        a[5] += mi * vy[i];
-        a[6] += mi * vz[i];
-    }
-    // the tree of warp_sum without the levels that add nothing but zeros
-    for (int o = 16; o > 0; o >>= 1) {
-        if (o >= nrem) continue;
-#pragma unroll
-        for (int k = 0; k < 7; ++k) a[k] += __shfl_down_sync(0xffffffffu, a[k], o);
-    }
-}
-
-// The halo's state after a pass that removed something: keep_run particles remain, a are the removed ones' sums.
-__device__ __forceinline__ void subtract_removed(HaloState &o, int keep_run, const double (&a)[7]) {
-    o.nb = keep_run;
-    if (keep_run == 0) {
-        o.M = o.sx = o.sy = o.sz = o.px = o.py = o.pz = 0.0;
-    } else {
-        o.M -= a[0];
-        o.sx -= a[1]; o.sy -= a[2]; o.sz -= a[3];
-        o.px -= a[4]; o.py -= a[5]; o.pz -= a[6];
-    }
-    const double M = o.M;
-    if (M > 0) {
-        o.cx = o.sx / M; o.cy = o.sy / M; o.cz = o.sz / M;
-        o.vx = o.px / M; o.vy = o.py / M; o.vz = o.pz / M;
-    } else {
-        o.cx = o.cy = o.cz = o.vx = o.vy = o.vz = 0.0;
-    }
-    o.wx = (float)(o.vx - o.v0x);
-    o.wy = (float)(o.vy - o.v0y);
-    o.wz = (float)(o.vz - o.v0z);
-}
-
 __device__ __forceinline__ float2 df_warp_sum(float2 v) {
     for (int o = 16; o > 0; o >>= 1)
         v = df_add(v, make_float2(__shfl_down_sync(0xffffffffu, v.x, o), __shfl_down_sync(0xffffffffu, v.y, o)));
@@ -1163,7 +1114,7 @@ __global__ void __launch_bounds__(kSegThreads) ub_energy_df_kernel(
             __syncthreads();
         }
         SegDF &o = seg_sums[seg];
-        if (w < kWarps - 1) {   // sum w, in the order of removed_sums
+        if (w < kWarps - 1) {   // sum w: lane-strided, then the warp tree
             double a = 0.0;
             for (int k = lane; k < nrem; k += 32) {
                 const int i = rlist[k];
@@ -1245,7 +1196,7 @@ __global__ void ub_finalize_df_kernel(int nh, const int *__restrict__ order, con
         else o.nb = keep_run;
     }
     if (rem_run == 0) return;
-    // the halo's sums less the removed particles', as subtract_removed has them
+    // the halo's sums less the removed particles' (a halo left empty has none), and the means
     double own = 0.0;
 #pragma unroll
     for (int k = 0; k < 7; ++k) {
@@ -1391,10 +1342,27 @@ __device__ __forceinline__ float4 get_pair_slot(const float4 *chunks, int r) {
     return make_float4(c[kp * 4 + hf], c[kp * 4 + 2 + hf], c[64 + kp * 4 + hf], c[64 + kp * 4 + 2 + hf]);
 }
 
-// 32 * T targets from group g0 on against the sources' chunks; the potentials go to phi (minus them when inc).
+// ---- a halo's blocks as a cluster (see kTeam)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// p of the block of the given rank.
+__device__ __forceinline__ void cluster_store(float2 *p, int rank, float2 v) {
+    unsigned at;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(at), "f"(v.x), "f"(v.y) : "memory");
+}
+
+// 32 * T targets from group g0 on against the sources' chunks; the potentials go to phi (minus them when inc), of every
+// block of a team of several.  All warps call it, those without a group too: the blocks' phi must be free to
+// write first (cluster_wait), which the pair terms hide.
 template <int T>
 __device__ __forceinline__ void small_pairs(const float4 *tgt, const float4 *src, int nb, int ns, int g0, bool inc,
-                                            float eps2, float2 *phi, int lane) {
+                                            float eps2, float2 *phi, int team, int lane) {
+    if (g0 * 32 >= nb) {
+        if (team > 1) cluster_wait();
+        return;
+    }
     f2x tx[T], ty[T], tz[T];
     float sum[T], comp[T];
 #pragma unroll
@@ -1423,18 +1391,30 @@ __device__ __forceinline__ void small_pairs(const float4 *tgt, const float4 *src
             two_sum_acc(sum[t], comp[t], a0 + a1);
         }
     }
+    if (team > 1) cluster_wait();
 #pragma unroll
     for (int t = 0; t < T; ++t) {
         const int r = (g0 + t) * 32 + lane;
         if (r >= nb) continue;
         const float2 d = df_add(make_float2(0.f, 0.f), df_from_acc(sum[t], comp[t]));   // as one slice is added
-        phi[r] = inc ? df_sub(phi[r], d) : d;
+        const float2 q = inc ? df_sub(phi[r], d) : d;
+        if (team == 1) phi[r] = q;
+        for (int k = 0; team > 1 && k < team; ++k) cluster_store(phi + r, k, q);
     }
 }
 
+// A few large haloes leave most SMs idle and wait for one block's pairs (939 members: 41 % of the block's time in the first
+// pass, 12 % in the second).  Clusters of kTeam blocks, or of two, then share a halo: every block keeps all of its
+// state and does every step, with the same bits, but only its share of the pair terms, and writes the potentials
+// to all of them; from the first pass of less than kTeamWork tiles of 32 x 32 pairs on the first goes on alone.  Taken while
+// all teams fit on the GPU at once.  24 haloes of 50 to 1,000: 97 us with a block each, 62 with four, 72 with two.
+// Where there are many haloes, the blocks that share an SM hide one another's latency: with two instead of one
+// (128 registers a thread) 10,000 haloes' largest class takes 352 us instead of 515.
+constexpr int kTeam = 4, kTeamWork = 64;
+
 template <int P, int THREADS>
-__global__ void __launch_bounds__(THREADS) ub_small_kernel(
-    const int *__restrict__ list, const int64_t *__restrict__ off, const double *__restrict__ x,
+__global__ void __launch_bounds__(THREADS, P == kSmallMax ? 2 : P == 256 ? 3 : 8) ub_small_kernel(
+    const int *__restrict__ list, int blocks, const int64_t *__restrict__ off, const double *__restrict__ x,
     const double *__restrict__ y, const double *__restrict__ z, const double *__restrict__ vx,
     const double *__restrict__ vy, const double *__restrict__ vz, const double *__restrict__ m, float eps2, double gfac,
     int max_iter, unsigned char *__restrict__ bound, double *__restrict__ phi_out, HaloState *__restrict__ hs) {
@@ -1446,7 +1426,10 @@ __global__ void __launch_bounds__(THREADS) ub_small_kernel(
     // the size classes' launches are independent: the next may start as soon as this one's blocks all run, and
     // ends after it (the wait below), so that what follows in the stream follows all of them
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int h = list[blockIdx.x];
+    constexpr bool kTeams = P == kSmallMax;
+    const int rank = kTeams ? blockIdx.x % blocks : 0;   // of the halo's blocks, a cluster when there are several
+    int team = kTeams ? blocks : 1;
+    const int h = list[kTeams ? blockIdx.x / blocks : blockIdx.x];
     const int64_t b = off[h];
     const int n = (int)(off[h + 1] - b);
     const float gfac_f = (float)gfac;
@@ -1525,14 +1508,21 @@ __global__ void __launch_bounds__(THREADS) ub_small_kernel(
         const bool inc = it > 0;
         const int groups = (nb + 31) >> 5, ns = inc ? nrem : nb;
         const float4 *src = inc ? sh.rem : sh.src;
-        if (groups <= W) {
-            if (w < groups) small_pairs<1>(sh.src, src, nb, ns, w, inc, eps2, sh.phi, lane);
-        } else if (groups <= 2 * W) {
-            if (2 * w < groups) small_pairs<2>(sh.src, src, nb, ns, 2 * w, inc, eps2, sh.phi, lane);
-        } else {
-            if (4 * w < groups) small_pairs<4>(sh.src, src, nb, ns, 4 * w, inc, eps2, sh.phi, lane);
+        if (team > 1 && groups * ((ns + 31) >> 5) < kTeamWork) {   // the same in all blocks
+            team = 1;
+            if (rank > 0) break;
         }
-        __syncthreads();
+        if (team > 1) cluster_arrive();   // this block's phi is complete and may be written
+        const int item = w * team + (team > 1 ? rank : 0), items = W * team;
+        if (groups <= items) small_pairs<1>(sh.src, src, nb, ns, item, inc, eps2, sh.phi, team, lane);
+        else if (groups <= 2 * items) small_pairs<2>(sh.src, src, nb, ns, 2 * item, inc, eps2, sh.phi, team, lane);
+        else small_pairs<4>(sh.src, src, nb, ns, 4 * item, inc, eps2, sh.phi, team, lane);
+        if (team > 1) {
+            cluster_arrive();
+            cluster_wait();
+        } else {
+            __syncthreads();
+        }
         // ---- energies and the cut (ub_energy_df_kernel)
         const float wx = sh.w[0], wy = sh.w[1], wz = sh.w[2];
         float ek_s = 0.f, ek_c = 0.f, ep_s = 0.f, ep_c = 0.f;
@@ -1555,7 +1545,7 @@ __global__ void __launch_bounds__(THREADS) ub_small_kernel(
                 if (keep) {
                     two_sum_acc(ek_s, ek_c, u[j].w * e.ek);
                     two_sum_acc(ep_s, ep_c, u[j].w * e.pf);
-                } else {
+                } else if (rank == 0) {
                     bound[id[j]] = 0;
                 }
             }
@@ -1609,16 +1599,23 @@ __global__ void __launch_bounds__(THREADS) ub_small_kernel(
         // ---- energies of the pass, and the next pass's mass and bulk velocity (ub_finalize_df_kernel)
         ++iter;
         const bool last = gone == 0 || it + 1 == max_iter;
-        if (w == 0) {
-            if (gone > 0) {   // subtract_removed, a lane per sum; the centre is formed after the last pass
-                double a[7], mine = 0.0;
-                removed_sums(sh.rlist, gone, x, y, z, vx, vy, vz, m, lane, a);
-#pragma unroll
-                for (int k = 0; k < 7; ++k) {
-                    const double t = __shfl_sync(0xffffffffu, a[k], 0);
-                    if (lane == k) mine = t;
+        if (gone > 0) {   // the removed particles' sums, in the order of the energy kernel, spread over the warps
+            for (int k = w; k < kRedSums - 1; k += W) {
+                const double *const of = k == 1 ? x : k == 2 ? y : k == 3 ? z : k == 4 ? vx : k == 5 ? vy : vz;
+                double a = 0.0;
+                for (int q = lane; q < gone; q += 32) {
+                    const int i = sh.rlist[q];
+                    a += m[i] * (k == 0 ? 1.0 : of[i]);
                 }
-                val = kept == 0 ? 0.0 : val - mine;
+                for (int t = 16; t > 0; t >>= 1)
+                    if (t < gone) a += __shfl_down_sync(0xffffffffu, a, t);
+                if (lane == 0) sh.q4[k][0] = a;
+            }
+            __syncthreads();
+        }
+        if (w == 0) {
+            if (gone > 0) {   // the halo's sums, one a lane; the centre is formed after the last pass
+                val = kept == 0 || lane >= kRedSums - 1 ? 0.0 : val - sh.q4[lane][0];
                 const double v = per_mass(__shfl_sync(0xffffffffu, val, 0));
                 if (lane >= 4 && lane < 7) sh.w[lane - 4] = (float)(v - v0);
             }
@@ -1638,9 +1635,9 @@ __global__ void __launch_bounds__(THREADS) ub_small_kernel(
         __syncthreads();
     }
     __syncthreads();
-    if (phi_out)
+    if (phi_out && rank == 0)
         for (int r = threadIdx.x; r < nb; r += THREADS) phi_out[sh.idx[r]] = df_to_double(sh.phi[r]);
-    if (w == 0) {
+    if (w == 0 && rank == 0) {
         const double v = per_mass(__shfl_sync(0xffffffffu, val, 0));
         HaloState o{};   // what ub_output_kernel reads
         o.M = __shfl_sync(0xffffffffu, val, 0);
@@ -1805,17 +1802,24 @@ static int launch_small(const int *list, int count, const int64_t *off, const do
     if (count <= 0) return HALMA_OK;
     constexpr int smem = (int)sizeof(SmallShared<P, THREADS>);
     HALMA_CUDA(cudaFuncSetAttribute(ub_small_kernel<P, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+    int per_sm = 1;
+    HALMA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ub_small_kernel<P, THREADS>, THREADS, smem));
+    int blocks = P == kSmallMax ? kTeam : 1;
+    while ((int64_t)count * blocks > (int64_t)device_sm_count() * per_sm && blocks > 1) blocks /= 2;
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = beside_last ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)blocks;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)count);
+    cfg.gridDim = dim3((unsigned)(count * blocks));
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = beside_last ? 1 : 0;
-    HALMA_CUDA(cudaLaunchKernelEx(&cfg, ub_small_kernel<P, THREADS>, list, off, x, y, z, vx, vy, vz, m,
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    HALMA_CUDA(cudaLaunchKernelEx(&cfg, ub_small_kernel<P, THREADS>, list, blocks, off, x, y, z, vx, vy, vz, m,
                                   (float)(p.eps * p.eps), gfac, p.max_iter, bound, phi_out, hs));
     count_launch();
     return HALMA_OK;

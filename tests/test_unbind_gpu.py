@@ -243,3 +243,31 @@ def test_work_list_of_many_haloes(cuda, count):
         autotune.set_table(upper, t, slice_len)
     for g, w in zip(got, want):
         np.testing.assert_array_equal(g, w)
+
+
+@pytest.mark.parametrize("count", [1, 100, 400])
+def test_teams_of_blocks(cuda, count):
+    """Haloes of 257 to 1,024 members with four blocks each (few haloes), two and one (many): bit for bit what the pass
+    kernels give, over haloes that lose members in several passes and one that loses none."""
+    from pyhalma_gb300 import autotune
+    rng = np.random.default_rng(11)
+    sizes = rng.integers(257, 300, count)
+    sizes[0] = 991
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    n = int(off[-1])
+    cols = [rng.normal(0.0, 0.01, n) for _ in range(3)] + [rng.normal(0.0, 60.0, n) for _ in range(3)]
+    cols.append(rng.uniform(0.5, 2.0, n) * 3e8)
+    if count > 1:
+        for k in range(3, 6):
+            cols[k][off[1]:off[2]] *= 1e-3
+    opt = UnbindOptions(eps=EPS)
+    upper, t, slice_len = autotune.get_table()
+    assert slice_len >= 1024
+    got = unbind_batched(off, *cols, opt, want_phi=True)
+    try:
+        autotune.set_table(upper, t, 992)
+        want = unbind_batched(off, *cols, opt, want_phi=True)
+    finally:
+        autotune.set_table(upper, t, slice_len)
+    for g, w in zip(got, want):
+        np.testing.assert_array_equal(g, w)
