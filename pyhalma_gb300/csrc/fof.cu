@@ -61,13 +61,25 @@ struct SegGeom {
     const long long *scol = nullptr;   // [4 * nseg] first virtual x column, columns in x, y, z
 };
 
+// SHARED: the parents lie in shared memory.
+template <bool SHARED>
+__device__ __forceinline__ int uf_load(const int *p) {
+    return SHARED ? *(const volatile int *)p : __ldcg(p);
+}
+template <bool SHARED>
+__device__ __forceinline__ void uf_store(int *p, int v) {
+    if (SHARED) *(volatile int *)p = v;
+    else __stcg(p, v);
+}
+
+template <bool SHARED = false>
 __device__ __forceinline__ int uf_find(int *parent, int v, int *err) {
-    int p = __ldcg(parent + v);
+    int p = uf_load<SHARED>(parent + v);
     int guard = 0;
     const int cap = c_uf_cap;
     while (p != v) {
-        const int gp = __ldcg(parent + p);
-        if (gp != p) __stcg(parent + v, gp);   // path halving: gp is an ancestor of v
+        const int gp = uf_load<SHARED>(parent + p);
+        if (gp != p) uf_store<SHARED>(parent + v, gp);   // path halving: gp is an ancestor of v
         v = p;
         p = gp;
         if (++guard > cap) {
@@ -119,12 +131,13 @@ __device__ __forceinline__ int uf_union(int *parent, int a, int b, int *err) {
 // The same for a whole warp: every lane with need joins its a and b, all lanes one step at a time (one step of
 // both walks, or the hook).  In nested loops of their own the lanes ran one after another (3.7 of 32
 // active).  Returns each lane's node as above.
+template <bool SHARED = false>
 __device__ __forceinline__ int uf_union_warp(int *parent, int a, int b, bool need, int *err) {
     const int cap = c_uf_cap;
     int guard = 0, xa = -1, xb = -1;   // the nodes before a and b on their walks
     while (__any_sync(0xffffffffu, need)) {
         if (need) {
-            const int pa = __ldcg(parent + a), pb = __ldcg(parent + b);
+            const int pa = uf_load<SHARED>(parent + a), pb = uf_load<SHARED>(parent + b);
             if (pa == a && pb == b) {
                 if (a != b) {
                     const bool swap = uf_rank(a) < uf_rank(b);
@@ -138,8 +151,8 @@ __device__ __forceinline__ int uf_union_warp(int *parent, int a, int b, bool nee
                     need = false;
                 }
             } else {   // path halving: pa and pb are ancestors of xa and xb
-                if (pa != a && xa >= 0) __stcg(parent + xa, pa);
-                if (pb != b && xb >= 0) __stcg(parent + xb, pb);
+                if (pa != a && xa >= 0) uf_store<SHARED>(parent + xa, pa);
+                if (pb != b && xb >= 0) uf_store<SHARED>(parent + xb, pb);
                 xa = a;
                 xb = b;
                 a = pa;
@@ -936,30 +949,30 @@ __global__ void __launch_bounds__(256) label_kernel(int n, const int *__restrict
 }
 
 // ---- small inputs ---------------------------------------------------------------------------
-// Up to kSmallFof particles, all pairs: no bounding box on the host, no sort, no cells -- seven launches and one
-// round trip instead of thirty and two.  A call takes 118 us at 5,000 particles (on cells 240, start 297) and 165 at
-// 8,192 (250); at 12,000 the two are level.
+// Up to kSmallFof particles, all pairs: no bounding box on the host, no sort, no cells -- five launches and one
+// round trip instead of thirty and two.  A call takes 88 us at 5,000 particles (on cells 245, start 297), 113 at
+// 8,192 (243) and 224 at 16,384 (256).
 // A particle is its position relative to particle 0 in linking lengths as two floats an axis (error below 2^-46 of
-// the largest); particles farther apart than 2^24 linking lengths, or a zero or subnormal linking length
-// on such coordinates, make the kernels test every pair in FP64 (flags[1]).
-constexpr int kSmallFof = 8192;
+// the largest); where some lie farther apart than 2^24 linking lengths (or the linking length is subnormal),
+// pairs that the first floats leave open are tested in FP64 (flags[1]).
+constexpr int kSmallFof = 16384;
 constexpr float kSmallReach = 16777216.f;
 
-struct SmallPos {
-    float4 hi;   // x, y, z
-    float4 lo;
+struct SmallArgs {
+    int n;
+    const double *x, *y, *z;
+    float4 *pos_hi, *pos_lo;   // pos_hi[i].w: the particle's root for the sweep
+    int *flags;                // [0] non-finite coordinate, [1] FP64 tests, [4] the largest |coordinate| (float bits)
+    int *parent, *first, *err;
+    float lo, hi;
+    double r2;
 };
 
-// flags: [0] non-finite coordinate, [1] FP64 tests
-__global__ void __launch_bounds__(256) small_prep_kernel(int n, const double *__restrict__ x, const double *__restrict__ y,
-                                                         const double *__restrict__ z, double scale,
-                                                         SmallPos *__restrict__ pos, int *__restrict__ parent,
-                                                         int *__restrict__ minidx, unsigned char *__restrict__ multi,
-                                                         int *__restrict__ flags) {
+__global__ void __launch_bounds__(256) small_prep_kernel(SmallArgs A, double scale) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int bad = 0, far = 0;
-    if (i < n) {
-        const double v[3] = {x[i], y[i], z[i]}, o[3] = {x[0], y[0], z[0]};
+    int bad = 0, far = 0, reach = 0;
+    if (i < A.n) {
+        const double v[3] = {A.x[i], A.y[i], A.z[i]}, o[3] = {A.x[0], A.y[0], A.z[0]};
         float hi[3], lo[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -968,127 +981,158 @@ __global__ void __launch_bounds__(256) small_prep_kernel(int n, const double *__
             hi[d] = (float)r;
             lo[d] = (float)(r - (double)hi[d]);
             if (!(fabsf(hi[d]) < kSmallReach)) far = 1;
+            reach = max(reach, __float_as_int(fabsf(hi[d])));
         }
-        pos[i].hi = make_float4(hi[0], hi[1], hi[2], 0.f);
-        pos[i].lo = make_float4(lo[0], lo[1], lo[2], 0.f);
-        parent[i] = i;
-        minidx[i] = i;
-        multi[i] = 0;
+        A.pos_hi[i] = make_float4(hi[0], hi[1], hi[2], 0.f);
+        A.pos_lo[i] = make_float4(lo[0], lo[1], lo[2], 0.f);
+        A.parent[i] = i;
+        A.first[i] = A.n;
     }
     bad = __any_sync(0xffffffffu, bad);
     far = __any_sync(0xffffffffu, far);
+    reach = __reduce_max_sync(0xffffffffu, reach);
     if ((threadIdx.x & 31) == 0) {
-        if (bad) atomicOr(flags, 1);
-        if (far) atomicOr(flags + 1, 1);
+        if (bad) atomicOr(A.flags, 1);
+        if (far) atomicOr(A.flags + 1, 1);
+        atomicMax(A.flags + 4, reach);
     }
 }
 
-struct SmallArgs {
-    int n;
-    const double *x, *y, *z;
-    const SmallPos *pos;
-    const int *flags;
-    int *parent, *err;
-    float lo, hi;
-    double r2;
-};
-
-// Whether particles i and j are friends: 1 or 0, and with !BAND also 0 in the band around the linking length.
-template <bool BAND>
-__device__ __forceinline__ bool small_friends(const SmallArgs &A, bool fp64, const float4 &ph, const float4 &pl, int i,
-                                              int j) {
+// Whether particles i and j are friends.
+__device__ __forceinline__ bool small_friends(const SmallArgs &A, bool fp64, int i, int j) {
     if (fp64) return exact_link(A.x, A.y, A.z, i, j, A.r2);
-    const float4 qh = A.pos[j].hi, ql = A.pos[j].lo;
+    const float4 ph = A.pos_hi[i], pl = A.pos_lo[i], qh = A.pos_hi[j], ql = A.pos_lo[j];
     const float dx = (qh.x - ph.x) + (ql.x - pl.x), dy = (qh.y - ph.y) + (ql.y - pl.y), dz = (qh.z - ph.z) + (ql.z - pl.z);
     const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
     if (d2 < A.lo) return true;
-    return BAND && d2 <= A.hi && exact_link(A.x, A.y, A.z, i, j, A.r2);
+    return d2 <= A.hi && exact_link(A.x, A.y, A.z, i, j, A.r2);
 }
 
-// One warp per particle: joins it with the first friends after it, two at most, among the next kHookReach particles
-// (the sweep finds the others).  Four groups of 32 at a time: their loads are in flight together, which is what
-// the small path is bound by.
-constexpr int kHookReach = 2048, kSweepLen = 512;
+// Bounds on the squared distance of the first floats alone: below x the pair is linked, above y it is not.  The second
+// floats are at most 2^-24 of the largest coordinate, two of them an axis.  Where the FP64 test's squares overflow or
+// underflow at the linking length, it decides every pair.
+__device__ __forceinline__ float2 small_bounds(const SmallArgs &A) {
+    const float e = __int_as_float(A.flags[4]) * 0x1p-22f + 1e-5f;
+    if (A.lo >= 0.f && !(A.r2 > 1e-280 && A.r2 < 1e300)) return make_float2(-1.f, INFINITY);   // (A.lo < 0: linking length 0)
+    const float in = sqrtf(fmaxf(A.lo, 0.f)) - e, out = sqrtf(fmaxf(A.hi, 0.f)) + e;
+    return make_float2(in > 0.f ? in * in * (1.f - 1e-6f) : -1.f, out * out * (1.f + 1e-6f));
+}
 
-__global__ void __launch_bounds__(256) small_hook_kernel(SmallArgs A) {
-    const int lane = threadIdx.x & 31;
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// All pairs, a particle a lane against a run of kNearLen later ones: the first and the last that are linked beyond doubt.
+// The last becomes the particle's parent: the indices rise along every path, so this forest needs no union.
+// Each lane remembers two, so no lane waits for another one's search (a warp per particle that stopped at two
+// friends took 25 us at 5,000 particles, as lonely ones scan to the end; 10 so).
+constexpr int kNearLen = 128, kSweepLen = 512, kSweepT = 4;
+
+__global__ void __launch_bounds__(256) small_near_kernel(SmallArgs A) {
+    __shared__ float4 run[kNearLen];
+    const int i = blockIdx.x * 256 + threadIdx.x, j0 = blockIdx.y * kNearLen;
+    const int len = min(kNearLen, A.n - j0);
+    if (j0 + len <= (int)blockIdx.x * 256 + 1) return;   // nothing after any of the block's particles
+    if (threadIdx.x < len) run[threadIdx.x] = A.pos_hi[j0 + threadIdx.x];
+    __syncthreads();
     if (i >= A.n) return;
-    const bool fp64 = A.flags[1] != 0;
-    const float4 ph = A.pos[i].hi, pl = A.pos[i].lo;
-    const int end = min(A.n, i + 1 + kHookReach);
-    int links = 0, t = i;   // lane k < links: the k-th friend
-    for (int j0 = i + 1; j0 < end && links < 2; j0 += 128) {
-        bool f[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int j = j0 + 32 * u + lane;
-            f[u] = j < end && small_friends<false>(A, fp64, ph, pl, i, j);
+    const float in = small_bounds(A).x;
+    const float4 p = A.pos_hi[i];
+    int first = A.n, last = -1;
+    auto linked = [&](int k) {
+        const float dx = run[k].x - p.x, dy = run[k].y - p.y, dz = run[k].z - p.z;
+        return fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < in;
+    };
+#pragma unroll 8
+    for (int k = max(0, i + 1 - j0); k < len; ++k)
+        if (linked(k)) {
+            first = min(first, j0 + k);
+            last = j0 + k;
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            unsigned hits = __ballot_sync(0xffffffffu, f[u]);
-            for (; hits && links < 2; hits &= hits - 1, ++links)
-                if (lane == links) t = j0 + 32 * u + __ffs(hits) - 1;
-        }
+    if (last >= 0) {
+        atomicMin(A.first + i, first);
+        atomicMax(A.parent + i, last);
     }
-    uf_union_warp(A.parent, i, t, lane < links, A.err);
 }
 
-__global__ void __launch_bounds__(256) small_flatten_kernel(int n, int *parent, int *__restrict__ root, int *err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) root[i] = uf_find(parent, i, err);
+// One block, the parents in shared memory: every particle joined with its first friend, and the roots, for the sweep.
+// (In global memory, every step of a path a trip to L2, the unions took 31 us at 5,000 particles; 10 so, roots included.)
+__global__ void __launch_bounds__(1024) small_union_kernel(SmallArgs A) {
+    extern __shared__ int su_parent[];
+    for (int i = threadIdx.x; i < A.n; i += 1024) su_parent[i] = A.parent[i];
+    __syncthreads();
+    for (int b = 0; b < A.n; b += 1024) {   // whole warps
+        const int i = b + threadIdx.x;
+        const int first = i < A.n ? A.first[i] : A.n;
+        uf_union_warp<true>(su_parent, min(first, A.n - 1), min(i, A.n - 1), first < A.n, A.err);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < A.n; i += 1024) {
+        const int r = uf_find<true>(su_parent, i, A.err);
+        A.parent[i] = r;
+        A.pos_hi[i].w = __int_as_float(r);
+    }
 }
 
-// One warp per particle i and run of kSweepLen particles (blockIdx.y): the friends after i whose roots differ are joined.
-__global__ void __launch_bounds__(256) small_sweep_kernel(SmallArgs A, const int *__restrict__ root) {
+// All pairs again, four particles a warp against runs of kSweepLen, one of them a lane: those that may be friends and
+// whose roots differ are looked at closely and joined.  A pair costs nine instructions (four particles share a
+// load; the roots come with the positions); with both floats of every position and a particle a warp
+// 5,000 particles took 30 us, 11 so.
+__global__ void __launch_bounds__(256) small_sweep_kernel(SmallArgs A) {
     const int lane = threadIdx.x & 31;
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int i0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kSweepT;
     const int j1 = min(A.n, (int)(blockIdx.y + 1) * kSweepLen);
-    if (i + 1 >= j1) return;
+    if (i0 >= A.n || i0 + 1 >= j1) return;
     const bool fp64 = A.flags[1] != 0;
-    const float4 ph = A.pos[i].hi, pl = A.pos[i].lo;
-    const int ri = root[i];
-    for (int j0 = max(i + 1, (int)blockIdx.y * kSweepLen); j0 < j1; j0 += 128) {
-        bool link[4];
+    const float out = small_bounds(A).y;
+    float4 p[kSweepT];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int j = j0 + 32 * u + lane;
-            link[u] = j < j1 && root[j] != ri && small_friends<true>(A, fp64, ph, pl, i, j);
+    for (int t = 0; t < kSweepT; ++t) p[t] = A.pos_hi[min(i0 + t, A.n - 1)];   // the last one's pairs again past the end
+#pragma unroll 2
+    for (int j0 = max(i0 & ~31, (int)blockIdx.y * kSweepLen); j0 < j1; j0 += 32) {
+        const int j = j0 + lane;
+        const float4 q = A.pos_hi[min(j, A.n - 1)];
+        unsigned may = 0;
+#pragma unroll
+        for (int t = 0; t < kSweepT; ++t) {
+            const float dx = q.x - p[t].x, dy = q.y - p[t].y, dz = q.z - p[t].z;
+            const bool near = !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > out);   // NaN where the floats overflow
+            if (near && __float_as_int(q.w) != __float_as_int(p[t].w)) may |= 1u << t;
         }
-        if (!__any_sync(0xffffffffu, link[0] | link[1] | link[2] | link[3])) continue;
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            uf_union_warp(A.parent, i, link[u] ? j0 + 32 * u + lane : i, link[u], A.err);
+        if (!__any_sync(0xffffffffu, may)) continue;
+#pragma unroll 1
+        for (int t = 0; t < kSweepT; ++t) {
+            const int i = min(i0 + t, A.n - 1), jj = min(j, A.n - 1);
+            const bool link = (may >> t & 1u) && small_friends(A, fp64, i, jj);
+            uf_union_warp(A.parent, i, link ? jj : i, link, A.err);
+        }
     }
 }
 
-__global__ void __launch_bounds__(256) small_root_kernel(int n, int *parent, int *__restrict__ root, int *minidx,
-                                                         unsigned char *__restrict__ multi, int *err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int r = uf_find(parent, i, err);
-    root[i] = r;
-    if (r != i) {
-        atomicMin(minidx + r, i);
-        multi[r] = 1;
+// One block, in shared memory: roots, smallest members and labels (-1 alone), and the number of groups.
+__global__ void __launch_bounds__(1024) small_label_kernel(int n, const int *__restrict__ parent,
+                                                           int *__restrict__ labels, int *__restrict__ ngroups,
+                                                           int *err) {
+    extern __shared__ int sl_smem[];
+    int *up = sl_smem, *least = sl_smem + n;   // least[r]: r's smallest member, n + that while r is alone
+    __shared__ int groups;
+    if (threadIdx.x == 0) groups = 0;
+    for (int i = threadIdx.x; i < n; i += 1024) {
+        up[i] = parent[i];
+        least[i] = n + i;
     }
-}
-
-__global__ void __launch_bounds__(256) small_label_kernel(int n, const int *__restrict__ root,
-                                                          const int *__restrict__ minidx,
-                                                          const unsigned char *__restrict__ multi,
-                                                          int *__restrict__ labels, int *__restrict__ ngroups) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool first = false;
-    if (i < n) {
-        const int r = root[i];
-        const int l = multi[r] ? minidx[r] : -1;
-        labels[i] = l;
-        first = l == i;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += 1024) {
+        const int r = uf_find<true>(up, i, err);
+        if (r != i) atomicMin(least + r, min(i, r));
     }
-    const unsigned b = __ballot_sync(0xffffffffu, first);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(ngroups, __popc(b));
+    __syncthreads();
+    int mine = 0;
+    for (int i = threadIdx.x; i < n; i += 1024) {
+        const int l = least[uf_find<true>(up, i, err)];
+        labels[i] = l < n ? l : -1;
+        mine += l == i;
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&groups, mine);
+    __syncthreads();
+    if (threadIdx.x == 0) *ngroups = groups;
 }
 
 int bits_for(uint64_t v) {
@@ -1378,29 +1422,29 @@ int fof_core(int n, const double *x, const double *y, const double *z, FofGeom g
 int fof_small(int n, const double *x, const double *y, const double *z, double ll, int *labels, int64_t *n_groups,
               cudaStream_t st) {
     Layout L;
-    const size_t o_pos = L.add(sizeof(SmallPos) * n), o_par = L.add(4ull * n), o_root = L.add(4ull * n);
-    const size_t o_min = L.add(4ull * n), o_multi = L.add(1ull * n), o_cnt = L.add(64);
+    const size_t o_hi = L.add(sizeof(float4) * n), o_lo = L.add(sizeof(float4) * n), o_par = L.add(4ull * n);
+    const size_t o_first = L.add(4ull * n), o_cnt = L.add(64);
     void *base = nullptr;
     HALMA_TRY(push_uf_cap(st));
     HALMA_TRY(workspace(L.total, &base, st));
     int *cnt = at<int>(base, o_cnt);   // [0] non-finite [1] FP64 tests [2] groups [3] error
-    int *parent = at<int>(base, o_par), *root = at<int>(base, o_root), *minidx = at<int>(base, o_min);
-    auto *multi = at<unsigned char>(base, o_multi);
+    int *parent = at<int>(base, o_par);
     Profile &prof = profile();
     FofGeom g{};
     set_scale(g, ll, 0.0);
     HALMA_CUDA(cudaMemsetAsync(cnt, 0, 64, st));
-    const int gt = grid_for(n, 256), gw = grid_for(n, 8);
-    SmallArgs A{n, x, y, z, at<SmallPos>(base, o_pos), cnt, parent, cnt + 3, g.lo, g.hi, g.r2};
-    HALMA_LAUNCH(small_prep_kernel, gt, 256, 0, st, n, x, y, z, g.inv_scale, at<SmallPos>(base, o_pos), parent, minidx,
-                 multi, cnt);
+    const int gt = grid_for(n, 256);
+    SmallArgs A{n,   x,      y,      z, at<float4>(base, o_hi), at<float4>(base, o_lo),
+                cnt, parent, at<int>(base, o_first), cnt + 3, g.lo, g.hi, g.r2};
+    HALMA_LAUNCH(small_prep_kernel, gt, 256, 0, st, A, g.inv_scale);
     for (int k = 1; k <= 5; ++k) HALMA_TRY(prof.fof_mark(k, st));
-    HALMA_LAUNCH(small_hook_kernel, gw, 256, 0, st, A);
-    HALMA_LAUNCH(small_flatten_kernel, gt, 256, 0, st, n, parent, root, cnt + 3);
-    HALMA_LAUNCH(small_sweep_kernel, dim3(gw, (n + kSweepLen - 1) / kSweepLen), 256, 0, st, A, root);
+    HALMA_LAUNCH(small_near_kernel, dim3(gt, (n + kNearLen - 1) / kNearLen), 256, 0, st, A);
+    HALMA_CUDA(cudaFuncSetAttribute(small_union_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kSmallFof));
+    HALMA_LAUNCH(small_union_kernel, 1, 1024, 4 * n, st, A);
+    HALMA_LAUNCH(small_sweep_kernel, dim3(grid_for(n, 8 * kSweepT), (n + kSweepLen - 1) / kSweepLen), 256, 0, st, A);
     HALMA_TRY(prof.fof_mark(6, st));
-    HALMA_LAUNCH(small_root_kernel, gt, 256, 0, st, n, parent, root, minidx, multi, cnt + 3);
-    HALMA_LAUNCH(small_label_kernel, gt, 256, 0, st, n, root, minidx, multi, labels, cnt + 2);
+    HALMA_CUDA(cudaFuncSetAttribute(small_label_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kSmallFof));
+    HALMA_LAUNCH(small_label_kernel, 1, 1024, 8 * n, st, n, parent, labels, cnt + 2, cnt + 3);
     HALMA_TRY(prof.fof_mark(7, st));
     int hc[4];
     HALMA_CUDA(cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));

@@ -222,7 +222,7 @@ def _filled(x, y, z, ll, total):
     return f(x, fx), f(y, np.zeros(k)), f(z, np.zeros(k))
 
 
-@pytest.mark.parametrize("total", [8192, 8193])
+@pytest.mark.parametrize("total", [8192, 8193, 16384, 16385])
 def test_both_sides_of_the_small_path(golden, cuda, total):
     """The reference's own cases on the all-pairs path and, filled up past its limit, on the cell path."""
     d = golden("fof_cases.npz")
