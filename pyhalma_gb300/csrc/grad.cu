@@ -21,7 +21,7 @@
 namespace halma {
 namespace {
 
-constexpr int kGWarps = 4, kGT = 2;
+constexpr int kGWarps = 4;
 constexpr float kFarG = 3.0e30f;
 
 __device__ __forceinline__ float4 load_b(const float *__restrict__ x, const float *__restrict__ y,
@@ -473,12 +473,20 @@ int launch_both(const BothPlan &P, const float *sx, const float *sy, const float
     return HALMA_OK;
 }
 
+// Targets a lane: four share the loads of a partner, but leave fewer items and, with the scalar sum, fewer warps an SM.
+// Vectors alone: 3,000 against 4,000 20 us with two and 23 with four, 20,000 x 25,000 233 and 232, 160,000 x 200,000 13.4 ms
+// and 12.7, 10^6 x 4e5 167 and 159; with the scalar two at every size (160,000 x 200,000: 14.2 and 14.5).
 template <bool WANT_S>
+int adjoint_targets(int64_t na) {
+    return !WANT_S && na >= 16384 ? 4 : 2;
+}
+
+template <bool WANT_S, int T>
 int launch_adjoint(const float *bx, const float *by, const float *bz, const float *bw, int64_t nb, const float *ax,
                    const float *ay, const float *az, int64_t na, float eps2, int self_mask, int64_t self_off,
                    int n_split, int64_t split_len, const float *vscale, float *out_s, float *out_v, double *part,
                    cudaStream_t st) {
-    constexpr int T = kGT, NV = WANT_S ? 4 : 3;
+    constexpr int NV = WANT_S ? 4 : 3;
     const int64_t items = (na + 32 * T - 1) / (32 * T) * n_split;
     HALMA_LAUNCH((adjoint_kernel<T, WANT_S>), (unsigned)((items + kGWarps - 1) / kGWarps), 32 * kGWarps, 0, st, bx, by,
                  bz, bw, nb, ax, ay, az, na, eps2, self_mask, self_off, n_split, split_len, vscale, out_s, out_v, part);
@@ -536,8 +544,8 @@ extern "C" int halma_potential_grad_f32(int64_t ns, const float *m_, const float
     sg.add((const float *)grad_tgt, grad_tgt ? 3 * nt : 0, false, true, &gt);
     int split_t = 1, split_s = 1;
     int64_t len_t = ns, len_s = nt;
-    if (grad_tgt) choose_slices(nt, ns, kGT, 3, &split_t, &len_t);
-    if (grad_m || grad_src) choose_slices(ns, nt, kGT, 4, &split_s, &len_s);
+    if (grad_tgt) choose_slices(nt, ns, adjoint_targets<false>(nt), 3, &split_t, &len_t);
+    if (grad_m || grad_src) choose_slices(ns, nt, adjoint_targets<true>(ns), 4, &split_s, &len_s);
     // both sides in one sweep from kBothPairs pairs on, and with a softening that keeps r^-2 finite
     const bool both = grad_tgt && (grad_m || grad_src) && (double)ns * (double)nt >= kBothPairs &&
                       (float)eps2 >= 0x1p-126f;
@@ -557,11 +565,13 @@ extern "C" int halma_potential_grad_f32(int64_t ns, const float *m_, const float
                               reinterpret_cast<float2 *>(part), st));
         return sg.download(st);
     }
-    if (gt)
-        HALMA_TRY(launch_adjoint<false>(sx, sy, sz, m, ns, tx, ty, tz, nt, (float)eps2, self, self_offset, split_t, len_t,
-                                        g, nullptr, gt, part, st));
+    if (gt) {
+        auto run = adjoint_targets<false>(nt) == 4 ? launch_adjoint<false, 4> : launch_adjoint<false, 2>;
+        HALMA_TRY(run(sx, sy, sz, m, ns, tx, ty, tz, nt, (float)eps2, self, self_offset, split_t, len_t, g, nullptr, gt,
+                      part, st));
+    }
     if (gm || gs)
-        HALMA_TRY(launch_adjoint<true>(tx, ty, tz, g, nt, sx, sy, sz, ns, (float)eps2, self, -self_offset, split_s, len_s,
-                                       m, gm, gs, part, st));
+        HALMA_TRY((launch_adjoint<true, 2>(tx, ty, tz, g, nt, sx, sy, sz, ns, (float)eps2, self, -self_offset, split_s,
+                                           len_s, m, gm, gs, part, st)));
     return sg.download(st);
 }
