@@ -84,13 +84,15 @@ int64_t     halma_kernel_launch_count(void);
  * fills out[] with [fof_ms, unbind_ms, n_passes, pairs_0, ms_0, sym_pairs_0, sym_ms_0,
  * pairs_1, ...] for the last call (per pass: pair terms, milliseconds of the pass's pair
  * kernels, the pair terms of the haloes that ran on the symmetric block kernel, where each
- * pair is evaluated once for both particles, and the milliseconds of that kernel alone) and
+ * pair is evaluated once for both particles, and the milliseconds of that kernel alone; haloes
+ * of up to 1,024 members run all their passes in one block and are not among them) and
  * returns the number of values available. */
 int         halma_set_profiling(int32_t on);
 int         halma_profile_stats(double *out, int32_t cap);
 /* With profiling on: milliseconds of the FoF stages of the last halma_find_haloes call
- * (bounding box + keys, key sort, sorted records + sub-cell runs, cell table + hash +
- * one-component cells, work items, linking, roots + labels, groups); returns the count (8). */
+ * (bounding box + keys, key sort, cells and nodes with their records, 0 (kept for its place),
+ * cell pairs, linking, roots + labels, groups); on the all-pairs path of small inputs all but
+ * the last three are 0; returns the count (8). */
 int         halma_profile_fof_stages(double *out, int32_t cap);
 /* Measurement hook (no reference counterpart): the FP32 FMA rate of the current device, from
  * a kernel of independent FMA chains (packed != 0: fma.rn.f32x2, else fma.rn.f32), iters
@@ -421,7 +423,7 @@ typedef struct {
     double  factor_v;   /* potential multiplied by factor_v^2 (halo_properties.py:353)  */
     int32_t max_iter;   /* passes at most (>= 1)                                        */
     int32_t precision;  /* HALMA_UNBIND_FP32C or HALMA_UNBIND_FP64                      */
-    int32_t use_graph;  /* FP32C: replay all passes as one captured CUDA graph          */
+    int32_t use_graph;  /* FP32C: passes as captured CUDA graphs where that is faster  */
     int32_t flags;      /* HALMA_UNBIND_FULL_RECOMPUTE or 0                             */
 } halma_unbind_params;
 

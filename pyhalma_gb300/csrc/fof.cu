@@ -21,6 +21,7 @@
 //      a link among their first tests go to a list that blocks work off;
 //   6. each component's label = the smallest ORIGINAL index among its members (atomicMin over nodes), -1
 //      for particles alone.
+// Inputs of up to kSmallFof particles take all pairs instead (fof_small).
 // The result is the reference's partition exactly: same components, same canonical labels.
 #include <math.h>
 #include <limits.h>
@@ -412,9 +413,8 @@ __global__ void keys_kernel(const double *__restrict__ x, const double *__restri
 // Sorted position k starts a cell when its cell key differs from its predecessor's, and a node when its
 // full key does (without half-cells in the key, every particle is a node).  A warp numbers kScanRun
 // consecutive positions with ballots; head_count_kernel leaves cells << 32 | nodes per warp, whose
-// exclusive scan is where head_apply_kernel's warp starts.  Together they replaced eight passes (records and
-// run heads, two scans, run joins, cell table, one-component flags): 0.50 of 11.5 ms at 2e7 particles
-// became 0.31.
+// exclusive scan is where head_apply_kernel's warp starts.  Together with the scan they take 0.50 ms at 2e7 particles,
+// where eight passes (records and run heads, two scans, run joins, cell table, one-component flags) took 0.83.
 constexpr int kScanRun = 512;
 
 struct Heads {

@@ -205,7 +205,7 @@ void choose_slices(int64_t na, int64_t nb, int T, int nv, int *n_split, int64_t 
 // A block of four warps holds 1,024 targets, eight a lane, and stages 512 sources; an item is one block of sources against
 // `tblocks` blocks of targets, the sources' sums kept in shared memory (compensated) over them.  Per item and
 // target, or source, one partial sum is written; they are added in order.
-// Bound: the FP32 pipe (18 lane-operations and a rsqrt a pair; it is 75 % busy).  160,000 targets x 200,000 sources:
+// Bound: the FP32 pipe (18 lane-operations and a rsqrt a pair; it is 70 % busy).  160,000 targets x 200,000 sources:
 // 27.5 ms in two sweeps, 22.0 in one (four targets a lane, two sources an instruction and r^-3 weighted twice: 23.5;
 // 256 sources, or ten or six targets a lane, 3 to 5 % more).
 constexpr int kBothT = 8, kBothTargets = 128 * kBothT, kBothSources = 512, kBothChunks = kBothSources / 32;

@@ -283,7 +283,7 @@ static int launch_reference(const float *m, const float *x, const float *y, cons
 //
 // Bound: the special-function unit (one rsqrt a term) and the FP32 pipe (7 lane-operations) together, as
 // the unbinding's tile kernel: two sources per two-lane instruction.  With one-lane instructions the
-// star terms of a 160,000-cell gas halo (6.4e9) took 2.29 ms, now 1.6.
+// star terms of a 160,000-cell gas halo (6.4e9) took 2.29 ms, now 1.69.
 template <bool FTZ>
 __device__ __forceinline__ float pot_rsqrt(float v) {
     return FTZ ? rsqrt_ftz(v) : rsqrtf(v);
@@ -449,7 +449,7 @@ constexpr int64_t kMaxPartials = 1ll << 21;   // partial sums of one call, from 
 
 // Number of source slices so that (target tiles x slices) keeps every SM busy.  Slices have at least
 // 2048 sources, or 128 while the partial sums stay within kMaxPartials: 3,000 targets x 4,000
-// sources took 248 us in one slice (24 warps), 13 us in 32.
+// sources took 248 us in one slice (24 warps), 12 us in 32.
 static void choose_split(int64_t ns, int64_t nt, int T, int *n_split, int64_t *split_len) {
     const int sms = device_sm_count();
     const int64_t ntiles = (nt + 32 * T - 1) / (32 * T);
@@ -549,13 +549,14 @@ __global__ void pack_sources_kernel(int64_t n, const float *__restrict__ m, cons
 }
 
 // phi_i = the set's slices in block order + the other sources (float32 or per-slice FP64
-// partials) + the self term m_i eps^-1 when the self pair is counted (mask NONE); FP64 sum.
+// partials) + the self term m_i eps^-1 when the self pair is counted (mask NONE); FP64 sum, which bounds it (232 us of
+// the 160,000-cell gas halo's forward, with one load in flight or eight).
 __global__ void sym_finish_kernel(int64_t nt, int nblk, int64_t npad, const float2 *__restrict__ part,
                                   const float *__restrict__ tail, const double *__restrict__ tail_part, int n_tail,
                                   const float *__restrict__ m, double self_scale, float *__restrict__ out) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nt; i += (int64_t)gridDim.x * blockDim.x) {
         double acc = 0.0;
-#pragma unroll 8   // loads in flight: one at a time took 232 us of the 160,000-cell gas halo's forward
+#pragma unroll 8
         for (int b = 0; b < nblk; ++b) {
             const float2 v = part[(int64_t)b * npad + i];
             acc += (double)v.x + (double)v.y;

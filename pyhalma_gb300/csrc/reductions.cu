@@ -582,7 +582,7 @@ int reductions_device(int64_t n, int nh, const int64_t *off, const double *x, co
 // The same for kRedSets sets of positions over the same n members of nh haloes, in one run: off has kRedSets * nh + 1
 // entries (set s, halo h: s * n + the member offset), about and out kRedSets * nh rows, about complete but for
 // R05.  out holds R05 and R_max, and sigma for the first set; the sums that about replaces are not formed.  One run
-// keeps four times as many walks in flight: 120 groups of 4e5 members took 4 x 0.17 ms for them, now 0.19.
+// keeps four times as many walks in flight: 120 groups of 4e5 members took 4 x 0.17 ms for them, now 0.14.
 int reductions_sets_device(int64_t n, int nh, const int64_t *off, const double *const (*pos)[3], const double *vx,
                            const double *vy, const double *vz, const double *m, const double *about, double *out,
                            cudaStream_t st) {

@@ -6,17 +6,18 @@
 //   reduce  - per halo, FP64 mass, centre of mass and bulk velocity;
 //   pack    - members re-centred on their halo's centre, float4 (x, y, z, m), padded to a
 //             multiple of 32 with zero-mass far points (halo-contiguous slots).
-// Every pass over all active haloes is then five kernels:
+// Haloes of up to kSmallMax members run all their passes in one block each (ub_small_kernel).  Every pass over the
+// other active haloes is four kernels, the first of these lists being written beside the last kernel of the pass before:
 //   items   - the implicit work list: per halo, (target tile of 32*T) x (source slice) items,
 //             biggest haloes first, and the energy segments of the pass;
 //   pairs   - persistent kernel: warps take items from an atomic counter, stream the slice's
 //             sources through a per-warp shared-memory chunk, two sources per f32x2
 //             instruction, 32-term FP32 partials folded into a TwoSum-compensated
 //             accumulator; the self pair is skipped by slot index;
-//   energy / compact / finalize - FP64 energy and sign test, survivors compacted into the
-//             other packed buffer, next pass's FP64 centre and bulk velocity; a halo whose pass
+//   energy / finalize / compact - energy and sign test, the next pass's FP64 mass, centre and bulk
+//             velocity, survivors compacted into the other packed buffer; a halo whose pass
 //             removed nothing becomes inactive and costs nothing later.
-// All passes are captured once into a CUDA graph and replayed (cached by shape).
+// Passes are launched as they are or as captured graphs (see kPassChunk).
 #include <math.h>
 #include <string.h>
 

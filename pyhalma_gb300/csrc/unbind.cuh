@@ -5,7 +5,7 @@
 namespace halma {
 
 // Optional measurement state (halma_set_profiling): CUDA events recorded on the launching
-// stream around every pair-kernel launch (captured into the pass graph as event nodes) and
+// stream around every pair-kernel launch (event nodes where the passes are captured) and
 // the pair count of each pass, read back at the end of the call.
 struct Profile {
     bool enabled = false;
