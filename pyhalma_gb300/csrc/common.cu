@@ -95,15 +95,77 @@ int workspace(size_t bytes, void **ptr, cudaStream_t stream, int slot) {
     return HALMA_OK;
 }
 
-bool is_device_pointer(const void *p) {
-    if (!p) return false;
+MemoryKind memory_kind(const void *p) {
+    if (!p) return MemoryKind::kUnknown;
     cudaPointerAttributes a;
     cudaError_t e = cudaPointerGetAttributes(&a, p);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return MemoryKind::kUnknown;
     }
-    return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
+    if (a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged) return MemoryKind::kDevice;
+    return a.type == cudaMemoryTypeHost ? MemoryKind::kPinned : MemoryKind::kPageable;
+}
+
+bool is_device_pointer(const void *p) { return memory_kind(p) == MemoryKind::kDevice; }
+
+bool host_page_tables() {
+    static std::map<int, bool> m;   // a property of the device
+    static std::mutex mu;
+    std::lock_guard<std::mutex> guard(mu);
+    const int d = current_device();
+    auto it = m.find(d);
+    if (it == m.end()) {
+        int v = 0;
+        if (cudaDeviceGetAttribute(&v, cudaDevAttrPageableMemoryAccessUsesHostPageTables, d) != cudaSuccess) {
+            cudaGetLastError();
+            v = 0;
+        }
+        it = m.emplace(d, v != 0).first;
+    }
+    return it->second;
+}
+
+namespace {
+
+// Array blockIdx.y, in the widest words its address allows (the destination is 256-byte aligned), then the bytes left over.
+template <class W>
+__device__ __forceinline__ size_t upload_words(const void *src, void *dst, size_t bytes) {
+    const W *from = static_cast<const W *>(src);
+    W *to = static_cast<W *>(dst);
+    const size_t n = bytes / sizeof(W), step = (size_t)gridDim.x * blockDim.x;
+    size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    for (; i + 3 * step < n; i += 4 * step) {
+        W v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = from[i + k * step];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) to[i + k * step] = v[k];
+    }
+    for (; i < n; i += step) to[i] = from[i];
+    return n * sizeof(W);
+}
+
+__global__ void __launch_bounds__(512) upload_kernel(Uploads u) {
+    const void *src = u.src[blockIdx.y];
+    void *dst = u.dst[blockIdx.y];
+    const size_t bytes = u.bytes[blockIdx.y];
+    const unsigned at = (unsigned)(uintptr_t)src;
+    const size_t done = at % 16 == 0  ? upload_words<uint4>(src, dst, bytes)
+                        : at % 8 == 0 ? upload_words<uint2>(src, dst, bytes)
+                        : at % 4 == 0 ? upload_words<unsigned>(src, dst, bytes)
+                                      : upload_words<unsigned char>(src, dst, bytes);
+    const size_t i = done + blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (i < bytes) static_cast<unsigned char *>(dst)[i] = static_cast<const unsigned char *>(src)[i];
+}
+
+}  // namespace
+
+int upload(const Uploads &u, cudaStream_t s) {
+    size_t most = 0;
+    for (int k = 0; k < u.n; ++k) most = std::max(most, u.bytes[k]);
+    HALMA_LAUNCH(upload_kernel, dim3((unsigned)grid_for((int64_t)(most / 16 + 1), 512, 64), (unsigned)u.n), 512, 0, s, u);
+    return HALMA_OK;
 }
 
 }  // namespace halma

@@ -70,7 +70,23 @@ int workspace(size_t bytes, void **ptr, cudaStream_t stream, int slot = 0);
 template <class T>
 inline T *at(void *base, size_t off) { return reinterpret_cast<T *>(static_cast<char *>(base) + off); }
 
+// Where an address lies: on the device (or managed), in page-locked host memory, or elsewhere on the host.
+enum class MemoryKind { kDevice, kPinned, kPageable, kUnknown };
+MemoryKind memory_kind(const void *p);
 bool is_device_pointer(const void *p);
+
+// One launch that copies up to kUploads arrays of the caller's from pageable host memory, which this GPU reads
+// over its link with the CPU's own page tables (host_page_tables()).  cudaMemcpyAsync takes 9 us of the host's time an array and
+// one after another: seven arrays of 80 kB 63 us, in one launch 16; of 3.2 MB 201 and 119, of 64 MB 2,602 and 2,152.
+constexpr int kUploads = 12;
+struct Uploads {
+    const void *src[kUploads];
+    void *dst[kUploads];
+    size_t bytes[kUploads];
+    int n = 0;
+};
+bool host_page_tables();
+int upload(const Uploads &u, cudaStream_t s);
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -86,16 +102,31 @@ struct Stager {
         void **slot;
         bool late;   // uploaded on the late stream of bind_and_upload, when one is given
         cudaEvent_t mark = nullptr;   // a marker, not an array: the event recorded at this point
+        bool pageable = false;        // readable by upload()
     };
     std::vector<Item> items;
     bool any_host = false;
+    cudaStream_t reading = nullptr;   // a launch on it may still read the caller's host memory
+    bool reads_host = false;
+
+    Stager() = default;
+    Stager(const Stager &) = delete;
+    Stager &operator=(const Stager &) = delete;
+    // On every way out: the caller's memory is not read after the call.
+    ~Stager() {
+        if (reads_host) cudaStreamSynchronize(reading);
+    }
 
     // `slot` receives the device pointer the kernels must use.
     template <class T, class U>
     void add(const T *user, size_t count, bool in, bool out, U **slot, bool late = false) {
         Item it{user, count * sizeof(T), in, out, false, 0,
                 reinterpret_cast<void **>(const_cast<typename std::remove_const<U>::type **>(slot)), late};
-        if (user && count > 0) it.host = !is_device_pointer(user);
+        if (user && count > 0) {
+            const MemoryKind kind = memory_kind(user);
+            it.host = kind != MemoryKind::kDevice;
+            it.pageable = kind == MemoryKind::kPageable && host_page_tables();
+        }
         any_host |= it.host;
         items.push_back(it);
     }
@@ -114,6 +145,16 @@ struct Stager {
     // s wait for before their first use.  With after_ev, the late copies start once the copies
     // on s have been done (after_ev is recorded on s and late_s waits for it).
     int bind_and_upload(void *base, cudaStream_t s, cudaStream_t late_s = nullptr, cudaEvent_t after_ev = nullptr) {
+        Uploads batch;
+        auto flush = [&]() -> int {
+            if (batch.n > 0) {
+                reading = s;
+                reads_host = true;
+                HALMA_TRY(upload(batch, s));
+            }
+            batch.n = 0;
+            return HALMA_OK;
+        };
         for (int pass = 0; pass < 2; ++pass) {   // the items on s first, then the late ones
             if (pass == 1 && late_s && after_ev) {
                 HALMA_CUDA(cudaEventRecord(after_ev, s));
@@ -123,6 +164,7 @@ struct Stager {
                 const bool late = it.late && late_s;
                 if (late != (pass == 1)) continue;
                 if (it.mark) {
+                    HALMA_TRY(flush());
                     HALMA_CUDA(cudaEventRecord(it.mark, late ? late_s : s));
                     continue;
                 }
@@ -132,13 +174,20 @@ struct Stager {
                 }
                 if (it.host) {
                     *it.slot = at<void>(base, it.off);
-                    if (it.in)
+                    if (it.in && it.pageable && !late) {
+                        batch.src[batch.n] = it.user;
+                        batch.dst[batch.n] = *it.slot;
+                        batch.bytes[batch.n++] = it.bytes;
+                        if (batch.n == kUploads) HALMA_TRY(flush());
+                    } else if (it.in) {
                         HALMA_CUDA(cudaMemcpyAsync(*it.slot, it.user, it.bytes, cudaMemcpyHostToDevice,
                                                    late ? late_s : s));
+                    }
                 } else {
                     *it.slot = const_cast<void *>(it.user);
                 }
             }
+            HALMA_TRY(flush());
         }
         return HALMA_OK;
     }
@@ -148,6 +197,7 @@ struct Stager {
                 HALMA_CUDA(cudaMemcpyAsync(const_cast<void *>(it.user), *it.slot, it.bytes,
                                            cudaMemcpyDeviceToHost, s));
         if (any_host) HALMA_CUDA(cudaStreamSynchronize(s));
+        if (reading == s) reads_host = false;
         return HALMA_OK;
     }
 };

@@ -178,3 +178,24 @@ def test_reference_mode_split_over_sources(cuda, kind, ns, nt):
     with np.errstate(all="ignore"):
         ref = oracle.bf_potential_f32(m, *s.T, *t.T)
     np.testing.assert_array_equal(got, ref)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 33, 2049, 70_001])
+def test_host_arrays_at_any_address(cuda, n):
+    """Host inputs are copied to the device whole, in the widest words their addresses allow: the same potentials for
+    arrays that start 0, 4, 8 and 12 bytes past a 16-byte boundary."""
+    rng = np.random.default_rng(n)
+    cols = [rng.normal(0, 1, n).astype(np.float32) for _ in range(3)] + [rng.uniform(1, 2, n).astype(np.float32)]
+    tgt = [rng.normal(0, 1, 19).astype(np.float32) for _ in range(3)]
+
+    def moved(a, k):
+        raw = np.zeros(len(a) + 8, dtype=np.float32)
+        first = (-raw.ctypes.data // 4) % 4 + k
+        out = raw[first:first + len(a)]
+        out[:] = a
+        assert out.ctypes.data % 16 == 4 * k
+        return out
+    want = halo_gas.bf_potential(cols[3], *cols[:3], *tgt, mode="reference")
+    for k in range(4):
+        c, t = [moved(a, (k + q) % 4) for q, a in enumerate(cols)], [moved(a, k) for a in tgt]
+        assert np.array_equal(halo_gas.bf_potential(c[3], *c[:3], *t, mode="reference"), want), k
