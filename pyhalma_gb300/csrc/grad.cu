@@ -74,6 +74,19 @@ __device__ __forceinline__ void fold2(float &s, float &c, f2x v) {
     two_sum_acc(s, c, lo + hi);
 }
 
+// One end of the pairs: na particles a, their sums over nb partners b with weights bw, in n_split slices of the partners.
+struct AdjointSide {
+    const float *bx, *by, *bz, *bw;
+    int64_t nb;
+    const float *ax, *ay, *az;
+    int64_t na, self_off;
+    int n_split;
+    int64_t split_len;
+    const float *vscale;
+    float *out_s, *out_v;
+    double *part;
+};
+
 // One warp per item: a tile of 32*T particles a against one slice of the partners b, streamed in
 // chunks of 32 through a per-warp shared buffer; chunk partials folded into TwoSum-compensated sums.
 // A slice's sums go to part[(slice * na + a) * NV + v] (v: the scalar sum if wanted, then the vector), added
@@ -82,15 +95,17 @@ __device__ __forceinline__ void fold2(float &s, float &c, f2x v) {
 // Bound: the FP32 pipe (12 or 13 lane-operations a pair, 10 pairs per SM-cycle).  The partners are sliced so
 // that several items wait for every warp slot (choose_slices): one item per tile left 94 warps for 3,000
 // cells (150 us a sweep, now 11) and 2.06 blocks an SM, the third round nearly empty, for 160,000
-// (19.6 ms, now 13.3).
+// (19.6 ms, now 12.7).
 template <int T, bool WANT_S>
-__global__ void __launch_bounds__(32 * kGWarps) adjoint_kernel(
-    const float *__restrict__ bx, const float *__restrict__ by, const float *__restrict__ bz,
-    const float *__restrict__ bw, int64_t nb, const float *__restrict__ ax, const float *__restrict__ ay,
-    const float *__restrict__ az, int64_t na, float eps2, int self_mask, int64_t self_off, int n_split,
-    int64_t split_len, const float *__restrict__ vscale, float *__restrict__ out_s, float *__restrict__ out_v,
-    double *__restrict__ part) {
-    __shared__ float4 buf[kGWarps][32];
+__device__ __forceinline__ void adjoint_items(const AdjointSide &S, float eps2, int self_mask, int64_t block,
+                                              float4 (*buf)[32]) {
+    const float *__restrict__ bx = S.bx, *__restrict__ by = S.by, *__restrict__ bz = S.bz, *__restrict__ bw = S.bw;
+    const float *__restrict__ ax = S.ax, *__restrict__ ay = S.ay, *__restrict__ az = S.az;
+    const float *__restrict__ vscale = S.vscale;
+    float *__restrict__ out_s = S.out_s, *__restrict__ out_v = S.out_v;
+    double *__restrict__ part = S.part;
+    const int64_t nb = S.nb, na = S.na, self_off = S.self_off, split_len = S.split_len;
+    const int n_split = S.n_split;
     constexpr int NV = WANT_S ? 4 : 3;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float *sa = reinterpret_cast<float *>(buf[w]);        // 16 float4: x/y pairs
@@ -98,7 +113,7 @@ __global__ void __launch_bounds__(32 * kGWarps) adjoint_kernel(
     const int kp = lane >> 1, hf = lane & 1;
     const f2x e2 = pack2(eps2, eps2);
     const int64_t ntiles = (na + 32 * T - 1) / (32 * T);
-    const int64_t item = (int64_t)blockIdx.x * kGWarps + w;
+    const int64_t item = block * kGWarps + w;
     if (item >= ntiles * n_split) return;
     const int64_t tile = item % ntiles;
     const int64_t slice = item / ntiles;
@@ -166,23 +181,43 @@ __global__ void __launch_bounds__(32 * kGWarps) adjoint_kernel(
     }
 }
 
+template <int T, bool WANT_S>
+__global__ void __launch_bounds__(32 * kGWarps) adjoint_kernel(AdjointSide side, float eps2, int self_mask) {
+    __shared__ float4 buf[kGWarps][32];
+    adjoint_items<T, WANT_S>(side, eps2, self_mask, blockIdx.x, buf);
+}
+
+// Both ends, one after the other's blocks: two sweeps too short for a launch each (a gradient of 3,000 cells is bound by the
+// host's launches).
+__global__ void __launch_bounds__(32 * kGWarps) adjoint_ends_kernel(AdjointSide t, AdjointSide s, unsigned t_blocks,
+                                                                    float eps2, int self_mask) {
+    __shared__ float4 buf[kGWarps][32];
+    if (blockIdx.x < t_blocks) adjoint_items<2, false>(t, eps2, self_mask, blockIdx.x, buf);
+    else adjoint_items<2, true>(s, eps2, self_mask, blockIdx.x - t_blocks, buf);
+}
+
 // The slices' sums in slice order (FP64), rounded to FP32 as a single slice's are, and scaled.
 template <bool WANT_S>
-__global__ void __launch_bounds__(256) adjoint_reduce_kernel(const double *__restrict__ part, int n_split, int64_t na,
-                                                             const float *__restrict__ vscale,
-                                                             float *__restrict__ out_s, float *__restrict__ out_v) {
+__device__ __forceinline__ void adjoint_reduce(const AdjointSide &S, int64_t k) {
     constexpr int NV = WANT_S ? 4 : 3;
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < na * NV; k += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t a = k / NV;
-        const int v = (int)(k - a * NV) - (NV - 3);   // -1: the scalar sum
-        double acc = 0.0;
+    const int64_t a = k / NV;
+    const int v = (int)(k - a * NV) - (NV - 3);   // -1: the scalar sum
+    double acc = 0.0;
 #pragma unroll 8
-        for (int s = 0; s < n_split; ++s) acc += part[(int64_t)s * na * NV + k];
-        if (v < 0) {
-            if (out_s) out_s[a] = (float)acc;
-        } else if (out_v) {
-            out_v[3 * a + v] = vscale[a] * (float)acc;
-        }
+    for (int s = 0; s < S.n_split; ++s) acc += S.part[(int64_t)s * S.na * NV + k];
+    if (v < 0) {
+        if (S.out_s) S.out_s[a] = (float)acc;
+    } else if (S.out_v) {
+        S.out_v[3 * a + v] = S.vscale[a] * (float)acc;
+    }
+}
+
+// Of the ends that have several slices (the other's na is 0).
+__global__ void __launch_bounds__(256) adjoint_reduce_kernel(AdjointSide t, AdjointSide s) {
+    const int64_t nt = 3 * t.na, ns = 4 * s.na;
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nt + ns; k += (int64_t)gridDim.x * blockDim.x) {
+        if (k < nt) adjoint_reduce<false>(t, k);
+        else adjoint_reduce<true>(s, k - nt);
     }
 }
 
@@ -481,18 +516,30 @@ int adjoint_targets(int64_t na) {
     return !WANT_S && na >= 16384 ? 4 : 2;
 }
 
-template <bool WANT_S, int T>
-int launch_adjoint(const float *bx, const float *by, const float *bz, const float *bw, int64_t nb, const float *ax,
-                   const float *ay, const float *az, int64_t na, float eps2, int self_mask, int64_t self_off,
-                   int n_split, int64_t split_len, const float *vscale, float *out_s, float *out_v, double *part,
-                   cudaStream_t st) {
-    constexpr int NV = WANT_S ? 4 : 3;
-    const int64_t items = (na + 32 * T - 1) / (32 * T) * n_split;
-    HALMA_LAUNCH((adjoint_kernel<T, WANT_S>), (unsigned)((items + kGWarps - 1) / kGWarps), 32 * kGWarps, 0, st, bx, by,
-                 bz, bw, nb, ax, ay, az, na, eps2, self_mask, self_off, n_split, split_len, vscale, out_s, out_v, part);
-    if (n_split > 1)
-        HALMA_LAUNCH(adjoint_reduce_kernel<WANT_S>, grid_for(na * NV, 256, device_sm_count() * 8), 256, 0, st, part,
-                     n_split, na, vscale, out_s, out_v);
+template <int T>
+unsigned adjoint_blocks(const AdjointSide &S) {
+    const int64_t items = (S.na + 32 * T - 1) / (32 * T) * S.n_split;
+    return (unsigned)((items + kGWarps - 1) / kGWarps);
+}
+
+// The wanted ends (na > 0) in a sweep each, or in one launch where two lanes' targets suit both.
+int launch_adjoint(AdjointSide t, AdjointSide s, float eps2, int self_mask, cudaStream_t st) {
+    const bool wide = adjoint_targets<false>(t.na) == 4;
+    if (t.na > 0 && s.na > 0 && !wide) {
+        const unsigned tb = adjoint_blocks<2>(t), sb = adjoint_blocks<2>(s);
+        HALMA_LAUNCH(adjoint_ends_kernel, tb + sb, 32 * kGWarps, 0, st, t, s, tb, eps2, self_mask);
+    } else {
+        if (t.na > 0 && wide)
+            HALMA_LAUNCH((adjoint_kernel<4, false>), adjoint_blocks<4>(t), 32 * kGWarps, 0, st, t, eps2, self_mask);
+        else if (t.na > 0)
+            HALMA_LAUNCH((adjoint_kernel<2, false>), adjoint_blocks<2>(t), 32 * kGWarps, 0, st, t, eps2, self_mask);
+        if (s.na > 0)
+            HALMA_LAUNCH((adjoint_kernel<2, true>), adjoint_blocks<2>(s), 32 * kGWarps, 0, st, s, eps2, self_mask);
+    }
+    if (t.n_split == 1) t.na = 0;
+    if (s.n_split == 1) s.na = 0;
+    if (t.na + s.na > 0)
+        HALMA_LAUNCH(adjoint_reduce_kernel, grid_for(3 * t.na + 4 * s.na, 256, device_sm_count() * 8), 256, 0, st, t, s);
     return HALMA_OK;
 }
 
@@ -552,9 +599,8 @@ extern "C" int halma_potential_grad_f32(int64_t ns, const float *m_, const float
     const BothPlan plan(ns, nt);
     Layout L;
     sg.plan(L);
-    const size_t o_part =
-        L.add(both ? plan.bytes(nt)
-                   : 8 * (size_t)std::max(split_t > 1 ? 3 * nt * split_t : 0, split_s > 1 ? 4 * ns * split_s : 0));
+    const size_t o_part = L.add(both ? plan.bytes(nt) : split_t > 1 ? 8 * (size_t)(3 * nt * split_t) : 0);
+    const size_t o_part_s = L.add(!both && split_s > 1 ? 8 * (size_t)(4 * ns * split_s) : 0);
     void *base = nullptr;
     HALMA_TRY(workspace(L.total, &base, st));
     HALMA_TRY(sg.bind_and_upload(base, st));
@@ -565,13 +611,9 @@ extern "C" int halma_potential_grad_f32(int64_t ns, const float *m_, const float
                               reinterpret_cast<float2 *>(part), st));
         return sg.download(st);
     }
-    if (gt) {
-        auto run = adjoint_targets<false>(nt) == 4 ? launch_adjoint<false, 4> : launch_adjoint<false, 2>;
-        HALMA_TRY(run(sx, sy, sz, m, ns, tx, ty, tz, nt, (float)eps2, self, self_offset, split_t, len_t, g, nullptr, gt,
-                      part, st));
-    }
-    if (gm || gs)
-        HALMA_TRY((launch_adjoint<true, 2>(tx, ty, tz, g, nt, sx, sy, sz, ns, (float)eps2, self, -self_offset, split_s,
-                                           len_s, m, gm, gs, part, st)));
+    HALMA_TRY(launch_adjoint({sx, sy, sz, m, ns, tx, ty, tz, gt ? nt : 0, self_offset, split_t, len_t, g, nullptr, gt, part},
+                             {tx, ty, tz, g, nt, sx, sy, sz, gm || gs ? ns : 0, -self_offset, split_s, len_s, m, gm, gs,
+                              at<double>(base, o_part_s)},
+                             (float)eps2, self, st));
     return sg.download(st);
 }
