@@ -236,19 +236,22 @@ void choose_slices(int64_t na, int64_t nb, int T, int nv, int *n_split, int64_t 
 // ---- both sides of a pair at once -----------------------------------------------------------
 // When the gradients of targets and sources are both wanted and there are enough pairs, one sweep gives them: distance,
 // rsqrt and r^-3 of a pair are formed once, 17 lane-operations instead of 12 + 13, and the sources' four
-// sums (r^-1 and the vector) are reduced over the warp's lanes (1 lane-operation a pair).
-// A block of four warps holds 1,024 targets, eight a lane, and stages 512 sources; an item is one block of sources against
-// `tblocks` blocks of targets, the sources' sums kept in shared memory (compensated) over them.  Per item and
-// target, or source, one partial sum is written; they are added in order.
-// Bound: the FP32 pipe (18 lane-operations and a rsqrt a pair; it is 70 % busy).  160,000 targets x 200,000 sources:
-// 27.5 ms in two sweeps, 22.0 in one (four targets a lane, two sources an instruction and r^-3 weighted twice: 23.5;
-// 256 sources, or ten or six targets a lane, 3 to 5 % more).
-constexpr int kBothT = 8, kBothTargets = 128 * kBothT, kBothSources = 512, kBothChunks = kBothSources / 32;
+// sums (r^-1 and the vector) are reduced over the warp's lanes (half a lane-operation a pair).
+// A block of four warps holds 2,304 targets, eighteen a lane, and stages 288 sources; an item is one block of sources
+// against `tblocks` blocks of targets, the sources' sums kept in shared memory (compensated) over them, the
+// targets' too, a column a thread, as they are touched once in 32 sources.  Per item and target, or source, one
+// partial sum is written; they are added in order.
+// Bound: the FP32 pipe (18 lane-operations and a rsqrt a pair; 77 % busy).  160,000 x 200,000: 27.5 ms in two sweeps,
+// 19.7 in one.  Fewer reductions and more independent pairs a warp gain more than warps: eight targets with their
+// sums in registers and three blocks an SM 22.0 (512 sources), with the sums in shared memory 21.2 (256), sixteen
+// and two blocks 20.5, eighteen with 192 to 320 sources 19.7 to 20.3; four targets, two sources an instruction 23.5.
+constexpr int kBothT = 18, kBothTargets = 128 * kBothT, kBothSources = 288, kBothChunks = kBothSources / 32;
 
 struct BothShared {
     float4 src[kBothSources][2];            // {x, x, y, y}, {z, z, m, m}
     float part[4][kBothSources][4];         // per warp: the sources' sums over the warp's targets of one block
     float sum[kBothSources][4], comp[kBothSources][4];
+    float2 vec[3 * kBothT][128];            // a thread's targets' vectors: compensated sums
 };
 
 // 32 sources against the lane's targets, two targets a two-lane instruction.  r^-3 is formed once for both ends of a pair;
@@ -259,7 +262,7 @@ constexpr float kBothReach = 0x1p40f;
 template <bool SELF, bool WIDE>
 __device__ __forceinline__ void both_chunk(const float4 (*src)[2], const f2x (&px)[kBothT / 2],
                                            const f2x (&py)[kBothT / 2], const f2x (&pz)[kBothT / 2],
-                                           const f2x (&g)[kBothT / 2], f2x e2, int j0, const int (&self)[kBothT],
+                                           const f2x (&g)[kBothT / 2], f2x e2, int self0,
                                            f2x (&vx)[kBothT / 2], f2x (&vy)[kBothT / 2], f2x (&vz)[kBothT / 2],
                                            float *out, int lane) {
 #pragma unroll 1
@@ -280,8 +283,8 @@ __device__ __forceinline__ void both_chunk(const float4 (*src)[2], const f2x (&p
                 unpack2(r2, r0, r1);
                 float i0 = rsqrt_ftz(r0), i1 = rsqrt_ftz(r1);
                 if (SELF) {
-                    if (j0 + k0 + k == self[2 * t]) i0 = 0.f;
-                    if (j0 + k0 + k == self[2 * t + 1]) i1 = 0.f;
+                    if (k0 + k == self0 + 64 * t) i0 = 0.f;
+                    if (k0 + k == self0 + 64 * t + 32) i1 = 0.f;
                 }
                 const f2x ri = pack2(i0, i1);
                 const f2x ri2 = mul2(ri, ri);
@@ -314,7 +317,7 @@ __device__ __forceinline__ void both_chunk(const float4 (*src)[2], const f2x (&p
 
 // part_t[(sb - sb0) * nt + i][3]: target i's vector over source block sb; part_s[tsb * nsrc + j - j0][4]: source j's sums
 // over the targets of item column tsb (nsrc sources from j0 = sb0 * kBothSources on).
-__global__ void __launch_bounds__(128, 3) adjoint_both_kernel(
+__global__ void __launch_bounds__(128, 2) adjoint_both_kernel(
     const float *__restrict__ sx, const float *__restrict__ sy, const float *__restrict__ sz,
     const float *__restrict__ sm, int64_t ns, const float *__restrict__ tx, const float *__restrict__ ty,
     const float *__restrict__ tz, const float *__restrict__ tg, int64_t nt, float eps2, int self_mask, int64_t self_off,
@@ -344,8 +347,6 @@ __global__ void __launch_bounds__(128, 3) adjoint_both_kernel(
         if (i0 >= nt) break;   // the same for the block
         const int64_t iw = i0 + w * 32 * kBothT;
         f2x px[kBothT / 2], py[kBothT / 2], pz[kBothT / 2], g[kBothT / 2];
-        float vs[kBothT][3], vc[kBothT][3];
-        int self[kBothT];
         bool far_target = false;
 #pragma unroll
         for (int t = 0; t < kBothT / 2; ++t) {
@@ -362,16 +363,11 @@ __global__ void __launch_bounds__(128, 3) adjoint_both_kernel(
             g[t] = pack2(p[0].w, p[1].w);
         }
 #pragma unroll
-        for (int t = 0; t < kBothT; ++t) {
-            const int64_t i = iw + t * 32 + lane;
-            const bool in = i < nt;
-            const int64_t sj = i + self_off - j0;   // the self pair's source in the block
-            self[t] = in && self_mask && sj >= 0 && sj < kBothSources ? (int)sj : -1;
-#pragma unroll
-            for (int v = 0; v < 3; ++v) vs[t][v] = vc[t][v] = 0.f;
-        }
+        for (int v = 0; v < 3 * kBothT; ++v) sh.vec[v][threadIdx.x] = make_float2(0.f, 0.f);
         const bool wide = far_sources || __any_sync(0xffffffffu, far_target);
         const int64_t lo = iw + self_off - j0;   // self pairs: sources lo .. lo + 32 T - 1 of the block
+        // the lane's first target's own source in the block; its t-th's is 32 t further (never, without self pairs)
+        const int self0 = self_mask ? (int)std::max<int64_t>(std::min<int64_t>(lo + lane, 1 << 29), -(1 << 29)) : 1 << 29;
         for (int c = 0; c < kBothChunks; ++c) {
             f2x vx[kBothT / 2], vy[kBothT / 2], vz[kBothT / 2];
 #pragma unroll
@@ -380,11 +376,11 @@ __global__ void __launch_bounds__(128, 3) adjoint_both_kernel(
             float *out = &sh.part[w][c * 32][0];
             const bool own = self_mask && lo < c * 32 + 32 && lo + 32 * kBothT > c * 32;
             if (wide)
-                both_chunk<true, true>(buf, px, py, pz, g, e2, c * 32, self, vx, vy, vz, out, lane);
+                both_chunk<true, true>(buf, px, py, pz, g, e2, self0 - c * 32, vx, vy, vz, out, lane);
             else if (own)
-                both_chunk<true, false>(buf, px, py, pz, g, e2, c * 32, self, vx, vy, vz, out, lane);
+                both_chunk<true, false>(buf, px, py, pz, g, e2, self0 - c * 32, vx, vy, vz, out, lane);
             else
-                both_chunk<false, false>(buf, px, py, pz, g, e2, c * 32, self, vx, vy, vz, out, lane);
+                both_chunk<false, false>(buf, px, py, pz, g, e2, self0 - c * 32, vx, vy, vz, out, lane);
 #pragma unroll
             for (int t = 0; t < kBothT; t += 2) {
                 const f2x q[3] = {vx[t / 2], vy[t / 2], vz[t / 2]};
@@ -392,8 +388,12 @@ __global__ void __launch_bounds__(128, 3) adjoint_both_kernel(
                 for (int v = 0; v < 3; ++v) {
                     float a, b;
                     unpack2(q[v], a, b);
-                    two_sum_acc(vs[t][v], vc[t][v], a);
-                    two_sum_acc(vs[t + 1][v], vc[t + 1][v], b);
+                    float2 &s0 = sh.vec[3 * t + v][threadIdx.x], &s1 = sh.vec[3 * t + 3 + v][threadIdx.x];
+                    float2 u = s0, w2 = s1;
+                    two_sum_acc(u.x, u.y, a);
+                    two_sum_acc(w2.x, w2.y, b);
+                    s0 = u;
+                    s1 = w2;
                 }
             }
         }
@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(128, 3) adjoint_both_kernel(
             if (i >= nt) continue;
             float2 *p = part_t + ((int64_t)sbl * nt + i) * 3;
 #pragma unroll
-            for (int v = 0; v < 3; ++v) p[v] = make_float2(vs[t][v], vc[t][v]);
+            for (int v = 0; v < 3; ++v) p[v] = sh.vec[3 * t + v][threadIdx.x];
         }
         __syncthreads();
         for (int k = threadIdx.x; k < kBothSources * 4; k += 128) {   // the warps in order, compensated
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(128, 3) adjoint_both_kernel(
 // After a band of source blocks: the targets' vectors over the band added to tot (first: set), and, after the last
 // band, the gradients; the band's sources' sums over the item columns in order, and their gradients.  A partial sum is a
 // compensated FP32 sum and its errors; they are added up the same way (in FP64 that pipe was the bound: 452 and
-// 140 us of 160,000 targets x 200,000 sources, now 335 and 87).
+// 140 us of 160,000 targets x 200,000 sources, now, with more partial sums, 528 and 94).
 __global__ void __launch_bounds__(256) both_targets_kernel(const float2 *__restrict__ part_t, int nsb, int64_t nt,
                                                            int first, int last, float2 *__restrict__ tot,
                                                            const float *__restrict__ scale, float *__restrict__ out) {
@@ -466,10 +466,10 @@ __global__ void __launch_bounds__(256) both_sources_kernel(const float2 *__restr
 }
 
 // Scratch: the targets' partial sums of one band within kBothBand bytes (one source block at least).
-constexpr int64_t kBothBand = 256ll << 20;
-// Below kBothPairs pairs its blocks, 1,024 x 512 pairs for an item of four warps, are too few for the GPU: 4.8e7
-// pairs take 89 us against 78 in two sweeps, 1.2e8 140 against 150, 5e8 407 against 479.
-constexpr double kBothPairs = 1e8;
+constexpr int64_t kBothBand = 512ll << 20;
+// Below kBothPairs pairs its blocks, 2,304 x 288 pairs for an item of four warps, are too few for the GPU: 1.2e8
+// pairs take 144 us against 138 with an end's sums each on its own, 5e8 383 against 474.
+constexpr double kBothPairs = 1.5e8;
 
 struct BothPlan {
     int64_t nsb = 0, band = 0, ntsb = 0;   // source blocks, source blocks of a band, item columns
@@ -478,8 +478,8 @@ struct BothPlan {
         nsb = (ns + kBothSources - 1) / kBothSources;
         band = std::min(nsb, std::max<int64_t>(1, kBothBand / (24 * nt)));
         const int64_t tb = (nt + kBothTargets - 1) / kBothTargets;
-        // about eight items for every block that fits on the GPU (three an SM)
-        const int64_t columns = std::min(tb, std::max<int64_t>(1, ((int64_t)device_sm_count() * 24 + band - 1) / band));
+        // about 32 items for every block that fits on the GPU (two an SM), so that the last ones are short
+        const int64_t columns = std::min(tb, std::max<int64_t>(1, ((int64_t)device_sm_count() * 64 + band - 1) / band));
         tblocks = (int)((tb + columns - 1) / columns);
         ntsb = (tb + tblocks - 1) / tblocks;
     }

@@ -134,10 +134,11 @@ def test_gas_halo_adjoint_at_full_scale(cuda):
 
 @pytest.mark.parametrize("ns,nt,self_offset", [
     (10_001, 10_007, None), (512 * 40, 512 * 10, 0), (512 * 40 + 1, 512 * 10 + 1, 7), (511, 200_003, 0),
-    (200_003, 513, -300), (300_000, 1, None), (1, 120_000_000 // 200, None), (4_097, 40_001, 4_000)])
+    (200_003, 513, -300), (300_000, 1, None), (1, 120_000_000 // 200, None), (4_097, 40_001, 4_000),
+    (288 * 60, 2304 * 4, 0), (288 * 60 + 1, 2304 * 4 + 1, -2), (287, 530_001, 0), (70_001, 2_303, 5)])
 def test_both_gradients_in_one_sweep(cuda, ns, nt, self_offset):
     """Enough pairs for the kernel that gives both ends' gradients at once (and shapes short of it), at the edges of
-    its blocks of 512 sources, with and without a skipped pair, against the FP64 gradient."""
+    its blocks (of 288 sources and 2,304 targets), with and without a skipped pair, against the FP64 gradient."""
     import torch
     from pyhalma_gb300.autograd import softened_potential
     rng = np.random.default_rng(8)
@@ -171,7 +172,7 @@ def test_both_gradients_in_other_units(cuda, shift):
     import torch
     from pyhalma_gb300.autograd import softened_potential
     rng = np.random.default_rng(9)
-    ns, nt, unit = 10_300, 10_100, 2.0 ** shift
+    ns, nt, unit = 12_700, 12_300, 2.0 ** shift
     s, t = rng.normal(0, 0.02, (3, ns)).astype(np.float32), rng.normal(0, 0.02, (3, nt)).astype(np.float32)
     m, g = rng.uniform(1.0, 2.0, ns).astype(np.float32), torch.tensor(rng.normal(size=nt).astype(np.float32), device=cuda)
 
