@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256) red_dist_kernel(int nh, const int64_t *__
 
 // The sorted rows with the runs of equal keys in order of the full distance (equal distances stay in row
 // order): a row of a run goes to the run's start plus the number of rows before it.  Runs are short (the
-// leading bits tell distances apart to 2^-27 or better); a long one costs its length per row.
+// leading bits tell distances apart to 1 / members or 2^-26); a long one costs its length per row.
 __global__ void __launch_bounds__(256) red_ties_kernel(int n, const uint64_t *__restrict__ key,
                                                        const int *__restrict__ val, const double *__restrict__ dist,
                                                        const unsigned char *__restrict__ mask, int *__restrict__ order) {
@@ -534,8 +534,13 @@ static int reductions_run(int64_t n, int nh, const int64_t *off, const RedIn &in
     const int cmax = nh + (int)(n / kRedChunk) + 1;   // chunks: sum over haloes of max(1, ceil(n_h / kRedChunk))
     int hbits = 1;
     while (hbits < 32 && ((uint64_t)(nh - 1) >> hbits) != 0) ++hbits;
-    // whole radix digits (8 bits), at least 37 bits of distance: sign 0, 11 of exponent, 26 of mantissa
-    const int kbits = std::min(64, (hbits + 37 + 7) / 8 * 8), dbits = std::min(63, kbits - hbits);
+    // Whole radix digits (8 bits), at least 11 bits of exponent and as many of mantissa as number the members, 26 at most:
+    // then even the members of one octave of one halo seldom share a key, and red_ties_kernel orders those that do.  (26 for
+    // all: one more pass, 22 us of the 1.6e6 rows of four half-mass radii of 4e5 members; one set of 120 haloes 333 us, now 306.)
+    const int64_t members = in.period > 0 ? in.period : n;
+    int mbits = 8;
+    while (mbits < 26 && (members >> mbits) != 0) ++mbits;
+    const int kbits = std::min(64, (hbits + 11 + mbits + 7) / 8 * 8), dbits = std::min(63, kbits - hbits);
     const size_t s64 = sort_pairs_u64_i32_bytes(N, hbits + dbits), sc = exclusive_sum_i32_bytes(nh + 1);
     Layout L;
     const size_t o_red = L.add(sizeof(Red) * nh);
