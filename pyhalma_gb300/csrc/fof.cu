@@ -951,7 +951,7 @@ __global__ void __launch_bounds__(256) label_kernel(int n, const int *__restrict
 // ---- small inputs ---------------------------------------------------------------------------
 // Up to kSmallFof particles, all pairs: no bounding box on the host, no sort, no cells -- five launches and one
 // round trip instead of thirty and two.  A call takes 88 us at 5,000 particles (on cells 245, start 297), 113 at
-// 8,192 (243) and 224 at 16,384 (256).
+// 8,192 (243) and 204 at 16,384 (256).
 // A particle is its position relative to particle 0 in linking lengths as two floats an axis (error below 2^-46 of
 // the largest); where some lie farther apart than 2^24 linking lengths (or the linking length is subnormal),
 // pairs that the first floats leave open are tested in FP64 (flags[1]).
@@ -1022,7 +1022,7 @@ __device__ __forceinline__ float2 small_bounds(const SmallArgs &A) {
 // The last becomes the particle's parent: the indices rise along every path, so this forest needs no union.
 // Each lane remembers two, so no lane waits for another one's search (a warp per particle that stopped at two
 // friends took 25 us at 5,000 particles, as lonely ones scan to the end; 10 so).
-constexpr int kNearLen = 128, kSweepLen = 512, kSweepT = 4;
+constexpr int kNearLen = 128, kSweepLen = 512, kSweepT = 8;
 
 __global__ void __launch_bounds__(256) small_near_kernel(SmallArgs A) {
     __shared__ float4 run[kNearLen];
@@ -1070,10 +1070,10 @@ __global__ void __launch_bounds__(1024) small_union_kernel(SmallArgs A) {
     }
 }
 
-// All pairs again, four particles a warp against runs of kSweepLen, one of them a lane: those that may be friends and
-// whose roots differ are looked at closely and joined.  A pair costs nine instructions (four particles share a
+// All pairs again, eight particles a warp against runs of kSweepLen, one of them a lane: those that may be friends and
+// whose roots differ are looked at closely and joined.  A pair costs nine instructions (eight particles share a
 // load; the roots come with the positions); with both floats of every position and a particle a warp
-// 5,000 particles took 30 us, 11 so.
+// 5,000 particles took 30 us, 11 so (four particles 11, and 223 us for a call on 16,384 instead of 204).
 __global__ void __launch_bounds__(256) small_sweep_kernel(SmallArgs A) {
     const int lane = threadIdx.x & 31;
     const int i0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kSweepT;
