@@ -180,9 +180,12 @@ __global__ void red_center_kernel(int nh, const int *__restrict__ cstart, const 
     }
 }
 
-// What the members are sorted by inside a halo: excluded particles after every member.
+// What the members are sorted by inside a halo, in 63 bits: excluded particles after every finite distance, NaN last.
+// A NaN may come with its sign set (infinity - infinity does), which has no place here: above the leading bits of
+// the distance stands the halo.  (A minimum, not a mask: the compiler takes it for granted that a square root has none.)
 __device__ __forceinline__ uint64_t full_key(double d, bool member) {
-    return member ? (uint64_t)__double_as_longlong(d) : 0x7ff0000000000000ull;
+    const uint64_t bits = (uint64_t)__double_as_longlong(d);
+    return !member ? 0x7ff0000000000000ull : bits < 0x7ff8000000000000ull ? bits : 0x7ff8000000000000ull;
 }
 
 // Per chunk: distances, sort keys (halo, leading dbits bits of the distance's bit pattern, which orders

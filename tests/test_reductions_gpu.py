@@ -117,3 +117,31 @@ def test_device_offsets_outside_the_rows_are_refused(cuda):
     out = hp.halo_reductions(torch.tensor([0, 1, 4], device=cuda), *[x] * 6, torch.ones(4, dtype=torch.float64,
                                                                                               device=cuda))
     assert out[:, 0].cpu().tolist() == [1.0, 3.0]
+
+
+@pytest.mark.parametrize("bad", [np.nan, -np.nan, np.inf, -np.inf])
+def test_non_finite_positions_stay_in_their_halo(cuda, bad):
+    """A distance that is not finite (NaN of either sign, infinity) sorts last in its own halo: the other haloes' rows are
+    bit for bit those of a call in which that member has an ordinary position."""
+    rng = np.random.default_rng(6)
+    off = np.array([0, 40, 95, 160, 161, 300], dtype=np.int64)
+    cols = [rng.normal(0.0, 1.0, off[-1]) for _ in range(6)]
+    m = rng.uniform(0.5, 2.0, off[-1])
+    good = hp.halo_reductions(off, *cols, m)
+    for h in (0, 2, 4):   # the halo number's last bit clear: one more bit there is the next halo
+        x = cols[0].copy()
+        x[off[h] + 3] = bad
+        x[off[h] + 7] = np.inf
+        out = hp.halo_reductions(off, x, *cols[1:], m)
+        keep = [k for k in range(5) if k != h]
+        assert np.array_equal(out[keep], good[keep]), h
+        # about a given centre, the members at a finite distance are walked first
+        about = np.full((5, hp.N_ABOUT), np.nan)
+        about[:, :3] = 0.0
+        about[:, 6] = good[:, 0]
+        out = hp.halo_reductions(off, x, *cols[1:], m, about=about)
+        sl = slice(off[h], off[h + 1])
+        d = np.sqrt(((0.0 - x[sl]) ** 2 + (0.0 - cols[1][sl]) ** 2) + (0.0 - cols[2][sl]) ** 2)
+        order = np.argsort(d, kind="stable")   # NaN last
+        f = int(np.argmax(np.cumsum(m[sl][order]) > 0.5 * good[h, 0]))
+        assert out[h, 8] == d[order[max(f - 1, 0)]], h
