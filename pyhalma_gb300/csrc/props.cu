@@ -78,21 +78,23 @@ __device__ __forceinline__ void block_sums(double (&v)[NV], double (*sh)[8]) {
 // Bulk velocity (sum m v / M with the given mass, zeros when M <= 0) and the "about" rows of
 // the four half-mass-radius reductions: 3-D around (cx, cy, cz), and the projections along x,
 // y, z as 3-D distances of (y, z, 0), (x, z, 0), (x, y, 0) around (cy, cz, 0), (cx, cz, 0),
-// (cx, cy, 0).
+// (cx, cy, 0).  A bulk velocity that is NaN (a velocity that is not finite) is 0 in those rows when the members' masses
+// do not add up to more than 0, as the reductions have it for a velocity that they form themselves.
 __global__ void __launch_bounds__(256) pr_bulk_kernel(int G, const int64_t *__restrict__ off,
                                                       const double *__restrict__ g, int64_t nm,
                                                       const double *__restrict__ cen, double *__restrict__ out,
                                                       double *__restrict__ about /* 4 x G x 8 */) {
-    __shared__ double sh[3][8];
+    __shared__ double sh[4][8];
     for (int h = blockIdx.x; h < G; h += gridDim.x) {
-        double v[3] = {0, 0, 0};
+        double v[4] = {0, 0, 0, 0};
         for (int64_t k = off[h] + threadIdx.x; k < off[h + 1]; k += blockDim.x) {
             const double mi = g[6 * nm + k];
             v[0] += mi * g[3 * nm + k];
             v[1] += mi * g[4 * nm + k];
             v[2] += mi * g[5 * nm + k];
+            v[3] += mi;
         }
-        block_sums<3>(v, sh);
+        block_sums<4>(v, sh);
         if (threadIdx.x == 0) {
             const double *c = cen + (int64_t)h * kCenFields;
             const double M = c[3];
@@ -107,9 +109,9 @@ __global__ void __launch_bounds__(256) pr_bulk_kernel(int G, const int64_t *__re
                 a[HALMA_ABOUT_CX] = cc[r][0];
                 a[HALMA_ABOUT_CY] = cc[r][1];
                 a[HALMA_ABOUT_CZ] = cc[r][2];
-                a[HALMA_ABOUT_VX] = ux;
-                a[HALMA_ABOUT_VY] = uy;
-                a[HALMA_ABOUT_VZ] = uz;
+                a[HALMA_ABOUT_VX] = isnan(ux) && !(v[3] > 0.0) ? 0.0 : ux;
+                a[HALMA_ABOUT_VY] = isnan(uy) && !(v[3] > 0.0) ? 0.0 : uy;
+                a[HALMA_ABOUT_VZ] = isnan(uz) && !(v[3] > 0.0) ? 0.0 : uz;
                 a[HALMA_ABOUT_MASS] = M;
                 a[HALMA_ABOUT_R05] = NAN;
             }

@@ -147,7 +147,9 @@ __global__ void __launch_bounds__(256) red_part_kernel(int nh, const int64_t *__
 }
 
 // One thread per halo: the chunks' sums in order, centre, bulk velocity (or the caller's),
-// reference mass and R05; rmax starts at 0 for the distance kernel's atomic maximum.
+// reference mass and R05; rmax starts at 0 for the distance kernel's atomic maximum.  NaN in the caller's row is a value to
+// be computed here; with SUMS = false, where no sums were formed, the row is complete and a NaN is its value.
+template <bool SUMS>
 __global__ void red_center_kernel(int nh, const int *__restrict__ cstart, const double *__restrict__ part,
                                   const double *__restrict__ about, Red *__restrict__ red) {
     for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < nh; h += gridDim.x * blockDim.x) {
@@ -164,13 +166,16 @@ __global__ void red_center_kernel(int nh, const int *__restrict__ cstart, const 
         double Mref = M, r05_in = NAN;
         if (about) {
             const double *a = about + (int64_t)h * HALMA_ABOUT_NFIELDS;
-            if (!isnan(a[HALMA_ABOUT_CX])) cx = a[HALMA_ABOUT_CX];
-            if (!isnan(a[HALMA_ABOUT_CY])) cy = a[HALMA_ABOUT_CY];
-            if (!isnan(a[HALMA_ABOUT_CZ])) cz = a[HALMA_ABOUT_CZ];
-            if (!isnan(a[HALMA_ABOUT_VX])) ux = a[HALMA_ABOUT_VX];
-            if (!isnan(a[HALMA_ABOUT_VY])) uy = a[HALMA_ABOUT_VY];
-            if (!isnan(a[HALMA_ABOUT_VZ])) uz = a[HALMA_ABOUT_VZ];
-            if (!isnan(a[HALMA_ABOUT_MASS])) Mref = a[HALMA_ABOUT_MASS];
+            auto take = [&](double &v, int f) {
+                if (!SUMS || !isnan(a[f])) v = a[f];
+            };
+            take(cx, HALMA_ABOUT_CX);
+            take(cy, HALMA_ABOUT_CY);
+            take(cz, HALMA_ABOUT_CZ);
+            take(ux, HALMA_ABOUT_VX);
+            take(uy, HALMA_ABOUT_VY);
+            take(uz, HALMA_ABOUT_VZ);
+            take(Mref, HALMA_ABOUT_MASS);
             r05_in = a[HALMA_ABOUT_R05];
         }
         Red o;
@@ -565,9 +570,13 @@ static int reductions_run(int64_t n, int nh, const int64_t *off, const RedIn &in
     HALMA_LAUNCH(red_chunks_kernel, gh, 256, 0, st, nh, off, cnum);
     HALMA_TRY(exclusive_sum_i32(tmp, sc, cnum, cst, nh + 1, st));
     HALMA_LAUNCH(red_owner_kernel, gh, 256, 0, st, nh, cst, chunk_h);
-    if (sums) HALMA_LAUNCH(red_part_kernel<true>, cmax, 256, 0, st, nh, off, cst, chunk_h, in, part);
-    else HALMA_LAUNCH(red_part_kernel<false>, cmax, 256, 0, st, nh, off, cst, chunk_h, in, part);
-    HALMA_LAUNCH(red_center_kernel, gh, 256, 0, st, nh, cst, part, about, red);
+    if (sums) {
+        HALMA_LAUNCH(red_part_kernel<true>, cmax, 256, 0, st, nh, off, cst, chunk_h, in, part);
+        HALMA_LAUNCH(red_center_kernel<true>, gh, 256, 0, st, nh, cst, part, about, red);
+    } else {
+        HALMA_LAUNCH(red_part_kernel<false>, cmax, 256, 0, st, nh, off, cst, chunk_h, in, part);
+        HALMA_LAUNCH(red_center_kernel<false>, gh, 256, 0, st, nh, cst, part, about, red);
+    }
     HALMA_LAUNCH(red_dist_kernel, cmax, 256, 0, st, nh, off, cst, chunk_h, in, dbits, red, key, v0, dist);
     if (n > 0) {
         HALMA_TRY(sort_pairs_u64_i32(tmp, s64, key, key2, v0, v1, (int)n, hbits + dbits, st));

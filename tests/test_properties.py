@@ -193,3 +193,32 @@ def test_member_index_out_of_range(cuda, bad):
     with pytest.raises(ValueError, match="outside"):
         halo_properties.halo_property_table(off, wrong, *cols, cen, 0.1)
     assert _same(halo_properties.halo_property_table(off, mem, *cols, cen, 0.1), good)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", ["velocity", "mass"])
+def test_non_finite_bulk_velocity(cuda, what):
+    """A member outside the half-mass radius whose velocity is NaN: the bulk velocity is, and so is the dispersion about
+    it.  With a NaN mass the masses have no sum, and the dispersion is that about a velocity of 0."""
+    from pyhalma_gb300 import _lib, halo_properties
+    rng = np.random.default_rng(12)
+    n = 60
+    x, y, z = rng.normal(0.0, 0.01, (3, n))
+    vx, vy, vz = rng.normal(50.0, 100.0, (3, n))
+    m = rng.uniform(0.5, 2.0, n)
+    x[29] = 5.0
+    cen = np.array([[0.0, 0.0, 0.0, m[:30].sum(), 5.0], [0.0, 0.0, 0.0, m[30:].sum(), 1.0]])
+    args = lambda: (np.array([0, 30, 60]), np.arange(n, dtype=np.int32), x, y, z, vx, vy, vz, m, cen, 0.05)
+    F = {k: i for i, k in enumerate(_lib.PROP_FIELDS)}
+    good = halo_properties.halo_property_table(*args())
+    (vx if what == "velocity" else m)[29] = np.nan
+    t = halo_properties.halo_property_table(*args())
+    assert _same(t[1], good[1])
+    assert np.isnan(t[0, F["vx"]])
+    if what == "velocity":
+        assert np.isnan(t[0, F["sig_3d"]])
+    else:
+        d = np.sqrt(x[:30] ** 2 + y[:30] ** 2 + z[:30] ** 2)
+        inside = d < t[0, F["r05"]]
+        v2 = (vx[:30][inside] ** 2 + vy[:30][inside] ** 2 + vz[:30][inside] ** 2).sum()
+        np.testing.assert_allclose(t[0, F["sig_3d"]], np.sqrt(v2 / 3.0 / inside.sum()), rtol=RTOL)
