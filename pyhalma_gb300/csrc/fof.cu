@@ -962,7 +962,7 @@ struct SmallArgs {
     int n;
     const double *x, *y, *z;
     float4 *pos_hi, *pos_lo;   // pos_hi[i].w: the particle's root for the sweep
-    int *flags;                // [0] non-finite coordinate, [1] FP64 tests, [4] the largest |coordinate| (float bits)
+    int *flags;                // [0] non-finite coordinate, [1] coordinates for FP64 tests, [4] the largest |coordinate| (float bits)
     int *parent, *first, *err;
     float lo, hi;
     double r2;
@@ -1010,10 +1010,14 @@ __device__ __forceinline__ bool small_friends(const SmallArgs &A, bool fp64, int
 
 // Bounds on the squared distance of the first floats alone: below x the pair is linked, above y it is not.  The second
 // floats are at most 2^-24 of the largest coordinate, two of them an axis.  Where the FP64 test's squares overflow or
-// underflow at the linking length, it decides every pair.
+// underflow at the linking length, it decides every pair (small_in_fp64).
+__device__ __forceinline__ bool small_in_fp64(const SmallArgs &A) {
+    return A.flags[1] != 0 || (A.lo >= 0.f && !(A.r2 > 1e-280 && A.r2 < 1e300));   // (A.lo < 0: linking length 0)
+}
+
 __device__ __forceinline__ float2 small_bounds(const SmallArgs &A) {
     const float e = __int_as_float(A.flags[4]) * 0x1p-22f + 1e-5f;
-    if (A.lo >= 0.f && !(A.r2 > 1e-280 && A.r2 < 1e300)) return make_float2(-1.f, INFINITY);   // (A.lo < 0: linking length 0)
+    if (A.lo >= 0.f && !(A.r2 > 1e-280 && A.r2 < 1e300)) return make_float2(-1.f, INFINITY);
     const float in = sqrtf(fmaxf(A.lo, 0.f)) - e, out = sqrtf(fmaxf(A.hi, 0.f)) + e;
     return make_float2(in > 0.f ? in * in * (1.f - 1e-6f) : -1.f, out * out * (1.f + 1e-6f));
 }
@@ -1079,7 +1083,7 @@ __global__ void __launch_bounds__(256) small_sweep_kernel(SmallArgs A) {
     const int i0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kSweepT;
     const int j1 = min(A.n, (int)(blockIdx.y + 1) * kSweepLen);
     if (i0 >= A.n || i0 + 1 >= j1) return;
-    const bool fp64 = A.flags[1] != 0;
+    const bool fp64 = small_in_fp64(A);
     const float out = small_bounds(A).y;
     float4 p[kSweepT];
 #pragma unroll

@@ -283,3 +283,12 @@ def test_groups_of_given_labels(cuda, n):
         assert len(off) == len(heads) + 1
         for g, h in enumerate(heads):
             assert np.array_equal(mem[off[g]:off[g + 1]], np.nonzero(lab == h)[0])
+
+
+@pytest.mark.parametrize("ll", [1e200, 1e-170])
+def test_small_path_where_the_predicate_leaves_the_range(cuda, ll):
+    """The FP64 predicate overflows (or underflows) on both sides at the linking length: it, not the floats, decides."""
+    rng = np.random.default_rng(4)
+    p = rng.uniform(0.0, 12.0, (1500, 3)) * ll
+    x, y, z = (np.ascontiguousarray(c) for c in p.T)
+    assert np.array_equal(fof.fof_labels(x, y, z, ll), _brute(p, ll))
