@@ -315,11 +315,12 @@ __device__ __forceinline__ void pot_chunk(const float4 *sa, const float4 *sb, co
                 if (!((a.x != qx) & (a.z != qy) & (b.x != qz))) i0 = 0.f;
                 if (!((a.y != qx) & (a.w != qy) & (b.y != qz))) i1 = 0.f;
             }
-            if (SELF) {
-                if (2 * kp == self[t]) i0 = 0.f;
-                if (2 * kp + 1 == self[t]) i1 = 0.f;
+            if (SELF) {   // the term, not its factor: the mass may be infinite
+                const bool skip0 = 2 * kp == self[t], skip1 = 2 * kp + 1 == self[t];
+                acc[t] = fma2(pack2(skip0 ? 0.f : b.z, skip1 ? 0.f : b.w), pack2(skip0 ? 0.f : i0, skip1 ? 0.f : i1), acc[t]);
+            } else {
+                acc[t] = fma2(M, pack2(i0, i1), acc[t]);
             }
-            acc[t] = fma2(M, pack2(i0, i1), acc[t]);
         }
     }
 }

@@ -199,3 +199,24 @@ def test_host_arrays_at_any_address(cuda, n):
     for k in range(4):
         c, t = [moved(a, (k + q) % 4) for q, a in enumerate(cols)], [moved(a, k) for a in tgt]
         assert np.array_equal(halo_gas.bf_potential(c[3], *c[:3], *t, mode="reference"), want), k
+
+
+@pytest.mark.parametrize("n", [40, 300, 5000])
+def test_skipped_pair_of_an_infinite_mass(cuda, n):
+    """Mask SELF leaves the self pair out whatever its mass: a particle of infinite mass has the potential of the others."""
+    rng = np.random.default_rng(21)
+    p, m = _cloud(rng, n)
+    x, y, z, m = (np.ascontiguousarray(a, dtype=np.float32) for a in (*p.T, m))
+    at = n // 3
+    m[at] = np.inf
+    phi = np.zeros(n, dtype=np.float32)
+    P = _lib.ptr
+    _lib.check(_lib.lib().halma_potential_f32(n, P(m), P(x), P(y), P(z), n, P(x), P(y), P(z), 1e-8, _lib.MASK_SELF, 0, P(phi),
+                                              None), "halma_potential_f32")
+    others = np.arange(n) != at
+    assert np.all(np.isnan(phi[others]) | np.isinf(phi[others]))
+    d = lambda a: a.astype(np.float64)
+    m[at] = 0.0
+    ref = oracle.potential_f64(d(m), d(x), d(y), d(z), d(x[at:at + 1]), d(y[at:at + 1]), d(z[at:at + 1]), eps2=1e-8,
+                               mask=oracle.MASK_NONE)
+    assert abs(phi[at] / ref[0] - 1.0) < RTOL_FAST
