@@ -2,8 +2,9 @@
 //   total_mass (:16-24), center_of_mass (:26-43), CM_velocity (:45-60),
 //   furthest_particle (:98-111), half_mass_radius (:365-392), sigma_effective (:607-625).
 // The half-mass radius needs the members in increasing distance from the centre: one stable radix sort over all
-// particles by (halo, leading bits of the FP64 distance), the few runs of equal leading bits put in order
+// particles by (halo, leading bits of the FP64 distance), the runs of equal leading bits put in order
 // by the full distance, after which each halo walks its own segment.
+#include <cooperative_groups.h>
 #include <limits.h>
 #include <math.h>
 #include <string.h>
@@ -72,7 +73,9 @@ struct RedIn {
 constexpr int kRedChunk = 4096;
 constexpr int kRedParts = 9;   // M, Mx, My, Mz, Mvx, Mvy, Mvz, count, masses the integer walk cannot take
 
-__global__ void red_chunks_kernel(int nh, const int64_t *__restrict__ off, int *__restrict__ cnum) {
+__global__ void red_chunks_kernel(int nh, const int64_t *__restrict__ off, int *__restrict__ cnum,
+                                  int *__restrict__ longest) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *longest = 0;   // see red_ties_kernel
     for (int h = blockIdx.x * blockDim.x + threadIdx.x; h <= nh; h += gridDim.x * blockDim.x) {
         const int64_t n = h < nh ? off[h + 1] - off[h] : 0;
         cnum[h] = h < nh ? (int)(n > 0 ? (n + kRedChunk - 1) / kRedChunk : 1) : 0;
@@ -232,31 +235,123 @@ __global__ void __launch_bounds__(256) red_dist_kernel(int nh, const int64_t *__
 }
 
 // The sorted rows with the runs of equal keys in order of the full distance (equal distances stay in row
-// order): a row of a run goes to the run's start plus the number of rows before it.  Runs are short (the
-// leading bits tell distances apart to 1 / members or 2^-26); a long one costs its length per row.
+// order).  In a run of up to kShortRun rows, nearly all of them, a row goes to the run's start plus the number of
+// rows before it.  Longer ones (members at one distance, on a shell, about a far centre) keep their
+// order here, which the stable sort has made right where their distances are all the same; *longest is
+// the length of the longest that has to be put in order (red_runs_kernel), run[p] a long run's start and length (0 elsewhere).
+// Rows at no finite distance and excluded ones keep their place: what they are sorted by is one value.
+// (Counted by every row, the masses of 2e6 members, a call without positions, took 3.9 s, now 11 ms with their copies.)
+constexpr int kShortRun = 32;
+
 __global__ void __launch_bounds__(256) red_ties_kernel(int n, const uint64_t *__restrict__ key,
                                                        const int *__restrict__ val, const double *__restrict__ dist,
-                                                       const unsigned char *__restrict__ mask, int *__restrict__ order) {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
+                                                       const unsigned char *__restrict__ mask, int *__restrict__ order,
+                                                       int2 *__restrict__ run, int *__restrict__ longest) {
+    for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t k = key[p];
         const int i = val[p];
-        int to = p;
+        int64_t to = p;
+        int2 r = make_int2(0, 0);
         if ((p > 0 && key[p - 1] == k) || (p + 1 < n && key[p + 1] == k)) {
-            int lo = 0, hi = p;   // the run's first row
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (key[mid] < k) lo = mid + 1;
-                else hi = mid;
-            }
             const uint64_t fi = full_key(dist[i], !mask || mask[i]);
-            to = lo;
-            for (int q = lo; q < n && key[q] == k; ++q) {
-                const int j = val[q];
-                const uint64_t fj = full_key(dist[j], !mask || mask[j]);
-                if (fj < fi || (fj == fi && q < p)) ++to;
+            if (fi < 0x7ff0000000000000ull) {
+                // the run's first row and the one past its last: doubling steps away from p, then bisection
+                int64_t lo = p, hi = p, step = 1;   // lo is in the run
+                while (lo - step >= 0 && key[lo - step] == k) {
+                    lo -= step;
+                    step <<= 1;
+                }
+                for (; step > 0; step >>= 1)
+                    if (lo - step >= 0 && key[lo - step] == k) lo -= step;
+                step = 1;
+                while (hi + step < n && key[hi + step] == k) {
+                    hi += step;
+                    step <<= 1;
+                }
+                for (; step > 0; step >>= 1)
+                    if (hi + step < n && key[hi + step] == k) hi += step;
+                ++hi;
+                if (hi - lo <= kShortRun) {
+                    to = lo;
+                    for (int64_t q = lo; q < hi; ++q) {
+                        const int j = val[q];
+                        const uint64_t fj = full_key(dist[j], !mask || mask[j]);
+                        if (fj < fi || (fj == fi && q < p)) ++to;
+                    }
+                } else {
+                    r = make_int2((int)lo, (int)(hi - lo));
+                    if (p > lo) {
+                        const int j = val[p - 1];
+                        if (full_key(dist[j], !mask || mask[j]) > fi) atomicMax(longest, r.y);
+                    }
+                }
             }
         }
         order[to] = i;
+        run[p] = r;
+    }
+}
+
+// The long runs in order: tiles of kRunTile rows by counting, then merges of neighbours twice as long each time, a row
+// finding its place in the other half by bisection (n log^2 n steps in all, over the whole grid).  Nothing to do for nearly
+// every call.  All rows of long runs lie at finite distances, which order as doubles.  (da, a) and (db, b): the rows'
+// distances and numbers, from one to the other; order is a.  One cooperative launch, whose barriers separate the merges.
+constexpr int kRunTile = 64;
+
+__global__ void __launch_bounds__(256) red_runs_kernel(int n, const int *__restrict__ longest,
+                                                       const int2 *__restrict__ run, const int *__restrict__ val,
+                                                       const double *__restrict__ dist, double *da, int *a, double *db,
+                                                       int *b) {
+    const int most = *longest;
+    if (most == 0) return;   // the same for the whole grid
+    cooperative_groups::grid_group grid = cooperative_groups::this_grid();
+    const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    int merges = 0;
+    while (((int64_t)kRunTile << merges) < most) ++merges;
+    double *ds = merges & 1 ? db : da, *dd = merges & 1 ? da : db;   // the last merge ends in (da, a)
+    int *is = merges & 1 ? b : a, *id = merges & 1 ? a : b;
+    for (int64_t p = first; p < n; p += step) {
+        const int2 r = run[p];
+        if (r.y == 0) continue;
+        const int64_t t0 = r.x + (p - r.x) / kRunTile * kRunTile, t1 = min(t0 + kRunTile, (int64_t)r.x + r.y);
+        const int i = val[p];
+        const double d = dist[i];
+        int64_t to = t0;
+        for (int64_t q = t0; q < t1; ++q) {
+            const double e = dist[val[q]];
+            if (e < d || (e == d && q < p)) ++to;
+        }
+        ds[to] = d;
+        is[to] = i;
+    }
+    for (int64_t w = kRunTile; w < most; w <<= 1) {
+        grid.sync();
+        for (int64_t p = first; p < n; p += step) {
+            const int2 r = run[p];
+            if (r.y == 0) continue;
+            const int64_t end_run = (int64_t)r.x + r.y, base = r.x + (p - r.x) / (2 * w) * (2 * w);
+            const int64_t mid = min(base + w, end_run), end = min(base + 2 * w, end_run);
+            const double d = ds[p];
+            const bool left = p < mid;
+            // rows of the other half before this one: smaller, or of the left half equal
+            int64_t lo = left ? mid : base, hi = left ? end : mid;
+            const int64_t from = lo;
+            while (lo < hi) {
+                const int64_t m = (lo + hi) >> 1;
+                const double e = ds[m];
+                if (left ? e < d : e <= d) lo = m + 1;
+                else hi = m;
+            }
+            const int64_t to = base + (p - (left ? base : mid)) + (lo - from);
+            dd[to] = d;
+            id[to] = is[p];
+        }
+        double *const td = ds;
+        ds = dd;
+        dd = td;
+        int *const ti = is;
+        is = id;
+        id = ti;
     }
 }
 
@@ -533,6 +628,16 @@ __global__ void red_out_kernel(int nh, const int *__restrict__ cstart, const dou
     }
 }
 
+int launch_runs(int n, const int *longest, const int2 *run, const int *val, const double *dist, double *da, int *a,
+                double *db, int *b, cudaStream_t st) {
+    const int grid = std::min(device_sm_count() * 2, grid_for(n, 256));   // all blocks are on the GPU at once
+    void *args[] = {&n, &longest, &run, &val, &dist, &da, &a, &db, &b};
+    HALMA_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(&red_runs_kernel), dim3((unsigned)grid), dim3(256), args,
+                                           0, st));
+    count_launch();
+    return HALMA_OK;
+}
+
 }  // namespace
 
 static int reductions_run(int64_t n, int nh, const int64_t *off, const RedIn &in, bool sums,
@@ -556,7 +661,10 @@ static int reductions_run(int64_t n, int nh, const int64_t *off, const RedIn &in
     const size_t o_v0 = L.add(4ull * N), o_v1 = L.add(4ull * N);
     const size_t o_cnum = L.add(4ull * (nh + 1)), o_cst = L.add(4ull * (nh + 1)), o_ch = L.add(4ull * cmax);
     const size_t o_part = L.add(8ull * kRedParts * cmax), o_part2 = L.add(16ull * cmax);
-    const size_t o_tmp = L.add(std::max(s64, sc));
+    const size_t o_run = L.add(8ull * N), o_long = L.add(4);
+    // of the sort, and afterwards of the long runs' merges
+    const size_t merge_d = align_up(8ull * N, 256);
+    const size_t o_tmp = L.add(std::max(std::max(s64, sc), merge_d + sizeof(int) * (size_t)N));
     void *base = nullptr;
     HALMA_TRY(workspace(L.total, &base, st));
     Red *red = at<Red>(base, o_red);
@@ -567,7 +675,9 @@ static int reductions_run(int64_t n, int nh, const int64_t *off, const RedIn &in
     double *part = at<double>(base, o_part), *part2 = at<double>(base, o_part2);
     void *tmp = at<void>(base, o_tmp);
     const int gh = grid_for(nh + 1, 256);
-    HALMA_LAUNCH(red_chunks_kernel, gh, 256, 0, st, nh, off, cnum);
+    auto *run = at<int2>(base, o_run);
+    int *longest = at<int>(base, o_long);
+    HALMA_LAUNCH(red_chunks_kernel, gh, 256, 0, st, nh, off, cnum, longest);
     HALMA_TRY(exclusive_sum_i32(tmp, sc, cnum, cst, nh + 1, st));
     HALMA_LAUNCH(red_owner_kernel, gh, 256, 0, st, nh, cst, chunk_h);
     if (sums) {
@@ -581,7 +691,9 @@ static int reductions_run(int64_t n, int nh, const int64_t *off, const RedIn &in
     if (n > 0) {
         HALMA_TRY(sort_pairs_u64_i32(tmp, s64, key, key2, v0, v1, (int)n, hbits + dbits, st));
         HALMA_LAUNCH(red_ties_kernel, std::min(device_sm_count() * 8, grid_for(n, 256)), 256, 0, st, (int)n, key2, v1,
-                     dist, in.mask, v0);
+                     dist, in.mask, v0, run, longest);
+        HALMA_TRY(launch_runs((int)n, longest, run, v1, dist, reinterpret_cast<double *>(key), v0, at<double>(base, o_tmp),
+                              at<int>(base, o_tmp + merge_d), st));
     }
     HALMA_LAUNCH(red_walk_kernel, nh, 256, 0, st, off, v0, dist, in, red);
     HALMA_LAUNCH(red_sigma_kernel, cmax, 256, 0, st, nh, off, cst, chunk_h, dist, in, red, part2);

@@ -145,3 +145,85 @@ def test_non_finite_positions_stay_in_their_halo(cuda, bad):
         order = np.argsort(d, kind="stable")   # NaN last
         f = int(np.argmax(np.cumsum(m[sl][order]) > 0.5 * good[h, 0]))
         assert out[h, 8] == d[order[max(f - 1, 0)]], h
+
+
+def _stable_r05(d, m, half):
+    """The half-mass walk over members sorted by distance, equal distances in member order."""
+    order = np.argsort(d, kind="stable")
+    over = np.cumsum(m[order]) > half
+    f = int(np.argmax(over)) if over.any() else len(d)
+    return d[order[max(f - 1, 0)]]
+
+
+@pytest.mark.parametrize("sizes", [(33,), (32, 1), (64, 65, 31, 127), (128, 129, 40, 1000, 2), (4097, 50_000)])
+@pytest.mark.parametrize("width", [0.0, 1e-9, 1e-4])
+def test_members_that_share_leading_distance_bits(cuda, sizes, width):
+    """Haloes about a centre 1e3 away with members in a shell of the given width: many members have the same leading bits
+    (all of them, down to all at one distance), up to and past the lengths of run at which the ordering changes its method."""
+    rng = np.random.default_rng(len(sizes))
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    n = int(off[-1])
+    x = 1.0e3 + width * rng.uniform(0.0, 1.0, n)
+    x[rng.integers(0, n, n // 3)] = x[0]          # equal distances among the others
+    z0 = np.zeros(n)
+    m = rng.uniform(0.5, 2.0, n)
+    mask = (rng.random(n) < 0.7).astype(np.uint8)
+    mask[off[:-1]] = 1
+    for mk in (None, mask):
+        about = np.full((len(sizes), hp.N_ABOUT), np.nan)
+        about[:, :3] = 0.0
+        want = []
+        for h in range(len(sizes)):
+            pl = np.arange(off[h], off[h + 1])
+            if mk is not None:
+                pl = pl[mk[pl] == 1]
+            about[h, 6] = np.cumsum(m[pl])[-1] * rng.uniform(0.2, 1.0)
+            want.append(_stable_r05(x[pl], m[pl], 0.5 * about[h, 6]))
+        out = hp.halo_reductions(off, x, z0, z0, z0, z0, z0, m, mask=mk, about=about)
+        assert np.array_equal(out[:, 8], want)
+
+
+def _device_ms(f):
+    import torch
+    f()
+    best = np.inf
+    for _ in range(3):
+        torch.cuda.synchronize()
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        f()
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b))
+    return best
+
+
+@pytest.mark.parametrize("case", ["coincident", "masked", "far centre"])
+def test_time_does_not_grow_with_the_square_of_a_run(cuda, case):
+    """One halo of 6e5 rows at one distance, nearly all masked out, or all with the same leading distance bits, against
+    the same rows spread out: the ordering adds passes, not a step per pair of rows (300 times as long)."""
+    import torch
+    n = 600_000
+    off = torch.tensor([0, n], device=cuda)
+    g = torch.Generator(device=cuda).manual_seed(5)
+    T = lambda: torch.rand(n, dtype=torch.float64, device=cuda, generator=g)
+    x, m, z = T(), T() + 0.5, torch.zeros(n, dtype=torch.float64, device=cuda)
+    about = torch.full((1, hp.N_ABOUT), np.nan, dtype=torch.float64, device=cuda)
+    about[:, :3] = 0.0
+    spread = _device_ms(lambda: hp.halo_reductions(off, x, x, x, z, z, z, m, about=about))
+    mask = None
+    if case == "coincident":
+        y = torch.zeros_like(x)
+    elif case == "masked":
+        y, mask = x, (T() < 0.01).to(torch.uint8)
+    else:
+        y = 1.0e3 + 1e-9 * x
+    out = []
+    took = _device_ms(lambda: out.append(hp.halo_reductions(off, y, z, z, z, z, z, m, mask=mask, about=about)))
+    assert took < 20.0 * spread + 2.0, (took, spread)
+    keep = slice(None) if mask is None else (mask.cpu().numpy() == 1)
+    d, mm = y.cpu().numpy()[keep], m.cpu().numpy()[keep]
+    # the device's reference mass is its own sum: the walk's end moves by no more than a few members
+    order = np.sort(d)
+    got, at = out[0][0, 8].item(), np.searchsorted(np.cumsum(mm[np.argsort(d, kind="stable")]), 0.5 * mm.sum())
+    assert order[max(at - 4, 0)] <= got <= order[min(at + 4, len(d) - 1)]
