@@ -954,7 +954,7 @@ __global__ void __launch_bounds__(256) label_kernel(int n, const int *__restrict
 // 8,192 (243) and 204 at 16,384 (256).
 // A particle is its position relative to particle 0 in linking lengths as two floats an axis (error below 2^-46 of
 // the largest); where some lie farther apart than 2^24 linking lengths (or the linking length is subnormal),
-// pairs that the first floats leave open are tested in FP64 (flags[1]).
+// pairs that the floats leave open are tested in FP64 (flags[1]).
 constexpr int kSmallFof = 16384;
 constexpr float kSmallReach = 16777216.f;
 
@@ -998,28 +998,49 @@ __global__ void __launch_bounds__(256) small_prep_kernel(SmallArgs A, double sca
     }
 }
 
-// Whether particles i and j are friends.
-__device__ __forceinline__ bool small_friends(const SmallArgs &A, bool fp64, int i, int j) {
-    if (fp64) return exact_link(A.x, A.y, A.z, i, j, A.r2);
-    const float4 ph = A.pos_hi[i], pl = A.pos_lo[i], qh = A.pos_hi[j], ql = A.pos_lo[j];
-    const float dx = (qh.x - ph.x) + (ql.x - pl.x), dy = (qh.y - ph.y) + (ql.y - pl.y), dz = (qh.z - ph.z) + (ql.z - pl.z);
-    const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    if (d2 < A.lo) return true;
-    return d2 <= A.hi && exact_link(A.x, A.y, A.z, i, j, A.r2);
-}
-
-// Bounds on the squared distance of the first floats alone: below x the pair is linked, above y it is not.  The second
-// floats are at most 2^-24 of the largest coordinate, two of them an axis.  Where the FP64 test's squares overflow or
-// underflow at the linking length, it decides every pair (small_in_fp64).
+// Where the FP64 test's squares overflow or underflow at the linking length, it decides every pair.
 __device__ __forceinline__ bool small_in_fp64(const SmallArgs &A) {
     return A.flags[1] != 0 || (A.lo >= 0.f && !(A.r2 > 1e-280 && A.r2 < 1e300));   // (A.lo < 0: linking length 0)
 }
 
-__device__ __forceinline__ float2 small_bounds(const SmallArgs &A) {
-    const float e = __int_as_float(A.flags[4]) * 0x1p-22f + 1e-5f;
-    if (A.lo >= 0.f && !(A.r2 > 1e-280 && A.r2 < 1e300)) return make_float2(-1.f, INFINITY);
-    const float in = sqrtf(fmaxf(A.lo, 0.f)) - e, out = sqrtf(fmaxf(A.hi, 0.f)) + e;
-    return make_float2(in > 0.f ? in * in * (1.f - 1e-6f) : -1.f, out * out * (1.f + 1e-6f));
+// How the kernels below look at a pair: by the first floats, or (low) by both; below `in` their squared distance says that
+// the pair is linked, above `out` that it is not.  The second floats are at most 2^-24 of the largest coordinate, two of them an
+// axis, so the bounds are 2^-22 of it apart from the linking length, or 2^-45 with both.  Coordinates beyond 2^20 linking
+// lengths of particle 0 take both: bounds a quarter of the linking length off would leave too many friends to small_friends
+// and a union each, and beyond 2^22 all of them.  With linking length 0 friends have the same floats.
+struct SmallRule {
+    float in, out;
+    bool low;
+    __device__ __forceinline__ SmallRule(const SmallArgs &A) {
+        const float reach = __int_as_float(A.flags[4]);
+        low = !(reach <= 0x1p20f);
+        if (A.lo < 0.f) {
+            in = -1.f;
+            out = 0.f;
+        } else if (!(A.r2 > 1e-280 && A.r2 < 1e300)) {
+            in = -1.f;
+            out = INFINITY;
+        } else {
+            const float e = reach * (low ? 0x1p-45f : 0x1p-22f) + 1e-5f;
+            const float near = sqrtf(A.lo) - e, far = sqrtf(A.hi) + e;
+            in = near > 0.f ? near * near * (1.f - 1e-6f) : -1.f;
+            out = far * far * (1.f + 1e-6f);   // NaN and infinity: every pair
+        }
+    }
+};
+
+// Squared distance of two particles by both floats.
+__device__ __forceinline__ float small_d2(const float4 &ph, const float4 &pl, const float4 &qh, const float4 &ql) {
+    const float dx = (qh.x - ph.x) + (ql.x - pl.x), dy = (qh.y - ph.y) + (ql.y - pl.y), dz = (qh.z - ph.z) + (ql.z - pl.z);
+    return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+}
+
+// Whether particles i and j are friends.
+__device__ __forceinline__ bool small_friends(const SmallArgs &A, bool fp64, int i, int j) {
+    if (fp64) return exact_link(A.x, A.y, A.z, i, j, A.r2);
+    const float d2 = small_d2(A.pos_hi[i], A.pos_lo[i], A.pos_hi[j], A.pos_lo[j]);
+    if (d2 < A.lo) return true;
+    return d2 <= A.hi && exact_link(A.x, A.y, A.z, i, j, A.r2);
 }
 
 // All pairs, a particle a lane against a run of kNearLen later ones: the first and the last that are linked beyond doubt.
@@ -1029,26 +1050,35 @@ __device__ __forceinline__ float2 small_bounds(const SmallArgs &A) {
 constexpr int kNearLen = 128, kSweepLen = 512, kSweepT = 8;
 
 __global__ void __launch_bounds__(256) small_near_kernel(SmallArgs A) {
-    __shared__ float4 run[kNearLen];
+    __shared__ float4 run[kNearLen], tail[kNearLen];
     const int i = blockIdx.x * 256 + threadIdx.x, j0 = blockIdx.y * kNearLen;
     const int len = min(kNearLen, A.n - j0);
     if (j0 + len <= (int)blockIdx.x * 256 + 1) return;   // nothing after any of the block's particles
-    if (threadIdx.x < len) run[threadIdx.x] = A.pos_hi[j0 + threadIdx.x];
+    const SmallRule rule(A);
+    if (threadIdx.x < len) {
+        run[threadIdx.x] = A.pos_hi[j0 + threadIdx.x];
+        if (rule.low) tail[threadIdx.x] = A.pos_lo[j0 + threadIdx.x];
+    }
     __syncthreads();
     if (i >= A.n) return;
-    const float in = small_bounds(A).x;
     const float4 p = A.pos_hi[i];
     int first = A.n, last = -1;
-    auto linked = [&](int k) {
-        const float dx = run[k].x - p.x, dy = run[k].y - p.y, dz = run[k].z - p.z;
-        return fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < in;
-    };
-#pragma unroll 8
-    for (int k = max(0, i + 1 - j0); k < len; ++k)
-        if (linked(k)) {
+    auto take = [&](int k, float d2) {
+        if (d2 < rule.in) {
             first = min(first, j0 + k);
             last = j0 + k;
         }
+    };
+    if (!rule.low) {
+#pragma unroll 8
+        for (int k = max(0, i + 1 - j0); k < len; ++k) {
+            const float dx = run[k].x - p.x, dy = run[k].y - p.y, dz = run[k].z - p.z;
+            take(k, fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+        }
+    } else {
+        const float4 pl = A.pos_lo[i];
+        for (int k = max(0, i + 1 - j0); k < len; ++k) take(k, small_d2(p, pl, run[k], tail[k]));
+    }
     if (last >= 0) {
         atomicMin(A.first + i, first);
         atomicMax(A.parent + i, last);
@@ -1084,7 +1114,7 @@ __global__ void __launch_bounds__(256) small_sweep_kernel(SmallArgs A) {
     const int j1 = min(A.n, (int)(blockIdx.y + 1) * kSweepLen);
     if (i0 >= A.n || i0 + 1 >= j1) return;
     const bool fp64 = small_in_fp64(A);
-    const float out = small_bounds(A).y;
+    const SmallRule rule(A);
     float4 p[kSweepT];
 #pragma unroll
     for (int t = 0; t < kSweepT; ++t) p[t] = A.pos_hi[min(i0 + t, A.n - 1)];   // the last one's pairs again past the end
@@ -1093,11 +1123,22 @@ __global__ void __launch_bounds__(256) small_sweep_kernel(SmallArgs A) {
         const int j = j0 + lane;
         const float4 q = A.pos_hi[min(j, A.n - 1)];
         unsigned may = 0;
+        if (!rule.low) {
 #pragma unroll
-        for (int t = 0; t < kSweepT; ++t) {
-            const float dx = q.x - p[t].x, dy = q.y - p[t].y, dz = q.z - p[t].z;
-            const bool near = !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > out);   // NaN where the floats overflow
-            if (near && __float_as_int(q.w) != __float_as_int(p[t].w)) may |= 1u << t;
+            for (int t = 0; t < kSweepT; ++t) {
+                const float dx = q.x - p[t].x, dy = q.y - p[t].y, dz = q.z - p[t].z;
+                const bool near = !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > rule.out);   // NaN where the floats overflow
+                if (near && __float_as_int(q.w) != __float_as_int(p[t].w)) may |= 1u << t;
+            }
+        } else {
+            const float4 ql = A.pos_lo[min(j, A.n - 1)];
+#pragma unroll 1
+            for (int t = 0; t < kSweepT; ++t) {   // read again: the registers are the other loop's
+                const int i = min(i0 + t, A.n - 1);
+                const float4 ph = A.pos_hi[i];
+                const bool near = !(small_d2(ph, A.pos_lo[i], q, ql) > rule.out);
+                if (near && __float_as_int(q.w) != __float_as_int(ph.w)) may |= 1u << t;
+            }
         }
         if (!__any_sync(0xffffffffu, may)) continue;
 #pragma unroll 1

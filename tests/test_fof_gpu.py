@@ -292,3 +292,53 @@ def test_small_path_where_the_predicate_leaves_the_range(cuda, ll):
     p = rng.uniform(0.0, 12.0, (1500, 3)) * ll
     x, y, z = (np.ascontiguousarray(c) for c in p.T)
     assert np.array_equal(fof.fof_labels(x, y, z, ll), _brute(p, ll))
+
+
+@pytest.mark.parametrize("reach", [2.0 ** 19, 2.0 ** 21, 3.0 ** 14, 2.0 ** 23.5, 2.0 ** 27, 2.0 ** 36, 2.0 ** 45])
+def test_small_path_with_an_outlier(cuda, reach):
+    """Friends around the linking length, half of them `reach` linking lengths from the other half: looked at by one
+    float, by both, and beyond that in FP64."""
+    rng = np.random.default_rng(14)
+    ll = 1.5e-3
+    p = rng.uniform(0.0, 12.0, (1500, 3)) * ll
+    p[::2] += reach * ll / np.sqrt(3.0)
+    p[3] = p[2] + np.array([ll, 0.0, 0.0])
+    p[5] = p[2] + np.array([0.0, ll * (1 + 1e-15), 0.0])
+    x, y, z = (np.ascontiguousarray(c) for c in p.T)
+    assert np.array_equal(fof.fof_labels(x, y, z, ll), _brute(p, ll))
+
+
+@pytest.mark.parametrize("what", ["outlier", "zero linking length"])
+def test_small_path_is_not_quadratic_in_friends(cuda, what):
+    """A crowd of 16,384 friends with one particle 1e8 linking lengths away takes about as long as the crowd alone, and
+    coordinates far below one unit with linking length 0 as long as ordinary ones."""
+    import torch
+    rng = np.random.default_rng(15)
+    n, ll = 16_384, 1.5e-3
+    p = rng.normal(0.0, 2.0 * ll, (3, n))
+    far = p.copy()
+    if what == "outlier":
+        far[:, 7] = 1e8 * ll
+    else:
+        ll, p, far = 0.0, 1e3 * p, 1e-9 * p
+
+    def ms(a):
+        x, y, z = (torch.tensor(c, device=cuda) for c in a)
+        fof.fof_labels(x, y, z, ll)
+        best = np.inf
+        for _ in range(3):
+            torch.cuda.synchronize()
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            lab = fof.fof_labels(x, y, z, ll)
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]))
+        return best, lab.cpu().numpy()
+    (alone, _), (took, lab) = ms(p), ms(far)
+    assert took < 3.0 * alone + 0.1, (took, alone)
+    x, y, z = (np.ascontiguousarray(c) for c in far)
+    keep = np.arange(n) != 7
+    want = oracle.fof_labels(x[keep], y[keep], z[keep], ll)
+    idx = np.nonzero(keep)[0]
+    assert np.array_equal(lab[keep], np.where(want >= 0, idx[want], -1))
