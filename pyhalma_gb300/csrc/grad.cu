@@ -221,12 +221,15 @@ __global__ void __launch_bounds__(256) adjoint_reduce_kernel(AdjointSide t, Adjo
     }
 }
 
-// Slices of the partners: about eight items per warp slot (16 warps an SM), at least 128 partners each, and
-// at most 2^23 partial sums (64 MB) in all.
+// Slices of the partners: about eight items per warp slot (16 warps an SM), at least 128 partners each, at most kMaxSlices,
+// which one thread adds up, and at most 2^23 partial sums (64 MB) in all.  (100 targets x 2e6 sources, 9,728 slices:
+// 1,470 us; 2,048 513, 1,024 383, 512 322, but 1,024 are 5 to 15 % faster for 5 to 20 sources x 10^7 targets.)
+constexpr int64_t kMaxSlices = 1024;
+
 void choose_slices(int64_t na, int64_t nb, int T, int nv, int *n_split, int64_t *split_len) {
     const int64_t ntiles = (na + 32 * T - 1) / (32 * T);
     int64_t s = ((int64_t)device_sm_count() * 16 * 8 + ntiles - 1) / ntiles;
-    s = std::min(s, std::min<int64_t>(nb / 128, (1ll << 23) / (na * nv)));
+    s = std::min(std::min(s, kMaxSlices), std::min<int64_t>(nb / 128, (1ll << 23) / (na * nv)));
     s = std::max<int64_t>(s, 1);
     const int64_t len = ((nb + s - 1) / s + 31) / 32 * 32;
     *n_split = (int)((nb + len - 1) / len);
@@ -468,8 +471,17 @@ __global__ void __launch_bounds__(256) both_sources_kernel(const float2 *__restr
 // Scratch: the targets' partial sums of one band within kBothBand bytes (one source block at least).
 constexpr int64_t kBothBand = 512ll << 20;
 // Below kBothPairs pairs its blocks, 2,304 x 288 pairs for an item of four warps, are too few for the GPU: 1.2e8
-// pairs take 144 us against 138 with an end's sums each on its own, 5e8 383 against 474.
-constexpr double kBothPairs = 1.5e8;
+// pairs take 144 us against 138 with an end's sums each on its own, 5e8 383 against 474.  Whole blocks are computed, so
+// neither end may be much short of one: 3,700 targets (4,608 computed) x 10^6 sources 3,278 and 3,307 us, 3,400 3,277 and
+// 3,078, 1,800 x 200,000 397 and 444, 1,000 x 200,000 393 and 361; 145 sources (288) x 1.4e6 targets 332 and 421, 100 x
+// 2e6 504 and 428, 100 targets x 2e6 sources 3,458 and 383.
+constexpr double kBothPairs = 1.5e8, kBothTargetPadding = 4.0 / 3.0, kBothSourcePadding = 2.0;
+
+bool both_at_once(int64_t ns, int64_t nt) {
+    auto padding = [](int64_t n, int64_t block) { return (double)((n + block - 1) / block * block) / (double)n; };
+    return (double)ns * (double)nt >= kBothPairs && padding(nt, kBothTargets) <= kBothTargetPadding &&
+           padding(ns, kBothSources) <= kBothSourcePadding;
+}
 
 struct BothPlan {
     int64_t nsb = 0, band = 0, ntsb = 0;   // source blocks, source blocks of a band, item columns
@@ -593,9 +605,8 @@ extern "C" int halma_potential_grad_f32(int64_t ns, const float *m_, const float
     int64_t len_t = ns, len_s = nt;
     if (grad_tgt) choose_slices(nt, ns, adjoint_targets<false>(nt), 3, &split_t, &len_t);
     if (grad_m || grad_src) choose_slices(ns, nt, adjoint_targets<true>(ns), 4, &split_s, &len_s);
-    // both sides in one sweep from kBothPairs pairs on, and with a softening that keeps r^-2 finite
-    const bool both = grad_tgt && (grad_m || grad_src) && (double)ns * (double)nt >= kBothPairs &&
-                      (float)eps2 >= 0x1p-126f;
+    // both sides in one sweep where that suits the sizes, and with a softening that keeps r^-2 finite
+    const bool both = grad_tgt && (grad_m || grad_src) && both_at_once(ns, nt) && (float)eps2 >= 0x1p-126f;
     const BothPlan plan(ns, nt);
     Layout L;
     sg.plan(L);

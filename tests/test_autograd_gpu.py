@@ -183,3 +183,41 @@ def test_both_gradients_in_other_units(cuda, shift):
         return [M.grad.double() * u] + [a.grad.double() * u * u for a in S + T]
     for a, b in zip(gradients(unit), gradients(1.0)):
         assert float((a - b).norm() / b.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("ns,nt", [(2_000_000, 100), (100, 2_000_000)])
+def test_few_against_many(cuda, ns, nt):
+    """Few particles at one end: the gradients against the FP64 ones, and no whole blocks computed for them -- the time is
+    of the order of as many pairs of two equal ends."""
+    import torch
+    from pyhalma_gb300 import _lib
+    g = torch.Generator(device=cuda).manual_seed(2)
+
+    def call(ns, nt):
+        T = lambda n: 0.02 * torch.randn(n, device=cuda, generator=g)
+        s, m, t, u = [T(ns) for _ in range(3)], T(ns).abs(), [T(nt) for _ in range(3)], T(nt)
+        out = [torch.empty(k, device=cuda) for k in (ns, 3 * ns, 3 * nt)]
+        P = _lib.ptr
+        run = lambda: _lib.check(_lib.lib().halma_potential_grad_f32(
+            ns, P(m), *[P(a) for a in s], nt, *[P(a) for a in t], P(u), 1e-8, _lib.MASK_NONE, 0, *[P(a) for a in out],
+            _lib.stream_of(m)), "halma_potential_grad_f32")
+        run()
+        ms = np.inf
+        for _ in range(3):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            run()
+            e[1].record()
+            torch.cuda.synchronize()
+            ms = min(ms, e[0].elapsed_time(e[1]))
+        return ms, s, m, t, u, out
+    square = call(14_142, 14_142)[0]
+    ms, s, m, t, u, out = call(ns, nt)
+    assert ms < 5.0 * square, (ms, square)
+    d = lambda a: a.double().cpu().numpy()
+    gm, gs, gt = oracle.potential_grad_f64(d(m), *[d(a) for a in s], *[d(a) for a in t], d(u), eps2=1e-8,
+                                           mask=oracle.MASK_NONE)
+    rel = lambda a, b: np.linalg.norm(a - b) / np.linalg.norm(b)
+    assert rel(d(out[0]), gm) < 1e-5
+    assert rel(d(out[1]).reshape(-1, 3), gs) < 1e-5
+    assert rel(d(out[2]).reshape(-1, 3), gt) < 1e-5
