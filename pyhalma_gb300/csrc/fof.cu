@@ -1150,10 +1150,12 @@ __global__ void __launch_bounds__(256) small_sweep_kernel(SmallArgs A) {
     }
 }
 
-// One block, in shared memory: roots, smallest members and labels (-1 alone), and the number of groups.
+// One block, in shared memory: roots, smallest members and labels (-1 alone), and the number of groups.  No labels where a
+// coordinate was not finite (*bad): the call is refused.
 __global__ void __launch_bounds__(1024) small_label_kernel(int n, const int *__restrict__ parent,
-                                                           int *__restrict__ labels, int *__restrict__ ngroups,
-                                                           int *err) {
+                                                           const int *__restrict__ bad, int *__restrict__ labels,
+                                                           int *__restrict__ ngroups, int *err) {
+    if (*bad) return;
     extern __shared__ int sl_smem[];
     int *up = sl_smem, *least = sl_smem + n;   // least[r]: r's smallest member, n + that while r is alone
     __shared__ int groups;
@@ -1489,7 +1491,7 @@ int fof_small(int n, const double *x, const double *y, const double *z, double l
     HALMA_LAUNCH(small_sweep_kernel, dim3(grid_for(n, 8 * kSweepT), (n + kSweepLen - 1) / kSweepLen), 256, 0, st, A);
     HALMA_TRY(prof.fof_mark(6, st));
     HALMA_CUDA(cudaFuncSetAttribute(small_label_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kSmallFof));
-    HALMA_LAUNCH(small_label_kernel, 1, 1024, 8 * n, st, n, parent, labels, cnt + 2, cnt + 3);
+    HALMA_LAUNCH(small_label_kernel, 1, 1024, 8 * n, st, n, parent, cnt, labels, cnt + 2, cnt + 3);
     HALMA_TRY(prof.fof_mark(7, st));
     int hc[4];
     HALMA_CUDA(cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, st));

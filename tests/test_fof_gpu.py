@@ -342,3 +342,16 @@ def test_small_path_is_not_quadratic_in_friends(cuda, what):
     want = oracle.fof_labels(x[keep], y[keep], z[keep], ll)
     idx = np.nonzero(keep)[0]
     assert np.array_equal(lab[keep], np.where(want >= 0, idx[want], -1))
+
+
+@pytest.mark.parametrize("n", [500, 16_384, 16_385])
+def test_labels_are_not_touched_by_a_refused_call(cuda, n):
+    import torch
+    from pyhalma_gb300 import _lib
+    rng = np.random.default_rng(16)
+    x, y, z = (torch.tensor(c, device=cuda) for c in rng.uniform(0.0, 1.0, (3, n)))
+    y[n // 3] = float("inf")
+    lab = torch.full((n,), 77, dtype=torch.int32, device=cuda)
+    st = _lib.lib().halma_fof(n, _lib.ptr(x), _lib.ptr(y), _lib.ptr(z), 0.05, _lib.ptr(lab), None, _lib.stream_of(x))
+    assert st == _lib.ERR_INVALID
+    assert bool((lab == 77).all())
