@@ -850,6 +850,14 @@ __global__ void pr_off4_kernel(int G, int64_t nm, const int64_t *__restrict__ of
         off4[k] = k == 4ll * G ? 4 * nm : (k / G) * nm + off[k % G];
 }
 
+// The table to the caller's device memory, unless a member index was out of range: a refused call writes nothing.
+__global__ void pr_store_kernel(int64_t count, const double *__restrict__ table, const int *__restrict__ bad,
+                                double *__restrict__ out) {
+    if (*bad) return;
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < count; k += (int64_t)gridDim.x * blockDim.x)
+        out[k] = table[k];
+}
+
 int nbits(uint64_t v) {
     int b = 0;
     while (b < 64 && (v >> b) != 0) ++b;
@@ -921,6 +929,8 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
     const bool sets = N0 > 0 && N0 <= (1 << 25) && G <= (1 << 25);
     Layout L;
     sg.plan(L);
+    const bool dev_out = is_device_pointer(out);
+    const size_t o_table = L.add(dev_out ? 8ull * G * HALMA_PROP_NFIELDS : 0);
     const size_t o_off4 = L.add(sets ? 8ull * (4ull * G + 1) : 8);
     const size_t o_g = L.add(64ull * NM), o_ab = L.add(8ull * 4 * G * HALMA_ABOUT_NFIELDS);
     const size_t o_red = L.add(8ull * 4 * G * HALMA_RED_NFIELDS), o_own = L.add(4ull * NM);
@@ -936,6 +946,8 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
     void *base = nullptr;
     HALMA_TRY(workspace(L.total, &base, st, 7));
     HALMA_TRY(sg.bind_and_upload(base, st));
+    double *const user_out = dout;
+    if (dev_out) dout = at<double>(base, o_table);
     double *gbuf = at<double>(base, o_g), *about = at<double>(base, o_ab), *red = at<double>(base, o_red);
     int *own = at<int>(base, o_own);
     auto *kin = at<uint64_t>(base, o_kin), *kout = at<uint64_t>(base, o_kout);
@@ -1007,6 +1019,9 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
         HALMA_LAUNCH(pr_proj_out_kernel, gH, 128, 0, st, G, res, dout);
     }
     HALMA_CUDA(cudaStreamWaitEvent(st, side->done, 0));
+    if (dev_out)
+        HALMA_LAUNCH(pr_store_kernel, grid_for((int64_t)G * HALMA_PROP_NFIELDS, 256, sms * 8), 256, 0, st,
+                     (int64_t)G * HALMA_PROP_NFIELDS, dout, cnt + 1, user_out);
     int bad = 0;
     HALMA_CUDA(cudaMemcpyAsync(&bad, cnt + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
     HALMA_CUDA(cudaStreamSynchronize(st));

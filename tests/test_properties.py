@@ -222,3 +222,27 @@ def test_non_finite_bulk_velocity(cuda, what):
         inside = d < t[0, F["r05"]]
         v2 = (vx[:30][inside] ** 2 + vy[:30][inside] ** 2 + vz[:30][inside] ** 2).sum()
         np.testing.assert_allclose(t[0, F["sig_3d"]], np.sqrt(v2 / 3.0 / inside.sum()), rtol=RTOL)
+
+
+@pytest.mark.gpu
+def test_device_table_is_not_touched_by_a_refused_call(cuda):
+    import torch
+    from pyhalma_gb300 import _lib
+    rng = np.random.default_rng(3)
+    cols = rng.uniform(0.1, 1.0, (7, 40))
+    cen = np.array([[0.5, 0.5, 0.5, cols[6, :20].sum(), 1.0]])
+    off, mem = np.array([0, 20]), np.arange(20, dtype=np.int32)
+    D = lambda a: torch.tensor(a, device=cuda)
+    arrs, dmem, doff, dcen = [D(c) for c in cols], D(mem), D(off), D(cen)
+    out = torch.full((1, len(_lib.PROP_FIELDS)), 77.0, dtype=torch.float64, device=cuda)
+
+    def call():
+        return _lib.lib().halma_halo_properties(40, *[_lib.ptr(a) for a in arrs], 1, _lib.ptr(doff), _lib.ptr(dmem),
+                                                _lib.ptr(dcen), 0.1, _lib.ptr(out), _lib.stream_of(out))
+    dmem[7] = 40
+    assert call() == _lib.ERR_INVALID
+    assert bool((out == 77.0).all())
+    dmem[7] = 7
+    assert call() == 0
+    from pyhalma_gb300 import halo_properties
+    assert _same(out.cpu().numpy(), halo_properties.halo_property_table(off, mem, *cols, cen, 0.1))
