@@ -1872,6 +1872,7 @@ extern "C" int halma_fof_groups(int64_t n, const int32_t *labels, int32_t min_me
         int64_t zero = 0;
         if (is_device_pointer(offsets)) HALMA_CUDA(cudaMemcpy(offsets, &zero, 8, cudaMemcpyHostToDevice));
         else offsets[0] = 0;
+        set_group_members(0);
         return HALMA_OK;
     }
     std::lock_guard<std::mutex> guard(api_mutex());
@@ -1902,6 +1903,6 @@ extern "C" int halma_fof_groups(int64_t n, const int32_t *labels, int32_t min_me
     }
     if (stage) cudaFreeAsync(stage, st);
     cudaStreamSynchronize(st);
-    set_group_members(nm);
+    if (s == HALMA_OK) set_group_members(nm);
     return s;
 }

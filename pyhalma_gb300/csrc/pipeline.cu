@@ -145,6 +145,7 @@ extern "C" int halma_find_haloes(int64_t n, const double *x, const double *y, co
             if (is_device_pointer(halo_offsets)) HALMA_CUDA(cudaMemcpy(halo_offsets, &zero, 8, cudaMemcpyHostToDevice));
             else halo_offsets[0] = 0;
         }
+        set_group_members(0);
         return HALMA_OK;
     }
     std::lock_guard<std::mutex> guard(api_mutex());
@@ -283,8 +284,8 @@ extern "C" int halma_find_haloes(int64_t n, const double *x, const double *y, co
     HALMA_CUDA(cudaStreamSynchronize(st));
     if (early.joinable()) early.join();
     else HALMA_CUDA(cudaStreamSynchronize(side->s));
-    set_group_members(nm);
     if (early_status != HALMA_OK) return fail(early_status, "%s", early_msg.c_str());
+    set_group_members(nm);
     return HALMA_OK;
 }
 

@@ -355,3 +355,23 @@ def test_labels_are_not_touched_by_a_refused_call(cuda, n):
     st = _lib.lib().halma_fof(n, _lib.ptr(x), _lib.ptr(y), _lib.ptr(z), 0.05, _lib.ptr(lab), None, _lib.stream_of(x))
     assert st == _lib.ERR_INVALID
     assert bool((lab == 77).all())
+
+
+def test_member_count_of_the_last_call(cuda):
+    """halma_last_group_members(): what the thread's last successful call stored; 0 after an empty one, and as it was after
+    one that failed."""
+    import ctypes
+    from pyhalma_gb300 import _lib
+    L = _lib.lib()
+    lab = np.array([0, 0, -1, 3, 3, 3], dtype=np.int32)
+    off, mem, ng = np.zeros(7, dtype=np.int64), np.zeros(6, dtype=np.int32), ctypes.c_int64()
+    call = lambda n, l: L.halma_fof_groups(n, _lib.ptr(l), 2, _lib.ptr(off), _lib.ptr(mem), ctypes.byref(ng), None)
+    assert call(6, lab) == 0 and L.halma_last_group_members() == 5
+    bad = np.array([0, 0, 9, 3, 3, 3], dtype=np.int32)
+    assert call(6, bad) == _lib.ERR_INVALID and L.halma_last_group_members() == 5
+    assert call(0, lab) == 0 and L.halma_last_group_members() == 0
+    from pyhalma_gb300.unbinding import find_haloes
+    assert call(6, lab) == 0 and L.halma_last_group_members() == 5
+    e = np.zeros(0)
+    find_haloes(e, e, e, e, e, e, e, 0.0015)
+    assert L.halma_last_group_members() == 0
