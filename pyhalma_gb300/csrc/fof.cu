@@ -27,6 +27,8 @@
 #include <limits.h>
 #include <string.h>
 
+#include <map>
+
 #include "common.cuh"
 #include "sort.cuh"
 #include "unbind.cuh"
@@ -432,18 +434,28 @@ __device__ __forceinline__ Heads heads_at(const uint64_t *__restrict__ keys, int
 }
 
 __global__ void __launch_bounds__(256) head_count_kernel(int n, int sb, const uint64_t *__restrict__ keys,
-                                                         int64_t *__restrict__ counts, int nruns) {
+                                                         int64_t *__restrict__ counts, int nruns,
+                                                         int *__restrict__ all_cells) {
+    __shared__ int block_cells;
+    if (threadIdx.x == 0) block_cells = 0;
+    __syncthreads();
     const int lane = threadIdx.x & 31;
     const int run = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (run >= nruns) return;
-    int cells = 0, nodes = 0;
+    if (run < nruns) {
+        int cells = 0, nodes = 0;
 #pragma unroll 4
-    for (int r = 0; r < kScanRun; r += 32) {
-        const Heads h = heads_at(keys, sb, run * kScanRun + r + lane, n);
-        cells += __popc(__ballot_sync(0xffffffffu, h.cell));
-        nodes += __popc(__ballot_sync(0xffffffffu, h.node));
+        for (int r = 0; r < kScanRun; r += 32) {
+            const Heads h = heads_at(keys, sb, run * kScanRun + r + lane, n);
+            cells += __popc(__ballot_sync(0xffffffffu, h.cell));
+            nodes += __popc(__ballot_sync(0xffffffffu, h.node));
+        }
+        if (lane == 0) {
+            counts[run] = (int64_t)cells << 32 | nodes;
+            atomicAdd(&block_cells, cells);
+        }
     }
-    if (lane == 0) counts[run] = (int64_t)cells << 32 | nodes;
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(all_cells, block_cells);
 }
 
 // Node m: first sorted position node_start[m], cell node_cell[m], first particle's record
@@ -1346,6 +1358,29 @@ int push_uf_cap(cudaStream_t st) {
     return HALMA_OK;
 }
 
+// From kPairsByCount particles on, the number of cells comes to the host by a stream of its own (into page-locked memory:
+// a copy elsewhere would keep the host from launching what runs meanwhile): in line it took 13 us of a call.
+constexpr int kPairsByCount = 1 << 20;
+
+struct CellSide {
+    cudaStream_t s = nullptr;
+    cudaEvent_t counted = nullptr, copied = nullptr;
+    int *cells = nullptr;
+};
+
+int cell_side(CellSide **out) {
+    static std::map<int, CellSide> m;   // per device, under api_mutex()
+    CellSide &c = m[current_device()];
+    if (!c.s) HALMA_CUDA(cudaStreamCreateWithFlags(&c.s, cudaStreamNonBlocking));
+    for (cudaEvent_t *e : {&c.counted, &c.copied})
+        if (!*e) HALMA_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    if (!c.cells) HALMA_CUDA(cudaMallocHost(reinterpret_cast<void **>(&c.cells), sizeof(int)));
+    *out = &c;
+    return HALMA_OK;
+}
+
+size_t pair_bytes(int ncell) { return sizeof(int2) * 14 * (size_t)std::max(ncell, 1); }
+
 // Keys, sort, cells, links and labels for a geometry whose cell grid is known.
 int fof_core(int n, const double *x, const double *y, const double *z, FofGeom g, SegGeom sg, int *labels,
              int64_t *n_groups, cudaStream_t st) {
@@ -1388,7 +1423,7 @@ int fof_core(int n, const double *x, const double *y, const double *z, FofGeom g
     auto *node_sub = at<unsigned char>(base, o_sub), *multi = at<unsigned char>(base, o_multi);
     int *cell_node = at<int>(base, o_cnode);
     auto *cell_key = at<uint64_t>(base, o_ckey);
-    int *cnt = at<int>(base, o_cnt);   // [0] cells [1] nodes [2] groups [3] error [4] heavy pairs [6..7] cell pairs [8..9] listed pairs of nodes
+    int *cnt = at<int>(base, o_cnt);   // [0] cells [1] nodes [2] groups [3] error [4] heavy pairs [6..7] cell pairs [8..9] listed pairs of nodes [10] cells, from their count
     auto *npairs = at<unsigned long long>(base, o_cnt + 24), *nlist = npairs + 1;
     auto *cell_list = at<long long>(base, o_clist);
     int *node_cell = at<int>(base, o_ncell);
@@ -1417,20 +1452,38 @@ int fof_core(int n, const double *x, const double *y, const double *z, FofGeom g
     HALMA_TRY(sort_pairs_u64_i32(tmp, sort_b, kin, kout, vin, vout, n, end_bit, st));
     HALMA_TRY(mark(2));
     const int gr = grid_for(nruns, 8);
-    HALMA_LAUNCH(head_count_kernel, gr, 256, 0, st, n, g.sb, kout, runs, nruns);
+    HALMA_LAUNCH(head_count_kernel, gr, 256, 0, st, n, g.sb, kout, runs, nruns, cnt + 10);
+    CellSide *side = nullptr;
+    if (n > kPairsByCount) {   // the cells' number, on its way to the host while the two kernels below run
+        HALMA_TRY(cell_side(&side));
+        HALMA_CUDA(cudaEventRecord(side->counted, st));
+        HALMA_CUDA(cudaStreamWaitEvent(side->s, side->counted, 0));
+        HALMA_CUDA(cudaMemcpyAsync(side->cells, cnt + 10, sizeof(int), cudaMemcpyDeviceToHost, side->s));
+        HALMA_CUDA(cudaEventRecord(side->copied, side->s));
+    }
     HALMA_TRY(exclusive_sum_i64(tmp, scan_b, runs, rbase, nruns, st));
     HALMA_LAUNCH(head_apply_kernel, gr, 256, 0, st, n, g.sb, kout, vout, pre, rbase, nruns, rec, node_of, node_start,
                  node_cell, node_sub, at<float4>(base, o_nrec), parent, minidx, multi, cell_node, cell_key, cnt);
     HALMA_TRY(mark(3));
-    // the list of cell pairs (at most 14 x 8 bytes per occupied cell) in its own cached buffer, sized from the cell
-    // count; up to 2^25 particles (3.8 GB) the particle count saves that round trip (25 us)
+    // The list of cell pairs (at most 14 x 8 bytes per occupied cell) in its own cached buffer: of a size for as many cells as
+    // particles up to kPairsByCount of them (117 MB), and for the cells there are above that, or where there is no room.
     int ncell = n;
-    if (n > (1 << 25)) {
-        HALMA_CUDA(cudaMemcpyAsync(&ncell, cnt + 0, sizeof(int), cudaMemcpyDeviceToHost, st));
-        HALMA_CUDA(cudaStreamSynchronize(st));
-    }
     void *pbase = nullptr;
-    HALMA_TRY(workspace(sizeof(int2) * 14 * (size_t)std::max(ncell, 1), &pbase, st, 10));
+    int got = HALMA_ERR_NOMEM;
+    if (n <= kPairsByCount) {
+        got = workspace(pair_bytes(n), &pbase, st, 10);
+    } else {
+        HALMA_CUDA(cudaEventSynchronize(side->copied));
+        ncell = *side->cells;
+    }
+    if (got == HALMA_ERR_NOMEM) {
+        if (n <= kPairsByCount) {
+            HALMA_CUDA(cudaMemcpyAsync(&ncell, cnt + 0, sizeof(int), cudaMemcpyDeviceToHost, st));
+            HALMA_CUDA(cudaStreamSynchronize(st));
+        }
+        got = workspace(pair_bytes(ncell), &pbase, st, 10);
+    }
+    HALMA_TRY(got);
     int2 *pairs = static_cast<int2 *>(pbase);
     const int gc = std::min(sms * 8, grid_for(ncell, 256));
     HALMA_TRY(mark(4));

@@ -1,0 +1,50 @@
+"""Device memory that calls keep or cannot do without: the scratch stays in proportion to what is computed, and a call
+whose faster form does not fit in what is left of the memory takes the smaller one."""
+import numpy as np
+import pytest
+
+import oracle
+from pyhalma_gb300 import _lib, fof, halo_gas, halo_properties, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _free():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def _scratch(call):
+    """Bytes of the library's scratch after one call on empty workspaces (the second, so that kernels are loaded)."""
+    call()
+    _lib.lib().halma_release_workspace()
+    before = _free()
+    call()
+    return before - _free()
+
+
+class _Leave:
+    """All of the device's memory taken but for `nbytes`, with empty workspaces."""
+    def __init__(self, nbytes):
+        self.nbytes = nbytes
+
+    def __enter__(self):
+        import torch
+        _lib.lib().halma_release_workspace()
+        torch.cuda.empty_cache()
+        self.held = torch.empty(max(_free() - self.nbytes, 0), dtype=torch.uint8, device="cuda")
+
+    def __exit__(self, *exc):
+        import torch
+        self.held = None
+        torch.cuda.empty_cache()
+        _lib.lib().halma_release_workspace()
+
+
+def test_fof_of_few_cells(cuda):
+    """The cell pairs take their place by the cells, not by the particles."""
+    import torch
+    s = synth.plummer_snapshot(4_000_000, 40, seed=1, box_mpc=10.0, contaminant_frac=0.05)
+    x, y, z = (torch.from_numpy(a).to(cuda) for a in (s.x, s.y, s.z))
+    assert _scratch(lambda: fof.fof_labels(x, y, z, 0.0015)) < 190 * s.n
