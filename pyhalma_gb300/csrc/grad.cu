@@ -606,14 +606,26 @@ extern "C" int halma_potential_grad_f32(int64_t ns, const float *m_, const float
     if (grad_tgt) choose_slices(nt, ns, adjoint_targets<false>(nt), 3, &split_t, &len_t);
     if (grad_m || grad_src) choose_slices(ns, nt, adjoint_targets<true>(ns), 4, &split_s, &len_s);
     // both sides in one sweep where that suits the sizes, and with a softening that keeps r^-2 finite
-    const bool both = grad_tgt && (grad_m || grad_src) && both_at_once(ns, nt) && (float)eps2 >= 0x1p-126f;
+    bool both = grad_tgt && (grad_m || grad_src) && both_at_once(ns, nt) && (float)eps2 >= 0x1p-126f;
     const BothPlan plan(ns, nt);
-    Layout L;
-    sg.plan(L);
-    const size_t o_part = L.add(both ? plan.bytes(nt) : split_t > 1 ? 8 * (size_t)(3 * nt * split_t) : 0);
-    const size_t o_part_s = L.add(!both && split_s > 1 ? 8 * (size_t)(4 * ns * split_s) : 0);
+    // where the partial sums do not fit in what is left of the memory: in slices, then without any (slower)
+    size_t o_part = 0, o_part_s = 0;
     void *base = nullptr;
-    HALMA_TRY(workspace(L.total, &base, st));
+    for (;;) {
+        Layout L;
+        sg.plan(L);
+        o_part = L.add(both ? plan.bytes(nt) : split_t > 1 ? 8 * (size_t)(3 * nt * split_t) : 0);
+        o_part_s = L.add(!both && split_s > 1 ? 8 * (size_t)(4 * ns * split_s) : 0);
+        const int s = workspace(L.total, &base, st);
+        if (s == HALMA_OK) break;
+        if (s != HALMA_ERR_NOMEM || (!both && split_t == 1 && split_s == 1)) return s;
+        if (!both) {
+            split_t = split_s = 1;
+            len_t = ns;
+            len_s = nt;
+        }
+        both = false;
+    }
     HALMA_TRY(sg.bind_and_upload(base, st));
     double *part = at<double>(base, o_part);
     const int self = mask == HALMA_MASK_SELF;

@@ -48,3 +48,33 @@ def test_fof_of_few_cells(cuda):
     s = synth.plummer_snapshot(4_000_000, 40, seed=1, box_mpc=10.0, contaminant_frac=0.05)
     x, y, z = (torch.from_numpy(a).to(cuda) for a in (s.x, s.y, s.z))
     assert _scratch(lambda: fof.fof_labels(x, y, z, 0.0015)) < 190 * s.n
+
+
+def test_gradients_where_partial_sums_do_not_fit(cuda):
+    """Both ends in one sweep (34 MB of partial sums), in slices (100 MB) or with none: 12 MB are left here."""
+    import torch
+    ns, nt = 20_000, 20_100
+    g = torch.Generator(device=cuda).manual_seed(3)
+    P = _lib.ptr
+
+    def make(ns, nt):
+        T = lambda n: 0.02 * torch.randn(n, device=cuda, generator=g)
+        ins = (ns, [T(ns).abs()] + [T(ns) for _ in range(3)], nt, [T(nt) for _ in range(4)])
+        return ins, [torch.empty(k, device=cuda) for k in (ns, 3 * ns, 3 * nt)]
+
+    def run(ins, out):
+        ns, s, nt, t = ins
+        _lib.check(_lib.lib().halma_potential_grad_f32(ns, *[P(a) for a in s], nt, *[P(a) for a in t], 1e-8, _lib.MASK_NONE,
+                                                       0, *[P(a) for a in out], _lib.stream_of(s[0])), "gradients")
+    ins, out = make(ns, nt)
+    run(ins, out)
+    want = [o.clone() for o in out]
+    for k in ((1000, nt), (300, 200)):   # the kernels that are called below, loaded while there is room
+        run(*make(*k))
+    for o in out:
+        o.zero_()
+    with _Leave(12 << 20):
+        run(ins, out)
+        torch.cuda.synchronize()
+    for o, w in zip(out, want):
+        assert float((o - w).norm() / w.norm()) < 1e-6
