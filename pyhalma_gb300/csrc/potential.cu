@@ -189,7 +189,8 @@ struct RefShape {
 template <int TL>
 __global__ void __launch_bounds__(RefShape<TL>::warps * 32) ref_potential_kernel(
     const Src4 *__restrict__ src, int64_t nstages, const float *__restrict__ tx, const float *__restrict__ ty,
-    const float *__restrict__ tz, int64_t nt, const int *__restrict__ flags, float nzero, float *__restrict__ out) {
+    const float *__restrict__ tz, int64_t nt, const int *__restrict__ flags, float nzero, int first,
+    float *__restrict__ out) {
     using S = RefShape<TL>;
     constexpr int N = S::take * TL / 32;    // quads of a lane in one stage
     extern __shared__ float4 ref_terms[];    // [2][S::quads][TL]
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(RefShape<TL>::warps * 32) ref_potential_kernel
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     if (share >= 0) fetch(0);
-    float acc = 0.f;
+    float acc = first ? 0.f : out[it];   // the sources before these
     for (int64_t st = 0; st <= nstages; ++st) {
         if (share >= 0 && st < nstages) {
             fetch(st + 1);
@@ -252,11 +253,13 @@ __global__ void __launch_bounds__(RefShape<TL>::warps * 32) ref_potential_kernel
     if (S::adds(w) && lane < TL && i < nt) out[i] = acc;
 }
 
-// Packs the sources and runs the kernel; src holds ref_quads_of(ntotal) quads.
+// Packs the sources and runs the kernel, kRefPiece sources at a time (64 MB of packed ones); src holds the quads of a piece.
+constexpr int64_t kRefPiece = 1ll << 22;
+
 template <int TL>
 static int64_t ref_quads_of(int64_t ns) {
     const int64_t q = RefShape<TL>::quads;
-    return ((ns + 3) / 4 + q - 1) / q * q;
+    return ((std::min(ns, kRefPiece) + 3) / 4 + q - 1) / q * q;
 }
 
 template <int TL>
@@ -264,14 +267,16 @@ static int launch_reference(const float *m, const float *x, const float *y, cons
                             const float *ty, const float *tz, int64_t nt, Src4 *src, int *flags, float *out,
                             cudaStream_t st) {
     using S = RefShape<TL>;
-    const int64_t nquads = ref_quads_of<TL>(ns);
-    HALMA_CUDA(cudaMemsetAsync(flags, 0, sizeof(int), st));
-    HALMA_LAUNCH(ref_pack_kernel, grid_for(std::max(nquads, nt), 256, device_sm_count() * 8), 256, 0, st, m, x, y, z, ns,
-                 nquads, tx, ty, tz, nt, src, flags);
     constexpr int smem = 2 * S::quads * TL * (int)sizeof(float4);
     HALMA_CUDA(cudaFuncSetAttribute(ref_potential_kernel<TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    HALMA_LAUNCH(ref_potential_kernel<TL>, (unsigned)((nt + TL - 1) / TL), S::warps * 32, smem, st, src,
-                 nquads / S::quads, tx, ty, tz, nt, flags, -0.0f, out);
+    for (int64_t j = 0; j < ns; j += kRefPiece) {
+        const int64_t n = std::min(kRefPiece, ns - j), nquads = ref_quads_of<TL>(n);
+        HALMA_CUDA(cudaMemsetAsync(flags, 0, sizeof(int), st));
+        HALMA_LAUNCH(ref_pack_kernel, grid_for(std::max(nquads, nt), 256, device_sm_count() * 8), 256, 0, st, m + j, x + j,
+                     y + j, z + j, n, nquads, tx, ty, tz, nt, src, flags);
+        HALMA_LAUNCH(ref_potential_kernel<TL>, (unsigned)((nt + TL - 1) / TL), S::warps * 32, smem, st, src,
+                     nquads / S::quads, tx, ty, tz, nt, flags, -0.0f, j == 0, out);
+    }
     return HALMA_OK;
 }
 

@@ -220,3 +220,17 @@ def test_skipped_pair_of_an_infinite_mass(cuda, n):
     ref = oracle.potential_f64(d(m), d(x), d(y), d(z), d(x[at:at + 1]), d(y[at:at + 1]), d(z[at:at + 1]), eps2=1e-8,
                                mask=oracle.MASK_NONE)
     assert abs(phi[at] / ref[0] - 1.0) < RTOL_FAST
+
+
+@pytest.mark.parametrize("ns", [2 ** 22 - 1, 2 ** 22, 2 ** 22 + 1, 2 ** 23 + 77])
+def test_reference_mode_in_pieces_of_the_sources(cuda, ns):
+    """More sources than are packed at a time, in one block of targets and with the plain operations in one piece alone (a
+    mass outside the fast terms' range)."""
+    rng = np.random.default_rng(22)
+    p, m = _cloud(rng, ns)
+    m[5] = 1e-20
+    m[ns - 1] = 2.0 ** 20
+    t, _ = _cloud(rng, 9)
+    t[3] = p[ns - 1]
+    got = halo_gas.bf_potential(m, *p.T, *t.T, mode="reference")
+    assert np.array_equal(got, oracle.bf_potential_f32(m, *p.T, *t.T))

@@ -78,3 +78,12 @@ def test_gradients_where_partial_sums_do_not_fit(cuda):
         torch.cuda.synchronize()
     for o, w in zip(out, want):
         assert float((o - w).norm() / w.norm()) < 1e-6
+
+
+def test_reference_potential_of_many_sources(cuda):
+    import torch
+    ns = 1 << 24
+    x, y, z = (torch.rand(ns, device=cuda) for _ in range(3))
+    m = x + 1.0
+    t = [torch.full((8,), 0.3 + k, device=cuda) for k in range(3)]
+    assert _scratch(lambda: halo_gas.bf_potential(m, x, y, z, *t, mode="reference")) < 100 << 20
