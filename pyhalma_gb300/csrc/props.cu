@@ -925,8 +925,9 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
     sg.add(centre, 5 * n_groups, true, false, &dcen);
     sg.add((const double *)out, n_groups * HALMA_PROP_NFIELDS, false, true, &dout);
     const int64_t NM = std::max<int64_t>(N0, 1), N3 = 3 * NM;
-    // the four half-mass reductions in one run, up to 2^25 members (5 GB of scratch), else one after another
-    const bool sets = N0 > 0 && N0 <= (1 << 25) && G <= (1 << 25);
+    // the four half-mass reductions in one run, up to 2^23 members (1.7 GB of scratch, as one of 2^25 takes), else, and where
+    // the memory is short, one after another
+    bool sets = N0 > 0 && N0 <= (1 << 23) && G <= (1 << 23);
     Layout L;
     sg.plan(L);
     const bool dev_out = is_device_pointer(out);
@@ -983,8 +984,11 @@ extern "C" int halma_halo_properties(int64_t n, const double *x, const double *y
     if (sets) {
         int64_t *off4 = at<int64_t>(base, o_off4);
         HALMA_LAUNCH(pr_off4_kernel, grid_for(4ll * G + 1, 256, sms * 8), 256, 0, st, G, N0, doff, off4);
-        HALMA_TRY(reductions_sets_device(N0, G, off4, pos, gvx, gvy, gvz, gm, about, red, st));
-    } else {
+        const int s = reductions_sets_device(N0, G, off4, pos, gvx, gvy, gvz, gm, about, red, st);
+        if (s == HALMA_ERR_NOMEM) sets = false;   // of its scratch, before anything was launched
+        else HALMA_TRY(s);
+    }
+    if (!sets) {
         for (int r = 0; r < 4; ++r)
             HALMA_TRY(reductions_device(N0, G, doff, pos[r][0], pos[r][1], pos[r][2], gvx, gvy, gvz, gm, nullptr,
                                         about + (int64_t)r * G * HALMA_ABOUT_NFIELDS,

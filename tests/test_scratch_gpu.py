@@ -87,3 +87,23 @@ def test_reference_potential_of_many_sources(cuda):
     m = x + 1.0
     t = [torch.full((8,), 0.3 + k, device=cuda) for k in range(3)]
     assert _scratch(lambda: halo_gas.bf_potential(m, x, y, z, *t, mode="reference")) < 100 << 20
+
+
+def test_half_mass_radii_where_four_sets_do_not_fit(cuda):
+    """The four half-mass radii one after another where one run for all has no room."""
+    rng = np.random.default_rng(4)
+    sizes = rng.integers(1000, 9000, 80)
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    n = int(off[-1])
+    cols = rng.normal(0.0, 0.01, (6, n))
+    m = rng.uniform(0.5, 2.0, n)
+    cen = np.zeros((len(sizes), 5))
+    cen[:, 3] = np.add.reduceat(m, off[:-1])
+    cen[:, 4] = 0.06
+    call = lambda: halo_properties.halo_property_table(off, np.arange(n, dtype=np.int32), *cols, m, cen, 0.002)
+    want = call()
+    used = _scratch(call)
+    one = 60 * n                       # one set's scratch, of which the run of four takes four
+    with _Leave(used - 2 * one):
+        got = call()
+    assert np.array_equal(got, want, equal_nan=True)
