@@ -330,6 +330,63 @@ __device__ __forceinline__ void pot_chunk(const float4 *sa, const float4 *sb, co
     }
 }
 
+// One item by a warp: 32 T targets from t0 on against the sources jb .. je; their compensated sums.
+template <int T, int MASK, bool FTZ>
+__device__ __forceinline__ void pot_item(const float *__restrict__ m, const float *__restrict__ x,
+                                         const float *__restrict__ y, const float *__restrict__ z, int64_t jb, int64_t je,
+                                         const float *__restrict__ tx, const float *__restrict__ ty,
+                                         const float *__restrict__ tz, int64_t t0, int64_t nt, float eps2,
+                                         int64_t self_offset, float4 *buf, int lane, float (&sum)[T], float (&comp)[T]) {
+    float *sa = reinterpret_cast<float *>(buf);        // 16 float4: x and y pairs
+    float *sb = reinterpret_cast<float *>(buf + 16);   // 16 float4: z and m pairs
+    const int kp = lane >> 1, hf = lane & 1;
+    const f2x e2 = pack2(eps2, eps2);
+    f2x px[T], py[T], pz[T];
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+        const int64_t i = t0 + t * 32 + lane;
+        const bool v = i < nt;
+        const float cx = v ? tx[i] : kPadCoord, cy = v ? ty[i] : kPadCoord, cz = v ? tz[i] : kPadCoord;
+        px[t] = pack2(cx, cx);
+        py[t] = pack2(cy, cy);
+        pz[t] = pack2(cz, cz);
+        sum[t] = 0.f;
+        comp[t] = 0.f;
+    }
+    // the tile's self pairs are with the sources lo_self .. lo_self + 32 T - 1
+    const int64_t lo_self = t0 + self_offset;
+    float4 nxt = load_source(m, x, y, z, jb + lane, je);
+    for (int64_t j0 = jb; j0 < je; j0 += 32) {
+        __syncwarp();
+        sa[kp * 4 + hf] = nxt.x;
+        sa[kp * 4 + 2 + hf] = nxt.y;
+        sb[kp * 4 + hf] = nxt.z;
+        sb[kp * 4 + 2 + hf] = nxt.w;
+        __syncwarp();
+        nxt = load_source(m, x, y, z, j0 + 32 + lane, je);
+        f2x acc[T];
+        int self[T];
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            acc[t] = pack2(0.f, 0.f);
+            self[t] = -1;
+        }
+        if (MASK == HALMA_MASK_SELF && j0 + 32 > lo_self && j0 < lo_self + 32 * T) {
+#pragma unroll
+            for (int t = 0; t < T; ++t) self[t] = (int)(lo_self + t * 32 + lane - j0);
+            pot_chunk<T, MASK, FTZ, true>(buf, buf + 16, px, py, pz, e2, self, acc);
+        } else {
+            pot_chunk<T, MASK, FTZ, false>(buf, buf + 16, px, py, pz, e2, self, acc);
+        }
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            float a0, a1;
+            unpack2(acc[t], a0, a1);
+            two_sum_acc(sum[t], comp[t], a0 + a1);
+        }
+    }
+}
+
 template <int T, int MASK, bool FTZ>
 __global__ void __launch_bounds__(256) bf_potential_fast_kernel(
     const float *__restrict__ m, const float *__restrict__ x, const float *__restrict__ y,
@@ -339,10 +396,6 @@ __global__ void __launch_bounds__(256) bf_potential_fast_kernel(
     double *__restrict__ partial) {
     __shared__ float4 buf[kWarpsPerBlock][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    float *sa = reinterpret_cast<float *>(buf[w]);        // 16 float4: x and y pairs
-    float *sb = reinterpret_cast<float *>(buf[w] + 16);   // 16 float4: z and m pairs
-    const int kp = lane >> 1, hf = lane & 1;
-    const f2x e2 = pack2(eps2, eps2);
     const int64_t gwarp = (int64_t)blockIdx.x * kWarpsPerBlock + w;
     const int64_t nwarps = (int64_t)gridDim.x * kWarpsPerBlock;
     const int64_t ntiles = (nt + 32 * T - 1) / (32 * T);
@@ -351,52 +404,9 @@ __global__ void __launch_bounds__(256) bf_potential_fast_kernel(
         const int64_t tile = item / n_split;
         const int s = (int)(item - tile * n_split);
         const int64_t jb = (int64_t)s * split_len;
-        const int64_t je = min(ns, jb + split_len);
-        f2x px[T], py[T], pz[T];
         float sum[T], comp[T];
-#pragma unroll
-        for (int t = 0; t < T; ++t) {
-            const int64_t i = tile * 32 * T + t * 32 + lane;
-            const bool v = i < nt;
-            const float cx = v ? tx[i] : kPadCoord, cy = v ? ty[i] : kPadCoord, cz = v ? tz[i] : kPadCoord;
-            px[t] = pack2(cx, cx);
-            py[t] = pack2(cy, cy);
-            pz[t] = pack2(cz, cz);
-            sum[t] = 0.f;
-            comp[t] = 0.f;
-        }
-        // the tile's self pairs are with the sources lo_self .. lo_self + 32 T - 1
-        const int64_t lo_self = tile * 32 * T + self_offset;
-        float4 nxt = load_source(m, x, y, z, jb + lane, je);
-        for (int64_t j0 = jb; j0 < je; j0 += 32) {
-            __syncwarp();
-            sa[kp * 4 + hf] = nxt.x;
-            sa[kp * 4 + 2 + hf] = nxt.y;
-            sb[kp * 4 + hf] = nxt.z;
-            sb[kp * 4 + 2 + hf] = nxt.w;
-            __syncwarp();
-            nxt = load_source(m, x, y, z, j0 + 32 + lane, je);
-            f2x acc[T];
-            int self[T];
-#pragma unroll
-            for (int t = 0; t < T; ++t) {
-                acc[t] = pack2(0.f, 0.f);
-                self[t] = -1;
-            }
-            if (MASK == HALMA_MASK_SELF && j0 + 32 > lo_self && j0 < lo_self + 32 * T) {
-#pragma unroll
-                for (int t = 0; t < T; ++t) self[t] = (int)(lo_self + t * 32 + lane - j0);
-                pot_chunk<T, MASK, FTZ, true>(buf[w], buf[w] + 16, px, py, pz, e2, self, acc);
-            } else {
-                pot_chunk<T, MASK, FTZ, false>(buf[w], buf[w] + 16, px, py, pz, e2, self, acc);
-            }
-#pragma unroll
-            for (int t = 0; t < T; ++t) {
-                float a0, a1;
-                unpack2(acc[t], a0, a1);
-                two_sum_acc(sum[t], comp[t], a0 + a1);
-            }
-        }
+        pot_item<T, MASK, FTZ>(m, x, y, z, jb, min(ns, jb + split_len), tx, ty, tz, tile * 32 * T, nt, eps2, self_offset,
+                               buf[w], lane, sum, comp);
 #pragma unroll
         for (int t = 0; t < T; ++t) {
             const int64_t i = tile * 32 * T + t * 32 + lane;
@@ -405,6 +415,34 @@ __global__ void __launch_bounds__(256) bf_potential_fast_kernel(
                 else partial[(int64_t)s * nt + i] = (double)sum[t] + (double)comp[t];
             }
         }
+    }
+}
+
+// The slices of 32 targets by one block, their sums added there in the same order: for up to kBlockSlices slices, without
+// memory for the partial sums (the allocation-free entry point).
+constexpr int kBlockSlices = 32;
+
+template <bool FTZ>
+__global__ void __launch_bounds__(256) bf_potential_block_kernel(
+    const float *__restrict__ m, const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
+    int64_t ns, const float *__restrict__ tx, const float *__restrict__ ty, const float *__restrict__ tz, int64_t nt,
+    float eps2, int n_split, int64_t split_len, float *__restrict__ out) {
+    __shared__ float4 buf[kWarpsPerBlock][32];
+    __shared__ double part[kBlockSlices][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t t0 = (int64_t)blockIdx.x * 32;
+    for (int s = w; s < n_split; s += kWarpsPerBlock) {
+        const int64_t jb = (int64_t)s * split_len;
+        float sum[1], comp[1];
+        pot_item<1, HALMA_MASK_COORD, FTZ>(m, x, y, z, jb, min(ns, jb + split_len), tx, ty, tz, t0, nt, eps2, 0, buf[w],
+                                           lane, sum, comp);
+        part[s][lane] = (double)sum[0] + (double)comp[0];
+    }
+    __syncthreads();
+    if (w == 0 && t0 + lane < nt) {
+        double acc = 0.0;
+        for (int s = 0; s < n_split; ++s) acc += part[s][lane];
+        out[t0 + lane] = (float)acc;
     }
 }
 
@@ -452,6 +490,8 @@ __global__ void __launch_bounds__(256) potential_f64_kernel(
 }
 
 constexpr int64_t kMaxPartials = 1ll << 21;   // partial sums of one call, from the finer slices below
+constexpr int64_t kCoarseSlice = 2048, kFineSlice = 128;   // sources of a slice at least
+static_assert(2 * kCoarseSlice <= kBlockSlices * kFineSlice, "fewer sources have at most kBlockSlices slices");
 
 // Number of source slices so that (target tiles x slices) keeps every SM busy.  Slices have at least
 // 2048 sources, or 128 while the partial sums stay within kMaxPartials: 3,000 targets x 4,000
@@ -463,8 +503,8 @@ static void choose_split(int64_t ns, int64_t nt, int T, int *n_split, int64_t *s
     int64_t s = 1;
     if (ntiles < want_items) s = (want_items + ntiles - 1) / ntiles;
     s = std::min<int64_t>(s, 1024);
-    const int64_t coarse = std::min(s, std::max<int64_t>(1, ns / 2048));
-    const int64_t fine = std::min(s, std::min(ns / 128, kMaxPartials / nt));
+    const int64_t coarse = std::min(s, std::max<int64_t>(1, ns / kCoarseSlice));
+    const int64_t fine = std::min(s, std::min(ns / kFineSlice, kMaxPartials / nt));
     s = std::max(coarse, fine);
     int64_t len = (ns + s - 1) / s;
     len = (len + 31) / 32 * 32;
@@ -736,13 +776,13 @@ extern "C" int halma_potential_f64(int64_t ns, const double *mm, const double *s
 // 2,097,152 partial sums (source slices x targets) the call is rejected with
 // HALMA_ERR_CAPACITY.
 //
-// Every GPU that loads this library holds the 16 MiB array until the process exits.  All calls
-// share it and it keeps the previous call's contents; each partial sum a call reads is written
+// Every GPU that loads this library holds the 16 MiB array until the process exits.  All calls with 4,096 sources or more
+// share it (the slices of fewer are added up inside a block) and it keeps the previous call's contents; each partial sum a call reads is written
 // by the same call first, so nothing needs clearing.  Calls that overlap on the GPU (two
 // streams, or two host threads without ordering) race on the array and give wrong results.
 // The first call on each device looks up the array's device address (cudaGetSymbolAddress with
 // that device current); make that first call before any stream capture begins.
-constexpr int64_t kNoAllocScratchDoubles = 1ll << 21;
+constexpr int64_t kNoAllocScratchDoubles = kMaxPartials;   // what the finer slices of any call take
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocScratchDoubles];
 
 namespace {
@@ -801,6 +841,16 @@ extern "C" int halma_bf_potential_f32_noalloc(int64_t ntotal, const float *total
     int n_split = 1;
     int64_t split_len = ntotal;
     choose_split(ntotal, ntest, T, &n_split, &split_len);
+    if (n_split > 1 && ntotal < 2 * kCoarseSlice) {   // few enough slices for a block, with nothing that calls share
+        const unsigned blocks = (unsigned)((ntest + 31) / 32);
+        if ((float)eps2 >= 0x1p-126f)
+            HALMA_LAUNCH(bf_potential_block_kernel<true>, blocks, 256, 0, st, total_mass, total_x, total_y, total_z, ntotal,
+                         test_x, test_y, test_z, ntest, (float)eps2, n_split, split_len, binding_energy);
+        else
+            HALMA_LAUNCH(bf_potential_block_kernel<false>, blocks, 256, 0, st, total_mass, total_x, total_y, total_z, ntotal,
+                         test_x, test_y, test_z, ntest, (float)eps2, n_split, split_len, binding_energy);
+        return HALMA_OK;
+    }
     if (n_split > 1 && (int64_t)n_split * ntest > kNoAllocScratchDoubles)
         return fail(HALMA_ERR_CAPACITY,
                     "this call needs %lld partial sums (%d source slices x %lld targets); the allocation-free "

@@ -74,3 +74,40 @@ def test_noalloc_rejects_host_arrays_and_oversized_splits(cuda):
     st = L.halma_bf_potential_f32_noalloc(ns, ps, ps, ps, ps, nt, pt, pt, pt, pt, 0.0, None)
     assert st == _lib.ERR_CAPACITY
     assert b"partial sums" in L.halma_last_error()
+
+
+@pytest.mark.parametrize("ns", [200, 256, 257, 1000, 4095, 4096])
+@pytest.mark.parametrize("nt", [1, 33, 3000])
+@pytest.mark.parametrize("eps2", [0.0, 1e-8])
+def test_noalloc_of_few_sources(cuda, ns, nt, eps2):
+    """The same values as the regular entry point on both sides of the 4,096 sources below which no partial sums are written
+    (one kernel instead of two), and then with calls on two streams at a time."""
+    import torch
+    L = _lib.lib()
+    srcs, tgts = _case(ns + nt, ns, nt, cuda)
+    tgts = [torch.where(torch.arange(nt, device=cuda) % 7 == 0, s[:1].expand(nt), t) for s, t in zip(srcs[1:], tgts)]
+    a = torch.empty(nt, dtype=torch.float32, device=cuda)
+    b = torch.empty(nt, dtype=torch.float32, device=cuda)
+    before = L.halma_kernel_launch_count()
+    _call(L.halma_bf_potential_f32_noalloc, srcs, tgts, a, ctypes.c_double(eps2))
+    launches = L.halma_kernel_launch_count() - before
+    _call(L.halma_bf_potential_f32, srcs, tgts, b, ctypes.c_int32(_lib.POT_FAST), ctypes.c_double(eps2))
+    assert np.array_equal(a.cpu().numpy(), b.cpu().numpy())
+    if ns >= 4096:
+        return
+    assert launches == 1
+    more = [_case(k, ns - k, nt, cuda) for k in range(2)]
+    outs = [[torch.empty(nt, dtype=torch.float32, device=cuda) for _ in range(8)] for _ in range(2)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+    for r in range(8):
+        for k in range(2):
+            p = [ctypes.c_void_p(t.data_ptr()) for t in more[k][0] + more[k][1] + [outs[k][r]]]
+            st = L.halma_bf_potential_f32_noalloc(ns - k, *p[:4], nt, *p[4:], ctypes.c_double(eps2),
+                                                  ctypes.c_void_p(streams[k].cuda_stream))
+            assert st == 0
+    torch.cuda.synchronize()
+    for k in range(2):
+        _call(L.halma_bf_potential_f32, *more[k], b, ctypes.c_int32(_lib.POT_FAST), ctypes.c_double(eps2))
+        for o in outs[k]:
+            assert torch.equal(o, b)
