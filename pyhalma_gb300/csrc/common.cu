@@ -1,6 +1,7 @@
 // Status strings, per-thread error text, cached workspace and launch accounting.
 #include <stdarg.h>
 #include <stdio.h>
+#include <unistd.h>
 
 #include <atomic>
 #include <map>
@@ -124,6 +125,14 @@ bool host_page_tables() {
         it = m.emplace(d, v != 0).first;
     }
     return it->second;
+}
+
+void touch_pages(const void *p, size_t bytes) {
+    static const size_t page = (size_t)std::max(sysconf(_SC_PAGESIZE), 1l);
+    if (bytes == 0) return;
+    const volatile unsigned char *c = static_cast<const unsigned char *>(p);
+    (void)c[0];
+    for (size_t k = page - reinterpret_cast<uintptr_t>(p) % page; k < bytes; k += page) (void)c[k];
 }
 
 namespace {

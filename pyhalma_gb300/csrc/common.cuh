@@ -88,6 +88,11 @@ struct Uploads {
 bool host_page_tables();
 int upload(const Uploads &u, cudaStream_t s);
 
+// Reads a byte of every page of host memory.  Pages that nobody has touched yet (zeros fresh from the allocator, a mapped
+// file) are so mapped by the CPU, which a GPU that meets them waits 9 us a page of 64 kB for; and an address that is not the
+// caller's memory ends the process here, as a copy by the CPU would, not the GPU's context.
+void touch_pages(const void *p, size_t bytes);
+
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 // Collects the caller's arrays of one call.  Host arrays get a slice of the workspace
@@ -175,6 +180,7 @@ struct Stager {
                 if (it.host) {
                     *it.slot = at<void>(base, it.off);
                     if (it.in && it.pageable && !late) {
+                        touch_pages(it.user, it.bytes);
                         batch.src[batch.n] = it.user;
                         batch.dst[batch.n] = *it.slot;
                         batch.bytes[batch.n++] = it.bytes;

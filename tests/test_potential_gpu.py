@@ -234,3 +234,25 @@ def test_reference_mode_in_pieces_of_the_sources(cuda, ns):
     t[3] = p[ns - 1]
     got = halo_gas.bf_potential(m, *p.T, *t.T, mode="reference")
     assert np.array_equal(got, oracle.bf_potential_f32(m, *p.T, *t.T))
+
+
+def test_host_pages_that_nobody_touched(cuda):
+    """Inputs fresh from the allocator (zeros whose pages are not there yet) take no longer than a CPU needs to map them."""
+    import time
+    n = 1 << 24
+    t = np.ones(1, dtype=np.float32)
+
+    def ms(fresh):
+        best = np.inf
+        for _ in range(3):
+            cols = [np.zeros(n, dtype=np.float32) for _ in range(4)]
+            if not fresh:
+                for c in cols:
+                    c += 0.0
+            t0 = time.perf_counter()
+            assert halo_gas.bf_potential(*cols, t, t, t, mode="fast", eps2=1.0)[0] == 0.0
+            best = min(best, 1e3 * (time.perf_counter() - t0))
+        return best
+    ms(False)
+    touched, fresh = ms(False), ms(True)
+    assert fresh < 2.0 * touched + 8.0, (fresh, touched)
