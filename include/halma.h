@@ -90,9 +90,10 @@ int64_t     halma_kernel_launch_count(void);
 int         halma_set_profiling(int32_t on);
 int         halma_profile_stats(double *out, int32_t cap);
 /* With profiling on: milliseconds of the FoF stages of the last halma_find_haloes call
- * (bounding box + keys, key sort, cells and nodes with their records, 0 (kept for its place),
- * cell pairs, linking, roots + labels, groups); on the all-pairs path of small inputs all but
- * the last three are 0; returns the count (8). */
+ * (bounding box + keys, key sort, cells and nodes with their records, cell pairs, first links and
+ * the pairs of nodes left to test, their tests, roots + labels, groups); on the all-pairs path of
+ * small inputs the first takes in the preparation, the second to fifth are 0 and the sixth is all
+ * the linking; returns the count (8). */
 int         halma_profile_fof_stages(double *out, int32_t cap);
 /* Measurement hook (no reference counterpart): the FP32 FMA rate of the current device, from
  * a kernel of independent FMA chains (packed != 0: fma.rn.f32x2, else fma.rn.f32), iters

@@ -173,6 +173,8 @@ def profile_stats():
             "sym_ms": sym_ms}
 
 
+# records: cells and nodes with their records; cells: the pairs of cells; items: first links, and the pairs of nodes
+# left to test; link: their tests
 FOF_STAGES = ["bbox_keys", "sort", "records", "cells", "items", "link", "labels", "groups"]
 
 

@@ -1486,14 +1486,13 @@ int fof_core(int n, const double *x, const double *y, const double *z, FofGeom g
     HALMA_TRY(got);
     int2 *pairs = static_cast<int2 *>(pbase);
     const int gc = std::min(sms * 8, grid_for(ncell, 256));
-    HALMA_TRY(mark(4));
     if (g.sb)
         HALMA_LAUNCH(cell_pair_kernel<true>, gc, 256, 0, st, cnt, cell_node, cell_key, g.ky, g.kz, pairs, cell_list,
                      npairs);
     else
         HALMA_LAUNCH(cell_pair_kernel<false>, gc, 256, 0, st, cnt, cell_node, cell_key, g.ky, g.kz, pairs, cell_list,
                      npairs);
-    HALMA_TRY(mark(5));
+    HALMA_TRY(mark(4));
     LinkArgs A{cnt, pairs, npairs, cell_list, cell_node, node_start, node_cell, node_sub, cell_key, rec,
                at<float4>(base, o_nrec), x, y, z, parent, cnt + 3, at<HeavyPair>(base, o_heavy), cnt + 4, heavy_cap};
     if (g.sb) {
@@ -1501,8 +1500,10 @@ int fof_core(int n, const double *x, const double *y, const double *z, FofGeom g
         HALMA_LAUNCH(hook_kernel, g1, 256, 0, st, A, g);
         HALMA_LAUNCH(flatten_kernel, g1, 256, 0, st, cnt, parent, root, cnt + 3);
         HALMA_LAUNCH(sweep_kernel, g1, 256, 0, st, A, g, root, list, (long long)n, nlist);
+        HALMA_TRY(mark(5));
         HALMA_LAUNCH(link_kernel, g1, 256, 0, st, A, g, list, (long long)n, nlist);
     } else {
+        HALMA_TRY(mark(5));
         HALMA_LAUNCH(link_particles_kernel, std::min(sms * 8, grid_for(4ll * ncell, 256)), 256, 0, st, A, g);
     }
     HALMA_LAUNCH(heavy_kernel, sms * 4, 256, 0, st, A, g, node_of);
