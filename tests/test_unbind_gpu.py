@@ -271,3 +271,28 @@ def test_teams_of_blocks(cuda, count):
         autotune.set_table(upper, t, slice_len)
     for g, w in zip(got, want):
         np.testing.assert_array_equal(g, w)
+
+
+@pytest.mark.parametrize("sizes", [(993,), (1023,), (1024,), (1025,), (1024, 1025, 700, 1024)])
+def test_both_sides_of_the_one_block_limit(cuda, sizes):
+    """Haloes of up to 1,024 members run in one block, larger ones on the pass kernels: the first pass bit for bit what the
+    pass kernels give (incremental=False keeps every halo there), all passes against FP64."""
+    rng = np.random.default_rng(sizes[0])
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    n = int(off[-1])
+    cols = [rng.normal(0.0, 0.01, n) for _ in range(3)] + [rng.normal(0.0, 40.0, n) for _ in range(3)]
+    cols.append(rng.uniform(0.5, 2.0, n) * 2e7)
+    got = unbind_batched(off, *cols, UnbindOptions(eps=EPS, max_iter=1), want_phi=True)
+    want = unbind_batched(off, *cols, UnbindOptions(eps=EPS, max_iter=1, incremental=False), want_phi=True)
+    for g, w in zip(got, want):
+        np.testing.assert_array_equal(g, w)
+    assert np.all(got[1][:, 7] > 0) and got[0].sum() < n   # some removed in the first pass, no halo emptied
+    got = unbind_batched(off, *cols, UnbindOptions(eps=EPS, max_iter=30), want_phi=True)
+    want = unbind_batched(off, *cols, UnbindOptions(eps=EPS, max_iter=30, precision="fp64"), want_phi=True)
+    assert np.all(want[1][:, 7] > 0)
+    same = got[0] == want[0]
+    assert (~same).sum() <= 2
+    if same.all():
+        np.testing.assert_array_equal(got[1][:, 7:9], want[1][:, 7:9])
+        both = got[0] == 1
+        assert np.max(np.abs(got[2][both] / want[2][both] - 1.0)) < RTOL_PHI
