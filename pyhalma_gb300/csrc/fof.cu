@@ -18,7 +18,7 @@
 //      A pair of particles whose float32 distance is clearly inside (outside) the linking length is accepted
 //      (rejected); pairs in a +-1e-5 band are re-tested with the exact FP64 predicate
 //      ((dx*dx + dy*dy) + dz*dz) <= ll*ll, every operation rounded on its own.  Pairs of crowded nodes without
-//      a link among their first tests go to a list that blocks work off;
+//      a link among their first tests go to lists that warps, and for the largest blocks, work off;
 //   6. each component's label = the smallest ORIGINAL index among its members (atomicMin over nodes), -1
 //      for particles alone.
 // Inputs of up to kSmallFof particles take all pairs instead (fof_small).
@@ -510,16 +510,20 @@ __global__ void __launch_bounds__(256) head_apply_kernel(
     }
 }
 
-__device__ __forceinline__ bool exact_link(const double *__restrict__ x, const double *__restrict__ y,
-                                           const double *__restrict__ z, int i, int j, double r2) {
-    // scipy's p = 2 distance: ((dx*dx + dy*dy) + dz*dz) <= r*r, each operation rounded
-    const double dx = __dsub_rn(x[i], x[j]);
-    const double dy = __dsub_rn(y[i], y[j]);
-    const double dz = __dsub_rn(z[i], z[j]);
+// scipy's p = 2 distance: ((dx*dx + dy*dy) + dz*dz) <= r*r, each operation rounded
+__device__ __forceinline__ bool exact_pair(double xi, double yi, double zi, double xj, double yj, double zj, double r2) {
+    const double dx = __dsub_rn(xi, xj);
+    const double dy = __dsub_rn(yi, yj);
+    const double dz = __dsub_rn(zi, zj);
     double s = __dmul_rn(dx, dx);
     s = __dadd_rn(s, __dmul_rn(dy, dy));
     s = __dadd_rn(s, __dmul_rn(dz, dz));
     return s <= r2;
+}
+
+__device__ __forceinline__ bool exact_link(const double *__restrict__ x, const double *__restrict__ y,
+                                           const double *__restrict__ z, int i, int j, double r2) {
+    return exact_pair(x[i], y[i], z[i], x[j], y[j], z[j], r2);
 }
 
 // Lower bound of q in the sorted keys[lo, n), searched forward from lo: doubling steps, then
@@ -636,8 +640,11 @@ struct __align__(8) HeavyPair {
     int a, na, b, nb, off, pad;
 };
 
-constexpr int kQuickTests = 1024;   // tests a thread makes for one pair of nodes before it leaves it to a block
-constexpr int kQuickNodes = 4096;   // pairs of particles a thread goes through for one cell pair (particles as nodes)
+// Tests that one pair of nodes gets from a lane: all when they are at most kLaneTests, else a glance, and a warp goes on with
+// what is open (up to kWarpTests; kWarpPairs pairs of particles, when they are the nodes, as each may be a union), and
+// a block with the rest.  With 1,024 from a lane and the others from a block, crowded nodes kept one lane of a warp at
+// work: 2e5 particles in clumps of 200 a twentieth of the linking length wide took 1.99 ms, now 0.34.
+constexpr int kLaneTests = 64, kLaneGlance = 8, kWarpTests = 1 << 15, kWarpPairs = 1 << 12;
 constexpr int kHookLinks = 2, kHookTests = 16;   // links and candidates of a node in hook_kernel
 
 struct LinkArgs {
@@ -651,6 +658,9 @@ struct LinkArgs {
     const float4 *rec, *node_rec;
     const double *x, *y, *z;
     int *parent, *err;
+    unsigned long long *crowd;      // pairs left to a warp each: nodes h << 32 | t, or the place of a pair of cells
+    unsigned long long *ncrowd;
+    int crowd_cap;
     HeavyPair *heavy;
     int *nheavy;
     int heavy_cap;
@@ -687,6 +697,18 @@ __device__ __forceinline__ int node_link(const LinkArgs &A, const FofGeom &g, in
         }
     }
     return 0;
+}
+
+// A warp's pairs (of the lanes with one) to the list for warps; false for those that find it full.
+__device__ __forceinline__ bool push_crowd_warp(const LinkArgs &A, bool mine, unsigned long long pr, int lane) {
+    const unsigned who = __ballot_sync(0xffffffffu, mine);
+    if (!who) return false;
+    unsigned long long first = 0;
+    if (lane == __ffs(who) - 1) first = atomicAdd(A.ncrowd, (unsigned long long)__popc(who));
+    const unsigned long long k = __shfl_sync(0xffffffffu, first, __ffs(who) - 1) + __popc(who & ((1u << lane) - 1u));
+    if (!mine || k >= (unsigned long long)A.crowd_cap) return false;
+    A.crowd[k] = pr;
+    return true;
 }
 
 __device__ __forceinline__ bool push_heavy(const LinkArgs &A, int a, int na, int b, int nb, int3 o) {
@@ -744,29 +766,141 @@ __global__ void __launch_bounds__(256) flatten_kernel(const int *__restrict__ cn
         root[k] = uf_find(parent, (int)k, err);
 }
 
-// Whether two nodes (of roots rh and rt) are in different sets and linked.
-__device__ __forceinline__ bool nodes_linked(const LinkArgs &A, const FofGeom &g, int h, int t, int3 o, int &rh,
-                                             int &rt) {
+// Whether two nodes are in different sets (of roots rh and rt) and linked, by one lane: 1, 0, or -1 when there are too many
+// tests for it.
+__device__ __forceinline__ int nodes_linked(const LinkArgs &A, const FofGeom &g, int h, int t, int3 o, int &rh, int &rt) {
     rh = uf_find(A.parent, h, A.err);
     rt = uf_find(A.parent, t, A.err);
-    if (rh == rt) return false;
-    const float sx = (float)o.x * g.cs, sy = (float)o.y * g.cs, sz = (float)o.z * g.cs;
+    if (rh == rt) return 0;
     const int p0 = A.node_start[h], p1 = A.node_start[h + 1], q0 = A.node_start[t], q1 = A.node_start[t + 1];
-    int left = kQuickTests;
-    int hit = node_link(A, g, p0, p1, q0, q1, sx, sy, sz, left);
-    if (hit < 0 && !push_heavy(A, p0, p1 - p0, q0, q1 - q0, o)) {
-        hit = 0;   // the blocks' list is full: row by row in place
-        for (int p = p0; p < p1 && hit <= 0; ++p) {
-            left = q1 - q0;
-            hit = node_link(A, g, p, p + 1, q0, q1, sx, sy, sz, left);
-        }
-    }
-    return hit > 0;
+    int left = (long long)(p1 - p0) * (q1 - q0) <= kLaneTests ? kLaneTests : kLaneGlance;
+    return node_link(A, g, p0, p1, q0, q1, (float)o.x * g.cs, (float)o.y * g.cs, (float)o.z * g.cs, left);
 }
 
+// The same where no warp is at hand: what a lane leaves open goes to the list for warps, or is decided row by row when that
+// is full.
 __device__ __forceinline__ void link_nodes(const LinkArgs &A, const FofGeom &g, int h, int t, int3 o) {
     int rh, rt;
-    if (nodes_linked(A, g, h, t, o, rh, rt)) uf_union(A.parent, rh, rt, A.err);
+    int hit = nodes_linked(A, g, h, t, o, rh, rt);
+    if (hit < 0) {
+        const int p0 = A.node_start[h], p1 = A.node_start[h + 1], q0 = A.node_start[t], q1 = A.node_start[t + 1];
+        const unsigned long long k = atomicAdd(A.ncrowd, 1ull);
+        if (k < (unsigned long long)A.crowd_cap) {
+            A.crowd[k] = (unsigned long long)h << 32 | (unsigned)t;
+            return;
+        }
+        for (int p = p0; p < p1 && hit <= 0; ++p) {
+            int left = q1 - q0;
+            hit = node_link(A, g, p, p + 1, q0, q1, (float)o.x * g.cs, (float)o.y * g.cs, (float)o.z * g.cs, left);
+        }
+    }
+    if (hit > 0) uf_union(A.parent, rh, rt, A.err);
+}
+
+// A box in a cell's coordinates, and the squared distance of a point from it.
+struct Box {
+    float lo[3], hi[3];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            lo[d] = INFINITY;
+            hi[d] = -INFINITY;
+        }
+    }
+    __device__ __forceinline__ void add(float x, float y, float z) {
+        const float v[3] = {x, y, z};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            lo[d] = fminf(lo[d], v[d]);
+            hi[d] = fmaxf(hi[d], v[d]);
+        }
+    }
+    __device__ __forceinline__ void join(const Box &b) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            lo[d] = fminf(lo[d], b.lo[d]);
+            hi[d] = fmaxf(hi[d], b.hi[d]);
+        }
+    }
+    __device__ __forceinline__ void warp_join() {
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+            for (int k = 16; k > 0; k >>= 1) {
+                lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], k));
+                hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], k));
+            }
+    }
+    __device__ __forceinline__ float d2(float x, float y, float z) const {
+        const float v[3] = {x, y, z};
+        float s = 0.f;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const float e = fmaxf(fmaxf(lo[d] - v[d], v[d] - hi[d]), 0.f);
+            s = fmaf(e, e, s);
+        }
+        return s;
+    }
+};
+
+// Whether two nodes are linked, by a warp: the particles of the larger a lane each, 32 at a time, against those of the smaller,
+// one after another; of many, only those near the smaller's box.
+__device__ __forceinline__ bool warp_nodes_linked(const LinkArgs &A, const FofGeom &g, int h, int t, int3 o, int lane) {
+    int a0 = A.node_start[h], na = A.node_start[h + 1] - a0, b0 = A.node_start[t], nb = A.node_start[t + 1] - b0;
+    float sx = (float)o.x * g.cs, sy = (float)o.y * g.cs, sz = (float)o.z * g.cs;   // added to b's coordinates
+    if (nb > na) {
+        const int s0 = a0, sn = na;
+        a0 = b0;
+        na = nb;
+        b0 = s0;
+        nb = sn;
+        sx = -sx;
+        sy = -sy;
+        sz = -sz;
+    }
+    const bool boxed = (long long)na * nb > 1024;
+    Box box;
+    box.clear();
+    if (boxed) {
+        for (int k = lane; k < nb; k += 32) {
+            const float4 b = A.rec[b0 + k];
+            box.add(b.x + sx, b.y + sy, b.z + sz);
+        }
+        box.warp_join();
+    }
+    for (int k0 = 0; k0 < na; k0 += 32) {
+        bool in = k0 + lane < na, known = false;
+        const float4 a = A.rec[a0 + min(k0 + lane, na - 1)];
+        if (boxed) in = in && box.d2(a.x, a.y, a.z) <= g.hi;
+        if (!__any_sync(0xffffffffu, in)) continue;
+        const float ax = a.x - sx, ay = a.y - sy, az = a.z - sz;
+        double ex = 0.0, ey = 0.0, ez = 0.0;   // the position for exact tests, read at the first of them
+        for (int q0 = 0; q0 < nb; q0 += 4) {
+            bool hit = false;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float4 b = A.rec[b0 + min(q0 + u, nb - 1)];
+                const float dx = b.x - ax, dy = b.y - ay, dz = b.z - az;
+                const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                if (!(in && d2 <= g.hi)) continue;
+                if (d2 < g.lo) {
+                    hit = true;
+                    continue;
+                }
+                if (!known) {
+                    const int i = __float_as_int(a.w);
+                    ex = A.x[i];
+                    ey = A.y[i];
+                    ez = A.z[i];
+                    known = true;
+                }
+                const int j = __float_as_int(b.w);
+                hit |= exact_pair(ex, ey, ez, A.x[j], A.y[j], A.z[j], g.r2);
+            }
+            if (__any_sync(0xffffffffu, hit)) return true;
+        }
+    }
+    return false;
 }
 
 // One thread per node: the pairs with nodes ahead of it that are near enough and whose roots differ, to the list
@@ -831,48 +965,151 @@ __global__ void __launch_bounds__(256) sweep_kernel(LinkArgs A, FofGeom g, const
     }
 }
 
-// One thread per listed pair of nodes.
+// A pair of nodes by a warp, or the largest listed for a block: whether they are linked.
+__device__ __forceinline__ bool warp_decides(const LinkArgs &A, const FofGeom &g, int h, int t, int lane) {
+    const int3 o = cell_offset(A.cell_key[A.node_cell[h]], A.cell_key[A.node_cell[t]], g.ky, g.kz);
+    const int p0 = A.node_start[h], np = A.node_start[h + 1] - p0, q0 = A.node_start[t], nq = A.node_start[t + 1] - q0;
+    if ((long long)np * nq > kWarpTests) {
+        bool listed = false;
+        if (lane == 0) listed = push_heavy(A, p0, np, q0, nq, o);
+        if (__shfl_sync(0xffffffffu, listed, 0)) return false;
+    }
+    return warp_nodes_linked(A, g, h, t, o, lane);
+}
+
+// One lane per listed pair of nodes; the pairs that it leaves open go to the list for warps (its own, when that is full).
 __global__ void __launch_bounds__(256) link_kernel(LinkArgs A, FofGeom g, const unsigned long long *__restrict__ list,
                                                    long long cap, const unsigned long long *__restrict__ nlist) {
+    const int lane = threadIdx.x & 31;
     const long long nl = (long long)*nlist < cap ? (long long)*nlist : cap;
     for (long long k0 = blockIdx.x * (long long)blockDim.x; k0 < nl; k0 += (long long)gridDim.x * blockDim.x) {
         const long long k = k0 + threadIdx.x;
-        int rh = 0, rt = 0;
-        bool join = false;
+        const unsigned long long pr = k < nl ? list[k] : 0;
+        const int h = (int)(pr >> 32), t = (int)(pr & 0xffffffffu);
+        int rh = 0, rt = 0, hit = 0;
         if (k < nl) {
-            const int h = (int)(list[k] >> 32), t = (int)(list[k] & 0xffffffffu);
             const int3 o = cell_offset(A.cell_key[A.node_cell[h]], A.cell_key[A.node_cell[t]], g.ky, g.kz);
-            join = nodes_linked(A, g, h, t, o, rh, rt);
+            hit = nodes_linked(A, g, h, t, o, rh, rt);
         }
-        uf_union_warp(A.parent, rh, rt, join, A.err);
+        if (push_crowd_warp(A, hit < 0, pr, lane)) hit = 0;
+        for (unsigned todo = __ballot_sync(0xffffffffu, hit < 0); todo; todo &= todo - 1) {
+            const int l = __ffs(todo) - 1;
+            const bool linked = warp_decides(A, g, __shfl_sync(0xffffffffu, h, l), __shfl_sync(0xffffffffu, t, l), lane);
+            if (lane == l) hit = linked;
+        }
+        uf_union_warp(A.parent, rh, rt, hit > 0, A.err);
     }
 }
 
-// Particles as nodes (coincident points only, or no room for half-cells in the key): one thread per cell pair
-// tests all its particles; crowded pairs go to the blocks' list.
+// Particles as nodes: the pairs of two cells' particles (of one, when they are the same) by a warp, a first particle a lane.
+__device__ __forceinline__ void warp_join_particles(const LinkArgs &A, const FofGeom &g, int h0, int h1, int t0, int t1,
+                                                    int3 o, bool same, int lane) {
+    const float sx = (float)o.x * g.cs, sy = (float)o.y * g.cs, sz = (float)o.z * g.cs;
+    for (int k0 = h0; k0 < h1; k0 += 32) {
+        const int p = min(k0 + lane, h1 - 1);
+        const float4 a = A.rec[p];
+        int rp = uf_find(A.parent, p, A.err);
+        for (int q = same ? k0 + 1 : t0; q < t1; ++q) {
+            const float4 b = A.rec[q];
+            const float dx = (b.x + sx) - a.x, dy = (b.y + sy) - a.y, dz = (b.z + sz) - a.z;
+            const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            bool join = k0 + lane < h1 && (!same || q > p) && d2 <= g.hi;
+            if (!__any_sync(0xffffffffu, join)) continue;
+            const int rq = uf_find(A.parent, q, A.err);
+            join = join && rq != rp &&
+                   (d2 < g.lo || exact_link(A.x, A.y, A.z, __float_as_int(a.w), __float_as_int(b.w), g.r2));
+            const int r = uf_union_warp(A.parent, rp, rq, join, A.err);
+            if (join) rp = r;
+        }
+    }
+}
+
+// A pair of cells' particles by a warp, or listed for a block.
+__device__ __forceinline__ void warp_joins_cells(const LinkArgs &A, const FofGeom &g, int2 pr, int lane) {
+    const int h0 = A.cell_node[pr.x], h1 = A.cell_node[pr.x + 1], t0 = A.cell_node[pr.y], t1 = A.cell_node[pr.y + 1];
+    const int3 o = pr.x == pr.y ? make_int3(0, 0, 0) : cell_offset(A.cell_key[pr.x], A.cell_key[pr.y], g.ky, g.kz);
+    if ((long long)(h1 - h0) * (t1 - t0) > kWarpPairs) {
+        bool listed = false;
+        if (lane == 0) listed = push_heavy(A, h0, h1 - h0, t0, t1 - t0, o);
+        if (__shfl_sync(0xffffffffu, listed, 0)) return;
+    }
+    warp_join_particles(A, g, h0, h1, t0, t1, o, pr.x == pr.y, lane);
+}
+
+// Particles as nodes (coincident points only, or no room for half-cells in the key): one lane per cell pair
+// tests all its particles; pairs with more than kLaneTests go to the list for warps.
 __global__ void __launch_bounds__(256) link_particles_kernel(LinkArgs A, FofGeom g) {
+    const int lane = threadIdx.x & 31;
     const long long np = (long long)*A.npairs;
-    for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < np; w += (long long)gridDim.x * blockDim.x) {
-        const int2 pr = A.pairs[w];
-        const bool same = pr.x == pr.y;
-        const int h0 = A.cell_node[pr.x], h1 = A.cell_node[pr.x + 1];
-        const int t0 = A.cell_node[pr.y], t1 = A.cell_node[pr.y + 1];
-        int3 o = make_int3(0, 0, 0);
-        if (!same) o = cell_offset(A.cell_key[pr.x], A.cell_key[pr.y], g.ky, g.kz);
-        if ((long long)(h1 - h0) * (t1 - t0) > kQuickNodes && push_heavy(A, h0, h1 - h0, t0, t1 - t0, o)) continue;
-        for (int h = h0; h < h1; ++h)
-            for (int t = same ? h + 1 : t0; t < t1; ++t) link_nodes(A, g, h, t, o);
+    for (long long w0 = blockIdx.x * (long long)blockDim.x; w0 < np; w0 += (long long)gridDim.x * blockDim.x) {
+        const long long w = w0 + threadIdx.x;
+        const int2 pr = w < np ? A.pairs[w] : make_int2(0, 0);
+        bool many = false;
+        if (w < np) {
+            const bool same = pr.x == pr.y;
+            const int h0 = A.cell_node[pr.x], h1 = A.cell_node[pr.x + 1], t0 = A.cell_node[pr.y], t1 = A.cell_node[pr.y + 1];
+            many = (long long)(h1 - h0) * (t1 - t0) > kLaneTests;
+            if (!many) {
+                int3 o = make_int3(0, 0, 0);
+                if (!same) o = cell_offset(A.cell_key[pr.x], A.cell_key[pr.y], g.ky, g.kz);
+                for (int h = h0; h < h1; ++h)
+                    for (int t = same ? h + 1 : t0; t < t1; ++t) link_nodes(A, g, h, t, o);
+            }
+        }
+        __syncwarp();
+        if (push_crowd_warp(A, many, (unsigned long long)w, lane)) many = false;
+        for (unsigned todo = __ballot_sync(0xffffffffu, many); todo; todo &= todo - 1) {
+            const int l = __ffs(todo) - 1;
+            warp_joins_cells(A, g, make_int2(__shfl_sync(0xffffffffu, pr.x, l), __shfl_sync(0xffffffffu, pr.y, l)), lane);
+        }
+    }
+}
+
+// One warp per pair on the list for warps.
+__global__ void __launch_bounds__(256) crowd_kernel(LinkArgs A, FofGeom g, int nodes) {
+    const int lane = threadIdx.x & 31;
+    const int n = (int)min(*A.ncrowd, (unsigned long long)A.crowd_cap);
+    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += (gridDim.x * blockDim.x) >> 5) {
+        const unsigned long long pr = A.crowd[k];
+        if (nodes) {
+            const int h = (int)(pr >> 32), t = (int)(pr & 0xffffffffu);
+            const int rh = uf_find(A.parent, h, A.err), rt = uf_find(A.parent, t, A.err);
+            // the lanes may have walked to different ancestors: one lane's word decides
+            if (__shfl_sync(0xffffffffu, rh == rt, 0)) continue;
+            const bool linked = warp_decides(A, g, h, t, lane);
+            if (lane == 0 && linked) uf_union(A.parent, rh, rt, A.err);
+            __syncwarp();
+        } else {
+            warp_joins_cells(A, g, A.pairs[pr], lane);
+        }
     }
 }
 
 // The list's entries: tiles of 256 x 256 particles, an entry of more than kHuge tiles spread over all blocks, the
-// others one block each.  A thread holds one particle of the first range; the second range's records
-// and roots are staged in shared memory.  Candidates already in the thread's set need no test.
+// others one block each.  A thread holds one particle of the first range; those of the second range that lie near the first
+// one's box are staged in shared memory with their roots, and a thread looks at them when its particle lies near
+// theirs.  Two nodes (nodes) are done with their first link: a tile of theirs starts with a look at their roots, and the
+// block stops when one of its threads finds a link.  Particles as nodes are joined one by one; candidates already in the thread's
+// set need no test.
+// Two sheets of 5e5 particles 1.3 linking lengths apart, one pair of nodes: 285 ms with every pair of particles tested, now 22.
 constexpr int kHuge = 64;
 
-__global__ void __launch_bounds__(256) heavy_kernel(LinkArgs A, FofGeom g, const int *__restrict__ node_of) {
+__device__ __forceinline__ Box block_box(Box box, Box *sh, int lane, int w) {
+    box.warp_join();
+    if (lane == 0) sh[w] = box;
+    __syncthreads();
+    Box all = sh[0];
+    for (int k = 1; k < 8; ++k) all.join(sh[k]);
+    __syncthreads();   // sh is reused
+    return all;
+}
+
+__global__ void __launch_bounds__(256) heavy_kernel(LinkArgs A, FofGeom g, const int *__restrict__ node_of, int nodes) {
     __shared__ float4 qrec[256];
-    __shared__ int qroot[256];
+    __shared__ int qroot[256], qat[256], wcnt[8];
+    __shared__ Box boxes[8];
+    __shared__ volatile int done;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int ne = min(*A.nheavy, A.heavy_cap);
     for (int e = 0; e < ne; ++e) {
         const HeavyPair hp = A.heavy[e];
@@ -882,29 +1119,89 @@ __global__ void __launch_bounds__(256) heavy_kernel(LinkArgs A, FofGeom g, const
         const bool same = hp.a == hp.b;
         const float sx = (float)((hp.off & 3) - 1) * g.cs, sy = (float)(((hp.off >> 2) & 3) - 1) * g.cs,
                     sz = (float)(((hp.off >> 4) & 3) - 1) * g.cs;
+        const int node_a = node_of[hp.a], node_b = node_of[hp.b];
         for (long long tile = huge ? blockIdx.x : 0; tile < tiles; tile += huge ? gridDim.x : 1) {
             const int p = hp.a + (int)(tile / tb) * 256 + threadIdx.x;
             const int q = hp.b + (int)(tile % tb) * 256 + threadIdx.x;
             const bool pv = p < hp.a + hp.na, qv = q < hp.b + hp.nb;
-            __syncthreads();   // the last tile's staging has been read
-            qrec[threadIdx.x] = qv ? A.rec[q] : make_float4(0.f, 0.f, 0.f, 0.f);
-            qroot[threadIdx.x] = qv ? uf_find(A.parent, node_of[q], A.err) : -1;
-            __syncthreads();
-            if (!pv) continue;
-            const float4 a = A.rec[p];
-            const int np = node_of[p];
-            int rp = uf_find(A.parent, np, A.err);
-            const int q0 = q - threadIdx.x, cnt = min(256, hp.b + hp.nb - q0);
-            for (int k = 0; k < cnt; ++k) {
-                if (qroot[k] == rp || (same && q0 + k <= p)) continue;
-                const float4 b = qrec[k];
-                const float dx = (b.x + sx) - a.x, dy = (b.y + sy) - a.y, dz = (b.z + sz) - a.z;
-                const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                if (!(d2 <= g.hi) ||
-                    !(d2 < g.lo || exact_link(A.x, A.y, A.z, __float_as_int(a.w), __float_as_int(b.w), g.r2)))
-                    continue;
-                rp = uf_union(A.parent, rp, qroot[k], A.err);
+            if (nodes) {
+                if (threadIdx.x == 0)
+                    done = uf_find(A.parent, node_a, A.err) == uf_find(A.parent, node_b, A.err);
+                __syncthreads();
+                const bool joined = done != 0;
+                __syncthreads();   // every thread has read it before it is written again
+                if (joined) break;
             }
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+            Box box;
+            box.clear();
+            if (pv) {
+                a = A.rec[p];
+                box.add(a.x, a.y, a.z);
+            }
+            const Box abox = block_box(box, boxes, lane, w);
+            bool keep = false;
+            if (qv) {
+                b = A.rec[q];
+                b.x += sx;
+                b.y += sy;
+                b.z += sz;
+                keep = abox.d2(b.x, b.y, b.z) <= g.hi;
+            }
+            const unsigned kept = __ballot_sync(0xffffffffu, keep);
+            if (lane == 0) wcnt[w] = __popc(kept);
+            box.clear();
+            if (keep) box.add(b.x, b.y, b.z);
+            const Box bbox = block_box(box, boxes, lane, w);   // its barriers publish wcnt
+            int at = __popc(kept & ((1u << lane) - 1u)), cnt = 0;
+            for (int k = 0; k < 8; ++k) {
+                if (k < w) at += wcnt[k];
+                cnt += wcnt[k];
+            }
+            if (keep) {
+                qrec[at] = b;
+                qat[at] = q;
+                qroot[at] = nodes ? node_b : uf_find(A.parent, node_of[q], A.err);
+            }
+            __syncthreads();
+            const bool near = pv && bbox.d2(a.x, a.y, a.z) <= g.hi;
+            auto linked = [&](int k) {
+                const float4 c = qrec[k];
+                const float dx = c.x - a.x, dy = c.y - a.y, dz = c.z - a.z;
+                const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                return d2 <= g.hi &&
+                       (d2 < g.lo || exact_link(A.x, A.y, A.z, __float_as_int(a.w), __float_as_int(c.w), g.r2));
+            };
+            if (nodes) {
+                for (int k0 = 0; k0 < cnt; k0 += 32) {
+                    if (!__any_sync(0xffffffffu, near && !done)) break;   // the same for the warp
+                    const int k1 = min(k0 + 32, cnt);
+                    for (int k = k0; near && k < k1; ++k)
+                        if (linked(k)) {
+                            uf_union(A.parent, node_a, node_b, A.err);
+                            done = 1;
+                            break;
+                        }
+                    __syncwarp();
+                }
+            } else {
+                // every thread starts at another candidate, the next particle in a pair of the same cell: coincident ones
+                // are one set after the first step, and known to be after the roots have been looked up again
+                int rp = near ? uf_find(A.parent, node_of[p], A.err) : 0;
+                int k = cnt > 0 ? (threadIdx.x + 1) % cnt : 0;
+                for (int j = 0; j < cnt; ++j) {
+                    if (near && qroot[k] != rp && !(same && qat[k] <= p) && linked(k))
+                        rp = uf_union(A.parent, rp, qroot[k], A.err);
+                    k = k + 1 < cnt ? k + 1 : 0;
+                    if ((j & (j + 1)) == 0) {
+                        __syncthreads();
+                        if ((int)threadIdx.x < cnt) qroot[threadIdx.x] = uf_find(A.parent, qroot[threadIdx.x], A.err);
+                        if (near) rp = uf_find(A.parent, rp, A.err);
+                        __syncthreads();
+                    }
+                }
+            }
+            __syncthreads();   // the staging and `done` are written again
         }
     }
 }
@@ -1400,9 +1697,10 @@ int fof_core(int n, const double *x, const double *y, const double *z, FofGeom g
     const size_t sort_b = sort_pairs_u64_i32_bytes(n, end_bit);
     const size_t scan_b = exclusive_sum_i64_bytes(nruns);
     Layout M;
-    const size_t o_kin = M.add(8ull * n), o_kout = M.add(8ull * n);
+    // the first three are free for the lists of pairs once the cells and nodes are known
+    const size_t o_kin = M.add(8ull * n), o_kout = M.add(8ull * n), o_pre = M.add(16ull * n);
     const size_t o_vin = M.add(4ull * n), o_vout = M.add(4ull * n);
-    const size_t o_rec = M.add(16ull * n), o_pre = M.add(16ull * n);
+    const size_t o_rec = M.add(16ull * n);
     const size_t o_run = M.add(8ull * nruns), o_base = M.add(8ull * nruns);
     const size_t o_nof = M.add(4ull * n), o_nst = M.add(4ull * (n + 1)), o_sub = M.add(1ull * n);
     const size_t o_nrec = M.add(16ull * n), o_ncell = M.add(4ull * n), o_clist = M.add(8ull * n);
@@ -1423,7 +1721,7 @@ int fof_core(int n, const double *x, const double *y, const double *z, FofGeom g
     auto *node_sub = at<unsigned char>(base, o_sub), *multi = at<unsigned char>(base, o_multi);
     int *cell_node = at<int>(base, o_cnode);
     auto *cell_key = at<uint64_t>(base, o_ckey);
-    int *cnt = at<int>(base, o_cnt);   // [0] cells [1] nodes [2] groups [3] error [4] heavy pairs [6..7] cell pairs [8..9] listed pairs of nodes [10] cells, from their count
+    int *cnt = at<int>(base, o_cnt);   // [0] cells [1] nodes [2] groups [3] error [4] heavy pairs [6..7] cell pairs [8..9] listed pairs of nodes [10] cells, from their count [12..13] pairs for warps
     auto *npairs = at<unsigned long long>(base, o_cnt + 24), *nlist = npairs + 1;
     auto *cell_list = at<long long>(base, o_clist);
     int *node_cell = at<int>(base, o_ncell);
@@ -1494,19 +1792,22 @@ int fof_core(int n, const double *x, const double *y, const double *z, FofGeom g
                      npairs);
     HALMA_TRY(mark(4));
     LinkArgs A{cnt, pairs, npairs, cell_list, cell_node, node_start, node_cell, node_sub, cell_key, rec,
-               at<float4>(base, o_nrec), x, y, z, parent, cnt + 3, at<HeavyPair>(base, o_heavy), cnt + 4, heavy_cap};
+               at<float4>(base, o_nrec), x, y, z, parent, cnt + 3, at<unsigned long long>(base, o_kin), npairs + 3, n,
+               at<HeavyPair>(base, o_heavy), cnt + 4, heavy_cap};
     if (g.sb) {
-        auto *list = reinterpret_cast<unsigned long long *>(kin);   // the sort's input is no longer needed: n entries
+        auto *list = at<unsigned long long>(base, o_kout);   // kout and pre: 3 n entries
+        const long long cap = 3ll * n;
         HALMA_LAUNCH(hook_kernel, g1, 256, 0, st, A, g);
         HALMA_LAUNCH(flatten_kernel, g1, 256, 0, st, cnt, parent, root, cnt + 3);
-        HALMA_LAUNCH(sweep_kernel, g1, 256, 0, st, A, g, root, list, (long long)n, nlist);
+        HALMA_LAUNCH(sweep_kernel, g1, 256, 0, st, A, g, root, list, cap, nlist);
         HALMA_TRY(mark(5));
-        HALMA_LAUNCH(link_kernel, g1, 256, 0, st, A, g, list, (long long)n, nlist);
+        HALMA_LAUNCH(link_kernel, g1, 256, 0, st, A, g, list, cap, nlist);
     } else {
         HALMA_TRY(mark(5));
         HALMA_LAUNCH(link_particles_kernel, std::min(sms * 8, grid_for(4ll * ncell, 256)), 256, 0, st, A, g);
     }
-    HALMA_LAUNCH(heavy_kernel, sms * 4, 256, 0, st, A, g, node_of);
+    HALMA_LAUNCH(crowd_kernel, sms * 8, 256, 0, st, A, g, g.sb ? 1 : 0);
+    HALMA_LAUNCH(heavy_kernel, sms * 4, 256, 0, st, A, g, node_of, g.sb ? 1 : 0);
     HALMA_TRY(mark(6));
     HALMA_LAUNCH(root_kernel, g1, 256, 0, st, cnt, node_start, parent, root, minidx, multi, cnt + 3);
     HALMA_LAUNCH(label_kernel, g1, 256, 0, st, n, vout, node_of, root, minidx, multi, labels, cnt + 2);

@@ -375,3 +375,69 @@ def test_member_count_of_the_last_call(cuda):
     e = np.zeros(0)
     find_haloes(e, e, e, e, e, e, e, 0.0015)
     assert L.halma_last_group_members() == 0
+
+
+@pytest.mark.parametrize("n", [8, 9, 60, 181, 182, 300])
+@pytest.mark.parametrize("sep", [1.4e-3, 1.4999999e-3, 1.50001e-3])
+def test_pairs_of_nodes_by_a_lane_a_warp_and_a_block(cuda, n, sep):
+    """Many pairs of clumps at the numbers of tests where a lane (64), a warp (32,768) and a block take over, linked by few
+    particles, by pairs at the linking length, or not at all."""
+    rng = np.random.default_rng(n)
+    ll, k = 1.5e-3, max(20, 20_000 // n)
+    c = np.stack(np.meshgrid(np.arange(40), np.arange(40), np.arange(40), indexing="ij"), -1).reshape(-1, 3)[:k] * (8 * ll)
+    a = c[:, None, :] + rng.uniform(-1.0, 1.0, (k, n, 3)) * [0.0, 2e-4, 2e-4]
+    b = c[:, None, :] + [sep, 0.0, 0.0] + rng.uniform(-1.0, 1.0, (k, n, 3)) * [1e-8, 2e-4, 2e-4]
+    p = np.concatenate([a.reshape(-1, 3), b.reshape(-1, 3)])
+    if len(p) <= 16_384:   # past the all-pairs limit
+        p = np.concatenate([p, np.stack([1.0 + 0.01 * np.arange(17_000 - len(p))] * 3, 1)])
+    p = p[rng.permutation(len(p))]
+    x, y, z = (np.ascontiguousarray(q) for q in p.T)
+    assert np.array_equal(fof.fof_labels(x, y, z, ll), oracle.fof_labels(x, y, z, ll))
+
+
+@pytest.mark.parametrize("copies", [8, 9, 64, 65, 256, 257, 1000])
+@pytest.mark.parametrize("ll", [0.0, 1e-6])
+def test_copies_of_particles(cuda, copies, ll):
+    """Coincident particles, with linking length 0 (particles as nodes) and a small one, around the sizes at which a lane, a warp
+    and a block take a pair of cells; some copies a little apart."""
+    rng = np.random.default_rng(copies)
+    p = np.repeat(rng.uniform(0.0, 1.0, (24_000 // copies, 3)), copies, axis=0)
+    p[rng.random(len(p)) < 0.1] += 0.5e-6
+    p = p[rng.permutation(len(p))]
+    x, y, z = (np.ascontiguousarray(q) for q in p.T)
+    assert np.array_equal(fof.fof_labels(x, y, z, ll), oracle.fof_labels(x, y, z, ll))
+
+
+@pytest.mark.parametrize("what", ["clumps", "lattice", "sheets", "copies"])
+def test_crowded_cells_take_no_longer_than_spread_ones(cuda, what):
+    """Particles crowded in half-cells that are not linked to their neighbours, or only here and there, against as many
+    spread out."""
+    import torch
+    rng = np.random.default_rng(18)
+    n, ll = 400_000, 1.0
+    if what == "clumps":
+        p = np.repeat(rng.uniform(0.0, 45.0, (n // 200, 3)), 200, axis=0) + rng.normal(0.0, 0.05, (n, 3))
+    elif what == "lattice":
+        p = np.round(rng.uniform(0.0, 20.0, (n, 3))) * 0.5
+    elif what == "sheets":
+        n = 100_000
+        p = rng.uniform(0.0, 0.3, (n, 3)) * [0.0, 1.0, 1.0]
+        p[::2, 0] = 1.3
+    else:
+        p, ll = np.repeat(rng.uniform(0.0, 10.0, (n // 500, 3)), 500, axis=0), 0.0
+
+    def ms(q, ll):
+        x, y, z = (torch.tensor(np.ascontiguousarray(c), device=cuda) for c in q.T)
+        fof.fof_labels(x, y, z, ll)
+        best = np.inf
+        for _ in range(3):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            torch.cuda.synchronize()
+            e[0].record()
+            fof.fof_labels(x, y, z, ll)
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]))
+        return best
+    spread, took = ms(rng.uniform(0.0, 70.0, (n, 3)), 1.0), ms(p, ll)
+    assert took < 4.0 * spread, (took, spread)
