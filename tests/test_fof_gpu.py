@@ -441,3 +441,14 @@ def test_crowded_cells_take_no_longer_than_spread_ones(cuda, what):
         return best
     spread, took = ms(rng.uniform(0.0, 70.0, (n, 3)), 1.0), ms(p, ll)
     assert took < 4.0 * spread, (took, spread)
+
+
+@pytest.mark.parametrize("sigma", [0.3, 1.0, 3.0])
+def test_crowded_cells_of_a_grid_without_room_for_half_cells(cuda, sigma):
+    """A crowd whose box is 1.5e6 linking lengths wide for the sake of one particle: particles are the nodes."""
+    rng = np.random.default_rng(19)
+    n, ll = 60_000, 1.0
+    p = rng.normal(0.0, sigma, (3, n))
+    p[:, 7] = 1.5e6
+    x, y, z = (np.ascontiguousarray(c) for c in p)
+    assert np.array_equal(fof.fof_labels(x, y, z, ll), oracle.fof_labels(x, y, z, ll))
