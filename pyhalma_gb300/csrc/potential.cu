@@ -189,7 +189,7 @@ struct RefShape {
 template <int TL>
 __global__ void __launch_bounds__(RefShape<TL>::warps * 32) ref_potential_kernel(
     const Src4 *__restrict__ src, int64_t nstages, const float *__restrict__ tx, const float *__restrict__ ty,
-    const float *__restrict__ tz, int64_t nt, const int *__restrict__ flags, float nzero, int first,
+    const float *__restrict__ tz, int64_t nt, const int *__restrict__ flags, float nzero, int first, int leave_plain,
     float *__restrict__ out) {
     using S = RefShape<TL>;
     constexpr int N = S::take * TL / 32;    // quads of a lane in one stage
@@ -202,6 +202,7 @@ __global__ void __launch_bounds__(RefShape<TL>::warps * 32) ref_potential_kernel
     const int64_t it = i < nt ? i : nt - 1;
     const float px = tx[it], py = ty[it], pz = tz[it];
     const int fl = *flags;
+    if (leave_plain && (fl & kRefPlain)) return;   // ref_direct_kernel's
     // every warp copies its own next sources while it computes
     auto fetch = [&](int64_t st) {
         if (st < nstages) {
@@ -253,6 +254,39 @@ __global__ void __launch_bounds__(RefShape<TL>::warps * 32) ref_potential_kernel
     if (S::adds(w) && lane < TL && i < nt) out[i] = acc;
 }
 
+// The same with a target a thread and the plain operations, for few sources or many targets with values that need them: no
+// stage to fill, and every thread computes.  With kRefDirect sources or fewer it is the one launch: 40 sources x 300,000
+// targets 49 us, 113 through the stages; from kRefManyTargets targets on with kRefDirectMany (300 x 300,000 151 and 173,
+// 300 x 30,000 77 and 59).  Of those many targets it also takes the pieces whose values need the plain operations throughout
+// (only_plain: the flag says so, else it leaves): 3,000 x 300,000 1,328 us through the stages, 1,099 so; fewer targets are
+// better off with eight warps for the terms of 32 (3,000 x 30,000 374 us here, 207 there).
+constexpr int64_t kRefDirect = 64, kRefDirectMany = 320, kRefManyTargets = 100000;
+
+__global__ void __launch_bounds__(256) ref_direct_kernel(const float *__restrict__ m, const float *__restrict__ x,
+                                                         const float *__restrict__ y, const float *__restrict__ z,
+                                                         int64_t ns, const float *__restrict__ tx,
+                                                         const float *__restrict__ ty, const float *__restrict__ tz,
+                                                         int64_t nt, const int *__restrict__ only_plain, int first,
+                                                         float *__restrict__ out) {
+    if (only_plain && !(*only_plain & kRefPlain)) return;
+    __shared__ float4 buf[256];
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const bool in = i < nt;
+    const float px = in ? tx[i] : 0.f, py = in ? ty[i] : 0.f, pz = in ? tz[i] : 0.f;
+    float acc = first || !in ? 0.f : out[i];
+    for (int64_t j0 = 0; j0 < ns; j0 += 256) {
+        const int cnt = (int)min((int64_t)256, ns - j0);
+        __syncthreads();
+        if ((int)threadIdx.x < cnt) {
+            const int64_t j = j0 + threadIdx.x;
+            buf[threadIdx.x] = make_float4(x[j], y[j], z[j], m[j]);
+        }
+        __syncthreads();
+        for (int k = 0; k < cnt; ++k) acc = __fadd_rn(acc, pair_term_reference(buf[k], px, py, pz));
+    }
+    if (in) out[i] = acc;
+}
+
 // Packs the sources and runs the kernel, kRefPiece sources at a time (64 MB of packed ones); src holds the quads of a piece.
 constexpr int64_t kRefPiece = 1ll << 22;
 
@@ -275,7 +309,10 @@ static int launch_reference(const float *m, const float *x, const float *y, cons
         HALMA_LAUNCH(ref_pack_kernel, grid_for(std::max(nquads, nt), 256, device_sm_count() * 8), 256, 0, st, m + j, x + j,
                      y + j, z + j, n, nquads, tx, ty, tz, nt, src, flags);
         HALMA_LAUNCH(ref_potential_kernel<TL>, (unsigned)((nt + TL - 1) / TL), S::warps * 32, smem, st, src,
-                     nquads / S::quads, tx, ty, tz, nt, flags, -0.0f, j == 0, out);
+                     nquads / S::quads, tx, ty, tz, nt, flags, -0.0f, j == 0, nt >= kRefManyTargets, out);
+        if (nt >= kRefManyTargets)
+            HALMA_LAUNCH(ref_direct_kernel, grid_for(nt, 256), 256, 0, st, m + j, x + j, y + j, z + j, n, tx, ty, tz, nt,
+                         flags, j == 0, out);
     }
     return HALMA_OK;
 }
@@ -693,6 +730,9 @@ extern "C" int halma_bf_potential_f32(int64_t ntotal, const float *total_mass, c
     HALMA_TRY(sg.bind_and_upload(base, st));
     if (ntotal == 0) {
         HALMA_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * ntest, st));
+    } else if (ntotal <= (ntest < kRefManyTargets ? kRefDirect : kRefDirectMany)) {
+        HALMA_LAUNCH(ref_direct_kernel, grid_for(ntest, 256), 256, 0, st, m, x, y, z, ntotal, tx, ty, tz, ntest,
+                     (const int *)nullptr, 1, out);
     } else {
         Src4 *src = at<Src4>(base, o_src);
         int *flags = at<int>(base, o_flags);

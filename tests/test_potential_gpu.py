@@ -256,3 +256,47 @@ def test_host_pages_that_nobody_touched(cuda):
     ms(False)
     touched, fresh = ms(False), ms(True)
     assert fresh < 2.0 * touched + 8.0, (fresh, touched)
+
+
+@pytest.mark.parametrize("ns", [1, 63, 64, 65, 257, 320, 321, 600])
+@pytest.mark.parametrize("nt", [1, 255, 257, 99_999, 100_000])
+@pytest.mark.parametrize("plain", [False, True])
+def test_reference_mode_of_few_sources_and_many_targets(cuda, ns, nt, plain):
+    """Both sides of the 64 sources up to which a thread takes a target, of the 320 for 100,000 targets and more, and of that
+    number, from which it does when the plain operations are needed (a mass outside the others' range)."""
+    rng = np.random.default_rng(ns + nt)
+    p, m = _cloud(rng, ns)
+    t, _ = _cloud(rng, nt)
+    t[::5] = p[rng.integers(0, ns, len(t[::5]))]
+    if plain:
+        m[ns // 2] = 1e-30
+    got = halo_gas.bf_potential(m, *p.T, *t.T, mode="reference")
+    assert np.array_equal(got, oracle.bf_potential_f32(m, *p.T, *t.T))
+
+
+def test_reference_mode_has_no_stages_for_few_sources(cuda):
+    """One launch with 64 sources or fewer; many targets take about as long with the plain operations as with the others."""
+    import torch
+    T = lambda n: torch.rand(n, device=cuda)
+    x, y, z, m = T(400), T(400), T(400), T(400) + 1.0
+    t = [T(300_000) for _ in range(3)]
+    count = _lib.lib().halma_kernel_launch_count
+    before = count()
+    halo_gas.bf_potential(m[:64].clone(), x[:64].clone(), y[:64].clone(), z[:64].clone(), *t, mode="reference")
+    assert count() - before == 1
+
+    def ms():
+        halo_gas.bf_potential(m, x, y, z, *t, mode="reference")
+        best = np.inf
+        for _ in range(5):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            torch.cuda.synchronize()
+            e[0].record()
+            halo_gas.bf_potential(m, x, y, z, *t, mode="reference")
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]))
+        return best
+    usual = ms()
+    m[7] = 1e-30
+    assert ms() < 1.5 * usual
