@@ -93,17 +93,15 @@ __device__ __forceinline__ int uf_find(int *parent, int v, int *err) {
     return v;
 }
 
-// A random order of the nodes (a bijection of 32-bit integers by multiplications and shifts).  Neighbouring nodes
-// have neighbouring numbers: hooked in the order of their numbers they make chains as long as a group, and
-// a walk is one dependent memory access a step; hooked in random order, trees are logarithmically deep (A. Goel,
-// S. Khanna, D. Larkin, R. E. Tarjan, Disjoint set union with randomized linking, SODA 2014).
+// A scattered order of the nodes: a bijection of 32-bit integers, multiplicative hashing by the golden ratio (D. E. Knuth, The Art
+// of Computer Programming 3, 6.4) twice, with the upper half folded in between.  Neighbouring nodes have neighbouring
+// numbers: hooked in the order of their numbers they make chains as long as a group, and a walk is one dependent memory
+// access a step; hooked in random order, trees are logarithmically deep (A. Goel, S. Khanna, D. Larkin, R. E. Tarjan,
+// Disjoint set union with randomized linking, SODA 2014).
 __device__ __forceinline__ unsigned uf_rank(int v) {
-    unsigned h = (unsigned)v;
-    h ^= h >> 16;
-    h *= 0x85ebca6bu;
-    h ^= h >> 13;
-    h *= 0xc2b2ae35u;
-    return h ^ (h >> 16);
+    constexpr unsigned kGolden = 2654435769u;   // 2^32 / 1.618.., odd
+    const unsigned h = (unsigned)v * kGolden;
+    return (h ^ (h >> 16)) * kGolden;
 }
 
 // Joins the sets of two ancestors a and b (roots or not): hooks the root of the larger rank under that of
