@@ -343,8 +343,8 @@ int halma_bf_potential_f32(int64_t ntotal, const float *total_mass, const float 
  * library.  Same source split, same kernels and identical results as
  * halma_bf_potential_f32(HALMA_POT_FAST); returns HALMA_ERR_CAPACITY when the split needs more
  * than 2,097,152 partial sums (source slices x targets).  The first call on a device looks up
- * the array's address: make it before any stream capture.  Calls share the array: calls that
- * overlap on the GPU race. */
+ * the array's address: make it before any stream capture.  Calls with 4,096 sources or more
+ * share the array: two of them that overlap on the GPU race (fewer sources are added up without it). */
 int halma_bf_potential_f32_noalloc(int64_t ntotal, const float *total_mass, const float *total_x,
                                    const float *total_y, const float *total_z, int64_t ntest,
                                    const float *test_x, const float *test_y, const float *test_z,

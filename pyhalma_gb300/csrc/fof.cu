@@ -93,8 +93,8 @@ __device__ __forceinline__ int uf_find(int *parent, int v, int *err) {
     return v;
 }
 
-// A scattered order of the nodes: a bijection of 32-bit integers, multiplicative hashing by the golden ratio (D. E. Knuth, The Art
-// of Computer Programming 3, 6.4) twice, with the upper half folded in between.  Neighbouring nodes have neighbouring
+// A scattered order of the nodes: a bijection of 32-bit integers, multiplicative hashing by the golden ratio (D. E. Knuth,
+// The Art of Computer Programming 3, 6.4) twice, with the upper half folded in between.  Neighbouring nodes have neighbouring
 // numbers: hooked in the order of their numbers they make chains as long as a group, and a walk is one dependent memory
 // access a step; hooked in random order, trees are logarithmically deep (A. Goel, S. Khanna, D. Larkin, R. E. Tarjan,
 // Disjoint set union with randomized linking, SODA 2014).
@@ -464,8 +464,9 @@ __global__ void __launch_bounds__(256) head_apply_kernel(
     int n, int sb, const uint64_t *__restrict__ keys, const int *__restrict__ idx, const float4 *__restrict__ pre,
     const int64_t *__restrict__ base, int nruns, float4 *__restrict__ rec, int *__restrict__ node_of,
     int *__restrict__ node_start, int *__restrict__ node_cell, unsigned char *__restrict__ node_sub,
-    float4 *__restrict__ node_rec, int *__restrict__ parent, int *__restrict__ minidx, unsigned char *__restrict__ multi, int *__restrict__ cell_node,
-    uint64_t *__restrict__ cell_key, int *__restrict__ cnt) {
+    float4 *__restrict__ node_rec, int *__restrict__ parent, int *__restrict__ minidx,
+    unsigned char *__restrict__ multi, int *__restrict__ cell_node, uint64_t *__restrict__ cell_key,
+    int *__restrict__ cnt) {
     const int lane = threadIdx.x & 31;
     const unsigned upto = 0xffffffffu >> (31 - lane);
     const int run = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1284,8 +1285,8 @@ __global__ void __launch_bounds__(256) label_kernel(int n, const int *__restrict
 
 // ---- small inputs ---------------------------------------------------------------------------
 // Up to kSmallFof particles, all pairs: no bounding box on the host, no sort, no cells -- five launches and one
-// round trip instead of thirty and two.  A call takes 88 us at 5,000 particles (on cells 245, start 297), 113 at
-// 8,192 (243) and 204 at 16,384 (256).
+// round trip instead of thirty and two.  A call takes 92 us at 5,000 particles (on cells 245), 113 at
+// 8,192 (243) and 214 at 16,384 (250).
 // A particle is its position relative to particle 0 in linking lengths as two floats an axis (error below 2^-46 of
 // the largest); where some lie farther apart than 2^24 linking lengths (or the linking length is subnormal),
 // pairs that the floats leave open are tested in FP64 (flags[1]).
@@ -1296,7 +1297,8 @@ struct SmallArgs {
     int n;
     const double *x, *y, *z;
     float4 *pos_hi, *pos_lo;   // pos_hi[i].w: the particle's root for the sweep
-    int *flags;                // [0] non-finite coordinate, [1] coordinates for FP64 tests, [4] the largest |coordinate| (float bits)
+    // [0] non-finite coordinate, [1] coordinates for FP64 tests, [4] the largest |coordinate| (float bits)
+    int *flags;
     int *parent, *first, *err;
     float lo, hi;
     double r2;
@@ -1746,7 +1748,9 @@ int fof_core(int n, const double *x, const double *y, const double *z, FofGeom g
     auto *node_sub = at<unsigned char>(base, o_sub), *multi = at<unsigned char>(base, o_multi);
     int *cell_node = at<int>(base, o_cnode);
     auto *cell_key = at<uint64_t>(base, o_ckey);
-    int *cnt = at<int>(base, o_cnt);   // [0] cells [1] nodes [2] groups [3] error [4] heavy pairs [6..7] cell pairs [8..9] listed pairs of nodes [10] cells, from their count [12..13] pairs for warps
+    // [0] cells [1] nodes [2] groups [3] error [4] pairs for blocks [6..7] cell pairs [8..9] listed pairs of nodes
+    // [10] cells, from their count [12..13] pairs for warps
+    int *cnt = at<int>(base, o_cnt);
     auto *npairs = at<unsigned long long>(base, o_cnt + 24), *nlist = npairs + 1;
     auto *cell_list = at<long long>(base, o_clist);
     int *node_cell = at<int>(base, o_ncell);
@@ -2084,8 +2088,9 @@ __global__ void group_offsets_kernel(int nm, const uint32_t *__restrict__ keys, 
 
 // All of the grouping for up to kSmallGroups particles in one block of 1024 threads, the labels' counts and the groups'
 // first places in shared memory: one launch and one round trip instead of ten and two.  A call takes 105 us at 5,000
-// particles (124 at the start) and as much as the general path at 12,000.  A member's place in its group is the number of earlier members: per chunk of 1024 particles the warps
-// take their places one after another, from counters that hold the members of earlier chunks and warps.
+// particles (124 on the general path) and as much as that at 12,000.  A member's place in its group is the number of earlier
+// members: per chunk of 1024 particles the warps take their places one after another, from counters that hold the members
+// of earlier chunks and warps.
 // cnt: [0] label outside [-1, n), [1] labels that are not their groups' members (the caller then takes the general
 // path), [2] groups, [3] members.
 constexpr int kSmallGroups = 8192;
@@ -2278,8 +2283,10 @@ extern "C" int halma_fof_groups(int64_t n, const int32_t *labels, int32_t min_me
     int64_t ng = 0, nm = 0;
     int s = fof_groups_device((int)n, dl, min_members, doff, dmem, &ng, &nm, st);
     if (s == HALMA_OK) {
-        if (h_off) s = cudaMemcpyAsync(offsets, doff, 8ull * (ng + 1), cudaMemcpyDeviceToHost, st) == cudaSuccess ? s : fail(HALMA_ERR_CUDA, "copy of group offsets failed");
-        if (h_mem && nm > 0) s = cudaMemcpyAsync(members, dmem, 4ull * nm, cudaMemcpyDeviceToHost, st) == cudaSuccess ? s : fail(HALMA_ERR_CUDA, "copy of group members failed");
+        if (h_off && cudaMemcpyAsync(offsets, doff, 8ull * (ng + 1), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+            s = fail(HALMA_ERR_CUDA, "copy of group offsets failed");
+        if (h_mem && nm > 0 && cudaMemcpyAsync(members, dmem, 4ull * nm, cudaMemcpyDeviceToHost, st) != cudaSuccess)
+            s = fail(HALMA_ERR_CUDA, "copy of group members failed");
         *n_groups = ng;
     }
     if (stage) cudaFreeAsync(stage, st);

@@ -244,8 +244,8 @@ void choose_slices(int64_t na, int64_t nb, int T, int nv, int *n_split, int64_t 
 // against `tblocks` blocks of targets, the sources' sums kept in shared memory (compensated) over them, the
 // targets' too, a column a thread, as they are touched once in 32 sources.  Per item and target, or source, one
 // partial sum is written; they are added in order.
-// Bound: the FP32 pipe (18 lane-operations and a rsqrt a pair; 77 % busy).  160,000 x 200,000: 27.5 ms in two sweeps,
-// 19.7 in one.  Fewer reductions and more independent pairs a warp gain more than warps: eight targets with their
+// Bound: the FP32 pipe (17.5 lane-operations, the reduction with them, and a rsqrt a pair; 77 % busy).
+// 160,000 x 200,000: 27.5 ms in two sweeps, 19.7 in one.  Fewer reductions and more independent pairs a warp gain more than warps: eight targets with their
 // sums in registers and three blocks an SM 22.0 (512 sources), with the sums in shared memory 21.2 (256), sixteen
 // and two blocks 20.5, eighteen with 192 to 320 sources 19.7 to 20.3; four targets, two sources an instruction 23.5.
 constexpr int kBothT = 18, kBothTargets = 128 * kBothT, kBothSources = 288, kBothChunks = kBothSources / 32;

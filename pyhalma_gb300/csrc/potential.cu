@@ -35,9 +35,10 @@ __device__ __forceinline__ float4 load_source(const float *__restrict__ m, const
 //
 // So: 0.065 ms and 3.7 ms.
 //
-// Bound of the terms: the FP32 pipe, 18 two-lane instructions for two terms (measured: 57 % of it
-// busy, 3.6 terms per SM-cycle).  Square root and
-// quotient come from one rsqrt y of s by Markstein's correction steps (P. Markstein, Computation
+// The terms take 18 two-lane instructions for two, 3.5 terms per SM-cycle at 40,000 x 100,000, where no unit is full: FMA
+// pipe 56 % busy, issue slots 54 %, shared memory 44 %.  Of 11 warp-cycles an issue 3.2 are spent at the barrier of a
+// stage, 1.6 each on waits for shared memory and for the operation before, 1.5 on the pipe.
+// Square root and quotient come from one rsqrt y of s by Markstein's correction steps (P. Markstein, Computation
 // of elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990):
 // g = s y, r = g + (s - g g) y / 2;  z = y + y (1 - r y);  q = m z, t = q + (m - r q) z.  r is the
 // rounded square root for every mantissa (checked over all 2^24 of two binades, in five

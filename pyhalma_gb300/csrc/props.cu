@@ -201,7 +201,8 @@ __global__ void __launch_bounds__(256) pr_shape_kernel(int G, const int64_t *__r
                                                        const double *__restrict__ g, int64_t nm,
                                                        const double *__restrict__ cen, double *__restrict__ out) {
     constexpr int kRow = kTile + 8;   // rows start in different banks
-    __shared__ float sr[2][4][kRow];  // x, y, z relative to the centre (FP32), mass; one tile filled while the other is added
+    // x, y, z relative to the centre (FP32), mass; one tile filled while the other is added
+    __shared__ float sr[2][4][kRow];
     __shared__ float acc[10];
     for (int h = blockIdx.x; h < G; h += gridDim.x) {
         const double *c = cen + (int64_t)h * kCenFields;
@@ -273,8 +274,8 @@ __global__ void __launch_bounds__(256) pr_shape_kernel(int G, const int64_t *__r
 // Tully-Fisher velocity about it.
 // A group's members are split over up to S blocks of at least kKinMin (the FP64 work per member
 // is heavy and GB300's FP64 pipe is narrow, so one block per group would leave the biggest
-// group's SM as the critical path; parts of 2,048 still left two blocks on some SMs and one on others); each block writes partial sums and the last block of the
-// group to finish (a per-group counter, no waiting) adds them in block order.
+// group's SM as the critical path; parts of 2,048 still left two blocks on some SMs and one on others); each block
+// writes partial sums and the last block of the group to finish (a per-group counter, no waiting) adds them in block order.
 constexpr int kKinMin = 512;
 
 __device__ __forceinline__ bool kin_part_of(int bid, int S, int G, const int64_t *__restrict__ off, int &h, int &sh,

@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(256) red_walk_kernel(const int64_t *__restrict
     const int64_t nmem = (int64_t)r.n;
     const double half = 0.5 * r.mref;
     const int lane = threadIdx.x & 31;
-    __shared__ double tile[2][1024];   // warp 0 walks one while the other warps fill the next
+    __shared__ double tile[2][1024];   // the next one's masses are written before this one is walked
     __shared__ long long first;
     if (threadIdx.x == 0) first = LLONG_MAX;
     SeqSum q;   // lane 0's state (warp 0)
