@@ -240,8 +240,10 @@ __global__ void __launch_bounds__(256) red_dist_kernel(int nh, const int64_t *__
 // order here, which the stable sort has made right where their distances are all the same; *longest is
 // the length of the longest that has to be put in order (red_runs_kernel), run[p] a long run's start and length (0 elsewhere).
 // Rows at no finite distance and excluded ones keep their place: what they are sorted by is one value.
-// (Counted by every row, the masses of 2e6 members, a call without positions, took 3.9 s, now 11 ms with their copies.)
-constexpr int kShortRun = 32;
+// (Counted by every row, the masses of 2e6 members, a call without positions, took 3.9 s, now 11 ms with their copies.
+// 100 haloes of 10,000 about a centre at 10^5 times their size, runs of some hundred: 689 us with runs of up to 32 counted, 555
+// so and with 256; at 10^7 times, one run a halo, 1.29 ms with two blocks an SM in red_runs_kernel, 1.17 with four.)
+constexpr int kShortRun = 128;
 
 __global__ void __launch_bounds__(256) red_ties_kernel(int n, const uint64_t *__restrict__ key,
                                                        const int *__restrict__ val, const double *__restrict__ dist,
@@ -630,7 +632,7 @@ __global__ void red_out_kernel(int nh, const int *__restrict__ cstart, const dou
 
 int launch_runs(int n, const int *longest, const int2 *run, const int *val, const double *dist, double *da, int *a,
                 double *db, int *b, cudaStream_t st) {
-    const int grid = std::min(device_sm_count() * 2, grid_for(n, 256));   // all blocks are on the GPU at once
+    const int grid = std::min(device_sm_count() * 4, grid_for(n, 256));   // all blocks are on the GPU at once (five an SM fit)
     void *args[] = {&n, &longest, &run, &val, &dist, &da, &a, &db, &b};
     HALMA_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(&red_runs_kernel), dim3((unsigned)grid), dim3(256), args,
                                            0, st));
