@@ -241,8 +241,9 @@ __global__ void __launch_bounds__(256) red_dist_kernel(int nh, const int64_t *__
 // the length of the longest that has to be put in order (red_runs_kernel), run[p] a long run's start and length (0 elsewhere).
 // Rows at no finite distance and excluded ones keep their place: what they are sorted by is one value.
 // (Counted by every row, the masses of 2e6 members, a call without positions, took 3.9 s, now 11 ms with their copies.
-// 100 haloes of 10,000 about a centre at 10^5 times their size, runs of some hundred: 689 us with runs of up to 32 counted, 555
-// so and with 256; at 10^7 times, one run a halo, 1.29 ms with two blocks an SM in red_runs_kernel, 1.17 with four.)
+// 100 haloes of 10,000 about a centre at 10^5 times their size, runs of up to 75 rows: 689 us with runs of up to 32 counted, 555
+// with 128, 550 with 256; at 10^7 times, runs of up to 4,500, 1.28 ms with two blocks an SM in red_runs_kernel, 1.17 with four.
+// 10 haloes of 30,000 at 10^7 times, up to 2,400: 695 us with 32, 710 with 128, 725 with 256, all with two blocks an SM.)
 constexpr int kShortRun = 128;
 
 __global__ void __launch_bounds__(256) red_ties_kernel(int n, const uint64_t *__restrict__ key,
